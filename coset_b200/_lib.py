@@ -1,21 +1,26 @@
-"""ctypes binding of libcoset_b200.so, the C-ABI CUDA library.
+"""Bindings of libcoset_b200.so, the C-ABI CUDA library: `lib()` is the ctypes binding of every declared
+function, `native()` the module with the native entry points of the calls whose host time matters.
 
 There is no CPU fallback: if the library is missing or a tensor is not on a CUDA device the
 call fails loudly.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libcoset_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "lib", "_coset_torch.so")
 
 DTYPE_F32, DTYPE_BF16 = 0, 1
 SCALE_NONE, SCALE_DIV_SCALAR, SCALE_MUL_TILE = 0, 1, 2
 SEM_CORE, SEM_REF, SEM_CORE_LITERAL, SEM_CORE_SATURATE = 0, 1, 2, 3
 
 _lib = None
+_native = None
 
 _vp, _i64, _i32, _f32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float
 
@@ -30,6 +35,8 @@ SIGNATURES = {
     "coset_e8_quantize": [_vp, _i32, _vp, _i32, _i64, _i64, _i32, _i32, _f32, _vp, _i32, _vp, _vp],
     "coset_e8_unpack_codes_f32": [_vp, _i64, _i32, _i32, _vp, _vp],
     "coset_e8_pack_codes_f32": [_vp, _i64, _i32, _i32, _vp, _vp],
+    "coset_e8_encode_digits_f32": [_vp, _f32, _i64, _i32, _i32, _vp, _vp],
+    "coset_e8_decode_digits_f32": [_vp, _f32, _i64, _i32, _i32, _vp, _vp],
     "coset_host_ctx_create": [_i64, _i32, ctypes.POINTER(ctypes.c_void_p)],
     "coset_host_ctx_destroy": [_vp],
     "coset_e8_encode_host": [_vp, _vp, _i32, _vp, _i32, _i64, _i64, _i32, _i32, _vp],
@@ -77,6 +84,20 @@ def lib():
                           else ctypes.c_int64 if name.endswith(("_scratch_bytes", "_max_blocks")) else ctypes.c_int)
         _lib = L
     return _lib
+
+
+def native():
+    """Loads the native module (csrc/torch_binding.cpp) once; raises if it has not been built."""
+    global _native
+    if _native is None:
+        lib()
+        if not os.path.exists(NATIVE_PATH):
+            raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m coset_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_coset_torch", NATIVE_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_coset_torch", loader))
+        loader.exec_module(module)
+        _native = module
+    return _native
 
 
 def check(rc, what):

@@ -1,4 +1,5 @@
-"""Builds libcoset_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libcoset_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and _coset_torch.so
+(the native PyTorch entry points on top of it) with g++.
 
     python -m coset_b200.build [--force] [--verbose]
 
@@ -9,11 +10,15 @@ multiply-add would change codes.
 import os
 import subprocess
 import sys
+import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libcoset_b200.so")
+TORCH_PATH = os.path.join(LIB_DIR, "_coset_torch.so")
+TORCH_SOURCE = "torch_binding.cpp"
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = [
@@ -44,32 +49,49 @@ def _nvcc():
     return "nvcc"
 
 
-def _stale():
-    if not os.path.exists(LIB_PATH):
-        return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(INCLUDE, "coset_b200.h"), __file__]
-    return any(os.path.getmtime(d) > t for d in deps)
+def _newer(target, deps):
+    """True if `target` exists and is no older than any of `deps`."""
+    return os.path.exists(target) and all(os.path.getmtime(d) <= os.path.getmtime(target) for d in deps)
 
 
-def build(force=False, verbose=False):
-    """Compile every .cu under csrc/ into lib/libcoset_b200.so; returns its path."""
-    if not force and not _stale():
-        return LIB_PATH
-    os.makedirs(LIB_DIR, exist_ok=True)
-    objs = []
-    for src in SOURCES:
-        obj = os.path.join(LIB_DIR, src.replace(".cu", ".o"))
-        cmd = [_nvcc(), *NVCC_FLAGS, "-I", INCLUDE, "-c", os.path.join(CSRC, src), "-o", obj]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
-            print(" ".join(cmd), flush=True)
-        subprocess.check_call(cmd)
-        objs.append(obj)
-    cmd = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"]
+def _run(cmd, verbose):
     if verbose:
         print(" ".join(cmd), flush=True)
     subprocess.check_call(cmd)
+
+
+def _build_torch_module(verbose):
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    inc = [f for d in (*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]) for f in ("-isystem", d)]
+    libs = [f for d in cpp_extension.library_paths() for f in ("-L", d)]
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc,
+          os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_PATH, "-L", LIB_DIR, "-lcoset_b200", "-Wl,-rpath,$ORIGIN", *libs,
+          "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"], verbose)
+
+
+def build(force=False, verbose=False):
+    """Compile every .cu under csrc/ that changed (or whose headers did) into lib/libcoset_b200.so, then the
+    PyTorch module; returns the library's path."""
+    os.makedirs(LIB_DIR, exist_ok=True)
+    header = os.path.join(INCLUDE, "coset_b200.h")
+    shared = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")] + [header, __file__]
+    todo, objs = [], []
+    for src in SOURCES:
+        obj = os.path.join(LIB_DIR, src.replace(".cu", ".o"))
+        objs.append(obj)
+        if not force and _newer(obj, [os.path.join(CSRC, src), *shared]):
+            continue
+        verb = ["-Xptxas=-v"] if verbose else []
+        todo.append([_nvcc(), *verb, *NVCC_FLAGS, "-I", INCLUDE, "-c", os.path.join(CSRC, src), "-o", obj])
+    with ThreadPoolExecutor(max_workers=max(1, min(len(todo), os.cpu_count() or 1))) as pool:
+        list(pool.map(lambda cmd: _run(cmd, verbose), todo))
+    if force or not _newer(LIB_PATH, objs):
+        _run([_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"], verbose)
+    # the module finds the library's functions at load time: only its own source and the header matter to it
+    if force or not _newer(TORCH_PATH, [os.path.join(CSRC, TORCH_SOURCE), header, __file__]):
+        _build_torch_module(verbose)
     return LIB_PATH
 
 

@@ -13,6 +13,9 @@ from ... import _lib
 from .lattice import E8Lattice
 
 
+_DTYPE_CODES = {torch.float32: _lib.DTYPE_F32, torch.bfloat16: _lib.DTYPE_BF16}
+
+
 def _as_blocks(x: torch.Tensor, name="x"):
     _lib.require_cuda(x, name)
     squeeze = x.dim() == 1
@@ -58,20 +61,8 @@ def e8_encode_packed(x: torch.Tensor, q: int = 4, M: int = 2, scale=None, scale_
     multiplies block b by scale[b // blocks_per_tile] (layer convention).
     literal=True forces the op-by-op search for every block (validation of the fast path).
     """
-    x2, _ = _as_blocks(x)
-    n = x2.shape[0]
-    nbytes = _code_dtype(q, M)
-    scale_t, mode, bpt = _scale_args(scale, scale_mode, n, blocks_per_tile, x2.device)
-    if out is None:
-        out = torch.empty((n, nbytes), dtype=torch.uint8, device=x2.device)
-    elif out.numel() * out.element_size() != n * nbytes or not out.is_contiguous() or out.device != x2.device:
-        raise ValueError("out has the wrong size, layout or device")
-    with torch.cuda.device(x2.device):
-        rc = _lib.lib().coset_e8_encode(_lib.ptr(x2), _lib.dtype_code(x2, "x"), _lib.ptr(scale_t), mode, n, bpt,
-                                        q, M, _lib.SEM_CORE_LITERAL if literal else _lib.SEM_CORE, _lib.ptr(out),
-                                        _lib.stream())
-    _lib.check(rc, "coset_e8_encode")
-    return out
+    return _lib.native().encode_packed(x, q, M, scale, scale_mode, blocks_per_tile, out,
+                                       _lib.SEM_CORE_LITERAL if literal else _lib.SEM_CORE)
 
 
 def e8_decode_packed(codes: torch.Tensor, q: int = 4, M: int = 2, scale=None, scale_mode: int = _lib.SCALE_NONE,
@@ -82,29 +73,18 @@ def e8_decode_packed(codes: torch.Tensor, q: int = 4, M: int = 2, scale=None, sc
     depth (1 .. M): coarse-to-fine reconstruction from the `depth` coarsest levels only, the
     float32 counterpart of ref/hnlq.py:447-507.  The residual of an all-zero level word is the
     zero vector, so the finer level words are cleared and the full decoder runs."""
-    _lib.require_cuda(codes, "codes")
-    nbytes = _code_dtype(q, M)
-    total = codes.numel() * codes.element_size()
-    if total % nbytes or not codes.is_contiguous():
-        raise ValueError("codes is not a contiguous array of packed block codes")
-    n = total // nbytes
     if depth is not None:
+        _lib.require_cuda(codes, "codes")
+        nbytes = _code_dtype(q, M)
         if not (1 <= depth <= M):
             raise ValueError(f"depth must be between 1 and {M}, got {depth}")
         if depth < M:
-            levels = codes.view(torch.uint8).reshape(n, M, nbytes // M).clone()
+            if codes.numel() * codes.element_size() % nbytes or not codes.is_contiguous():
+                raise ValueError("codes is not a contiguous array of packed block codes")
+            levels = codes.view(torch.uint8).reshape(-1, M, nbytes // M).clone()
             levels[:, :M - depth] = 0
             codes = levels.view(-1)
-    scale_t, mode, bpt = _scale_args(scale, scale_mode, n, blocks_per_tile, codes.device)
-    if out is None:
-        out = torch.empty((n, 8), dtype=dtype, device=codes.device)
-    elif out.shape != (n, 8) or not out.is_contiguous() or out.device != codes.device:
-        raise ValueError("out has the wrong shape, layout or device")
-    with torch.cuda.device(codes.device):
-        rc = _lib.lib().coset_e8_decode(_lib.ptr(codes), _lib.ptr(scale_t), mode, n, bpt, q, M, _lib.SEM_CORE,
-                                        _lib.ptr(out), _lib.dtype_code(out, "out"), _lib.stream())
-    _lib.check(rc, "coset_e8_decode")
-    return out
+    return _lib.native().decode_packed(codes, q, M, scale, scale_mode, blocks_per_tile, _DTYPE_CODES.get(dtype, -1), out)
 
 
 def e8_encode(x: torch.Tensor, config, lattice=None, dither: Optional[torch.Tensor] = None,
@@ -116,28 +96,21 @@ def e8_encode(x: torch.Tensor, config, lattice=None, dither: Optional[torch.Tens
     """
     if device is not None:
         x = x.to(device)
-    x2, squeeze = _as_blocks(x)
-    if x2.dtype != torch.float32:
-        raise TypeError(f"e8_encode expects float32 like the reference; got {x2.dtype} "
-                        "(use e8_encode_packed for bfloat16 input)")
     q, M, beta = int(config.q), int(config.M), float(config.beta)
-    if getattr(config, "with_dither", False) and dither is not None:
+    if dither is not None and getattr(config, "with_dither", False):
         # codecs.py:64-69: x / beta + dither, then quantise without further scaling.  The
         # division uses a device tensor so that it is an IEEE division, as on the CPU.
+        x2, squeeze = _as_blocks(x)
+        if x2.dtype != torch.float32:
+            raise TypeError(f"e8_encode expects float32 like the reference; got {x2.dtype} "
+                            "(use e8_encode_packed for bfloat16 input)")
         d = dither.to(x2.device)
         if d.dim() == 1:
             d = d.unsqueeze(0)
         xs = x2 / torch.tensor(beta, dtype=torch.float32, device=x2.device) + d
-        packed = e8_encode_packed(xs.contiguous(), q, M)
-    else:
-        packed = e8_encode_packed(x2, q, M, scale=beta, scale_mode=_lib.SCALE_DIV_SCALAR)
-    digits = torch.empty((x2.shape[0], M, 8), dtype=torch.float32, device=x2.device)
-    with torch.cuda.device(x2.device):
-        rc = _lib.lib().coset_e8_unpack_codes_f32(_lib.ptr(packed), x2.shape[0], q, M, _lib.ptr(digits), _lib.stream())
-    _lib.check(rc, "coset_e8_unpack_codes_f32")
-    if squeeze:
-        digits = digits.squeeze(0)
-    return digits, 0
+        digits = _lib.native().encode_digits(xs, q, M, 1.0)
+        return (digits.squeeze(0) if squeeze else digits), 0
+    return _lib.native().encode_digits(x, q, M, beta), 0
 
 
 class DecodingMethod(Enum):
@@ -147,21 +120,7 @@ class DecodingMethod(Enum):
 
 
 def _decode_digits(b: torch.Tensor, config) -> torch.Tensor:
-    _lib.require_cuda(b, "b")
-    squeeze = b.dim() == 2
-    b3 = b.unsqueeze(0) if squeeze else b
-    if b3.dim() != 3 or b3.shape[2] != 8:
-        raise ValueError(f"encoding vectors must have shape [N, M, 8] or [M, 8], got {tuple(b.shape)}")
-    n, M, _ = b3.shape
-    q, beta = int(config.q), float(config.beta)
-    nbytes = _code_dtype(q, M)
-    digits = b3.to(torch.float32).contiguous()
-    packed = torch.empty((n, nbytes), dtype=torch.uint8, device=b3.device)
-    with torch.cuda.device(b3.device):
-        rc = _lib.lib().coset_e8_pack_codes_f32(_lib.ptr(digits), n, q, M, _lib.ptr(packed), _lib.stream())
-    _lib.check(rc, "coset_e8_pack_codes_f32")
-    out = e8_decode_packed(packed, q, M, scale=beta, scale_mode=_lib.SCALE_DIV_SCALAR)
-    return out.squeeze(0) if squeeze else out
+    return _lib.native().decode_digits(b, int(config.q), float(config.beta))
 
 
 class E8Decoder:
@@ -190,14 +149,7 @@ def e8_decode(b: torch.Tensor, config, method: str = "full", device: Optional[to
 def e8_quantize(x: torch.Tensor, q: int, lattice: Optional[E8Lattice] = None) -> torch.Tensor:
     """decode(encode(x)) with M = 2 and beta = 1, as the reference hard-wires
     (coset/core/e8/codecs.py:221-286), in one fused kernel."""
-    x2, squeeze = _as_blocks(x)
-    _code_dtype(q, 2)
-    out = torch.empty((x2.shape[0], 8), dtype=torch.float32, device=x2.device)
-    with torch.cuda.device(x2.device):
-        rc = _lib.lib().coset_e8_quantize(_lib.ptr(x2), _lib.dtype_code(x2, "x"), None, _lib.SCALE_NONE, x2.shape[0],
-                                          1, q, 2, 0.0, _lib.ptr(out), _lib.DTYPE_F32, None, _lib.stream())
-    _lib.check(rc, "coset_e8_quantize")
-    return out.squeeze(0) if squeeze else out
+    return _lib.native().quantize(x, q)
 
 
 def e8_quant_stats(x: torch.Tensor, scale=None, scale_mode: int = _lib.SCALE_NONE, blocks_per_tile: int = 1) -> dict:

@@ -96,59 +96,6 @@ class _E8FakeQuant(torch.autograd.Function):
         return grad_w, (grad_beta.view(beta_shape) if need_beta else None), None, None, None, None
 
 
-class _E8LayerFakeQuant(torch.autograd.Function):
-    """The layer's whole weight path in one call each way: the per-tile scale
-    beta = beta_min + sigmoid(theta) * (beta_max - beta_min) is computed on the device
-    (coset_e8_layer_fake_quant_fwd), and the backward call returns dL/dW and dL/dtheta directly
-    (coset_e8_layer_fake_quant_bwd), so no small torch kernels sit around the two CUDA kernels."""
-
-    @staticmethod
-    def forward(ctx, weight, theta, beta_min, beta_range, blocks_per_tile, q, clip, out_dtype):
-        _lib.require_float32(weight, "weight")
-        _lib.require_cuda(weight, "weight")
-        w = weight.contiguous()
-        th = theta.detach().to(torch.float32).contiguous().view(-1)
-        n_blocks = w.numel() // 8
-        lib = _lib.lib()
-        code_bytes = lib.coset_e8_code_bytes(q, 2)
-        if code_bytes == 0:
-            raise ValueError(f"unsupported q={q} for the fused E8 weight quantiser (2 <= q <= 16)")
-        codes = torch.empty((n_blocks, code_bytes), dtype=torch.uint8, device=w.device)
-        out = torch.empty(w.shape, dtype=out_dtype, device=w.device)
-        beta = torch.empty_like(th)
-        with torch.cuda.device(w.device):
-            rc = lib.coset_e8_layer_fake_quant_fwd(_lib.ptr(w), _lib.ptr(th), _lib.ptr(beta_min), _lib.ptr(beta_range), n_blocks,
-                                                   blocks_per_tile, q, float(clip), _lib.ptr(out), _lib.dtype_code(out, "out"),
-                                                   _lib.ptr(codes), _lib.ptr(beta), _lib.stream())
-        _lib.check(rc, "coset_e8_layer_fake_quant_fwd")
-        ctx.save_for_backward(w, th, beta, codes)
-        # the bounds tensors are refreshed in place once every stat_update_interval steps (so that a captured
-        # graph keeps reading them); kept outside save_for_backward, whose version check would turn a refresh
-        # between this forward and its backward into an error
-        ctx.beta_range = beta_range
-        ctx.meta = (blocks_per_tile, q, float(clip), theta.shape)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        w, th, beta, codes = ctx.saved_tensors
-        beta_range = ctx.beta_range
-        blocks_per_tile, q, clip, theta_shape = ctx.meta
-        g = grad_out.contiguous()
-        if g.dtype not in (torch.float32, torch.bfloat16):
-            g = g.float()
-        grad_w = torch.empty_like(w)
-        need_theta = ctx.needs_input_grad[1]
-        grad_theta = torch.empty_like(th) if need_theta else None
-        with torch.cuda.device(w.device):
-            rc = _lib.lib().coset_e8_layer_fake_quant_bwd(_lib.ptr(g), _lib.dtype_code(g, "grad"), _lib.ptr(w), _lib.ptr(codes),
-                                                          _lib.ptr(beta), _lib.ptr(th), _lib.ptr(beta_range), w.numel() // 8,
-                                                          blocks_per_tile, q, clip, _lib.ptr(grad_w), _lib.ptr(grad_theta),
-                                                          _lib.stream())
-        _lib.check(rc, "coset_e8_layer_fake_quant_bwd")
-        return grad_w, (grad_theta.view(theta_shape) if need_theta else None), None, None, None, None, None, None
-
-
 def e8_fake_quantize(weight, beta, blocks_per_tile, q=4, clip=2.0, out_dtype=torch.float32):
     """Differentiable fused weight quantiser used by HNLQLinearQAT (see _E8FakeQuant)."""
     return _E8FakeQuant.apply(weight, beta, int(blocks_per_tile), int(q), float(clip), out_dtype)
@@ -348,9 +295,10 @@ class HNLQLinearQAT(nn.Module):
         The bounds depend only on the two statistics buffers, which change once every 256 quantised
         forwards, so they are kept until one of the buffers is written (in place or replaced) or a
         hyper-parameter changes; the arithmetic and its order are the reference's."""
-        key = (self.sigma_ema._version, self.xmax_ema._version, self.sigma_ema.data_ptr(), self.xmax_ema.data_ptr(),
-               self.Delta0, self.eta, self.q, self.M)
-        if getattr(self, "_bounds_key", None) != key:
+        state = self.__dict__
+        sigma, xmax = state["_buffers"]["sigma_ema"], state["_buffers"]["xmax_ema"]
+        key = (sigma._version, xmax._version, sigma.data_ptr(), xmax.data_ptr(), state["Delta0"], state["eta"], state["q"], state["M"])
+        if state.get("_bounds_key") != key:
             with torch.no_grad():
                 qM = float(self.q ** self.M)
                 ginv = self._gamma_inv_host
@@ -389,23 +337,28 @@ class HNLQLinearQAT(nn.Module):
         return exact + (soft - soft.detach())  # value of the kernel, gradient of the torch expression
 
     # ------------------------------------------------------------------ quantised weights
+    def _count_step(self, W):
+        """One quantised forward pass more; every stat_update_interval of them the statistics follow the weights.
+        The step counter lives on the host; the `step_count` buffer is brought up to date when it is
+        read (state_dict, int(layer.step_count) through the property above) -- one launch less per step."""
+        self._step_host += 1
+        if self._step_host % self.stat_update_interval == 0:
+            self._sync_step_count()
+            self._gather_stats(W.detach().view(self.out_features, self.blocks_per_row, self.block_size))
+
     def _quantize_weights(self, out_dtype=torch.float32):
         W = self.weight
         if not self.quantization_enabled:
             if self.enable_diagnostics:
                 self._weight_history.append(W.detach().clone())
             return W
-        # the step counter lives on the host; the `step_count` buffer is brought up to date when it is
-        # read (state_dict, int(layer.step_count) through the property below) -- one launch less per step
-        self._step_host += 1
-        if self._step_host % self.stat_update_interval == 0:
-            self._sync_step_count()
-            self._gather_stats(W.detach().view(self.out_features, self.blocks_per_row, self.block_size))
+        self._count_step(W)
         bpt = self.blocks_per_row if self.tiling == "row" else 1
         if self._fused and W.is_cuda:
             beta_min, _ = self._bounds()
-            W_q = _E8LayerFakeQuant.apply(W, self.theta_beta, beta_min, self._bounds_cache[2], bpt, int(self.q),
-                                          float(self.weight_clip_value), out_dtype)
+            W_q = _lib.native().layer_fake_quant(W, self.theta_beta, beta_min, self._bounds_cache[2], bpt, int(self.q),
+                                                 float(self.weight_clip_value),
+                                                 _lib.DTYPE_BF16 if out_dtype == torch.bfloat16 else _lib.DTYPE_F32)
         elif self._fused_d4 and W.is_cuda:
             from .d4.layers import d4_fake_quantize
             W_q = d4_fake_quantize(W, self._beta(), bpt, self.weight_clip_value, out_dtype)
@@ -427,8 +380,30 @@ class HNLQLinearQAT(nn.Module):
         Wq = Wq.view(self.out_features, self.blocks_per_row, self.block_size) / b3
         return torch.clamp(Wq.reshape(self.out_features, self.in_features), -self.weight_clip_value, self.weight_clip_value)
 
+    def _one_node(self, x, low):
+        """Whether the whole product can run as one native autograd node: the plain case of a quantised E8 layer
+        on the GPU.  Warm-up, diagnostics (which look at the quantised weights), autocast, parametrised weights and
+        a quantize_fn of the caller's own take the composed path."""
+        state = self.__dict__
+        params = state["_parameters"]
+        return (state["_fused"] and state["quantization_enabled"] and not state["enable_diagnostics"] and x.is_cuda
+                and (low or x.dtype == torch.float32) and not torch.is_autocast_enabled("cuda")
+                and "weight" in params and ("theta_beta" in params or not state["theta_trainable"]) and params["weight"].is_cuda)
+
     def forward(self, x):
         low = x.dtype == torch.bfloat16
+        if self._one_node(x, low):
+            # quantised weights, product and bias as one autograd node in native code
+            params = self.__dict__["_parameters"]
+            W = params["weight"]
+            self._count_step(W)
+            beta_min, _ = self._bounds()
+            theta = params["theta_beta"] if self.theta_trainable else self.__dict__["_buffers"]["theta_beta"]
+            x = _lib.native().qat_linear(x, W, theta, params["bias"], beta_min, self._bounds_cache[2],
+                                         self.blocks_per_row if self.tiling == "row" else 1, int(self.q), float(self.weight_clip_value))
+            if self.quantize_activations and self.actq is not None:
+                x = self.actq(x)
+            return x
         W_q = self._quantize_weights(torch.bfloat16 if low else torch.float32)
         bias = self.bias
         if low:

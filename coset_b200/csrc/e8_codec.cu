@@ -53,9 +53,12 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// one divisor as a kernel argument instead of a device pointer (the digit entry points)
+constexpr int kScaleDivValue = 3;
+
 template <int MODE>
 __device__ __forceinline__ float scale_in(float v, float s) {
-    if (MODE == COSET_SCALE_DIV_SCALAR) return __fdiv_rn(v, s);
+    if (MODE == COSET_SCALE_DIV_SCALAR || MODE == kScaleDivValue) return __fdiv_rn(v, s);
     if (MODE == COSET_SCALE_MUL_TILE) return __fmul_rn(v, s);
     return v;
 }
@@ -237,28 +240,42 @@ inline unsigned encoder_grid(int64_t n_blocks) {
     return (unsigned)(need < cap ? (need < 1 ? 1 : need) : cap);
 }
 
-// RECON = false: codes only (e8_encode).  RECON = true: the fused round trip -- every finished code is
-// decoded through the residual table, unscaled, clamped and written as [n, 8] of type DTO; the
-// packed code is stored only if `codes` is not null (e8_quantize / the layer's weight path).
-template <int DT, int MODE, bool RECON, int DTO, bool SAT>
+// KIND = kRecon: the fused round trip -- every finished code is decoded through the residual table, unscaled,
+// clamped and written as [n, 8] of type DTO; the packed code is stored only if `codes` is not null (e8_quantize /
+// the layer's weight path).  KIND = kDigits: the code is written as the reference's float32 digits [n, 2, 8].
+// `value` is the divisor of MODE == kScaleDivValue and the clamp otherwise.
+constexpr int kRecon = 0, kDigits = 1;
+
+__device__ __forceinline__ void store_digits(float* __restrict__ digits, int64_t row, uint32_t word) {
+    int d[8];
+    float f[8];
+    e8::unpack_level<2>(word, d);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = (float)d[i];
+    e8::Row8<0>::store(digits, row, f);
+}
+
+template <int DT, int MODE, int KIND, int DTO, bool SAT>
 __global__ void __launch_bounds__(kThreads, 4)
 k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n,
-                     uint32_t* __restrict__ codes, const uint2* __restrict__ table, void* __restrict__ out, float clip) {
+                     uint32_t* __restrict__ codes, const uint2* __restrict__ table, void* __restrict__ out, float value) {
     __shared__ uint32_t q_index[kEncWarps][2][kQueueSlots];  // block index lo / hi
     __shared__ int q_count[kEncWarps];
     auto emit = [&](int64_t b, uint32_t code, float s) {
-        if (!RECON) {
-            __stcs(codes + b, code);
+        if constexpr (KIND == kDigits) {
+            store_digits((float*)out, 2 * b, code & 0xffffu);
+            store_digits((float*)out, 2 * b + 1, code >> 16);
         } else {
             if (codes) __stcs(codes + b, code);
             float v2[8], xh[8];
             e8::decode_q4m2_twice(code, table, v2);
             e8::scale_twice<MODE>(v2, s, xh);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) xh[i] = clampf(xh[i], clip);
+            for (int i = 0; i < 8; ++i) xh[i] = clampf(xh[i], value);
             e8::Row8<DTO>::store(out, b, xh);
         }
     };
+    auto scale_of = [&](int64_t b) { return MODE == kScaleDivValue ? value : load_scale<MODE>(scale, td, b); };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) q_count[warp] = 0;
     __syncwarp();
@@ -272,7 +289,7 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
             const int64_t b = (int64_t)(((uint64_t)q_index[warp][1][e] << 32) | q_index[warp][0][e]);
             float v[8];
             e8::Row8<DT>::load(x, b, v);
-            const float s = load_scale<MODE>(scale, td, b);
+            const float s = scale_of(b);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 v[i] = scale_in<MODE>(v[i], s);
@@ -303,7 +320,7 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
                 sc[j] = 1.0f;
                 if (b < n) {
                     e8::Row8<DT>::load(x, b, v[j]);
-                    sc[j] = load_scale<MODE>(scale, td, b);
+                    sc[j] = scale_of(b);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) v[j][i] = 0.0f;
@@ -640,6 +657,67 @@ k_pack_f32(const float* __restrict__ digits, int64_t n_words, int q, void* __res
     reinterpret_cast<typename LevelWord<BPD>::type*>(codes)[i] = (typename LevelWord<BPD>::type)e8::pack_level<BPD>(d);
 }
 
+// Digits of any (q, M) from the literal search, and values from digits: what coset_e8_encode / _decode do with packed
+// codes in between, without the packed array (4 launches and 72 bytes per block less for q = 4, M = 2).
+__global__ void __launch_bounds__(kThreads)
+k_encode_digits_generic(const float* __restrict__ x, float beta, int64_t n, int q, int M, float* __restrict__ digits) {
+    const int64_t b = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (b >= n) return;
+    float xl[8];
+    e8::Row8<0>::load(x, b, xl);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) xl[i] = __fdiv_rn(xl[i], beta);
+    const float qf = (float)q;
+    for (int m = 0; m < M; ++m) {
+        float y[8], f[8];
+        int d[8];
+        const bool half = e8::projection(xl, y);
+        e8::encode_coords(y, half, q, d);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = (float)d[i];
+        e8::Row8<0>::store(digits, b * M + m, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) xl[i] = __fdiv_rn(xl[i], qf);
+    }
+}
+
+// Q4: the residual of a level comes from the table; the sum over the levels is exact in float32 (multiples of 1/2
+// below 2^18), so its order does not matter.
+template <bool Q4>
+__global__ void __launch_bounds__(kThreads)
+k_decode_digits(const float* __restrict__ digits, float beta, int64_t n, int q, int M, const uint2* __restrict__ table, float* __restrict__ out) {
+    const int64_t b = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (b >= n) return;
+    float xh[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) xh[i] = 0.0f;
+    const float qf = (float)q;
+    float w = 1.0f;
+    for (int m = 0; m < M; ++m) {
+        float f[8], r[8];
+        int d[8];
+        e8::Row8<0>::load(digits, b * M + m, f);
+        if (Q4) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d[j] = __float2int_rn(f[j]) & 3;
+            const uint2 t = __ldg(table + e8::pack_level<2>(d));
+            const uint32_t tw[2] = {t.x, t.y};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = 0.5f * (float)((int)((tw[j >> 2] >> (8 * (j & 3))) & 0xffu) - e8::kTableBias);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d[j] = e8::floored_mod(__float2int_rn(f[j]), q);
+            e8::level_residual(d, qf, r);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) xh[i] = __fadd_rn(xh[i], __fmul_rn(w, r[i]));
+        w = __fmul_rn(w, qf);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) xh[i] = __fmul_rn(xh[i], beta);
+    e8::Row8<0>::store(out, b, xh);
+}
+
 inline unsigned grid_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
 int check_common(const void* a, const void* b, int64_t n_blocks, int q, int M) {
@@ -879,7 +957,7 @@ int coset_e8_quantize(const void* x, int x_dtype, const float* scale, int scale_
         const uint2* table = residual_table_q4(st);
         if (!table) return COSET_E_STATE;
         unsigned qgrid = encoder_grid(n_blocks);
-        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_encode_q4m2_queued<DTI, MODE, true, DTO, false><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)))))
+        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, false><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)))))
     } else if (q <= 4) {
         DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_quantize_generic<DTI, DTO, MODE, 2><<<grid, kThreads, 0, st>>>(x, scale, td, n_blocks, q, M, clip, out, codes_out)))))
     } else {
@@ -906,6 +984,39 @@ int coset_e8_pack_codes_f32(const float* digits, int64_t n_blocks, int q, int M,
     if (q <= 4) k_pack_f32<2><<<grid_for(nw), kThreads, 0, (cudaStream_t)stream>>>(digits, nw, q, codes);
     else k_pack_f32<4><<<grid_for(nw), kThreads, 0, (cudaStream_t)stream>>>(digits, nw, q, codes);
     return check_launch("e8_pack_codes_f32");
+}
+
+int coset_e8_encode_digits_f32(const float* x, float beta, int64_t n_blocks, int q, int M, float* digits, void* stream) {
+    if (int e = check_common(x, digits, n_blocks, q, M)) return e;
+    if (n_blocks == 0) return 0;
+    if (!aligned(x, 16) || !aligned(digits, 16)) return fail(COSET_E_ALIGN, "x and digits must be 16-byte aligned");
+    cudaStream_t st = (cudaStream_t)stream;
+    if (q == 4 && M == 2) {
+        const e8::TileDiv td = e8::make_tile_div(1, n_blocks);
+        const unsigned grid = encoder_grid(n_blocks);
+        if (beta == 1.0f)  // x / 1 is x
+            k_encode_q4m2_queued<0, COSET_SCALE_NONE, kDigits, 0, false><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, 0.0f);
+        else
+            k_encode_q4m2_queued<0, kScaleDivValue, kDigits, 0, false><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, beta);
+    } else {
+        k_encode_digits_generic<<<grid_for(n_blocks), kThreads, 0, st>>>(x, beta, n_blocks, q, M, digits);
+    }
+    return check_launch("e8_encode_digits_f32");
+}
+
+int coset_e8_decode_digits_f32(const float* digits, float beta, int64_t n_blocks, int q, int M, float* out, void* stream) {
+    if (int e = check_common(digits, out, n_blocks, q, M)) return e;
+    if (n_blocks == 0) return 0;
+    if (!aligned(digits, 16) || !aligned(out, 16)) return fail(COSET_E_ALIGN, "digits and out must be 16-byte aligned");
+    cudaStream_t st = (cudaStream_t)stream;
+    if (q == 4) {
+        const uint2* table = residual_table_q4(st);
+        if (!table) return COSET_E_STATE;
+        k_decode_digits<true><<<grid_for(n_blocks), kThreads, 0, st>>>(digits, beta, n_blocks, q, M, table, out);
+    } else {
+        k_decode_digits<false><<<grid_for(n_blocks), kThreads, 0, st>>>(digits, beta, n_blocks, q, M, nullptr, out);
+    }
+    return check_launch("e8_decode_digits_f32");
 }
 
 }  // extern "C"

@@ -1,0 +1,449 @@
+// Native entry points for PyTorch callers: argument checks, output allocation and the launch of one C-ABI
+// call in a single Python -> C++ step.
+//
+// What bounds a small call is the host: through ctypes an encode of a few thousand blocks took 25-30 us of
+// argument conversion, device context and allocation in Python against 3-9 us on the device.  The functions
+// here are plain METH_FASTCALL entry points of a CPython module (no argument parsing library) that read the
+// tensors directly; they add nothing to what the C ABI computes.  The library itself (libcoset_b200.so) stays
+// free of torch symbols; this module links against both.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/coset_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+// ---------------------------------------------------------------- small helpers
+void* stream_of(const Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+void* data(const Tensor& t) { return t.defined() && t.numel() > 0 ? t.data_ptr() : nullptr; }
+float* fdata(const Tensor& t) { return (float*)data(t); }
+
+void check_rc(int rc, const char* what) {
+    TORCH_CHECK(rc == 0, what, " failed with status ", rc, ": ", coset_last_error_string());
+}
+
+const Tensor& tensor_arg(PyObject* o, const char* name) {
+    TORCH_CHECK_TYPE(THPVariable_Check(o), name, " must be a torch.Tensor, got ", Py_TYPE(o)->tp_name);
+    return THPVariable_Unpack(o);
+}
+const Tensor& cuda_arg(PyObject* o, const char* name) {
+    const Tensor& t = tensor_arg(o, name);
+    TORCH_CHECK_VALUE(t.is_cuda(), name, " must live on a CUDA device (coset_b200 has no CPU path); got ", t.device());
+    return t;
+}
+Tensor optional_arg(PyObject* o, const char* name) { return o == Py_None ? Tensor() : tensor_arg(o, name); }
+
+int64_t int_arg(PyObject* o) {
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw python_error();
+    return (int64_t)v;
+}
+double float_arg(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw python_error();
+    return v;
+}
+void nargs_are(Py_ssize_t got, Py_ssize_t want) { TORCH_CHECK_TYPE(got == want, "expected ", want, " arguments, got ", got); }
+
+int dtype_code(const Tensor& t, const char* name) {
+    if (t.scalar_type() == at::kFloat) return COSET_DTYPE_F32;
+    TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, name, " must be float32 or bfloat16, got ", t.scalar_type());
+    return COSET_DTYPE_BF16;
+}
+at::ScalarType scalar_type(int code) { return code == COSET_DTYPE_F32 ? at::kFloat : at::kBFloat16; }
+
+Tensor empty(at::IntArrayRef size, at::ScalarType type, const Tensor& like) {
+    return at::detail::empty_cuda(size, type, like.device(), std::nullopt);
+}
+// The tensor as contiguous float32, itself when it already is.
+Tensor as_f32(const Tensor& t) {
+    if (!t.defined()) return t;
+    Tensor f = t.scalar_type() == at::kFloat ? t : t.to(at::kFloat);
+    return f.is_contiguous() ? f : f.contiguous();
+}
+Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+
+// rows of 8: a vector is one row
+Tensor as_blocks(PyObject* o, const char* name, bool* squeeze) {
+    const Tensor& x = cuda_arg(o, name);
+    *squeeze = x.dim() == 1;
+    Tensor x2 = *squeeze ? x.unsqueeze(0) : x;
+    TORCH_CHECK_VALUE(x2.dim() == 2, name, " must be 1-D or 2-D, got ", x2.dim(), " dimensions");
+    TORCH_CHECK_VALUE(x2.size(1) == 8, "Input dimension ", x2.size(1), " doesn't match E8 dimension 8");
+    return contiguous(x2);
+}
+int64_t code_bytes(int64_t q, int64_t M) {
+    const int b = coset_e8_code_bytes((int)q, (int)M);
+    TORCH_CHECK_VALUE(b != 0, "unsupported (q=", q, ", M=", M, "); the CUDA library handles 2 <= q <= 16, 1 <= M <= 8");
+    return b;
+}
+
+struct Scale {
+    Tensor t;
+    int mode = COSET_SCALE_NONE;
+    int64_t bpt = 1;
+};
+Scale scale_arg(PyObject* o, int64_t mode, int64_t n_blocks, int64_t bpt, const Tensor& x) {
+    Scale s;
+    if (o == Py_None || mode == COSET_SCALE_NONE) return s;
+    if (THPVariable_Check(o)) s.t = as_f32(cuda_arg(o, "scale"));
+    else s.t = at::full({1}, float_arg(o), x.options().dtype(at::kFloat));  // filled on the device: no copy from the host
+    if (mode == COSET_SCALE_DIV_SCALAR) {
+        TORCH_CHECK_VALUE(s.t.numel() == 1, "the codec (divide) convention takes one scalar beta");
+    } else {
+        const int64_t tiles = bpt > 0 ? (n_blocks + bpt - 1) / bpt : 0;
+        TORCH_CHECK_VALUE(s.t.numel() == tiles, "expected ", tiles, " per-tile scales, got ", s.t.numel());
+    }
+    s.mode = (int)mode;
+    s.bpt = bpt;
+    return s;
+}
+
+// ---------------------------------------------------------------- codec
+// encode_packed(x, q, M, scale, scale_mode, blocks_per_tile, out, sem)
+PyObject* encode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 8);
+    bool squeeze;
+    const Tensor x = as_blocks(a[0], "x", &squeeze);
+    const int64_t q = int_arg(a[1]), M = int_arg(a[2]), nb = x.size(0);
+    const int64_t bytes = code_bytes(q, M);
+    c10::cuda::CUDAGuard guard(x.device());
+    const Scale s = scale_arg(a[3], int_arg(a[4]), nb, int_arg(a[5]), x);
+    Tensor out;
+    if (a[6] == Py_None) {
+        out = empty({nb, bytes}, at::kByte, x);
+    } else {
+        out = tensor_arg(a[6], "out");
+        TORCH_CHECK_VALUE((int64_t)out.nbytes() == nb * bytes && out.is_contiguous() && out.device() == x.device(),
+                          "out has the wrong size, layout or device");
+    }
+    check_rc(coset_e8_encode(data(x), dtype_code(x, "x"), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, (int)int_arg(a[7]), data(out),
+                             stream_of(x)), "coset_e8_encode");
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// decode_packed(codes, q, M, scale, scale_mode, blocks_per_tile, dtype_code, out)
+PyObject* decode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 8);
+    const Tensor& codes = cuda_arg(a[0], "codes");
+    const int64_t q = int_arg(a[1]), M = int_arg(a[2]);
+    const int64_t bytes = code_bytes(q, M), total = (int64_t)codes.nbytes();
+    TORCH_CHECK_VALUE(total % bytes == 0 && codes.is_contiguous(), "codes is not a contiguous array of packed block codes");
+    const int64_t nb = total / bytes;
+    c10::cuda::CUDAGuard guard(codes.device());
+    const Scale s = scale_arg(a[3], int_arg(a[4]), nb, int_arg(a[5]), codes);
+    Tensor out;
+    if (a[7] == Py_None) {
+        out = empty({nb, 8}, scalar_type((int)int_arg(a[6])), codes);
+    } else {
+        out = tensor_arg(a[7], "out");
+        TORCH_CHECK_VALUE(out.dim() == 2 && out.size(0) == nb && out.size(1) == 8 && out.is_contiguous() && out.device() == codes.device(),
+                          "out has the wrong shape, layout or device");
+    }
+    check_rc(coset_e8_decode(data(codes), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, COSET_SEM_CORE, data(out), dtype_code(out, "out"),
+                             stream_of(codes)), "coset_e8_decode");
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// encode_digits(x, q, M, beta) -> float32 digits [N, M, 8]
+PyObject* encode_digits(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 4);
+    bool squeeze;
+    const Tensor x = as_blocks(a[0], "x", &squeeze);
+    TORCH_CHECK_TYPE(x.scalar_type() == at::kFloat, "e8_encode expects float32 like the reference; got ", x.scalar_type(),
+                     " (use e8_encode_packed for bfloat16 input)");
+    const int64_t q = int_arg(a[1]), M = int_arg(a[2]);
+    code_bytes(q, M);
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor digits = squeeze ? empty({M, 8}, at::kFloat, x) : empty({x.size(0), M, 8}, at::kFloat, x);
+    check_rc(coset_e8_encode_digits_f32(fdata(x), (float)float_arg(a[3]), x.size(0), (int)q, (int)M, fdata(digits), stream_of(x)),
+             "coset_e8_encode_digits_f32");
+    return THPVariable_Wrap(digits);
+    END_HANDLE_TH_ERRORS
+}
+
+// decode_digits(digits [N, M, 8] or [M, 8], q, beta) -> float32 [N, 8] or [8]
+PyObject* decode_digits(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 3);
+    const Tensor& b = cuda_arg(a[0], "b");
+    const bool squeeze = b.dim() == 2;
+    TORCH_CHECK_VALUE((squeeze || b.dim() == 3) && b.size(-1) == 8, "encoding vectors must have shape [N, M, 8] or [M, 8], got ", b.sizes());
+    const int64_t q = int_arg(a[1]), M = b.size(-2), nb = squeeze ? 1 : b.size(0);
+    code_bytes(q, M);
+    c10::cuda::CUDAGuard guard(b.device());
+    const Tensor digits = as_f32(b);
+    Tensor out = squeeze ? empty({8}, at::kFloat, b) : empty({nb, 8}, at::kFloat, b);
+    check_rc(coset_e8_decode_digits_f32(fdata(digits), (float)float_arg(a[2]), nb, (int)q, (int)M, fdata(out), stream_of(b)),
+             "coset_e8_decode_digits_f32");
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// quantize(x, q): e8_quantize, float32 result
+PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 2);
+    bool squeeze;
+    const Tensor x = as_blocks(a[0], "x", &squeeze);
+    const int64_t q = int_arg(a[1]);
+    code_bytes(q, 2);
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = squeeze ? empty({8}, at::kFloat, x) : empty({x.size(0), 8}, at::kFloat, x);
+    check_rc(coset_e8_quantize(data(x), dtype_code(x, "x"), nullptr, COSET_SCALE_NONE, x.size(0), 1, (int)q, 2, 0.0f, data(out),
+                               COSET_DTYPE_F32, nullptr, stream_of(x)), "coset_e8_quantize");
+    return THPVariable_Wrap(out);
+    END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- gradient exchange
+// grad_encode(blocks [n, 8], scale (1-element tensor), out, sem)
+PyObject* grad_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 4);
+    const Tensor &x = tensor_arg(a[0], "grad"), &s = tensor_arg(a[1], "scale"), &out = tensor_arg(a[2], "out");
+    const int64_t nb = x.size(0);
+    c10::cuda::CUDAGuard guard(x.device());
+    check_rc(coset_e8_encode(data(x), dtype_code(x, "grad"), fdata(s), COSET_SCALE_MUL_TILE, nb, nb > 0 ? nb : 1, 4, 2,
+                             (int)int_arg(a[3]), data(out), stream_of(x)), "coset_e8_encode");
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
+// decode_mean(codes [world, stride], world, n_blocks, scale, out)
+PyObject* decode_mean(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 5);
+    const Tensor &codes = tensor_arg(a[0], "codes"), &out = tensor_arg(a[4], "out");
+    c10::cuda::CUDAGuard guard(codes.device());
+    check_rc(coset_e8_decode_mean(data(codes), (int)int_arg(a[1]), int_arg(a[2]), codes.size(1), (float)float_arg(a[3]), data(out),
+                                  dtype_code(out, "out"), stream_of(codes)), "coset_e8_decode_mean");
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- code-domain product
+void check_codes(const Tensor& codes) {
+    TORCH_CHECK_VALUE(codes.scalar_type() == at::kInt && codes.dim() == 2 && codes.is_contiguous(),
+                      "codes must be a contiguous int32 tensor [n_out, n_in / 8]");
+}
+// [..., n_in] -> [T, n_in] and the shape of the result
+Tensor token_rows(const Tensor& x, int64_t n_in, int64_t n_out, c10::SmallVector<int64_t, 6>* y_shape) {
+    for (int64_t i = 0; i + 1 < x.dim(); ++i) y_shape->push_back(x.size(i));
+    y_shape->push_back(n_out);
+    Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, n_in});
+    return contiguous(x2);
+}
+
+// vlut_linear(x [..., n_in], codes, beta or None, blocks_per_tile, bias or None, clip, out_dtype_code)
+PyObject* vlut_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 7);
+    const Tensor &codes = cuda_arg(a[1], "codes"), &x = cuda_arg(a[0], "x");
+    check_codes(codes);
+    const int64_t n_out = codes.size(0), n_in = codes.size(1) * 8;
+    TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in, "x must be [T, ", n_in, "], got ", x.sizes());
+    c10::cuda::CUDAGuard guard(x.device());
+    c10::SmallVector<int64_t, 6> shape;
+    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
+    const Tensor beta = as_f32(optional_arg(a[2], "beta")), bias = as_f32(optional_arg(a[4], "bias"));
+    const int y_code = (int)int_arg(a[6]);
+    Tensor y = empty(shape, scalar_type(y_code), x);
+    check_rc(coset_e8_vlut_gemv(data(codes), fdata(beta), int_arg(a[3]), (int)n_out, (int)n_in, data(x2), dtype_code(x2, "x"), n_in,
+                                (int)x2.size(0), fdata(bias), data(y), y_code, n_out, (float)float_arg(a[5]), stream_of(x)),
+             "coset_e8_vlut_gemv");
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
+// decode_gemm(x [..., n_in] bf16, codes, beta or None, blocks_per_tile, bias or None, clip, scratch or None, out_dtype_code, status or None)
+// -> (y, status)
+PyObject* decode_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 9);
+    const Tensor &codes = cuda_arg(a[1], "codes"), &x = cuda_arg(a[0], "x");
+    TORCH_CHECK_TYPE(x.scalar_type() == at::kBFloat16, "e8_decode_gemm takes bfloat16 activations");
+    check_codes(codes);
+    const int64_t n_out = codes.size(0), n_in = codes.size(1) * 8;
+    TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in && n_in % 64 == 0, "x must be [T, ", n_in, "] with n_in a multiple of 64, got ", x.sizes());
+    c10::cuda::CUDAGuard guard(x.device());
+    c10::SmallVector<int64_t, 6> shape;
+    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
+    Tensor scratch = optional_arg(a[6], "scratch");
+    if (!scratch.defined()) scratch = empty({n_out * n_in}, at::kBFloat16, x);
+    else
+        TORCH_CHECK_VALUE(scratch.scalar_type() == at::kBFloat16 && scratch.numel() >= n_out * n_in && scratch.is_contiguous() && scratch.device() == x.device(),
+                          "scratch must be a contiguous bfloat16 tensor of at least ", n_out * n_in, " values on ", x.device());
+    const int y_code = (int)int_arg(a[7]);
+    Tensor y = empty(shape, scalar_type(y_code), x);
+    Tensor status = optional_arg(a[8], "status");
+    if (!status.defined()) status = at::zeros({1}, x.options().dtype(at::kInt));
+    const Tensor beta = as_f32(optional_arg(a[2], "beta")), bias = as_f32(optional_arg(a[4], "bias"));
+    check_rc(coset_e8_decode_gemm(data(codes), fdata(beta), int_arg(a[3]), (int)n_out, (int)n_in, data(x2), n_in, (int)x2.size(0),
+                                  fdata(bias), data(y), y_code, n_out, (float)float_arg(a[5]), data(scratch), (int64_t)scratch.nbytes(),
+                                  (int*)data(status), stream_of(x)), "coset_e8_decode_gemm");
+    return Py_BuildValue("NN", THPVariable_Wrap(y), THPVariable_Wrap(status));
+    END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- training layer
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// W_q = clamp(e8_quantize(W beta) / beta, +-clip) with beta = beta_min + sigmoid(theta) range per tile, and the
+// straight-through gradients of the reference graph (coset/core/layers.py:62-110, 415-470).
+struct FakeQuant : torch::autograd::Function<FakeQuant> {
+    static void launch(const Tensor& w, const Tensor& th, const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip,
+                       at::ScalarType out_type, Tensor& wq, Tensor& codes, Tensor& beta) {
+        const int bytes = coset_e8_code_bytes((int)q, 2);
+        TORCH_CHECK_VALUE(bytes != 0, "unsupported q=", q, " for the fused E8 weight quantiser (2 <= q <= 16)");
+        const int64_t nb = w.numel() / 8;
+        codes = empty({nb, bytes}, at::kByte, w);
+        wq = empty(w.sizes(), out_type, w);
+        beta = empty({th.numel()}, at::kFloat, w);
+        check_rc(coset_e8_layer_fake_quant_fwd(fdata(w), fdata(th), fdata(beta_min), fdata(beta_range), nb, bpt, (int)q, (float)clip, data(wq),
+                                               out_type == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16, data(codes), fdata(beta), stream_of(w)),
+                 "coset_e8_layer_fake_quant_fwd");
+    }
+    // dL/dW and dL/dtheta (undefined unless asked for) from dL/dW_q
+    static std::pair<Tensor, Tensor> backward_launch(Tensor g, const Tensor& w, const Tensor& theta, const Tensor& beta, const Tensor& codes,
+                                                     const Tensor& beta_range, int64_t bpt, int64_t q, double clip, bool need_theta) {
+        g = contiguous(g);
+        if (g.scalar_type() != at::kFloat && g.scalar_type() != at::kBFloat16) g = g.to(at::kFloat);
+        const Tensor th = as_f32(theta);
+        Tensor gw = empty(w.sizes(), at::kFloat, w), gt;
+        if (need_theta) gt = empty(theta.sizes(), at::kFloat, w);
+        check_rc(coset_e8_layer_fake_quant_bwd(data(g), dtype_code(g, "grad"), fdata(w), data(codes), fdata(beta), fdata(th), fdata(beta_range),
+                                               w.numel() / 8, bpt, (int)q, (float)clip, fdata(gw), fdata(gt), stream_of(w)),
+                 "coset_e8_layer_fake_quant_bwd");
+        return {gw, gt};
+    }
+    static Tensor forward(AutogradContext* ctx, const Tensor& weight, const Tensor& theta, const Tensor& beta_min, const Tensor& beta_range,
+                          int64_t bpt, int64_t q, double clip, int64_t out_code) {
+        const Tensor w = contiguous(weight);
+        Tensor wq, codes, beta;
+        launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, scalar_type((int)out_code), wq, codes, beta);
+        ctx->save_for_backward({w, theta, beta, codes});
+        // the bounds are refreshed in place once every stat_update_interval steps (a captured graph keeps reading
+        // them), so they are kept outside save_for_backward, whose version check would refuse that
+        ctx->saved_data["range"] = beta_range;
+        ctx->saved_data["bpt"] = bpt;
+        ctx->saved_data["q"] = q;
+        ctx->saved_data["clip"] = clip;
+        return wq;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        c10::cuda::CUDAGuard guard(saved[0].device());
+        auto r = backward_launch(grads[0], saved[0], saved[1], saved[2], saved[3], ctx->saved_data["range"].toTensor(), ctx->saved_data["bpt"].toInt(),
+                                 ctx->saved_data["q"].toInt(), ctx->saved_data["clip"].toDouble(), ctx->needs_input_grad(1));
+        return {r.first, r.second, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+// y = x W_q^T + bias as ONE autograd node: the forward quantises and multiplies, the backward forms dx, dW, dtheta
+// and dbias.  An eager step of a small layer is bound by the host; one node instead of five (cast, quantise,
+// transpose, product, bias) and native code on both sides took the step of the [3072, 768] layer with 4096
+// tokens from 312 us to the time of its kernels.
+struct QatLinear : torch::autograd::Function<QatLinear> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& theta, const Tensor& bias,
+                          const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip) {
+        const Tensor w = contiguous(weight);
+        Tensor wq, codes, beta;
+        FakeQuant::launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, x.scalar_type(), wq, codes, beta);
+        Tensor b = bias;
+        if (b.defined() && b.scalar_type() != x.scalar_type()) b = b.to(x.scalar_type());
+        Tensor y = at::linear(x, wq, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
+        ctx->save_for_backward({x, w, theta, beta, codes, wq});
+        ctx->saved_data["range"] = beta_range;
+        ctx->saved_data["min"] = beta_min;
+        ctx->saved_data["bpt"] = bpt;
+        ctx->saved_data["q"] = q;
+        ctx->saved_data["clip"] = clip;
+        if (bias.defined()) ctx->saved_data["bias_type"] = (int64_t)bias.scalar_type();
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x = saved[0], &w = saved[1], &theta = saved[2], &beta = saved[3], &codes = saved[4];
+        c10::cuda::CUDAGuard guard(x.device());
+        const int64_t bpt = ctx->saved_data["bpt"].toInt(), q = ctx->saved_data["q"].toInt();
+        const double clip = ctx->saved_data["clip"].toDouble();
+        const Tensor range = ctx->saved_data["range"].toTensor();
+        Tensor wq = saved[5];
+        // create_graph: the gradient of x has to depend on the weight, so the weight is quantised again under autograd
+        if (at::GradMode::is_enabled())
+            wq = FakeQuant::apply(w, theta, ctx->saved_data["min"].toTensor(), range, bpt, q, clip,
+                                  (int64_t)(x.scalar_type() == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16));
+        const Tensor g2 = grads[0].reshape({-1, w.size(0)}), x2 = x.reshape({-1, w.size(1)});
+        variable_list out(9);
+        if (ctx->needs_input_grad(0)) out[0] = at::mm(g2, wq).view(x.sizes());
+        const bool need_theta = ctx->needs_input_grad(2);
+        if (ctx->needs_input_grad(1) || need_theta) {
+            auto r = FakeQuant::backward_launch(at::mm(g2.t(), x2), w, theta, beta, codes, range, bpt, q, clip, need_theta);
+            out[1] = r.first;
+            out[2] = r.second;
+        }
+        if (ctx->needs_input_grad(3)) {
+            const auto type = (at::ScalarType)ctx->saved_data["bias_type"].toInt();
+            out[3] = at::sum(g2, at::IntArrayRef{0}, false, g2.scalar_type() == type ? std::nullopt : std::optional<at::ScalarType>(type));
+        }
+        return out;
+    }
+};
+
+void check_weight(const Tensor& w) {
+    TORCH_CHECK_TYPE(w.scalar_type() == at::kFloat, "weight must be float32 (the fused weight kernels read float32 rows), got ", w.scalar_type(),
+                     "; keep the layer's parameters in float32 and pass low-precision activations instead");
+}
+
+// layer_fake_quant(weight, theta, beta_min, beta_range, blocks_per_tile, q, clip, out_dtype_code)
+PyObject* layer_fake_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 8);
+    const Tensor& w = tensor_arg(a[0], "weight");
+    check_weight(w);
+    cuda_arg(a[0], "weight");
+    c10::cuda::CUDAGuard guard(w.device());
+    return THPVariable_Wrap(FakeQuant::apply(w, tensor_arg(a[1], "theta"), tensor_arg(a[2], "beta_min"), tensor_arg(a[3], "beta_range"),
+                                             int_arg(a[4]), int_arg(a[5]), float_arg(a[6]), int_arg(a[7])));
+    END_HANDLE_TH_ERRORS
+}
+
+// qat_linear(x, weight, theta, bias or None, beta_min, beta_range, blocks_per_tile, q, clip)
+PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 9);
+    const Tensor &x = tensor_arg(a[0], "x"), &w = tensor_arg(a[1], "weight");
+    check_weight(w);
+    cuda_arg(a[1], "weight");
+    c10::cuda::CUDAGuard guard(w.device());
+    return THPVariable_Wrap(QatLinear::apply(x, w, tensor_arg(a[2], "theta"), optional_arg(a[3], "bias"), tensor_arg(a[4], "beta_min"),
+                                             tensor_arg(a[5], "beta_range"), int_arg(a[6]), int_arg(a[7]), float_arg(a[8])));
+    END_HANDLE_TH_ERRORS
+}
+
+#define COSET_METHOD(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
+PyMethodDef kMethods[] = {
+    COSET_METHOD(encode_packed), COSET_METHOD(decode_packed), COSET_METHOD(encode_digits), COSET_METHOD(decode_digits), COSET_METHOD(quantize),
+    COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(decode_gemm),
+    COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_coset_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__coset_torch(void) { return PyModule_Create(&kModule); }

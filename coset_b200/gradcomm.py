@@ -42,24 +42,15 @@ class CudaCodec:
         self._scales = {}  # (device, scale) -> 1-element tensor: no allocation or host-to-device copy per call
 
     def encode(self, blocks: torch.Tensor, scale: float, out: torch.Tensor) -> torch.Tensor:
-        n = blocks.shape[0]
         key = (blocks.device, float(scale))
         s = self._scales.get(key)
         if s is None:
             s = self._scales[key] = torch.full((1,), float(scale), dtype=torch.float32, device=blocks.device)
-        sem = _lib.SEM_CORE_SATURATE if self.saturate else _lib.SEM_CORE
-        with torch.cuda.device(blocks.device):
-            rc = _lib.lib().coset_e8_encode(_lib.ptr(blocks), _lib.dtype_code(blocks, "grad"), _lib.ptr(s),
-                                            _lib.SCALE_MUL_TILE, n, max(n, 1), 4, 2, sem, _lib.ptr(out),
-                                            _lib.stream())
-        _lib.check(rc, "coset_e8_encode")
+        _lib.native().grad_encode(blocks, s, out, _lib.SEM_CORE_SATURATE if self.saturate else _lib.SEM_CORE)
         return out
 
     def decode_mean(self, codes: torch.Tensor, world: int, n_blocks: int, scale: float, out: torch.Tensor):
-        with torch.cuda.device(codes.device):
-            rc = _lib.lib().coset_e8_decode_mean(_lib.ptr(codes), world, n_blocks, codes.shape[1], float(scale),
-                                                 _lib.ptr(out), _lib.dtype_code(out, "out"), _lib.stream())
-        _lib.check(rc, "coset_e8_decode_mean")
+        _lib.native().decode_mean(codes, world, n_blocks, scale, out)
         return out
 
 

@@ -18,32 +18,17 @@ import torch
 import torch.nn as nn
 
 from . import _lib
-from .core.e8.codecs import e8_decode_packed, e8_encode_packed
+from .core.e8.codecs import _DTYPE_CODES, e8_decode_packed, e8_encode_packed
 
 
 def e8_vlut_matmul(codes: torch.Tensor, beta: Optional[torch.Tensor], blocks_per_tile: int, x: torch.Tensor,
                    bias: Optional[torch.Tensor] = None, clip: float = 0.0, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """y = x @ Wq.T + bias with Wq = decode(codes) / beta (clamped to +-clip when clip > 0);
     codes int32 [n_out, n_in / 8]; x [T, n_in]; y float32, or bf16 rounded once from the float32 sums."""
-    _lib.require_cuda(codes, "codes")
     _lib.require_cuda(x, "x")
-    if codes.dtype != torch.int32 or codes.dim() != 2 or not codes.is_contiguous():
-        raise ValueError("codes must be a contiguous int32 tensor [n_out, n_in / 8]")
-    n_out, kb = codes.shape
-    if x.dim() != 2 or x.shape[1] != kb * 8:
-        raise ValueError(f"x must be [T, {kb * 8}], got {tuple(x.shape)}")
-    x = x.contiguous()
-    T = x.shape[0]
-    y = torch.empty((T, n_out), dtype=out_dtype, device=x.device)
-    b = beta.to(torch.float32).contiguous().view(-1) if beta is not None else None
-    bias32 = bias.to(torch.float32).contiguous() if bias is not None else None
-    with torch.cuda.device(x.device):
-        rc = _lib.lib().coset_e8_vlut_gemv(_lib.ptr(codes), _lib.ptr(b) if b is not None else None, int(blocks_per_tile),
-                                           n_out, kb * 8, _lib.ptr(x), _lib.dtype_code(x, "x"), x.stride(0), T,
-                                           _lib.ptr(bias32) if bias32 is not None else None, _lib.ptr(y),
-                                           _lib.dtype_code(y, "y"), y.stride(0), float(clip), _lib.stream())
-    _lib.check(rc, "coset_e8_vlut_gemv")
-    return y
+    if x.dim() != 2:
+        raise ValueError(f"x must be [T, n_in], got {tuple(x.shape)}")
+    return _lib.native().vlut_linear(x, codes, beta, int(blocks_per_tile), bias, float(clip), _DTYPE_CODES.get(out_dtype, -1))
 
 
 def e8_dequant_gemm(codes: torch.Tensor, beta: Optional[torch.Tensor], blocks_per_tile: int, x: torch.Tensor,
@@ -88,36 +73,12 @@ def e8_decode_gemm(codes: torch.Tensor, beta: Optional[torch.Tensor], blocks_per
     of CTAs (cta_group::2).  Same bits as e8_dequant_gemm and, measured, the same speed up to 8192 tokens, a few
     percent more beyond; nothing dense survives the call.  out_dtype: float32 or bfloat16 (rounded once from the
     float32 accumulator)."""
-    if out_dtype not in (torch.float32, torch.bfloat16):
+    if out_dtype not in _DTYPE_CODES:
         raise TypeError("out_dtype must be float32 or bfloat16")
-    _lib.require_cuda(codes, "codes")
     _lib.require_cuda(x, "x")
-    if x.dtype != torch.bfloat16:
-        raise TypeError("e8_decode_gemm takes bfloat16 activations")
-    if codes.dtype != torch.int32 or codes.dim() != 2 or not codes.is_contiguous():
-        raise ValueError("codes must be a contiguous int32 tensor [n_out, n_in / 8]")
-    n_out, kb = codes.shape
-    if x.dim() != 2 or x.shape[1] != kb * 8 or (kb * 8) % 64:
-        raise ValueError(f"x must be [T, {kb * 8}] with n_in a multiple of 64, got {tuple(x.shape)}")
-    x = x.contiguous()
-    T = x.shape[0]
-    need = n_out * kb * 8
-    if scratch is None:
-        scratch = torch.empty(need, dtype=torch.bfloat16, device=x.device)
-    elif scratch.dtype != torch.bfloat16 or scratch.numel() < need or not scratch.is_contiguous() or scratch.device != x.device:
-        raise ValueError(f"scratch must be a contiguous bfloat16 tensor of at least {need} values on {x.device}")
-    y = torch.empty((T, n_out), dtype=out_dtype, device=x.device)
-    if status is None:
-        status = torch.zeros(1, dtype=torch.int32, device=x.device)
-    b = beta.to(torch.float32).contiguous().view(-1) if beta is not None else None
-    bias32 = bias.to(torch.float32).contiguous() if bias is not None else None
-    with torch.cuda.device(x.device):
-        rc = _lib.lib().coset_e8_decode_gemm(_lib.ptr(codes), _lib.ptr(b) if b is not None else None,
-                                             int(blocks_per_tile), n_out, kb * 8, _lib.ptr(x), x.stride(0), T,
-                                             _lib.ptr(bias32) if bias32 is not None else None, _lib.ptr(y),
-                                             _lib.dtype_code(y, "y"), y.stride(0), float(clip), _lib.ptr(scratch), scratch.numel() * 2,
-                                             _lib.ptr(status), _lib.stream())
-    _lib.check(rc, "coset_e8_decode_gemm")
+    if x.dim() != 2:
+        raise ValueError(f"x must be [T, n_in] with n_in a multiple of 64, got {tuple(x.shape)}")
+    y, status = _lib.native().decode_gemm(x, codes, beta, int(blocks_per_tile), bias, float(clip), scratch, _DTYPE_CODES[out_dtype], status)
     if check and int(status.item()) != 0:
         raise RuntimeError("coset_e8_decode_gemm: a barrier wait expired inside the kernel; the result is invalid")
     return y
@@ -160,6 +121,7 @@ class E8CodeLinear(nn.Module):
         self.blocks_per_tile = int(blocks_per_tile)
         self.weight_clip_value = float(weight_clip_value)
         self._dense, self._dense_key = None, None  # bf16 copy for the library GEMM, rebuilt when codes / scales change
+        self._bias16, self._bias16_key = None, None  # the bias in bf16 beside it
         self._status = None                         # device word the tensor-core kernels set when a bounded wait gave up
 
     def _load_from_state_dict(self, state_dict, prefix, *args, **kwargs):
@@ -212,11 +174,20 @@ class E8CodeLinear(nn.Module):
         return w.view(self.out_features, self.in_features)
 
     def _dense_bf16(self):
-        key = (self.codes._version, self.beta._version, self.codes.data_ptr(), self.beta.data_ptr(), self.codes.device,
-               self.weight_clip_value, self.blocks_per_tile)
+        codes, beta = self._buffers["codes"], self._buffers["beta"]
+        key = (codes._version, beta._version, codes.data_ptr(), beta.data_ptr(), codes.device, self.weight_clip_value, self.blocks_per_tile)
         if self._dense is None or self._dense_key != key:
             self._dense, self._dense_key = self.dense_weight(torch.bfloat16), key
         return self._dense
+
+    def _bias_bf16(self):
+        bias = self._buffers["bias"]
+        if bias is None or bias.dtype == torch.bfloat16:
+            return bias
+        key = (bias._version, bias.data_ptr(), bias.device)
+        if self._bias16 is None or self._bias16_key != key:
+            self._bias16, self._bias16_key = bias.to(torch.bfloat16), key
+        return self._bias16
 
     def check(self):
         """Synchronises and raises if a bounded barrier wait expired inside one of the tensor-core kernels since
@@ -226,30 +197,27 @@ class E8CodeLinear(nn.Module):
             raise RuntimeError("E8CodeLinear: a barrier wait expired inside a tensor-core kernel; results since the last check are invalid")
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
-        clip = self.weight_clip_value
-        if x2.shape[0] <= self.small_t_max:
-            out_dtype = torch.bfloat16 if x.dtype == torch.bfloat16 else torch.float32
-            y = e8_vlut_matmul(self.codes, self.beta, self.blocks_per_tile, x2, self.bias, clip, out_dtype)
-            y = y.to(x.dtype) if x.dtype != out_dtype else y
-        else:
-            if x2.dtype == torch.float32:
-                y = torch.nn.functional.linear(x2, self.dense_weight(torch.float32), self.bias)
-            elif x2.dtype == torch.bfloat16 and self.in_features % 64 == 0 and (
-                    self.large_t_path == "tcgen05" or (self.large_t_path == "auto" and x2.shape[0] >= self.PAIR_GEMM_MIN_T)):
-                if self._status is None or self._status.device != x2.device:
-                    self._status = torch.zeros(1, dtype=torch.int32, device=x2.device)
-                if x2.shape[0] >= 1024:
-                    y = e8_decode_gemm(self.codes, self.beta, self.blocks_per_tile, x2, self.bias, clip=clip, out_dtype=torch.bfloat16,
-                                       status=self._status)
-                else:
-                    y = e8_dequant_gemm(self.codes, self.beta, self.blocks_per_tile, x2, self.bias, clip=clip,
-                                        status=self._status).to(x2.dtype)
-            else:
-                b = self.bias.to(x2.dtype) if self.bias is not None else None
-                y = torch.nn.functional.linear(x2, self._dense_bf16().to(x2.dtype), b)
-        return y.reshape(*lead, self.out_features)
+        # the module's attribute look-up is a Python call per buffer; the dictionaries are read directly
+        buf, n_in, dtype = self._buffers, self.in_features, x.dtype
+        T = x.numel() // n_in
+        if T <= self.small_t_max:
+            return _lib.native().vlut_linear(x, buf["codes"], buf["beta"], self.blocks_per_tile, buf["bias"], self.weight_clip_value,
+                                             _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
+        if dtype is torch.bfloat16:
+            if n_in % 64 == 0 and (self.large_t_path == "tcgen05" or (self.large_t_path == "auto" and T >= self.PAIR_GEMM_MIN_T)):
+                if self._status is None or self._status.device != x.device:
+                    self._status = torch.zeros(1, dtype=torch.int32, device=x.device)
+                if T >= 1024:
+                    return _lib.native().decode_gemm(x, buf["codes"], buf["beta"], self.blocks_per_tile, buf["bias"], self.weight_clip_value,
+                                                     None, _lib.DTYPE_BF16, self._status)[0]
+                y = e8_dequant_gemm(buf["codes"], buf["beta"], self.blocks_per_tile, x.reshape(-1, n_in), buf["bias"],
+                                    clip=self.weight_clip_value, status=self._status).to(dtype)
+                return y.reshape(*x.shape[:-1], self.out_features)
+            return torch.nn.functional.linear(x, self._dense_bf16(), self._bias_bf16())
+        if dtype is torch.float32:
+            return torch.nn.functional.linear(x, self.dense_weight(torch.float32), buf["bias"])
+        b = buf["bias"].to(dtype) if buf["bias"] is not None else None
+        return torch.nn.functional.linear(x, self._dense_bf16().to(dtype), b)
 
 
 def out_feature_shard(n_out: int, world: int, rank: int):

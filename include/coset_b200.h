@@ -126,6 +126,17 @@ int coset_e8_pack_codes_f32(const float* digits, int64_t n_blocks, int q, int M,
                             void* stream);
 
 /*
+ * The reference's own calling convention in one launch each (coset/core/e8/codecs.py:17-89 and :139-218):
+ * digits are float32 [n_blocks, M, 8], beta is one scalar passed by value.
+ *   encode: digits of x / beta;   decode: x_hat * beta (digits are rounded and reduced modulo q first)
+ * x, digits and out are 16-byte aligned.
+ */
+int coset_e8_encode_digits_f32(const float* x, float beta, int64_t n_blocks, int q, int M, float* digits,
+                               void* stream);
+int coset_e8_decode_digits_f32(const float* digits, float beta, int64_t n_blocks, int q, int M, float* out,
+                               void* stream);
+
+/*
  * Backward of the fake-quantised weight path of HNLQLinearQAT (straight-through estimator,
  * coset/core/layers.py:62-95, with torch autograd's rules for the surrounding
  * mul / div / clamp of coset/core/layers.py:429-463).  M is 2 (e8_quantize hard-wires it).

@@ -336,3 +336,18 @@ def test_encode_on_concurrent_streams_and_growing_sizes(e8):
     torch.cuda.synchronize()
     for (rep, i), c in got.items():
         assert torch.equal(c, want[i]), (rep, i, int((c != want[i]).sum()))
+
+
+@pytest.mark.parametrize("q,M", [(4, 2), (4, 3), (3, 2), (16, 1)])
+@pytest.mark.parametrize("n,beta", [(1, 1.0), (33, 0.7), (1000, 1.3)])
+def test_digits_in_one_launch(e8, cfgcls, q, M, n, beta):
+    """e8_encode / e8_decode on digit tensors against the oracle: ragged sizes, values beyond the code's range, digits
+    that are not reduced modulo q yet."""
+    rng = np.random.default_rng(n + q)
+    x = (rng.standard_normal((n, 8)) * 2.0).astype(np.float32)
+    want = O.encode(x, beta=np.float32([beta]), scale_mode=1, q=q, M=M)
+    got, T = e8.e8_encode(dev(x), cfg(cfgcls, q, M, beta))
+    assert T == 0 and np.array_equal(got.cpu().numpy(), want)
+    shifted = got + q * torch.randint(-2, 3, got.shape, device="cuda")
+    want_xh = O.decode(want, beta=np.float32([beta]), scale_mode=1, q=q)
+    assert np.array_equal(bits(e8.e8_decode(shifted, cfg(cfgcls, q, M, beta)).cpu().numpy()), bits(want_xh))

@@ -229,3 +229,25 @@ def test_graphed_train_step_keeps_the_statistics_schedule():
     assert torch.equal(la, lb)
     assert torch.equal(a.weight.grad, b.weight.grad)
     assert torch.allclose(a.theta_beta.grad, b.theta_beta.grad, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("tiling", ["row", "block"])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 1e-2)])
+def test_one_node_equals_the_composed_path(tiling, dtype, tol):
+    """The layer's single autograd node against the composed path (which diagnostics force: quantised weights as one
+    node, then F.linear), forward, backward and the gradient of a gradient (create_graph)."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    torch.manual_seed(3)
+    grads = []
+    for diagnostics in (False, True):
+        layer = create_e8_hnlq_linear(72, 40, device="cuda", tiling=tiling, init_method="zeros", enable_diagnostics=diagnostics)
+        torch.manual_seed(4)
+        layer.load_weights(torch.randn(40, 72) * 20.0, torch.randn(40))
+        x = torch.randn(3, 11, 72, device="cuda").to(dtype).requires_grad_()
+        y = layer(x)
+        gx, = torch.autograd.grad((y.float() ** 2).sum(), x, create_graph=True)
+        (y.float().sum() + (gx.float() ** 2).sum()).backward()
+        grads.append((y.detach(), gx.detach(), x.grad, layer.weight.grad, layer.theta_beta.grad, layer.bias.grad))
+    for one, composed in zip(*grads):
+        assert one.shape == composed.shape and one.dtype == composed.dtype
+        assert rel(one.float().cpu().numpy(), composed.float().cpu().numpy()) < tol
