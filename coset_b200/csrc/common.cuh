@@ -26,6 +26,10 @@ const uint2* residual_table_q4(cudaStream_t stream);
 // bound by instruction issue keep the 8-byte entries, which unpack with 12 fewer instructions.
 const uint32_t* residual_table_q4_packed(cudaStream_t stream);
 
+// The same residuals in 2 bytes per level word (layout at e8::compact_residues), 128 KB: for the kernels that keep
+// the whole table in shared memory.
+const uint16_t* residual_table_q4_compact(cudaStream_t stream);
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 }  // namespace coset

@@ -598,7 +598,7 @@ k_decode_q4m2(const uint32_t* __restrict__ codes, const float* __restrict__ scal
 
 // Residual table of the q=4 decoder, produced by the literal float32 decoder itself:
 // entry[w] = 2 * (G b - 4 Q(G b / 4)) + 7 for the 16-bit level word w, as 8 unsigned bytes.
-__global__ void k_build_table_q4(uint2* __restrict__ table, uint32_t* __restrict__ packed, int* __restrict__ bad) {
+__global__ void k_build_table_q4(uint2* __restrict__ table, uint32_t* __restrict__ packed, uint16_t* __restrict__ compact, int* __restrict__ bad) {
     int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= 65536) return;
     int d[8];
@@ -625,8 +625,21 @@ __global__ void k_build_table_q4(uint2* __restrict__ table, uint32_t* __restrict
         ok = ok && ((t[i] & 1) == p) && nib >= 0 && nib <= (i < 7 ? 15 : 7);
         e |= ((uint32_t)nib & 0xfu) << (4 * i);
     }
-    if (!ok) atomicAdd(bad, 1);
     packed[w] = e;
+    // compact entry (layout at e8::compact_residues)
+    const uint32_t res = e8::compact_residues((uint32_t)w);
+    uint32_t fields = 0;
+    bool marked = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int diff = t[i] + (i < 7 ? e8::kCompactBias : e8::kCompactBias7) - (int)((res >> (2 * i)) & 3u);
+        const int m = diff >> 2;
+        ok = ok && (diff & 3) == 0 && m >= 0 && m <= (i < 7 ? 4 : 2);
+        marked = marked || m == 4;
+        fields |= (uint32_t)(m & 3) << (2 * i);
+    }
+    compact[w] = (uint16_t)(marked ? fields | 0xc000u : fields);
+    if (!ok) atomicAdd(bad, 1);
 }
 
 // ---------------------------------------------------------------- digit views
@@ -747,22 +760,23 @@ const uint2* residual_table_q4(cudaStream_t stream) {
     if (dev < 0 || dev >= 64) { fail(COSET_E_STATE, "device index %d out of range", dev); return nullptr; }
     std::lock_guard<std::mutex> lock(mu);
     if (!tables[dev]) {
-        uint2* t = nullptr;  // 65536 x 8 B, then 65536 x 4 B packed, then the builder's self-check word
-        if (check_cuda(cudaMalloc(&t, 65536 * (sizeof(uint2) + sizeof(uint32_t)) + 16), "cudaMalloc(residual table)")) return nullptr;
+        uint2* t = nullptr;  // 65536 x 8 B, then 65536 x 4 B packed, 65536 x 2 B compact, the builder's self-check word
+        if (check_cuda(cudaMalloc(&t, 65536 * (sizeof(uint2) + sizeof(uint32_t) + sizeof(uint16_t)) + 16), "cudaMalloc(residual table)")) return nullptr;
         uint32_t* packed = reinterpret_cast<uint32_t*>(t + 65536);
-        int* bad = reinterpret_cast<int*>(packed + 65536);
+        uint16_t* compact = reinterpret_cast<uint16_t*>(packed + 65536);
+        int* bad = reinterpret_cast<int*>(compact + 65536);
         int bad_host = -1;
         // Built on the caller's stream: every later use on any stream must see it complete, so
         // the one-time build synchronises that stream.
         bool failed = check_cuda(cudaMemsetAsync(bad, 0, sizeof(int), stream), "table build") != 0;
         if (!failed) {
-            k_build_table_q4<<<65536 / 256, 256, 0, stream>>>(t, packed, bad);
+            k_build_table_q4<<<65536 / 256, 256, 0, stream>>>(t, packed, compact, bad);
             failed = check_launch("k_build_table_q4") ||
                      check_cuda(cudaMemcpyAsync(&bad_host, bad, sizeof(int), cudaMemcpyDeviceToHost, stream), "table build") ||
                      check_cuda(cudaStreamSynchronize(stream), "table build");
         }
         if (!failed && bad_host != 0) {
-            fail(COSET_E_STATE, "residual table: %d entries do not fit the packed layout", bad_host);
+            fail(COSET_E_STATE, "residual table: %d entries do not fit the packed layouts", bad_host);
             failed = true;
         }
         if (failed) {
@@ -777,6 +791,11 @@ const uint2* residual_table_q4(cudaStream_t stream) {
 const uint32_t* residual_table_q4_packed(cudaStream_t stream) {
     const uint2* t = residual_table_q4(stream);
     return t ? reinterpret_cast<const uint32_t*>(t + 65536) : nullptr;
+}
+
+const uint16_t* residual_table_q4_compact(cudaStream_t stream) {
+    const uint32_t* p = residual_table_q4_packed(stream);
+    return p ? reinterpret_cast<const uint16_t*>(p + 65536) : nullptr;
 }
 
 }  // namespace coset

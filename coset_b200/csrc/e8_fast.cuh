@@ -366,4 +366,26 @@ __device__ __forceinline__ void decode_q4m2(uint32_t code, const uint2* __restri
     scale_twice<0>(v2, 1.0f, xh);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Compact form of the same table: 2 bytes per level word, 128 KB, small enough for the shared memory of one CTA
+// (a random gather from there costs the bank conflicts of 32 addresses, ~4 cycles per warp; from the 512 KB table
+// through L1 and L2 ~27 were measured).
+//
+// Twice the residual is only unknown by a multiple of 4: with r(b) = G b - 4 Q and 2 Q integer, t_i = 2 r_i(b) equals
+// 2 (G b)_i modulo 4, and G is almost bidiagonal, so that residue follows from two digits and the last one.  The
+// biased value T_i = t_i + 7 (T_7 = t_7 + 5) is therefore 4 m_i + s_i with
+//     s_i = (c_i 2 + b_7 - 1) mod 4 (s_7: + 2),  c_i = low bit of b_i xor b_{i+1} (c_0 = b_1, c_6 = b_6, c_7 = 0)
+// and m_i in 0..4, m_7 in 0..2.  The entry holds the eight m_i in 2-bit fields; the 146 entries in which some m_i is 4
+// are marked by m_7 = 3 and have to be looked up in the 8-byte table (the encoder hardly ever produces their words).
+constexpr int kCompactBias = 7, kCompactBias7 = 5;
+
+// The 2-bit fields s_i of two level words at once, one per half of w.
+__device__ __forceinline__ uint32_t compact_residues(uint32_t w) {
+    const uint32_t c = (w & 0x15541554u) ^ ((w >> 2) & 0x05550555u);
+    const uint32_t b7 = (((w >> 14) & 0x00030003u) + 0x00030003u) & 0x00030003u;
+    return (b7 * 0x5555u) ^ ((c << 1) ^ 0x80008000u);
+}
+// Non-zero where an entry (in either half) is marked.
+__device__ __forceinline__ uint32_t compact_marked(uint32_t e) { return e & (e << 1) & 0x80008000u; }
+
 }  // namespace e8

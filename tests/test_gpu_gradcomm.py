@@ -270,3 +270,27 @@ def test_two_gpu_peer_memory_transport_equals_all_gather(tmp_path):
     res = subprocess.run(cmd, env=env, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stderr[-2000:]
     assert "PEER_OK" in res.stdout
+
+
+@pytest.mark.parametrize("world", [1, 2, 3, 8, 16, 17])
+@pytest.mark.parametrize("n", [1000, 2 * 148 * 1024 + 77])  # below and above the shared-memory table's threshold
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_decode_mean_equals_the_sum_of_decoded_streams(world, n, dtype):
+    """Both kernels behind coset_e8_decode_mean against decode, exact sum, one division: codes of an encoder, with words
+    that need the full table, non-zero top-level words and the all-zero word sprinkled in; a stride beyond n."""
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    from coset_b200.gradcomm import CudaCodec
+    g = torch.Generator(device="cuda").manual_seed(world)
+    codes = torch.full((world, n + 5), -1, dtype=torch.int32, device="cuda")
+    for r in range(world):
+        codes[r, :n] = e8_encode_packed(torch.randn(n, 8, device="cuda", generator=g) * 0.5).view(torch.int32).view(-1)
+        hit = torch.randint(0, 300, (n,), device="cuda", generator=g)
+        any_word = torch.randint(0, 1 << 32, (n,), device="cuda", generator=g)  # uniform words: 0.2 % are marked entries
+        word = torch.where(hit == 0, any_word, any_word & 0xffff)
+        codes[r, :n] = torch.where(hit < 20, (word - ((word >> 31) << 32)).to(torch.int32), codes[r, :n])
+        codes[r, :n] = torch.where(hit == 20, torch.zeros_like(codes[r, :n]), codes[r, :n])
+    out = torch.empty((n, 8), dtype=dtype, device="cuda")
+    CudaCodec().decode_mean(codes, world, n, 3.7, out)
+    total = sum(e8_decode_packed(codes[r, :n].contiguous()) for r in range(world))  # half-integers: exact in float32
+    divisor = torch.tensor(np.float32(np.float32(3.7) * np.float32(world)), device="cuda")
+    assert torch.equal(out, (total / divisor).to(dtype))
