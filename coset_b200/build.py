@@ -27,6 +27,7 @@ SOURCES = [
     "e8_host.cu",
     "e8_gradcomm.cu",
     "e8_vlut.cu",
+    "e8_vlut_bytes.cu",
     "e8_stats.cu",
     "e8_ref.cu",
     "e8_dequant_gemm.cu",

@@ -1,0 +1,492 @@
+// Few-token product of a layer that keeps its weight in a decode-ready layout: y[T, N] = x[T, K] * Wq^T (+ bias).
+//
+// The code-domain kernels of e8_vlut.cu rebuild every weight block from two table gathers and a few dozen integer
+// instructions per call (10-20 us for one token and a 4096 x 4096 weight).  Twice the reconstruction is an integer in
+// [-35, 55], so a layer can hold t + 64 as one byte per weight instead, laid out once in the order in which the tensor
+// cores want it.  The product then has no gather: a PRMT puts two bytes under the exponent 0x43 (bf16 128 + byte), one
+// bf16x2 subtraction leaves t exactly, and mma.sync multiplies it UNSCALED with the activations; the scale is applied to
+// the float32 inner products -- once per row when a scale covers whole rows, once per block otherwise (m16n8k8 then
+// spans exactly one block).  Every product is exact, nothing is rounded to bf16 but the result.
+//   * float32 activations are the exact sum of three bf16 terms and take three products;
+//   * a clamp that can bind (|t| > clip 2 beta for some possible t) is a second product of the clamped signs, so the
+//     clamped weights are exact too.
+// Bound: 1 byte per weight (+ 4 per 8 weights of per-block scales), 2.6-3.9 us of HBM traffic for 4096 x 4096.  Measured
+// there (graph replay, before -> now), one scale per row with a clamp: 14.4 -> 5.5 us for one token, 22.4 -> 9.5 for 16;
+// one per block: 9.9 -> 6.9, 22.8 -> 10.3; float32 tokens with a scale per row: 15.2 -> 9.7, 118 -> 20.6.  8192 x 8192, one
+// token, scale per row: 48 -> 16 us (4.2 TB/s).  What is left at 16 tokens is latency: two warps' worth of shared-memory
+// round trips per unit at 16 warps per SM (staging the activations once per CTA, deeper cp.async rings with the weights in
+// them and two-stage rings at higher occupancy were measured within 10 % of this form, and slower for few tokens).
+// A warp owns 16 rows and every KW-th unit of K; KW depends on K alone, so a row's sum does
+// not depend on how many rows the matrix has (a row-sharded layer returns the same bits), and the partial sums are added
+// in a fixed order through shared memory.
+//
+// Layout: [groups of 16 rows][units of 8 blocks][2][32 lanes] of 16 bytes; a lane's 32 bytes are eight words, word b =
+// coordinates 2c, 2c + 1 of block b of the unit for row g | the same for row g + 8, with g = lane / 4, c = lane % 4: the A
+// fragment of one m16n8k8 step, and two neighbouring words that of one m16n8k16 step.
+#include <cuda_bf16.h>
+
+#include "common.cuh"
+#include "e8_fast.cuh"
+#include "e8_io.cuh"
+
+using namespace coset;
+
+namespace {
+
+constexpr int kMaxTargets = 16;
+struct Targets {  // where a result row goes: one buffer, or the result buffer of every rank (peer memory, plain stores)
+    void* y[kMaxTargets];
+    int n;
+    int bf16;
+};
+__device__ __forceinline__ void store_result(const Targets& out, int64_t idx, float r) {
+    for (int k = 0; k < out.n; ++k) {
+        if (out.bf16) reinterpret_cast<__nv_bfloat16*>(out.y[k])[idx] = __float2bfloat16_rn(r);
+        else reinterpret_cast<float*>(out.y[k])[idx] = r;
+    }
+}
+
+constexpr float kMaxTwice = 55.0f;  // largest |2 x_hat| of any code
+constexpr int kByteBias = 64;
+
+// d = a b (FRESH) or d += a b
+template <bool FRESH>
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    if (FRESH)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool FRESH>
+__device__ __forceinline__ void mma_1688(float (&d)[4], const uint32_t (&a)[2], uint32_t b0) {
+    if (FRESH)
+        asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0), "f"(0.0f));
+    else
+        asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(b0));
+}
+
+// Bytes 0, 1 (HIGH: 2, 3) of a word as two exact bf16 integers byte - 64.
+template <bool HIGH>
+__device__ __forceinline__ uint32_t twice_pair(uint32_t w) {
+    uint32_t r;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(__byte_perm(w, 0x43434343u, HIGH ? 0x4342 : 0x4140)), "r"(0x43404340u));
+    return r;
+}
+// The clamp in units of t: lanes with |t| > k become 0 in `t` and +-1 in the result.
+__device__ __forceinline__ uint32_t clamp_signs(uint32_t& t, uint32_t k2) {
+    const uint32_t a = t & 0x7fff7fffu;
+    const uint32_t over = __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&k2));
+    const uint32_t sign = ((t & 0x80008000u) | 0x3f803f80u) & over;
+    t &= ~over;
+    return sign;
+}
+// floor(clip / |scale|) in both halves (64 where nothing can exceed it)
+__device__ __forceinline__ uint32_t clamp_limit(float clip, float scale) {
+    const __nv_bfloat162 h = __float2bfloat162_rn(fminf(floorf(__fdividef(clip, fabsf(scale))), 64.0f));
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float reciprocal(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+// The exact three-term bf16 split of two floats, packed: out[p] = (p-th term of a, p-th term of b).
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&out)[3]) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+        out[p] = __byte_perm(ua, ub, 0x7632);  // truncation keeps 8 significand bits, the rest is exact
+        const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
+        a = p > 0 || ra == ra ? ra : 0.0f;  // an infinity stays in the first term
+        b = p > 0 || rb == rb ? rb : 0.0f;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// codes -> layout, once per weight.  One warp per (group, unit).
+__device__ __forceinline__ uint2 code_bytes_of(const uint2* table, uint32_t code) {
+    const uint2 t0 = __ldg(table + (code & 0xffffu)), t1 = __ldg(table + (code >> 16));
+    const uint32_t shift = (kByteBias - 5 * e8::kTableBias) * 0x01010101u;  // 2 x_hat + 35 -> + 64, at most 119
+    return make_uint2(t0.x + 4u * t1.x + shift, t0.y + 4u * t1.y + shift);
+}
+
+__global__ void __launch_bounds__(256)
+k_vlut_layout(const uint32_t* __restrict__ codes, int n_out, int kb, int units, int64_t tiles, const uint2* __restrict__ table, uint4* __restrict__ out) {
+    const int64_t tile = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (tile >= tiles) return;
+    const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+    const int64_t group = tile / units;
+    const int unit = (int)(tile - group * units);
+    uint2 b[2][2];  // [row g, g + 8][block 2c, 2c + 1]
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int64_t row = group * 16 + g + 8 * h;
+            const int blk = unit * 8 + 2 * c + q;
+            const uint32_t code = row < n_out && blk < kb ? __ldg(codes + row * kb + blk) : 0u;
+            b[h][q] = code_bytes_of(table, code);
+        }
+    uint32_t w[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int src = (lane & ~3) + (k >> 1);
+        const uint32_t gx = __shfl_sync(0xffffffffu, b[0][k & 1].x, src), gy = __shfl_sync(0xffffffffu, b[0][k & 1].y, src);
+        const uint32_t hx = __shfl_sync(0xffffffffu, b[1][k & 1].x, src), hy = __shfl_sync(0xffffffffu, b[1][k & 1].y, src);
+        w[k] = __byte_perm(c < 2 ? gx : gy, c < 2 ? hx : hy, c & 1 ? 0x7632 : 0x5410);
+    }
+    out[tile * 64 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+    out[tile * 64 + 32 + lane] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// ---------------------------------------------------------------------------------------------
+struct Product {
+    const uint4* w;
+    const float* beta;
+    int rows_per_scale;   // rows kernel: rows that share a scale
+    e8::TileDiv td;       // blocks kernel: block index -> scale
+    int n_out, kb, units, T;
+    const void* x;
+    int64_t ldx, ldy;
+    const float* bias;
+    float clip;
+    int kw_log2;
+    Targets out;
+};
+
+// Adds the KW partial tiles of every row group of this CTA in a fixed order and stores the results.
+template <int NT, int WARPS>
+__device__ __forceinline__ void reduce_and_store(const float (*part)[16][8 * NT + 1], const Product& a, int t0) {
+    const int rw = WARPS >> a.kw_log2, kw = 1 << a.kw_log2;
+    __syncthreads();
+    for (int e = threadIdx.x; e < rw * 16 * 8 * NT; e += WARPS * 32) {
+        const int r = e & 15, t = (e >> 4) & (8 * NT - 1), group = (e >> 4) / (8 * NT);  // consecutive threads: consecutive rows of one token
+        const int row = (blockIdx.x * rw + group) * 16 + r;
+        if (row < a.n_out && t0 + t < a.T) {
+            float v = part[group << a.kw_log2][r][t];
+            for (int w = 1; w < kw; ++w) v += part[(group << a.kw_log2) + w][r][t];
+            store_result(a.out, (int64_t)(t0 + t) * a.ldy + row, v + (a.bias ? __ldg(a.bias + row) : 0.0f));
+        }
+    }
+}
+
+// How a weight is scaled: once per row; once per block with the scales of a row in order (rows of whole units, read as
+// vectors); once per block through the tile index.
+constexpr int kPerRow = 0, kPerBlock = 1, kPerTile = 2;
+
+// Shared memory of one warp: activations of a unit as bf16 [buffer][plane][token][8 blocks of 16 bytes], the block index
+// exclusive-ored with the token so that the eight rows of an ldmatrix fall into different banks, and the scales of a unit
+// [4 blocks][16 rows][4].
+template <int NT, int P, int SCALE>
+struct WarpSmem {
+    static constexpr int kBuffers = P == 1 ? 2 : 1, kPlane = 8 * NT * 128;
+    uint8_t x[kBuffers * P * kPlane];
+    float scale[SCALE == kPerRow ? 4 : 128];
+};
+
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// Four 8 x 8 b16 matrices; lane l gives the address of row l % 8 of matrix l / 8.
+__device__ __forceinline__ void load_matrices(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+template <int NT, int P, bool CLIP, int SCALE, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+k_product(const __grid_constant__ Product a) {
+    typedef WarpSmem<NT, P, SCALE> Smem;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+    Smem& mem = reinterpret_cast<Smem*>(smem)[warp];
+    float(*part)[16][8 * NT + 1] = reinterpret_cast<float(*)[16][8 * NT + 1]>(smem + WARPS * sizeof(Smem));
+    const int kw = 1 << a.kw_log2, rw = WARPS >> a.kw_log2, first = warp & (kw - 1), t0 = blockIdx.y * (8 * NT);
+    const int group = blockIdx.x * rw + (warp >> a.kw_log2);
+    const int tokens = a.T - t0 < 8 * NT ? a.T - t0 : 8 * NT;
+    float acc[NT][4], sign_acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][i] = sign_acc[n][i] = 0.0f;
+    float row_scale[2] = {0.5f, 0.5f};
+    if (group * 16 < a.n_out) {
+        const uint4* wp = a.w + ((int64_t)group * a.units + first) * 64 + lane;
+        uint4 next[2];
+        if (first < a.units) { next[0] = __ldcs(wp); next[1] = __ldcs(wp + 32); }
+
+        // Activations of unit u.  bf16: asynchronous 16-byte copies, eight lanes per token; float32: through registers (8
+        // floats per lane and step), split into three planes.  Tokens beyond T are not written (their columns of the result
+        // are not stored), blocks beyond K are zero.
+        constexpr int STEPS = 2 * NT;  // four tokens per step
+        float4 held[STEPS][2];  // unused for bf16
+        const uint32_t x_base = (uint32_t)__cvta_generic_to_shared(mem.x);
+        const int st = lane >> 3, sb = lane & 7;  // token of the step, block of the unit
+        const uint8_t* xp = reinterpret_cast<const uint8_t*>(a.x) + ((int64_t)(t0 + st) * a.ldx + (int64_t)first * 64 + sb * 8) * (P == 1 ? 2 : 4);
+        auto request = [&](int u, int buffer) {  // xp points at unit u
+#pragma unroll
+            for (int i = 0; i < STEPS; ++i) {
+                const int t = 4 * i + st;
+                const uint8_t* src = xp + (int64_t)(4 * i) * a.ldx * (P == 1 ? 2 : 4);
+                if constexpr (P == 1) {
+                    const uint32_t off = (uint32_t)(buffer * Smem::kPlane + t * 128 + ((sb ^ (t & 7)) << 4));
+                    if (t < tokens) {
+                        if (u * 8 + sb < a.kb) copy16_async(x_base + off, src);
+                        else *reinterpret_cast<uint4*>(mem.x + off) = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                } else {
+                    held[i][0] = held[i][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (t < tokens && u * 8 + sb < a.kb) {
+                        held[i][0] = __ldg(reinterpret_cast<const float4*>(src));
+                        held[i][1] = __ldg(reinterpret_cast<const float4*>(src) + 1);
+                    }
+                }
+            }
+            if (P == 1) asm volatile("cp.async.commit_group;" ::: "memory");
+            xp += (int64_t)(64 * (P == 1 ? 2 : 4)) << a.kw_log2;
+        };
+        // The scales of unit u: lane l holds four blocks of row l / 2.
+        float4 next_scale = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        const int srow = group * 16 + (lane >> 1) < a.n_out ? group * 16 + (lane >> 1) : a.n_out - 1;
+        int64_t sat = (int64_t)srow * a.kb + (int64_t)first * 8 + 4 * (lane & 1);
+        auto request_scales = [&](int u) {
+            if (SCALE == kPerBlock) {
+                next_scale = __ldcs(reinterpret_cast<const float4*>(a.beta + sat));
+            } else if (SCALE == kPerTile) {
+                float v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = u * 8 + 4 * (lane & 1) + k < a.kb ? __ldg(a.beta + e8::tile_of(a.td, sat + k)) : 1.0f;
+                next_scale = make_float4(v[0], v[1], v[2], v[3]);
+            }
+            sat += 8 * kw;
+        };
+
+        if (first < a.units) {
+            request(first, 0);
+            if (SCALE != kPerRow) request_scales(first);
+        }
+        if (SCALE == kPerRow && a.beta) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = group * 16 + g + 8 * h;
+                row_scale[h] = 0.5f * reciprocal(__ldg(a.beta + (row < a.n_out ? row : a.n_out - 1) / a.rows_per_scale));
+            }
+        }
+        bool bind = CLIP && SCALE == kPerRow && __any_sync(0xffffffffu, kMaxTwice * fmaxf(fabsf(row_scale[0]), fabsf(row_scale[1])) > a.clip);
+        int buffer = 0;
+        for (int u = first; u < a.units; u += kw) {
+            const uint32_t w[8] = {next[0].x, next[0].y, next[0].z, next[0].w, next[1].x, next[1].y, next[1].z, next[1].w};
+            const bool more = u + kw < a.units;
+            wp += 64 * kw;
+            if (more) { next[0] = __ldcs(wp); next[1] = __ldcs(wp + 32); }
+            if constexpr (P == 3) {
+#pragma unroll
+                for (int i = 0; i < STEPS; ++i) {
+                    const int t = 4 * i + st;
+                    const float4 lo = held[i][0], hi = held[i][1];
+                    uint32_t q[4][3];
+                    split3(lo.x, lo.y, q[0]); split3(lo.z, lo.w, q[1]); split3(hi.x, hi.y, q[2]); split3(hi.z, hi.w, q[3]);
+                    if (t < tokens) {
+#pragma unroll
+                        for (int p = 0; p < P; ++p)
+                            *reinterpret_cast<uint4*>(mem.x + p * Smem::kPlane + t * 128 + ((sb ^ (t & 7)) << 4)) = make_uint4(q[0][p], q[1][p], q[2][p], q[3][p]);
+                    }
+                }
+            }
+            if (SCALE != kPerRow) {
+                const float4 r = make_float4(reciprocal(2.0f * next_scale.x), reciprocal(2.0f * next_scale.y), reciprocal(2.0f * next_scale.z), reciprocal(2.0f * next_scale.w));
+                *reinterpret_cast<float4*>(mem.scale + (lane & 1) * 64 + (lane >> 1) * 4) = r;
+                if (CLIP) bind = __any_sync(0xffffffffu, kMaxTwice * fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w))) > a.clip);
+                if (more) request_scales(u + kw);
+            }
+            if (more) request(u + kw, buffer ^ 1);
+            if (P == 1) {
+                if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncwarp();
+            float d[NT][4], ds[NT][4];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {  // blocks 4 half .. + 3
+                float scale[2][4];
+                if (SCALE != kPerRow) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float4 v = *reinterpret_cast<const float4*>(mem.scale + half * 64 + (g + 8 * h) * 4);
+                        scale[h][0] = v.x; scale[h][1] = v.y; scale[h][2] = v.z; scale[h][3] = v.w;
+                    }
+                }
+                uint32_t b[NT][P][4];  // coordinates 2c, 2c + 1 of the four blocks, token 8 n + g
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int p = 0; p < P; ++p)
+                        load_matrices(x_base + (uint32_t)((P == 1 ? buffer : p) * Smem::kPlane + (8 * n + (lane & 7)) * 128 + (((4 * half + (lane >> 3)) ^ (lane & 7)) << 4)), b[n][p]);
+#pragma unroll
+                for (int k = 0; k < 4; k += 2) {
+                    const int b0 = 4 * half + k;
+                    uint32_t t[4] = {twice_pair<false>(w[b0]), twice_pair<true>(w[b0]), twice_pair<false>(w[b0 + 1]), twice_pair<true>(w[b0 + 1])};
+                    uint32_t sign[4];
+                    if (CLIP && bind) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            sign[i] = clamp_signs(t[i], clamp_limit(a.clip, SCALE == kPerRow ? row_scale[i & 1] : scale[i & 1][k + (i >> 1)]));
+                    }
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        if (SCALE == kPerRow) {
+#pragma unroll
+                            for (int p = 0; p < P; ++p) {
+                                if (b0 == 0 && p == 0) mma_16816<true>(d[n], t, b[n][p][k], b[n][p][k + 1]);
+                                else mma_16816<false>(d[n], t, b[n][p][k], b[n][p][k + 1]);
+                                if (CLIP && bind) {
+                                    if (b0 == 0 && p == 0) mma_16816<true>(ds[n], sign, b[n][p][k], b[n][p][k + 1]);
+                                    else mma_16816<false>(ds[n], sign, b[n][p][k], b[n][p][k + 1]);
+                                }
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 2; ++q) {
+                                const uint32_t tq[2] = {t[2 * q], t[2 * q + 1]};
+                                mma_1688<true>(d[n], tq, b[n][0][k + q]);
+#pragma unroll
+                                for (int p = 1; p < P; ++p) mma_1688<false>(d[n], tq, b[n][p][k + q]);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) acc[n][i] = __fmaf_rn(d[n][i], scale[i >> 1][k + q], acc[n][i]);
+                                if (CLIP && bind) {
+                                    const uint32_t sq[2] = {sign[2 * q], sign[2 * q + 1]};
+                                    mma_1688<true>(ds[n], sq, b[n][0][k + q]);
+#pragma unroll
+                                    for (int p = 1; p < P; ++p) mma_1688<false>(ds[n], sq, b[n][p][k + q]);
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) acc[n][i] = __fmaf_rn(ds[n][i], copysignf(a.clip, scale[i >> 1][k + q]), acc[n][i]);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            if (SCALE == kPerRow) {
+                // float32 additions between units: at most four chained tensor-core accumulations per term
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        acc[n][i] += d[n][i];
+                        if (CLIP && bind) sign_acc[n][i] += ds[n][i];
+                    }
+            }
+            __syncwarp();  // the next unit overwrites what this one read
+            buffer ^= 1;
+        }
+    }
+    // accumulator layout: [0], [1] = (row g, tokens 2c, 2c + 1); [2], [3] = (row g + 8, same tokens)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v = acc[n][i];
+            if (SCALE == kPerRow) {
+                v *= row_scale[i >> 1];
+                if (CLIP) v = __fmaf_rn(sign_acc[n][i], copysignf(a.clip, row_scale[i >> 1]), v);
+            }
+            part[warp][g + 8 * (i >> 1)][8 * n + 2 * c + (i & 1)] = v;
+        }
+    reduce_and_store<NT, WARPS>(part, a, t0);
+}
+
+// Whether one scale covers whole rows.
+bool scale_per_row(const float* beta, int64_t blocks_per_tile, int kb) { return !beta || kb == 0 || blocks_per_tile % kb == 0; }
+
+template <int NT, int P, bool CLIP, int SCALE, int WARPS>
+int launch_as(const Product& a, cudaStream_t st) {
+    const int groups = (a.n_out + 15) / 16, rw = WARPS >> a.kw_log2;
+    const dim3 grid((groups + rw - 1) / rw, (a.T + 8 * NT - 1) / (8 * NT));
+    if (grid.y > 65535) return fail(COSET_E_UNSUPPORTED, "T too large for the few-token product");
+    constexpr int smem = WARPS * (int)(sizeof(WarpSmem<NT, P, SCALE>) + 16 * (8 * NT + 1) * sizeof(float));
+    if (smem > 48 * 1024)
+        if (int e = check_cuda(cudaFuncSetAttribute(k_product<NT, P, CLIP, SCALE, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
+    k_product<NT, P, CLIP, SCALE, WARPS><<<grid, WARPS * 32, smem, st>>>(a);
+    return check_launch("e8_vlut_product");
+}
+
+template <int NT, int P, bool CLIP>
+int launch_product(Product a, int scale, cudaStream_t st) {
+    // Warps per row group, from K alone: a warp should have at least two units (its next loads overlap the arithmetic),
+    // and up to 16 warps share a row group of a long K (8 where a thread needs more registers).
+    constexpr int most = NT == 1 && P == 1 ? 4 : 3;
+    while (a.kw_log2 < most && (4 << a.kw_log2) <= a.units) ++a.kw_log2;
+#define PRODUCT_AS(SCALE)                                                                          \
+    if constexpr (most == 4)                                                                       \
+        if (a.kw_log2 == 4) return launch_as<NT, P, CLIP, SCALE, 16>(a, st);                       \
+    return launch_as<NT, P, CLIP, SCALE, 8>(a, st)
+    if (scale == kPerRow) { PRODUCT_AS(kPerRow); }
+    if (scale == kPerBlock) { PRODUCT_AS(kPerBlock); }
+    PRODUCT_AS(kPerTile);
+#undef PRODUCT_AS
+}
+
+template <int P>
+int launch_tokens(const Product& a, int scale, cudaStream_t st) {
+    if (a.T > 8) return a.clip > 0.0f ? launch_product<2, P, true>(a, scale, st) : launch_product<2, P, false>(a, scale, st);
+    return a.clip > 0.0f ? launch_product<1, P, true>(a, scale, st) : launch_product<1, P, false>(a, scale, st);
+}
+
+}  // namespace
+
+extern "C" int64_t coset_e8_vlut_layout_bytes(int n_out, int n_in) {
+    if (n_out < 0 || n_in < 0) return 0;
+    return (((int64_t)n_out + 15) / 16) * (((int64_t)n_in + 63) / 64) * 1024;
+}
+
+extern "C" int coset_e8_vlut_layout(const void* codes, int n_out, int n_in, void* layout, void* stream) {
+    if (n_out < 0 || n_in < 0 || (n_in % 8) != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
+    if (n_out == 0 || n_in == 0) return 0;
+    if (!codes || !layout) return fail(COSET_E_BADARG, "null pointer");
+    if (!aligned(codes, 4) || !aligned(layout, 16)) return fail(COSET_E_ALIGN, "codes must be 4-byte and the layout 16-byte aligned");
+    cudaStream_t st = (cudaStream_t)stream;
+    const uint2* table = residual_table_q4(st);
+    if (!table) return COSET_E_STATE;
+    const int kb = n_in / 8, units = (kb + 7) / 8;
+    const int64_t tiles = (((int64_t)n_out + 15) / 16) * units;
+    const unsigned grid = (unsigned)((tiles + 7) / 8);
+    k_vlut_layout<<<grid, 256, 0, st>>>((const uint32_t*)codes, n_out, kb, units, tiles, table, (uint4*)layout);
+    return check_launch("e8_vlut_layout");
+}
+
+extern "C" int coset_e8_vlut_product(const void* layout, const float* beta, int64_t blocks_per_tile, int n_out, int n_in, const void* x, int x_dtype,
+                                     int64_t ldx, int T, const float* bias, void* const* y_targets, int n_targets, int y_dtype, int64_t ldy,
+                                     float clip, void* stream) {
+    if (n_out < 0 || n_in < 0 || T < 0 || (n_in % 8) != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
+    if (n_targets < 1 || n_targets > kMaxTargets || !y_targets) return fail(COSET_E_BADARG, "need 1..16 result buffers");
+    if (n_out == 0 || T == 0) return 0;
+    if (!layout || !x) return fail(COSET_E_BADARG, "null pointer");
+    if ((x_dtype != COSET_DTYPE_F32 && x_dtype != COSET_DTYPE_BF16) || (y_dtype != COSET_DTYPE_F32 && y_dtype != COSET_DTYPE_BF16))
+        return fail(COSET_E_BADARG, "unknown dtype");
+    if (ldx < n_in || ldy < n_out) return fail(COSET_E_BADARG, "leading dimension too small");
+    if (!aligned(x, 16) || ((ldx * (x_dtype == COSET_DTYPE_F32 ? 4 : 2)) % 16) != 0 || !aligned(layout, 16))
+        return fail(COSET_E_ALIGN, "the layout and the rows of x must be 16-byte aligned");
+    if (beta && blocks_per_tile < 1) return fail(COSET_E_BADARG, "blocks_per_tile must be >= 1");
+    if (!(clip == clip)) return fail(COSET_E_BADARG, "clip is not a number");
+    const int kb = n_in / 8;
+    Product a = {};
+    a.w = (const uint4*)layout;
+    a.beta = beta;
+    a.n_out = n_out; a.kb = kb; a.units = (kb + 7) / 8; a.T = T;
+    a.x = x; a.ldx = ldx; a.ldy = ldy; a.bias = bias; a.clip = clip > 0.0f ? clip : 0.0f;
+    for (int k = 0; k < n_targets; ++k) {
+        if (!y_targets[k]) return fail(COSET_E_BADARG, "result buffer %d is null", k);
+        a.out.y[k] = y_targets[k];
+    }
+    a.out.n = n_targets;
+    a.out.bf16 = y_dtype == COSET_DTYPE_BF16 ? 1 : 0;
+    const bool rows = scale_per_row(beta, blocks_per_tile, kb), one = blocks_per_tile == 1 && (kb % 8) == 0 && aligned(beta, 16);
+    a.rows_per_scale = rows && beta && kb > 0 ? (int)(blocks_per_tile / kb) : 1;
+    if (!rows) a.td = e8::make_tile_div(blocks_per_tile, (int64_t)n_out * kb);
+    cudaStream_t st = (cudaStream_t)stream;
+    const int scale_kind = rows ? kPerRow : (one ? kPerBlock : kPerTile);
+    return x_dtype == COSET_DTYPE_BF16 ? launch_tokens<1>(a, scale_kind, st) : launch_tokens<3>(a, scale_kind, st);
+}

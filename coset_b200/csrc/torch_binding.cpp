@@ -270,6 +270,43 @@ PyObject* vlut_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// vlut_layout(codes) -> the decode-ready copy of the weight
+PyObject* vlut_layout(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 1);
+    const Tensor& codes = cuda_arg(a[0], "codes");
+    check_codes(codes);
+    const int n_out = (int)codes.size(0), n_in = (int)codes.size(1) * 8;
+    c10::cuda::CUDAGuard guard(codes.device());
+    Tensor layout = empty({coset_e8_vlut_layout_bytes(n_out, n_in)}, at::kByte, codes);
+    check_rc(coset_e8_vlut_layout(data(codes), n_out, n_in, data(layout), stream_of(codes)), "coset_e8_vlut_layout");
+    return THPVariable_Wrap(layout);
+    END_HANDLE_TH_ERRORS
+}
+
+// vlut_product(x [..., n_in], layout, n_out, n_in, beta or None, blocks_per_tile, bias or None, clip, out_dtype_code)
+PyObject* vlut_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 9);
+    const Tensor &x = cuda_arg(a[0], "x"), &layout = tensor_arg(a[1], "layout");
+    const int64_t n_out = int_arg(a[2]), n_in = int_arg(a[3]);
+    TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in, "x must be [T, ", n_in, "], got ", x.sizes());
+    TORCH_CHECK_VALUE(layout.device() == x.device(), "the weight is on ", layout.device(), ", x on ", x.device());
+    c10::cuda::CUDAGuard guard(x.device());
+    c10::SmallVector<int64_t, 6> shape;
+    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
+    const Tensor beta = as_f32(optional_arg(a[4], "beta")), bias = as_f32(optional_arg(a[6], "bias"));
+    const int y_code = (int)int_arg(a[8]);
+    Tensor y = empty(shape, scalar_type(y_code), x);
+    void* target = data(y);
+    if (target)
+        check_rc(coset_e8_vlut_product(data(layout), fdata(beta), int_arg(a[5]), (int)n_out, (int)n_in, data(x2), dtype_code(x2, "x"), n_in,
+                                       (int)x2.size(0), fdata(bias), &target, 1, y_code, n_out, (float)float_arg(a[7]), stream_of(x)),
+                 "coset_e8_vlut_product");
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
 // decode_gemm(x [..., n_in] bf16, codes, beta or None, blocks_per_tile, bias or None, clip, scratch or None, out_dtype_code, status or None)
 // -> (y, status)
 PyObject* decode_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -440,7 +477,7 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define COSET_METHOD(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     COSET_METHOD(encode_packed), COSET_METHOD(decode_packed), COSET_METHOD(encode_digits), COSET_METHOD(decode_digits), COSET_METHOD(quantize),
-    COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(decode_gemm),
+    COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(vlut_layout), COSET_METHOD(vlut_product), COSET_METHOD(decode_gemm),
     COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_coset_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

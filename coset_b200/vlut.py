@@ -3,8 +3,9 @@
 The weight of a trained HNLQLinearQAT layer is exported as packed q=4, M=2 codes (4 bytes per 8
 weights) plus the scales beta, and applied from the codes:
 
-  * few tokens  (T <= small_t_max): the code-domain kernels of coset_e8_vlut_gemv, which read the code
-    stream (8.4 - 16.8 MB for a 4096 x 4096 weight instead of 64 MB of float32);
+  * few tokens  (T <= small_t_max): by default a decode-ready copy of the codes, one byte per weight in tensor-core order
+    (coset_e8_vlut_layout, kept like the dense copy below), and coset_e8_vlut_product; `large_t_path="tcgen05"` keeps no
+    copy of any kind and reads the code stream (coset_e8_vlut_gemv);
   * many tokens (from 2048 by default): the weight is decoded into a transient bf16 buffer and multiplied by
     this library's tcgen05 GEMM (coset_e8_decode_gemm); nothing dense survives the call;
   * in between, by default, the library GEMM on a cached dense bf16 copy (`large_t_path` chooses).
@@ -94,6 +95,8 @@ class E8CodeLinear(nn.Module):
     cta_group::2 GEMM from 1024 tokens, the single-launch fused kernel below; "cublas" -- a cached dense bf16 copy
     and the library GEMM; "auto" (default) -- the own kernels from PAIR_GEMM_MIN_T tokens, the library path for
     the tokens in between, where decoding the whole weight per call costs more than the product itself.
+    Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 5.5-10 us for 1-16
+    tokens and a 4096 x 4096 weight; "tcgen05" keeps nothing and stays on the code-domain kernels (9.7-23 us).
     small_t_max defaults to 16 ("auto", "cublas") or 48 ("tcgen05"): measured on a 4096 x 4096 layer the
     code-domain kernels take 9.7 / 23 / 44 / 86 us for 1 / 16 / 32 / 64 tokens (they re-read and re-decode the
     codes for every 16 tokens), the library on the cached copy 7-13 us, the fused kernel 64 us.
@@ -122,6 +125,7 @@ class E8CodeLinear(nn.Module):
         self.weight_clip_value = float(weight_clip_value)
         self._dense, self._dense_key = None, None  # bf16 copy for the library GEMM, rebuilt when codes / scales change
         self._bias16, self._bias16_key = None, None  # the bias in bf16 beside it
+        self._layout, self._layout_key = None, None  # decode-ready bytes for few tokens, rebuilt likewise
         self._status = None                         # device word the tensor-core kernels set when a bounded wait gave up
 
     def _load_from_state_dict(self, state_dict, prefix, *args, **kwargs):
@@ -129,6 +133,7 @@ class E8CodeLinear(nn.Module):
         self.blocks_per_tile = int(self.blocks_per_tile_t.item())
         self.weight_clip_value = float(self.weight_clip_value_t.item())
         self._dense, self._dense_key = None, None
+        self._layout, self._layout_key = None, None
 
     @classmethod
     def from_weight(cls, weight: torch.Tensor, beta: torch.Tensor, blocks_per_tile: int, bias=None, **kw):
@@ -173,6 +178,15 @@ class E8CodeLinear(nn.Module):
             w = w.clamp_(-self.weight_clip_value, self.weight_clip_value).to(dtype)
         return w.view(self.out_features, self.in_features)
 
+    def _product_layout(self):
+        """The weight as bytes in tensor-core order (coset_e8_vlut_layout): 1 byte per weight, built on the first few-token
+        call and when the codes change."""
+        codes = self._buffers["codes"]
+        key = (codes._version, codes.data_ptr())
+        if self._layout_key != key:
+            self._layout, self._layout_key = _lib.native().vlut_layout(codes), key
+        return self._layout
+
     def _dense_bf16(self):
         codes, beta = self._buffers["codes"], self._buffers["beta"]
         key = (codes._version, beta._version, codes.data_ptr(), beta.data_ptr(), codes.device, self.weight_clip_value, self.blocks_per_tile)
@@ -201,6 +215,9 @@ class E8CodeLinear(nn.Module):
         buf, n_in, dtype = self._buffers, self.in_features, x.dtype
         T = x.numel() // n_in
         if T <= self.small_t_max:
+            if self.large_t_path != "tcgen05" and n_in:
+                return _lib.native().vlut_product(x, self._product_layout(), self.out_features, n_in, buf["beta"], self.blocks_per_tile, buf["bias"],
+                                                  self.weight_clip_value, _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
             return _lib.native().vlut_linear(x, buf["codes"], buf["beta"], self.blocks_per_tile, buf["bias"], self.weight_clip_value,
                                              _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
         if dtype is torch.bfloat16:
@@ -304,12 +321,18 @@ class ColumnParallelE8CodeLinear(nn.Module):
         x2 = x2.contiguous()
         bias32 = loc.bias.to(torch.float32).contiguous() if loc.bias is not None else None
         with torch.cuda.device(x2.device):
-            rc = _lib.lib().coset_e8_vlut_gemv_scatter(
-                _lib.ptr(loc.codes), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
-                _lib.ptr(x2), _lib.dtype_code(x2, "x"), x2.stride(0), T, _lib.ptr(bias32) if bias32 is not None else None,
-                ctypes.cast(targets, ctypes.c_void_p), self.world, self.out_features, float(loc.weight_clip_value),
-                _lib.stream())
-        _lib.check(rc, "coset_e8_vlut_gemv_scatter")
+            bias = _lib.ptr(bias32) if bias32 is not None else None
+            if loc.large_t_path != "tcgen05":  # the kernel of the unsharded layer, so that the results are the same bits
+                rc = _lib.lib().coset_e8_vlut_product(
+                    _lib.ptr(loc._product_layout()), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
+                    _lib.ptr(x2), _lib.dtype_code(x2, "x"), x2.stride(0), T, bias, ctypes.cast(targets, ctypes.c_void_p), self.world,
+                    _lib.DTYPE_F32, self.out_features, float(loc.weight_clip_value), _lib.stream())
+            else:
+                rc = _lib.lib().coset_e8_vlut_gemv_scatter(
+                    _lib.ptr(loc.codes), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
+                    _lib.ptr(x2), _lib.dtype_code(x2, "x"), x2.stride(0), T, bias, ctypes.cast(targets, ctypes.c_void_p), self.world,
+                    self.out_features, float(loc.weight_clip_value), _lib.stream())
+        _lib.check(rc, "few-token product into every rank's buffer")
         region.arrive()  # bounded: all ranks have written their columns into this rank's buffer
         # the half is written again two calls from now, after the arrival of the call in between
         mine = region.data(torch.float32)[parity * half_elems: parity * half_elems + T * self.out_features]

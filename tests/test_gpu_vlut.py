@@ -261,3 +261,41 @@ def test_two_gpu_column_parallel_equals_unsharded(tmp_path):
     res = subprocess.run(cmd, env=env, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stderr[-2000:]
     assert "SHARD_OK" in res.stdout
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bpt_of", [lambda kb: kb, lambda kb: 1, lambda kb: 3, lambda kb: 2 * kb], ids=["row", "block", "three_blocks", "two_rows"])
+@pytest.mark.parametrize("n_out,n_in", [(1, 8), (17, 72), (200, 1032), (16, 4096), (1200, 2048)])
+@pytest.mark.parametrize("T,clip", [(1, 0.0), (8, 0.05), (9, 4.0), (17, 0.0)])
+def test_few_token_product_edges(n_out, n_in, bpt_of, T, clip, dtype):
+    """The layer's few-token product: ragged rows, K that is no multiple of a unit, scale tiles that straddle rows, both
+    token tiles and the remainder, a clamp that binds on some weights and one that cannot, any code word and non-zero top
+    levels.  The weights are exact in the kernel and the sums are float32, for bf16 activations too, so 1e-5 holds for both."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    from coset_b200.vlut import E8CodeLinear
+    g = torch.Generator(device="cuda").manual_seed(n_out + T)
+    kb = n_in // 8
+    bpt = bpt_of(kb)
+    n = n_out * kb
+    beta = 25.0 * (0.75 + 0.5 * torch.rand((n + bpt - 1) // bpt, device="cuda", generator=g))
+    codes = e8_encode_packed(torch.randn(n, 8, device="cuda", generator=g) * 0.6).view(torch.int32).view(-1)
+    word = torch.randint(0, 1 << 32, (n,), device="cuda", generator=g)
+    hit = torch.randint(0, 100, (n,), device="cuda", generator=g)
+    word = torch.where(hit == 0, word, word & 0xffff)
+    codes = torch.where(hit < 20, (word - ((word >> 31) << 32)).to(torch.int32), codes)
+    w = e8_decode_packed(codes, scale=beta, scale_mode=_lib.SCALE_MUL_TILE, blocks_per_tile=bpt).view(n_out, n_in)
+    w = w.clamp(-clip, clip) if clip else w
+    bias = torch.randn(n_out, device="cuda", generator=g)
+    x = torch.randn(T, n_in, device="cuda", generator=g).to(dtype)
+    want = (x.double() @ w.double().T + bias.double()).cpu().numpy()
+    lin = E8CodeLinear(codes.view(n_out, kb), beta, bpt, bias, small_t_max=64, weight_clip_value=clip)
+    product = lambda l, code: _lib.native().vlut_product(x, l._product_layout(), l.out_features, n_in, l.beta, bpt, l.bias, clip, code)
+    got = product(lin, _lib.DTYPE_F32)
+    assert rel(got.cpu().numpy(), want) < 1e-5
+    assert torch.equal(product(lin, _lib.DTYPE_BF16), got.to(torch.bfloat16))
+    assert torch.equal(lin(x), got.to(dtype))
+    if bpt <= kb and n_out > 1 and bpt != 3:  # a shard of the rows returns the same bits
+        half = n_out // 2
+        part = E8CodeLinear(lin.codes[:half], beta[:half * (kb // bpt)], bpt, bias[:half], small_t_max=64, weight_clip_value=clip)
+        assert torch.equal(product(part, _lib.DTYPE_F32), got[:, :half])
