@@ -13,6 +13,7 @@ from typing import Any, Dict, List, Optional, Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from .. import _lib
 
@@ -382,12 +383,13 @@ class HNLQLinearQAT(nn.Module):
 
     def _one_node(self, x, low):
         """Whether the whole product can run as one native autograd node: the plain case of a quantised E8 layer
-        on the GPU.  Warm-up, diagnostics (which look at the quantised weights), autocast, parametrised weights and
-        a quantize_fn of the caller's own take the composed path."""
+        on the GPU.  Warm-up, diagnostics (which look at the quantised weights), autocast, forward-mode derivatives (the
+        node has none), parametrised weights and a quantize_fn of the caller's own take the composed path."""
         state = self.__dict__
         params = state["_parameters"]
         return (state["_fused"] and state["quantization_enabled"] and not state["enable_diagnostics"] and x.is_cuda
                 and (low or x.dtype == torch.float32) and not torch.is_autocast_enabled("cuda")
+                and forward_ad._current_level < 0
                 and "weight" in params and ("theta_beta" in params or not state["theta_trainable"]) and params["weight"].is_cuda)
 
     def forward(self, x):

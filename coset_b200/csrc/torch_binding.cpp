@@ -59,7 +59,10 @@ int dtype_code(const Tensor& t, const char* name) {
     TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, name, " must be float32 or bfloat16, got ", t.scalar_type());
     return COSET_DTYPE_BF16;
 }
-at::ScalarType scalar_type(int code) { return code == COSET_DTYPE_F32 ? at::kFloat : at::kBFloat16; }
+at::ScalarType scalar_type(int code) {
+    TORCH_CHECK_TYPE(code == COSET_DTYPE_F32 || code == COSET_DTYPE_BF16, "the result's dtype must be float32 or bfloat16");
+    return code == COSET_DTYPE_F32 ? at::kFloat : at::kBFloat16;
+}
 
 Tensor empty(at::IntArrayRef size, at::ScalarType type, const Tensor& like) {
     return at::detail::empty_cuda(size, type, like.device(), std::nullopt);
@@ -96,7 +99,13 @@ Scale scale_arg(PyObject* o, int64_t mode, int64_t n_blocks, int64_t bpt, const 
     Scale s;
     if (o == Py_None || mode == COSET_SCALE_NONE) return s;
     if (THPVariable_Check(o)) s.t = as_f32(cuda_arg(o, "scale"));
-    else s.t = at::full({1}, float_arg(o), x.options().dtype(at::kFloat));  // filled on the device: no copy from the host
+    else {  // filled on the device: no copy from the host
+        PyObject* number = PyNumber_Float(o);  // what float(scale) takes
+        if (!number) throw python_error();
+        const double value = PyFloat_AS_DOUBLE(number);
+        Py_DECREF(number);
+        s.t = at::full({1}, value, x.options().dtype(at::kFloat));
+    }
     if (mode == COSET_SCALE_DIV_SCALAR) {
         TORCH_CHECK_VALUE(s.t.numel() == 1, "the codec (divide) convention takes one scalar beta");
     } else {
@@ -296,11 +305,11 @@ PyObject* vlut_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
     c10::SmallVector<int64_t, 6> shape;
     const Tensor x2 = token_rows(x, n_in, n_out, &shape);
     const Tensor beta = as_f32(optional_arg(a[4], "beta")), bias = as_f32(optional_arg(a[6], "bias"));
-    const int y_code = (int)int_arg(a[8]);
+    const int y_code = (int)int_arg(a[8]), x_code = dtype_code(x2, "x");
     Tensor y = empty(shape, scalar_type(y_code), x);
     void* target = data(y);
     if (target)
-        check_rc(coset_e8_vlut_product(data(layout), fdata(beta), int_arg(a[5]), (int)n_out, (int)n_in, data(x2), dtype_code(x2, "x"), n_in,
+        check_rc(coset_e8_vlut_product(data(layout), fdata(beta), int_arg(a[5]), (int)n_out, (int)n_in, data(x2), x_code, n_in,
                                        (int)x2.size(0), fdata(bias), &target, 1, y_code, n_out, (float)float_arg(a[7]), stream_of(x)),
                  "coset_e8_vlut_product");
     return THPVariable_Wrap(y);
@@ -403,7 +412,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         Tensor wq, codes, beta;
         FakeQuant::launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, x.scalar_type(), wq, codes, beta);
         Tensor b = bias;
-        if (b.defined() && b.scalar_type() != x.scalar_type()) b = b.to(x.scalar_type());
+        if (b.defined() && x.scalar_type() == at::kBFloat16) b = b.to(at::kBFloat16);
         Tensor y = at::linear(x, wq, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
         ctx->save_for_backward({x, w, theta, beta, codes, wq});
         ctx->saved_data["range"] = beta_range;

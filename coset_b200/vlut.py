@@ -13,6 +13,7 @@ weights) plus the scales beta, and applied from the codes:
 The math is the reference's one-sided vLUT inner product (coset/legacy/quant/vlut.py:72-117) in
 the layer's scale convention W_q = decode(codes) / beta (coset/core/layers.py:453-460).
 """
+import operator
 from typing import Optional
 
 import torch
@@ -123,17 +124,21 @@ class E8CodeLinear(nn.Module):
         self.register_buffer("weight_clip_value_t", torch.tensor(float(weight_clip_value), dtype=torch.float32))
         self.blocks_per_tile = int(blocks_per_tile)
         self.weight_clip_value = float(weight_clip_value)
-        self._dense, self._dense_key = None, None  # bf16 copy for the library GEMM, rebuilt when codes / scales change
-        self._bias16, self._bias16_key = None, None  # the bias in bf16 beside it
-        self._layout, self._layout_key = None, None  # decode-ready bytes for few tokens, rebuilt likewise
-        self._status = None                         # device word the tensor-core kernels set when a bounded wait gave up
+        self._kept = {}      # copies of the weight in other forms, see _keep
+        self._status = None  # device word the tensor-core kernels set when a bounded wait gave up
 
     def _load_from_state_dict(self, state_dict, prefix, *args, **kwargs):
         super()._load_from_state_dict(state_dict, prefix, *args, **kwargs)
         self.blocks_per_tile = int(self.blocks_per_tile_t.item())
         self.weight_clip_value = float(self.weight_clip_value_t.item())
-        self._dense, self._dense_key = None, None
-        self._layout, self._layout_key = None, None
+        self._kept = {}
+
+    def __getstate__(self):  # a copied or pickled layer makes its own copies of the weight again
+        return {**self.__dict__, "_kept": {}}
+
+    def __setstate__(self, state):
+        super().__setstate__({k: v for k, v in state.items() if k not in ("_dense", "_dense_key")})
+        self.__dict__.setdefault("_kept", {})
 
     @classmethod
     def from_weight(cls, weight: torch.Tensor, beta: torch.Tensor, blocks_per_tile: int, bias=None, **kw):
@@ -178,30 +183,49 @@ class E8CodeLinear(nn.Module):
             w = w.clamp_(-self.weight_clip_value, self.weight_clip_value).to(dtype)
         return w.view(self.out_features, self.in_features)
 
+    def _keep(self, name, sources, settings, make):
+        """`make()`, kept until one of the buffers it was made from is written or replaced (the entry holds the buffers, so
+        their identity cannot be taken over by another tensor).  It is complete on the device before it is published, for a
+        later call may come from another stream or thread, and none of these may still read the one it replaces.  Inside a
+        graph capture it is recorded with the call and not kept: nothing is computed before the replay."""
+        entry = self._kept.get(name)
+        if any(t.is_inference() for t in sources):  # no version counter: a write would go unseen
+            return make()
+        versions = [(t._version, t.data_ptr()) for t in sources]
+        if entry is not None and entry[1] == versions and entry[2] == settings and all(map(operator.is_, entry[3], sources)):
+            return entry[0]
+        value = make()
+        if not torch.cuda.is_current_stream_capturing():
+            if entry is not None:
+                torch.cuda.synchronize(value.device)
+            else:
+                torch.cuda.current_stream(value.device).synchronize()
+            self._kept[name] = (value, versions, settings, sources)
+        return value
+
+    @property
+    def _dense(self):
+        return self._kept["dense"][0] if "dense" in self._kept else None
+
     def _product_layout(self):
-        """The weight as bytes in tensor-core order (coset_e8_vlut_layout): 1 byte per weight, built on the first few-token
-        call and when the codes change."""
+        """The weight as bytes in tensor-core order (coset_e8_vlut_layout), 1 byte per weight; None where the call has to
+        read the codes themselves: under capture, for a graph is replayed on whatever the codes then hold, and for codes
+        without a version counter."""
         codes = self._buffers["codes"]
-        key = (codes._version, codes.data_ptr())
-        if self._layout_key != key:
-            self._layout, self._layout_key = _lib.native().vlut_layout(codes), key
-        return self._layout
+        if torch.cuda.is_current_stream_capturing() or codes.is_inference():
+            return None
+        return self._keep("layout", (codes,), None, lambda: _lib.native().vlut_layout(codes))
 
     def _dense_bf16(self):
-        codes, beta = self._buffers["codes"], self._buffers["beta"]
-        key = (codes._version, beta._version, codes.data_ptr(), beta.data_ptr(), codes.device, self.weight_clip_value, self.blocks_per_tile)
-        if self._dense is None or self._dense_key != key:
-            self._dense, self._dense_key = self.dense_weight(torch.bfloat16), key
-        return self._dense
+        buf = self._buffers
+        return self._keep("dense", (buf["codes"], buf["beta"]), (self.weight_clip_value, self.blocks_per_tile),
+                          lambda: self.dense_weight(torch.bfloat16))
 
     def _bias_bf16(self):
         bias = self._buffers["bias"]
         if bias is None or bias.dtype == torch.bfloat16:
             return bias
-        key = (bias._version, bias.data_ptr(), bias.device)
-        if self._bias16 is None or self._bias16_key != key:
-            self._bias16, self._bias16_key = bias.to(torch.bfloat16), key
-        return self._bias16
+        return self._keep("bias", (bias,), None, lambda: bias.to(torch.bfloat16))
 
     def check(self):
         """Synchronises and raises if a bounded barrier wait expired inside one of the tensor-core kernels since
@@ -215,8 +239,9 @@ class E8CodeLinear(nn.Module):
         buf, n_in, dtype = self._buffers, self.in_features, x.dtype
         T = x.numel() // n_in
         if T <= self.small_t_max:
-            if self.large_t_path != "tcgen05" and n_in:
-                return _lib.native().vlut_product(x, self._product_layout(), self.out_features, n_in, buf["beta"], self.blocks_per_tile, buf["bias"],
+            layout = self._product_layout() if self.large_t_path != "tcgen05" and n_in else None
+            if layout is not None:
+                return _lib.native().vlut_product(x, layout, self.out_features, n_in, buf["beta"], self.blocks_per_tile, buf["bias"],
                                                   self.weight_clip_value, _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
             return _lib.native().vlut_linear(x, buf["codes"], buf["beta"], self.blocks_per_tile, buf["bias"], self.weight_clip_value,
                                              _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
@@ -322,9 +347,10 @@ class ColumnParallelE8CodeLinear(nn.Module):
         bias32 = loc.bias.to(torch.float32).contiguous() if loc.bias is not None else None
         with torch.cuda.device(x2.device):
             bias = _lib.ptr(bias32) if bias32 is not None else None
-            if loc.large_t_path != "tcgen05":  # the kernel of the unsharded layer, so that the results are the same bits
+            layout = loc._product_layout() if loc.large_t_path != "tcgen05" and loc.in_features else None
+            if layout is not None:  # the kernel of the unsharded layer, so that the results are the same bits
                 rc = _lib.lib().coset_e8_vlut_product(
-                    _lib.ptr(loc._product_layout()), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
+                    _lib.ptr(layout), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
                     _lib.ptr(x2), _lib.dtype_code(x2, "x"), x2.stride(0), T, bias, ctypes.cast(targets, ctypes.c_void_p), self.world,
                     _lib.DTYPE_F32, self.out_features, float(loc.weight_clip_value), _lib.stream())
             else:

@@ -351,3 +351,16 @@ def test_digits_in_one_launch(e8, cfgcls, q, M, n, beta):
     shifted = got + q * torch.randint(-2, 3, got.shape, device="cuda")
     want_xh = O.decode(want, beta=np.float32([beta]), scale_mode=1, q=q)
     assert np.array_equal(bits(e8.e8_decode(shifted, cfg(cfgcls, q, M, beta)).cpu().numpy()), bits(want_xh))
+
+
+def test_unknown_result_type_is_refused_and_scales_are_numbers():
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    codes = e8_encode_packed(torch.randn(16, 8, device="cuda"))
+    with pytest.raises(TypeError):
+        e8_decode_packed(codes, dtype=torch.float16)
+    want = e8_decode_packed(codes, scale=2.0, scale_mode=_lib.SCALE_DIV_SCALAR)
+    for two in (2, "2.0", torch.tensor(2.0, device="cuda")):
+        assert torch.equal(e8_decode_packed(codes, scale=two, scale_mode=_lib.SCALE_DIV_SCALAR), want)
+    with pytest.raises(ValueError):
+        e8_decode_packed(codes, scale="two", scale_mode=_lib.SCALE_DIV_SCALAR)

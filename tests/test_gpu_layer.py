@@ -251,3 +251,25 @@ def test_one_node_equals_the_composed_path(tiling, dtype, tol):
     for one, composed in zip(*grads):
         assert one.shape == composed.shape and one.dtype == composed.dtype
         assert rel(one.float().cpu().numpy(), composed.float().cpu().numpy()) < tol
+
+
+def test_forward_mode_derivative_in_the_input():
+    """The product is linear in x: the tangent is t W_q^T."""
+    import torch.autograd.forward_ad as fa
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 32, device="cuda")
+    layer.load_weights(torch.randn(32, 64, device="cuda") * 20.0, torch.randn(32, device="cuda"))
+    x, t = torch.randn(8, 64, device="cuda"), torch.randn(8, 64, device="cuda")
+    with fa.dual_level():
+        y, tangent = fa.unpack_dual(layer(fa.make_dual(x, t)))
+    torch.testing.assert_close(y.detach(), layer(x).detach(), rtol=1e-5, atol=1e-4)
+    torch.testing.assert_close(tangent.detach(), (layer(t) - layer.bias).detach(), rtol=1e-5, atol=1e-3)
+
+
+def test_bias_of_another_type_is_refused_for_float32():
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 32, device="cuda")
+    layer.bias.data = layer.bias.data.to(torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        layer(torch.randn(8, 64, device="cuda"))
+    assert layer(torch.randn(8, 64, device="cuda").to(torch.bfloat16)).dtype == torch.bfloat16

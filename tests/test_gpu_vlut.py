@@ -299,3 +299,78 @@ def test_few_token_product_edges(n_out, n_in, bpt_of, T, clip, dtype):
         half = n_out // 2
         part = E8CodeLinear(lin.codes[:half], beta[:half * (kb // bpt)], bpt, bias[:half], small_t_max=64, weight_clip_value=clip)
         assert torch.equal(product(part, _lib.DTYPE_F32), got[:, :half])
+
+
+def _kept_copy_layer(n_out=64, n_in=256, seed=5, **kw):
+    from coset_b200.vlut import E8CodeLinear
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randn(n_out, n_in, device="cuda", generator=g) * 0.05
+    return E8CodeLinear.from_weight(w, torch.full((n_out,), 25.0, device="cuda"), n_in // 8, **kw), torch.randn(3, n_in, device="cuda", generator=g)
+
+
+def test_few_tokens_under_capture_read_the_codes_of_the_replay():
+    """A graph captured before any eager call keeps nothing that only its replay would compute, and its replay follows
+    codes that were written after the capture."""
+    lin, x = _kept_copy_layer()
+    other, _ = _kept_copy_layer(seed=6)
+    want = x.double() @ lin.dense_weight().double().T
+    want_other = x.double() @ other.dense_weight().double().T
+    other(x)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        y = lin(x)
+    torch.cuda.synchronize()
+    assert rel(lin(x).cpu().numpy(), want.cpu().numpy()) < 1e-5
+    graph.replay()
+    assert rel(y.cpu().numpy(), want.cpu().numpy()) < 1e-5
+    lin.codes.copy_(other.codes)
+    graph.replay()
+    assert rel(y.cpu().numpy(), want_other.cpu().numpy()) < 1e-5
+    assert rel(lin(x).cpu().numpy(), want_other.cpu().numpy()) < 1e-5
+
+
+def test_kept_copies_follow_the_buffers():
+    """In-place writes, replaced buffers, copies of the layer and buffers without a version counter."""
+    import copy
+    import pickle
+    a, x = _kept_copy_layer()
+    b, _ = _kept_copy_layer(seed=6)
+    ya, yb = a(x), b(x)
+    assert not torch.equal(ya, yb)
+    for twin in (copy.deepcopy(a), pickle.loads(pickle.dumps(a))):
+        assert torch.equal(twin(x), ya)
+        twin.codes.copy_(b.codes)
+        assert torch.equal(twin(x), yb)
+    old = copy.deepcopy(a)
+    del old.__dict__["_kept"]  # a module pickled before it kept copies this way
+    assert torch.equal(pickle.loads(pickle.dumps(old))(x), ya)
+    a.codes = b.codes.clone()
+    assert torch.equal(a(x), yb)
+    with torch.inference_mode():
+        c, _ = _kept_copy_layer()
+        yc = c(x)
+        assert rel(yc.cpu().numpy(), ya.cpu().numpy()) < 1e-5
+        c.codes.copy_(b.codes)
+        assert rel(c(x).cpu().numpy(), yb.cpu().numpy()) < 1e-5
+
+
+def test_kept_copy_is_complete_for_every_stream():
+    """The first call lays the weight out on its own stream; a call on another stream right after reads it complete."""
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for seed in range(8):
+        lin, x = _kept_copy_layer(2048, 2048, seed)
+        torch.cuda.synchronize()
+        ys = []
+        for s in streams:
+            with torch.cuda.stream(s):
+                ys.append(lin(x))
+        torch.cuda.synchronize()
+        assert torch.equal(ys[0], ys[1])
+
+
+def test_few_tokens_refuse_other_types_at_any_count():
+    lin, x = _kept_copy_layer()
+    for T in (0, 3):
+        with pytest.raises(TypeError):
+            lin(x[:T].half())
