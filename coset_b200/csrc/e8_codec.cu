@@ -8,7 +8,6 @@
 #include <stdarg.h>
 
 #include <mutex>
-#include <vector>
 
 #include "common.cuh"
 #include "e8_fast.cuh"
@@ -368,53 +367,45 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
 }
 
 // ---------------------------------------------------------------- encode-only production path
-// The codes-only encoder is two launches.  Measured on this part, ANY state carried across the loop of
-// the persistent kernel above (a queue length, a vote per iteration, a second loop) costs 10-25 % of
-// its time through register pressure at the 64-register budget, so the main kernel carries none: a
-// lane whose block the cheapest tier cannot prove stores a marker code (top level word non-zero, which
-// that tier never produces) and appends the block index to a list in scratch memory with one atomic
-// in a rare branch.  The fix-up kernel then finishes the listed blocks densely with the always-valid
-// tiers.  When more blocks are deferred than the list holds (an overloaded quantiser) the fix-up kernel
-// instead sweeps all codes for the marker and compacts the marked blocks warp by warp.
+// The codes-only encoder.  Any state carried across the loop in registers (a queue length, a vote per iteration, a second
+// loop) costs 10-25 % of its time through register pressure at the 64-register budget, so the loop carries none: a lane
+// whose block the cheapest tier cannot prove puts the block's index on a list of its CTA in shared memory, in a rare
+// branch, and after its loop the CTA finishes the listed blocks with all lanes busy, while other CTAs of the SM are still
+// in their loops.  A CTA with more such blocks than its list holds (an overloaded quantiser) stores a marker code instead
+// (top level word non-zero, which the cheapest tier never produces) and sweeps its own codes for the marker.
+// Measured against a list in global memory that a second launch finished: a lane then waited for the return of a global
+// atomic (27 % of the warps of the benchmark data did) and the second launch took 10 us at any size.
 constexpr uint32_t kDeferredMark = 0x80000000u;
-// The list is split into kDeferLists sub-lists (CTA i of the main kernel appends to sub-list i mod
-// kDeferLists), each with its own counter in its own 32-byte sector: appends do not contend for one
-// address (a single counter serialises: 2.7e5 appends took 0.4 ms).
-constexpr int kDeferLists = 256;
-constexpr int kCounterStride = 8;  // uint32 words between counters
+constexpr int kListCap = 1024;  // the benchmark data defers 1 % of the 19000 blocks of a CTA
 
-struct EncodeScratch {
-    uint32_t* ctrl;   // [kDeferLists * kCounterStride] counters, then [0] overflow flag, [1] fix-up CTAs finished
-    int64_t* list;    // kDeferLists sub-lists of `cap` entries
-    uint32_t cap;     // entries per sub-list
-};
-__device__ __forceinline__ uint32_t* scratch_tail(const EncodeScratch& s) { return s.ctrl + kDeferLists * kCounterStride; }
-
-// rows per lane and iteration of the main kernel (with its rare deferral branch, 4 rows at 85 registers and
-// 3 CTAs per SM measured 5 % slower than 3 rows at 64 registers and 4 CTAs per SM)
-constexpr int kMainRows = 3;
-inline unsigned main_grid(int64_t n_blocks) {
-    const int64_t per_cta = (int64_t)kThreads * kMainRows;
-    const int64_t need = (n_blocks + per_cta - 1) / per_cta;
-    const int64_t cap = (int64_t)sm_count() * kEncCtasPerSm;
-    return (unsigned)(need < cap ? (need < 1 ? 1 : need) : cap);
+// One level of a deferred block: the cheapest tier when it applies, then the exact-rounding tier, then the
+// literal search.  amax, s1: max and sum of |x_i|.
+__device__ __forceinline__ uint32_t level_any_q4(const float (&x)[8], float amax, float s1, const uint4* rows) {
+    uint32_t digits;
+    if (amax <= 1.96f && s1 <= 7.96f && e8::level_fast2_q4(x, digits, rows)) return digits;
+    return e8::level_slow_q4(x, s1 == s1 && s1 - s1 == 0.0f ? amax : __int_as_float(0x7fc00000));
 }
 
-template <int DT, int MODE>
+// ROWS: rows per lane and iteration.
+template <int DT, int MODE, bool SAT, int ROWS>
 __global__ void __launch_bounds__(kThreads, 4)
-k_encode_q4m2_main(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n,
-                   uint32_t* __restrict__ codes, EncodeScratch sc_) {
+k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n, uint32_t* codes) {
     __shared__ uint4 flip_rows[8];
+    __shared__ int64_t list[kListCap];
+    __shared__ int64_t queue[kEncWarps][64];
+    __shared__ uint32_t listed;
     if (threadIdx.x < 8) flip_rows[threadIdx.x] = e8::kFlipRows[threadIdx.x];
+    if (threadIdx.x == 0) listed = 0u;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t span = 32 * kMainRows;
+    const int64_t span = 32 * ROWS;
     const int64_t stride = (int64_t)gridDim.x * kEncWarps * span;
-    for (int64_t base = ((int64_t)blockIdx.x * kEncWarps + warp) * span; base < n; base += stride) {
-        float v[kMainRows][8];
-        float sc[kMainRows];
+    const int64_t first = ((int64_t)blockIdx.x * kEncWarps + warp) * span;
+    for (int64_t base = first; base < n; base += stride) {
+        float v[ROWS][8];
+        float sc[ROWS];
 #pragma unroll
-        for (int j = 0; j < kMainRows; ++j) {
+        for (int j = 0; j < ROWS; ++j) {
             const int64_t b = base + j * 32 + lane;
             sc[j] = 1.0f;
             if (b < n) {
@@ -426,7 +417,7 @@ k_encode_q4m2_main(const void* __restrict__ x, const float* __restrict__ scale, 
             }
         }
 #pragma unroll
-        for (int j = 0; j < kMainRows; ++j) {
+        for (int j = 0; j < ROWS; ++j) {
             const int64_t b = base + j * 32 + lane;
             float s1 = 0.0f;
 #pragma unroll
@@ -442,37 +433,17 @@ k_encode_q4m2_main(const void* __restrict__ x, const float* __restrict__ scale, 
             const bool origin = amax <= 0.49f && s1 <= 1.99f;  // this level is the origin too: code 0
             uint32_t code;
             const bool proven = e8::level_fast2_q4(v[j], code, flip_rows);
-            const bool done = origin || (pre && proven);
             if (b < n) {
-                if (done) {
+                if (origin || (pre && proven)) {
                     __stcs(codes + b, origin ? 0u : code);
-                } else {  // rare: mark the block and append it to this CTA's sub-list
-                    codes[b] = kDeferredMark;
-                    const uint32_t l = blockIdx.x % kDeferLists;
-                    const uint32_t pos = atomicAdd(sc_.ctrl + l * kCounterStride, 1u);
-                    if (pos < sc_.cap) sc_.list[(int64_t)l * sc_.cap + pos] = b;
-                    else *scratch_tail(sc_) = 1u;  // full: the fix-up kernel will sweep for the markers instead
+                } else {  // rare
+                    const uint32_t pos = atomicAdd(&listed, 1u);
+                    if (pos < (uint32_t)kListCap) list[pos] = b;
+                    else codes[b] = kDeferredMark;
                 }
             }
         }
     }
-}
-
-// One level of a deferred block: the cheapest tier when it applies, then the exact-rounding tier, then the
-// literal search.  amax, s1: max and sum of |x_i|.
-__device__ __forceinline__ uint32_t level_any_q4(const float (&x)[8], float amax, float s1) {
-    uint32_t digits;
-    if (amax <= 1.96f && s1 <= 7.96f && e8::level_fast2_q4(x, digits)) return digits;
-    return e8::level_slow_q4(x, s1 == s1 && s1 - s1 == 0.0f ? amax : __int_as_float(0x7fc00000));
-}
-
-template <int DT, int MODE, bool SAT>
-__global__ void __launch_bounds__(kThreads)
-k_encode_q4m2_fix(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n,
-                  uint32_t* __restrict__ codes, EncodeScratch sc_) {
-    __shared__ uint32_t q_index[kEncWarps][2][64];
-    __shared__ uint32_t prefix[kDeferLists + 1];
-    const bool overflow = *reinterpret_cast<volatile uint32_t*>(scratch_tail(sc_)) != 0u;
     auto finish = [&](int64_t b) {
         float v[8];
         e8::Row8<DT>::load(x, b, v);
@@ -489,7 +460,7 @@ k_encode_q4m2_fix(const void* __restrict__ x, const float* __restrict__ scale, e
 #pragma unroll 1
         for (int m = 0; m < 2; ++m) {
             const bool origin = amax <= 0.49f && s1 <= 1.99f;
-            if (!origin) code |= level_any_q4(v, amax, s1) << (16 * m);
+            if (!origin) code |= level_any_q4(v, amax, s1, flip_rows) << (16 * m);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(v[i], 0.25f);
             amax *= 0.25f;
@@ -497,73 +468,37 @@ k_encode_q4m2_fix(const void* __restrict__ x, const float* __restrict__ scale, e
         }
         __stcs(codes + b, code);
     };
-    if (!overflow) {
-        // every deferred block is in a sub-list.  Flatten them: exclusive prefix of the kDeferLists
-        // counters (one per thread), then one thread per entry across the whole grid, all lanes busy.
-        uint32_t cnt = *reinterpret_cast<volatile uint32_t*>(sc_.ctrl + threadIdx.x * kCounterStride);
-        prefix[threadIdx.x + 1] = cnt < sc_.cap ? cnt : sc_.cap;
-        if (threadIdx.x == 0) prefix[0] = 0u;
-        __syncthreads();
-        for (int o = 1; o < kDeferLists; o <<= 1) {  // Hillis-Steele inclusive scan over prefix[1..]
-            const uint32_t add = threadIdx.x + 1 > (unsigned)o ? prefix[threadIdx.x + 1 - o] : 0u;
-            __syncthreads();
-            prefix[threadIdx.x + 1] += add;
-            __syncthreads();
-        }
-        const uint32_t total = prefix[kDeferLists];
-        for (uint32_t f = blockIdx.x * kThreads + threadIdx.x; f < total; f += gridDim.x * kThreads) {
-            int lo = 0, hi = kDeferLists;  // largest l with prefix[l] <= f
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (prefix[mid] <= f) lo = mid; else hi = mid;
-            }
-            finish(sc_.list[(int64_t)lo * sc_.cap + (f - prefix[lo])]);
-        }
-    } else {
-        // a sub-list overflowed: sweep all codes for the marker, 32 marked blocks at a time per warp
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();  // the list is complete and the markers of this CTA are visible to it
+    const uint32_t total = listed;
+    if (total > (uint32_t)kListCap) {
+        // every warp reads the codes that it wrote, 32 marked blocks at a time.  A listed block whose old content happens to
+        // be the marker is finished twice, with the same result; the sweep is over before the list is worked off, whose
+        // results may equal the marker.
         int count = 0;
         auto drain = [&](int take) {
-            if (lane < take) {
-                const int e = count - take + lane;
-                finish((int64_t)(((uint64_t)q_index[warp][1][e] << 32) | q_index[warp][0][e]));
-            }
+            if (lane < take) finish(queue[warp][count - take + lane]);
             count -= take;
             __syncwarp();
         };
-        const int64_t stride = (int64_t)gridDim.x * kEncWarps * 32;
-        for (int64_t base = ((int64_t)blockIdx.x * kEncWarps + warp) * 32; base < n; base += stride) {
-            const int64_t b = base + lane;
-            const bool marked = b < n && codes[b] == kDeferredMark;
-            const uint32_t bal = __ballot_sync(0xffffffffu, marked);
-            if (bal) {
-                if (marked) {
-                    const int pos = count + __popc(bal & ((1u << lane) - 1u));
-                    q_index[warp][0][pos] = (uint32_t)b;
-                    q_index[warp][1][pos] = (uint32_t)((uint64_t)b >> 32);
+        for (int64_t base = first; base < n; base += stride) {
+#pragma unroll 1
+            for (int j = 0; j < ROWS; ++j) {
+                const int64_t b = base + j * 32 + lane;
+                const bool marked = b < n && codes[b] == kDeferredMark;
+                const uint32_t bal = __ballot_sync(0xffffffffu, marked);
+                if (bal) {
+                    if (marked) queue[warp][count + __popc(bal & ((1u << lane) - 1u))] = b;
+                    count += __popc(bal);
+                    __syncwarp();
+                    if (count >= 32) drain(32);
                 }
-                count += __popc(bal);
-                __syncwarp();
-                if (count >= 32) drain(32);
             }
         }
         if (count > 0) drain(count);
+        __syncthreads();
     }
-    // the last CTA to finish clears the counters and the flag for the next call on this scratch
-    __syncthreads();
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(scratch_tail(sc_) + 1, 1u) == gridDim.x - 1u;
-    }
-    __syncthreads();
-    if (last) {
-        sc_.ctrl[threadIdx.x * kCounterStride] = 0u;
-        if (threadIdx.x == 0) { scratch_tail(sc_)[0] = 0u; scratch_tail(sc_)[1] = 0u; }
-        __threadfence();
-    }
+    for (uint32_t e = threadIdx.x; e < total && e < (uint32_t)kListCap; e += kThreads) finish(list[e]);
 }
-static_assert(kDeferLists == kThreads, "the fix-up kernel scans one counter per thread");
 
 // Four blocks per thread (kThreads apart, so every access stays coalesced): all codes are
 // loaded before the first table lookup, which multiplies the gathers in flight per thread
@@ -802,73 +737,16 @@ const uint16_t* residual_table_q4_compact(cudaStream_t stream) {
 
 namespace {
 
-// Scratch of the two-launch encoder, one per (device, stream): calls on one stream are ordered, so they
-// may share it; the mutex keeps the two launches of one call together when several host threads use the
-// same stream.  Allocated on first use and when a larger tensor arrives (never inside a stream capture:
-// make the first call of a given size before capturing).
-struct ScratchSlot {
-    int device;
-    cudaStream_t stream;
-    EncodeScratch s;
-};
-std::mutex g_scratch_mu;
-std::vector<ScratchSlot> g_scratch;
-
-constexpr size_t kCtrlBytes = (size_t)(kDeferLists * kCounterStride + 8) * sizeof(uint32_t);
-
-int alloc_scratch(EncodeScratch* s, uint32_t cap, cudaStream_t st) {
-    *s = EncodeScratch{nullptr, nullptr, 0};
-    if (int e = check_cuda(cudaMalloc(&s->ctrl, kCtrlBytes), "cudaMalloc(encode scratch)")) return e;
-    if (int e = check_cuda(cudaMalloc(&s->list, (size_t)kDeferLists * cap * sizeof(int64_t)), "cudaMalloc(encode scratch)")) return e;
-    if (int e = check_cuda(cudaMemsetAsync(s->ctrl, 0, kCtrlBytes, st), "cudaMemsetAsync(encode scratch)")) return e;
-    s->cap = cap;
-    return 0;
-}
-
-int encode_scratch(cudaStream_t st, int64_t n_blocks, EncodeScratch* out) {
-    int dev = 0;
-    if (int e = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return e;
-    // room for one block in 32 deferred (the benchmark data defers one in 125), at least 64 per sub-list
-    const uint32_t want = (uint32_t)(n_blocks / 32 / kDeferLists) + 64u;
-    if ((uint64_t)want * kDeferLists >= 0xffffffffull) return fail(COSET_E_BADARG, "n_blocks too large");
-    for (auto& slot : g_scratch) {
-        if (slot.device == dev && slot.stream == st) {
-            if (slot.s.cap >= want) { *out = slot.s; return 0; }
-            // grow: earlier launches on this stream may still use the old buffers
-            if (int e = check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize(encode scratch)")) return e;
-            cudaFree(slot.s.ctrl);
-            cudaFree(slot.s.list);
-            if (int e = alloc_scratch(&slot.s, want, st)) return e;
-            *out = slot.s;
-            return 0;
-        }
-    }
-    ScratchSlot slot{dev, st, EncodeScratch{nullptr, nullptr, 0}};
-    if (int e = alloc_scratch(&slot.s, want, st)) return e;
-    g_scratch.push_back(slot);
-    *out = slot.s;
-    return 0;
-}
-
-template <int DT, int MODE>
-int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_t n, uint32_t* codes, bool saturate,
-                       cudaStream_t st) {
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
-    EncodeScratch sc;
-    if (int e = encode_scratch(st, n, &sc)) return e;
-    const unsigned mgrid = main_grid(n);
-    k_encode_q4m2_main<DT, MODE><<<mgrid, kThreads, 0, st>>>(x, scale, td, n, codes, sc);
-    if (int e = check_launch("e8_encode (main)")) return e;
-    // the deferred blocks are few: a grid of four CTAs per SM shares them evenly (in sweep mode it strides
-    // over the whole tensor)
-    const int64_t need = (n + kThreads - 1) / kThreads;
-    const unsigned fgrid = (unsigned)(need < 4 * sm_count() ? (need < 1 ? 1 : need) : 4 * sm_count());
-    (void)mgrid;
-    if (saturate)
-        k_encode_q4m2_fix<DT, MODE, true><<<fgrid, kThreads, 0, st>>>(x, scale, td, n, codes, sc);
+// Rows per lane: three keep the loads of the later rows behind the arithmetic of the earlier ones (four at 85 registers
+// and 3 CTAs per SM were 5 % slower); one where three would leave resident CTAs of the chip without work.
+template <int DT, int MODE, bool SAT>
+int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_t n, uint32_t* codes, cudaStream_t st) {
+    const int64_t sms = sm_count(), need3 = (n + 3 * kThreads - 1) / (3 * kThreads), need1 = (n + kThreads - 1) / kThreads;
+    if (need3 >= 4 * sms)
+        k_encode_q4m2_listed<DT, MODE, SAT, 3><<<(unsigned)(need3 < kEncCtasPerSm * sms ? need3 : kEncCtasPerSm * sms), kThreads, 0, st>>>(x, scale, td, n, codes);
     else
-        k_encode_q4m2_fix<DT, MODE, false><<<fgrid, kThreads, 0, st>>>(x, scale, td, n, codes, sc);
-    return check_launch("e8_encode (fix-up)");
+        k_encode_q4m2_listed<DT, MODE, SAT, 1><<<(unsigned)(need1 < 4 * sms ? need1 : 4 * sms), kThreads, 0, st>>>(x, scale, td, n, codes);
+    return check_launch("e8_encode");
 }
 
 }  // namespace
@@ -914,13 +792,12 @@ int coset_e8_encode(const void* x, int x_dtype, const float* scale, int scale_mo
     e8::TileDiv td = e8::make_tile_div(scale_mode == COSET_SCALE_MUL_TILE ? blocks_per_tile : 1, n_blocks);
     unsigned grid = grid_for(n_blocks);
     if (q == 4 && M == 2 && sem == COSET_SEM_CORE) {
-        // persistent warps: at most kEncCtasPerSm CTAs per SM of grid (4 resident at a time)
         int rc = 0;
-        DISPATCH_DT(x_dtype, DT, DISPATCH_MODE(scale_mode, (rc = launch_encode_q4m2<DT, MODE>(x, scale, td, n_blocks, (uint32_t*)codes, false, st))))
+        DISPATCH_DT(x_dtype, DT, DISPATCH_MODE(scale_mode, (rc = launch_encode_q4m2<DT, MODE, false>(x, scale, td, n_blocks, (uint32_t*)codes, st))))
         return rc;
     } else if (q == 4 && M == 2 && sem == COSET_SEM_CORE_SATURATE) {
         int rc = 0;
-        DISPATCH_DT(x_dtype, DT, DISPATCH_MODE(scale_mode, (rc = launch_encode_q4m2<DT, MODE>(x, scale, td, n_blocks, (uint32_t*)codes, true, st))))
+        DISPATCH_DT(x_dtype, DT, DISPATCH_MODE(scale_mode, (rc = launch_encode_q4m2<DT, MODE, true>(x, scale, td, n_blocks, (uint32_t*)codes, st))))
         return rc;
     } else if (q == 4 && M == 2) {
         DISPATCH_DT(x_dtype, DT, DISPATCH_MODE(scale_mode, (k_encode_q4m2<DT, MODE, true><<<grid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes))))

@@ -86,11 +86,7 @@ int coset_e8_projection(const float* x, int64_t n_blocks, float* y, void* stream
  * e8_encode (coset/core/e8/codecs.py:17-89): scale, then M levels of
  * encode_coords(projection(x / q^m)) (coset/core/base.py:134-154), written as packed codes.
  * x: [n_blocks, 8] of x_dtype (16-byte aligned).  codes: packed, 4-byte aligned.
-  * For q = 4, M = 2 the call is two launches (main kernel + a short fix-up kernel for the blocks the
- * cheapest tier cannot prove) and uses a few MB of library-owned scratch per (device, stream), allocated
- * on the first call and when a larger tensor arrives: make the first call of a given size before a
- * stream capture begins.  Calls on one stream share the scratch (they are ordered); concurrent calls
- * on different streams have their own.
+ * One launch, no scratch memory and no state between calls.
  */
 int coset_e8_encode(const void* x, int x_dtype, const float* scale, int scale_mode,
                     int64_t n_blocks, int64_t blocks_per_tile, int q, int M, int sem,

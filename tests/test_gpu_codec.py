@@ -315,10 +315,8 @@ def test_bulk_config_properties(e8):
 
 
 def test_encode_on_concurrent_streams_and_growing_sizes(e8):
-    """The codes-only encoder keeps library-owned scratch per (device, stream): calls issued on several
-    streams at once must not disturb each other, a larger tensor on the same stream grows the scratch,
-    and an overloaded tensor (most blocks deferred: the fix-up kernel's sweep) leaves the scratch clean
-    for the next call."""
+    """Calls issued on several streams at once must not disturb each other, in any order of sizes, and neither does an
+    overloaded tensor (most blocks deferred: the sweep for markers)."""
     g = torch.Generator(device="cuda").manual_seed(5)
     sizes = [4096, 300_000, 70_001, 1_200_000]
     xs = [torch.randn(n, 8, device="cuda", generator=g) * (0.5 if i != 2 else 6.0) for i, n in enumerate(sizes)]
@@ -364,3 +362,16 @@ def test_unknown_result_type_is_refused_and_scales_are_numbers():
         assert torch.equal(e8_decode_packed(codes, scale=two, scale_mode=_lib.SCALE_DIV_SCALAR), want)
     with pytest.raises(ValueError):
         e8_decode_packed(codes, scale="two", scale_mode=_lib.SCALE_DIV_SCALAR)
+
+
+@pytest.mark.parametrize("n", [1, 257, 148 * 4 * 768 - 768, 148 * 4 * 768 + 1, 2_500_001])
+@pytest.mark.parametrize("spread", [0.5, 1.0, 6.0])
+def test_deferred_blocks_in_every_mode(e8, n, spread):
+    """Both row counts per lane around their switch, lists that stay short, fill and overflow (a CTA of the largest tensor
+    has 1400 blocks, its list 1024 entries), and an output buffer that already holds the marker."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, 8, device="cuda", generator=g) * spread
+    x[::53, 1] = 1.5
+    out = torch.full((n,), -(1 << 31), dtype=torch.int32, device="cuda")
+    e8.e8_encode_packed(x, out=out)
+    assert torch.equal(out, e8.e8_encode_packed(x, literal=True).view(torch.int32).view(-1))
