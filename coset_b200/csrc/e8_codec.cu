@@ -209,7 +209,7 @@ k_encode_q4m2(const void* __restrict__ x, const float* __restrict__ scale, e8::T
 
 // Queued encoder (the production path for q=4, M=2).
 //
-// Warps are persistent; one loop iteration of a warp covers kRowsPerIter * 32 consecutive blocks,
+// Warps are persistent; one loop iteration of a warp covers ROWS * 32 consecutive blocks,
 // one row per lane and sub-step.  Every lane runs the cheapest tier (level_fast2_q4: one rounding
 // pass, both cosets from it, digits on the FP32 pipe) behind one pre-test, max|x| <= 1.96 and
 // sum|x| <= 7.96, which makes the top level the origin and bounds every quantity of that tier.
@@ -225,17 +225,18 @@ k_encode_q4m2(const void* __restrict__ x, const float* __restrict__ scale, e8::T
 // SAT: every scaled coordinate is first clamped to +-kSaturate, which keeps the two-level code from
 // wrapping around (the top level stays the origin); only deferred blocks can exceed the bound, so the
 // clamp costs nothing on the common path.
-constexpr int kRowsPerIter = 3;   // rows per lane and loop iteration
-constexpr int kQueueSlots = 32 * (kRowsPerIter + 1);  // < 32 left after a drain + at most 32 per sub-step
 constexpr int kEncWarps = kThreads / 32;
 constexpr float kSaturate = 3.9f;  // 8 * 3.9 / 4 < 7.96 and 3.9 / 4 < 1.96: level 1 of a clamped block is the origin
 
-// CTAs of the queued encoder: enough for every warp to get one iteration, at most kEncCtasPerSm per SM.
+// Rows per lane and iteration of the encoders: three keep the loads of the later rows behind the arithmetic of the
+// earlier ones (four at 85 registers and 3 CTAs per SM were 5 % slower); one where three would leave resident CTAs of the
+// chip without work (digits of 65536 blocks 6.7 -> 5.5 us, a [768, 768] layer's weights 7.1 -> 5.8).  The grid gives every
+// warp an iteration, with at most kEncCtasPerSm CTAs per SM for three rows and the four resident ones for one.
 constexpr int kEncCtasPerSm = 12;
-inline unsigned encoder_grid(int64_t n_blocks) {
-    const int64_t per_cta = (int64_t)kThreads * kRowsPerIter;
-    const int64_t need = (n_blocks + per_cta - 1) / per_cta;
-    const int64_t cap = (int64_t)sm_count() * kEncCtasPerSm;
+inline unsigned encoder_grid(int64_t n_blocks, int* rows) {
+    const int64_t sms = sm_count(), need3 = (n_blocks + 3 * kThreads - 1) / (3 * kThreads), need1 = (n_blocks + kThreads - 1) / kThreads;
+    *rows = need3 >= 4 * sms ? 3 : 1;
+    const int64_t need = *rows == 3 ? need3 : need1, cap = (*rows == 3 ? kEncCtasPerSm : 4) * sms;
     return (unsigned)(need < cap ? (need < 1 ? 1 : need) : cap);
 }
 
@@ -254,10 +255,11 @@ __device__ __forceinline__ void store_digits(float* __restrict__ digits, int64_t
     e8::Row8<0>::store(digits, row, f);
 }
 
-template <int DT, int MODE, int KIND, int DTO, bool SAT>
+template <int DT, int MODE, int KIND, int DTO, bool SAT, int ROWS>
 __global__ void __launch_bounds__(kThreads, 4)
 k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n,
                      uint32_t* __restrict__ codes, const uint2* __restrict__ table, void* __restrict__ out, float value) {
+    constexpr int kQueueSlots = 32 * (ROWS + 1);  // < 32 left after a drain + at most 32 per sub-step
     __shared__ uint32_t q_index[kEncWarps][2][kQueueSlots];  // block index lo / hi
     __shared__ int q_count[kEncWarps];
     auto emit = [&](int64_t b, uint32_t code, float s) {
@@ -302,19 +304,19 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
         __syncwarp();
     };
 
-    const int64_t span = 32 * kRowsPerIter;
+    const int64_t span = 32 * ROWS;
     const int64_t stride = (int64_t)gridDim.x * kEncWarps * span;
     for (int64_t base = ((int64_t)blockIdx.x * kEncWarps + warp) * span; base < n; base += stride) {
-        bool defer[kRowsPerIter];
+        bool defer[ROWS];
         bool any_defer = false;
         {
             // All rows are requested first; the tier then runs row after row in straight-line code, so
             // the loads of the later rows overlap the arithmetic of the earlier ones.  The rows are not
             // kept beyond this scope.
-            float v[kRowsPerIter][8];
-            float sc[kRowsPerIter];
+            float v[ROWS][8];
+            float sc[ROWS];
 #pragma unroll
-            for (int j = 0; j < kRowsPerIter; ++j) {
+            for (int j = 0; j < ROWS; ++j) {
                 const int64_t b = base + j * 32 + lane;
                 sc[j] = 1.0f;
                 if (b < n) {
@@ -326,7 +328,7 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
                 }
             }
 #pragma unroll
-            for (int j = 0; j < kRowsPerIter; ++j) {
+            for (int j = 0; j < ROWS; ++j) {
                 const int64_t b = base + j * 32 + lane;
                 float s1 = 0.0f;
 #pragma unroll
@@ -350,7 +352,7 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
         }
         if (any_defer) {  // rare: one branch per iteration keeps the queue code off the common path
 #pragma unroll
-            for (int j = 0; j < kRowsPerIter; ++j) {
+            for (int j = 0; j < ROWS; ++j) {
                 if (defer[j]) {
                     const int64_t b = base + j * 32 + lane;
                     const int pos = atomicAdd(&q_count[warp], 1);
@@ -737,15 +739,12 @@ const uint16_t* residual_table_q4_compact(cudaStream_t stream) {
 
 namespace {
 
-// Rows per lane: three keep the loads of the later rows behind the arithmetic of the earlier ones (four at 85 registers
-// and 3 CTAs per SM were 5 % slower); one where three would leave resident CTAs of the chip without work.
 template <int DT, int MODE, bool SAT>
 int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_t n, uint32_t* codes, cudaStream_t st) {
-    const int64_t sms = sm_count(), need3 = (n + 3 * kThreads - 1) / (3 * kThreads), need1 = (n + kThreads - 1) / kThreads;
-    if (need3 >= 4 * sms)
-        k_encode_q4m2_listed<DT, MODE, SAT, 3><<<(unsigned)(need3 < kEncCtasPerSm * sms ? need3 : kEncCtasPerSm * sms), kThreads, 0, st>>>(x, scale, td, n, codes);
-    else
-        k_encode_q4m2_listed<DT, MODE, SAT, 1><<<(unsigned)(need1 < 4 * sms ? need1 : 4 * sms), kThreads, 0, st>>>(x, scale, td, n, codes);
+    int rows;
+    const unsigned grid = encoder_grid(n, &rows);
+    if (rows == 3) k_encode_q4m2_listed<DT, MODE, SAT, 3><<<grid, kThreads, 0, st>>>(x, scale, td, n, codes);
+    else k_encode_q4m2_listed<DT, MODE, SAT, 1><<<grid, kThreads, 0, st>>>(x, scale, td, n, codes);
     return check_launch("e8_encode");
 }
 
@@ -852,8 +851,9 @@ int coset_e8_quantize(const void* x, int x_dtype, const float* scale, int scale_
     if (q == 4 && M == 2) {
         const uint2* table = residual_table_q4(st);
         if (!table) return COSET_E_STATE;
-        unsigned qgrid = encoder_grid(n_blocks);
-        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, false><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)))))
+        int rows;
+        const unsigned qgrid = encoder_grid(n_blocks, &rows);
+        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (rows == 3 ? (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, false, 3><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)) : (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, false, 1><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip))))))
     } else if (q <= 4) {
         DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_quantize_generic<DTI, DTO, MODE, 2><<<grid, kThreads, 0, st>>>(x, scale, td, n_blocks, q, M, clip, out, codes_out)))))
     } else {
@@ -889,11 +889,15 @@ int coset_e8_encode_digits_f32(const float* x, float beta, int64_t n_blocks, int
     cudaStream_t st = (cudaStream_t)stream;
     if (q == 4 && M == 2) {
         const e8::TileDiv td = e8::make_tile_div(1, n_blocks);
-        const unsigned grid = encoder_grid(n_blocks);
-        if (beta == 1.0f)  // x / 1 is x
-            k_encode_q4m2_queued<0, COSET_SCALE_NONE, kDigits, 0, false><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, 0.0f);
-        else
-            k_encode_q4m2_queued<0, kScaleDivValue, kDigits, 0, false><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, beta);
+        int rows;
+        const unsigned grid = encoder_grid(n_blocks, &rows);
+#define DIGITS_AS(MODE, ROWS) k_encode_q4m2_queued<0, MODE, kDigits, 0, false, ROWS><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, beta)
+        if (beta == 1.0f) {  // x / 1 is x
+            if (rows == 3) DIGITS_AS(COSET_SCALE_NONE, 3); else DIGITS_AS(COSET_SCALE_NONE, 1);
+        } else {
+            if (rows == 3) DIGITS_AS(kScaleDivValue, 3); else DIGITS_AS(kScaleDivValue, 1);
+        }
+#undef DIGITS_AS
     } else {
         k_encode_digits_generic<<<grid_for(n_blocks), kThreads, 0, st>>>(x, beta, n_blocks, q, M, digits);
     }

@@ -375,3 +375,21 @@ def test_deferred_blocks_in_every_mode(e8, n, spread):
     out = torch.full((n,), -(1 << 31), dtype=torch.int32, device="cuda")
     e8.e8_encode_packed(x, out=out)
     assert torch.equal(out, e8.e8_encode_packed(x, literal=True).view(torch.int32).view(-1))
+
+
+@pytest.mark.parametrize("n", [255, 148 * 4 * 768 - 768, 148 * 4 * 768 + 1])
+@pytest.mark.parametrize("spread", [0.5, 3.0])
+def test_round_trip_and_digits_around_the_row_count_switch(e8, cfgcls, n, spread):
+    """e8_quantize and the digit calls share the queue of deferred blocks; one and three rows per lane give what the
+    op-by-op search gives."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, 8, device="cuda", generator=g) * spread
+    x[::53, 1] = 1.5
+    codes = e8.e8_encode_packed(x, literal=True)
+    want = e8.e8_decode_packed(codes)
+    config = cfgcls(lattice_type="E8", q=4, M=2, beta=1.0)
+    digits, _ = e8.e8_encode(x, config)
+    words = codes.view(torch.int32).view(-1, 1, 1) >> (16 * torch.arange(2, device="cuda").view(1, 2, 1) + 2 * torch.arange(8, device="cuda"))
+    assert torch.equal(digits, (words & 3).float())
+    assert torch.equal(e8.e8_quantize(x, 4), want)
+    assert torch.equal(e8.e8_decode(digits, config), want)
