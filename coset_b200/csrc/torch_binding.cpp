@@ -353,17 +353,20 @@ using torch::autograd::variable_list;
 // W_q = clamp(e8_quantize(W beta) / beta, +-clip) with beta = beta_min + sigmoid(theta) range per tile, and the
 // straight-through gradients of the reference graph (coset/core/layers.py:62-110, 415-470).
 struct FakeQuant : torch::autograd::Function<FakeQuant> {
+    // bias16: the bias in bf16, written by the launch that forms the scales, where the caller wants one
     static void launch(const Tensor& w, const Tensor& th, const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip,
-                       at::ScalarType out_type, Tensor& wq, Tensor& codes, Tensor& beta) {
+                       at::ScalarType out_type, Tensor& wq, Tensor& codes, Tensor& beta, const Tensor& bias = Tensor(), const Tensor& bias16 = Tensor()) {
         const int bytes = coset_e8_code_bytes((int)q, 2);
         TORCH_CHECK_VALUE(bytes != 0, "unsupported q=", q, " for the fused E8 weight quantiser (2 <= q <= 16)");
+        TORCH_CHECK(bpt >= 1, "blocks_per_tile must be >= 1");
         const int64_t nb = w.numel() / 8;
         codes = empty({nb, bytes}, at::kByte, w);
         wq = empty(w.sizes(), out_type, w);
         beta = empty({th.numel()}, at::kFloat, w);
-        check_rc(coset_e8_layer_fake_quant_fwd(fdata(w), fdata(th), fdata(beta_min), fdata(beta_range), nb, bpt, (int)q, (float)clip, data(wq),
-                                               out_type == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16, data(codes), fdata(beta), stream_of(w)),
-                 "coset_e8_layer_fake_quant_fwd");
+        check_rc(coset_layer_beta_bias(fdata(th), fdata(beta_min), fdata(beta_range), (nb + bpt - 1) / bpt, fdata(beta), fdata(bias),
+                                       bias16.defined() ? bias.numel() : 0, data(bias16), stream_of(w)), "coset_layer_beta_bias");
+        check_rc(coset_e8_quantize(fdata(w), COSET_DTYPE_F32, fdata(beta), COSET_SCALE_MUL_TILE, nb, bpt, (int)q, 2, (float)clip, data(wq),
+                                   out_type == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16, data(codes), stream_of(w)), "coset_e8_quantize");
     }
     // dL/dW and dL/dtheta (undefined unless asked for) from dL/dW_q
     static std::pair<Tensor, Tensor> backward_launch(Tensor g, const Tensor& w, const Tensor& theta, const Tensor& beta, const Tensor& codes,
@@ -409,10 +412,13 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& theta, const Tensor& bias,
                           const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip) {
         const Tensor w = contiguous(weight);
-        Tensor wq, codes, beta;
-        FakeQuant::launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, x.scalar_type(), wq, codes, beta);
-        Tensor b = bias;
-        if (b.defined() && x.scalar_type() == at::kBFloat16) b = b.to(at::kBFloat16);
+        Tensor wq, codes, beta, b = bias, b16;
+        if (b.defined() && x.scalar_type() == at::kBFloat16) {
+            if (b.scalar_type() == at::kFloat && b.is_contiguous() && b.device() == w.device()) b16 = empty(b.sizes(), at::kBFloat16, w);
+            else b = b.to(at::kBFloat16);
+        }
+        FakeQuant::launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, x.scalar_type(), wq, codes, beta, b, b16);
+        if (b16.defined()) b = b16;
         Tensor y = at::linear(x, wq, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
         ctx->save_for_backward({x, w, theta, beta, codes, wq});
         ctx->saved_data["range"] = beta_range;
@@ -446,7 +452,13 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         }
         if (ctx->needs_input_grad(3)) {
             const auto type = (at::ScalarType)ctx->saved_data["bias_type"].toInt();
-            out[3] = at::sum(g2, at::IntArrayRef{0}, false, g2.scalar_type() == type ? std::nullopt : std::optional<at::ScalarType>(type));
+            const bool own = g2.is_contiguous() && (type == at::kFloat || type == at::kBFloat16) && (g2.scalar_type() == at::kFloat || g2.scalar_type() == at::kBFloat16)
+                             && !at::GradMode::is_enabled();
+            if (own) {
+                out[3] = empty({g2.size(1)}, type, g2);
+                check_rc(coset_column_sum(data(g2), dtype_code(g2, "grad"), g2.size(0), g2.size(1), data(out[3]),
+                                          type == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16, stream_of(g2)), "coset_column_sum");
+            } else out[3] = at::sum(g2, at::IntArrayRef{0}, false, g2.scalar_type() == type ? std::nullopt : std::optional<at::ScalarType>(type));
         }
         return out;
     }

@@ -159,6 +159,12 @@ int coset_e8_fake_quant_bwd(const void* grad_out, int grad_dtype, const float* w
  */
 int coset_layer_beta(const float* theta, const float* beta_min, const float* beta_range, int64_t n_tiles,
                      float* beta, void* stream);
+/* coset_layer_beta and, in the same launch, bias_bf16 = bf16(bias) of n_bias values (0: none). */
+int coset_layer_beta_bias(const float* theta, const float* beta_min, const float* beta_range, int64_t n_tiles,
+                          float* beta, const float* bias, int64_t n_bias, void* bias_bf16, void* stream);
+/* out[c] = sum over r of x[r][c] of a row-major [rows, cols] matrix (the gradient of a bias), summed in
+ * float32 in a fixed order; float32 or bf16 in and out. */
+int coset_column_sum(const void* x, int x_dtype, int64_t rows, int64_t cols, void* out, int out_dtype, void* stream);
 int coset_e8_layer_fake_quant_fwd(const float* w, const float* theta, const float* beta_min, const float* beta_range,
                                   int64_t n_blocks, int64_t blocks_per_tile, int q, float clip, void* out,
                                   int out_dtype, void* codes, float* beta, void* stream);

@@ -273,3 +273,36 @@ def test_bias_of_another_type_is_refused_for_float32():
     with pytest.raises(RuntimeError):
         layer(torch.randn(8, 64, device="cuda"))
     assert layer(torch.randn(8, 64, device="cuda").to(torch.bfloat16)).dtype == torch.bfloat16
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(0, 8), (1, 1), (255, 31), (256, 32), (257, 33), (4096, 776), (3, 4100), (5000, 64)])
+def test_column_sum(rows, cols, dtype):
+    """Ragged row groups and column strips, rows that are and are not a multiple of 16 bytes, an unaligned matrix.  The sums
+    are float32 with at most rows / 256 + 40 additions in a chain."""
+    from coset_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    for offset in (0, 1):
+        x = torch.randn(rows * cols + offset, device="cuda", generator=g).to(dtype)[offset:].view(rows, cols)
+        want, size = x.double().sum(0), x.double().abs().sum(0)
+        for out_dtype, code in ((torch.float32, _lib.DTYPE_F32), (torch.bfloat16, _lib.DTYPE_BF16)):
+            y = torch.full((cols,), float("nan"), device="cuda", dtype=out_dtype)
+            rc = _lib.lib().coset_column_sum(x.data_ptr(), _lib.dtype_code(x, "x"), rows, cols, _lib.ptr(y), code, _lib.stream())
+            _lib.check(rc, "coset_column_sum")
+            bound = size * (rows / 256 + 40) * 2.0 ** -24 + (want.abs() * 2.0 ** -8 if out_dtype is torch.bfloat16 else 0)
+            assert bool(((y.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("grad", ["dense", "expanded"])
+def test_bias_gradient_of_any_layout(grad):
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 40, device="cuda")
+    x = torch.randn(3, 50, 64, device="cuda")
+    y = layer(x)
+    if grad == "dense":
+        gy = torch.randn_like(y)
+        y.backward(gy)
+    else:
+        gy = torch.ones_like(y)
+        y.sum().backward()
+    torch.testing.assert_close(layer.bias.grad, gy.sum((0, 1)), rtol=1e-5, atol=1e-4)
