@@ -19,13 +19,17 @@
 //     adds one table row; three bit-selects and a shift leave the 16-bit level word.
 // Guards: max|x| <= 1.96 and sum|x| <= 7.96 (which also makes the NEXT level the origin and keeps every
 // lane in range), max|d| < 1/2 - 2.96 * 2^-21 and min|d| > 2.96 * 2^-21 (rint equals the reference's
-// custom_round for x and x - 1/2), minimum of |d| unique by 2^-21, |dist1 - dist0| > 2^-14.
+// custom_round for x and x - 1/2), minimum of |d| unique by 2^-21 if coset 1 has a flip, |dist1 - dist0| > 2^-14.
+// Bound: instruction issue (77 % of the slots, ALU 68 %, FMA 36 %, 276 instructions per warp row in the encoder), so what
+// the FMA pipe does on all eight coordinates is done in pairs (f32x2), and floor comes from a round-down addition instead
+// of a saturated product: 2^25 float32 blocks 317 -> 307 us.  With the uniqueness of the minimum asked for only where it is
+// used, which halves the deferred blocks of data with equal magnitudes: 300 us, bf16 362 -> 351.
 #pragma once
 #include "e8_fast.cuh"
 
 namespace e8 {
 
-constexpr float kMagic0 = 8388608.0f + 64.0f * (1.0f + 512.0f);     // coordinate 0 starts digit word A
+constexpr float kMagicA = 8388608.0f + 64.0f * (1.0f + 512.0f);
 constexpr float kMagicB = 8388608.0f + 64.0f * (8.0f + 2048.0f);
 constexpr float kMagicC = 8388608.0f + 64.0f * (32.0f + 8192.0f);
 constexpr float kMagicD = 8388608.0f + 64.0f * (128.0f + 32768.0f);
@@ -53,20 +57,59 @@ __device__ __forceinline__ uint32_t bitselect(uint32_t a, uint32_t b, uint32_t m
     return r;
 }
 
+// Two floats in one 64-bit register pair: one instruction, each half rounded on its own.
+struct F2 {
+    uint64_t v;
+};
+__device__ __forceinline__ F2 pair2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void split2(F2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2_down(F2 a, F2 b) {  // towards minus infinity
+    F2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
 // x: scaled block with max|x| <= 1.96 and sum|x| <= 7.96 (the caller's pre-test).  Returns true and the
 // 16-bit level word, or false when a guard refuses.
 // rows: the eight kFlipRows entries, in shared memory when the caller has a copy there (lanes index it
 // with different values; constant memory would serialise those reads), else kFlipRows itself.
 __device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& digits, const uint4* rows = kFlipRows) {
     const float kTie = 2.96f * 4.76837158203125e-07f;
-    float w[8], f[8], d[8], g[8];
+    // Rounding, remainder and g = [d < 0] in pairs: g is rint - floor, for x is away from the integers (guarded).
+    float w[8], d[8];
+    F2 f2[4], g2[4];
+    const F2 M2 = pair2(kMagic, kMagic);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float M = i == 0 ? kMagic0 : kMagic;
-        w[i] = __fadd_rn(x[i], M);
-        f[i] = __fsub_rn(w[i], M);
-        d[i] = __fsub_rn(x[i], f[i]);
-        g[i] = __saturatef(__fmul_rn(d[i], -1.099511627776e12f));  // 1 where d < 0
+    for (int i = 0; i < 4; ++i) {
+        const F2 x2 = pair2(x[2 * i], x[2 * i + 1]), w2 = add2(x2, M2);
+        f2[i] = sub2(w2, M2);
+        g2[i] = sub2(w2, add2_down(x2, M2));
+        split2(w2, w[2 * i], w[2 * i + 1]);
+        split2(sub2(x2, f2[i]), d[2 * i], d[2 * i + 1]);
     }
     float l1 = 0.0f;
 #pragma unroll
@@ -84,10 +127,13 @@ __device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& di
     bool ok = (m0 < 0.5f - kTie) && (mn > kTie);
     // the minimum must be unique by ~2^-21: sum of sat(1 - (|d_i| - mn) 2^20) is 1 from the minimum itself
     const float cu = __fmaf_rn(mn, 1048576.0f, 1.0f);
-    float u = 0.0f;
+    F2 u2[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) u = __fadd_rn(u, __saturatef(__fmaf_rn(fabsf(d[i]), -1048576.0f, cu)));
-    ok = ok && (u < 1.5f);
+    for (int i = 0; i < 4; ++i)
+        u2[i] = pair2(__saturatef(__fmaf_rn(fabsf(d[2 * i]), -1048576.0f, cu)), __saturatef(__fmaf_rn(fabsf(d[2 * i + 1]), -1048576.0f, cu)));
+    float u, u_hi;
+    split2(add2(add2(u2[0], u2[1]), add2(u2[2], u2[3])), u, u_hi);
+    u = __fadd_rn(u, u_hi);
     // sign bytes of d and of x, one byte per coordinate in key-lane order
     const uint32_t sA = gather_bytes<0x0073>(d[7], d[6], d[5], d[4]), sB = gather_bytes<0x0073>(d[3], d[2], d[1], d[0]);
     const uint32_t xA = gather_bytes<0x0073>(x[7], x[6], x[5], x[4]), xB = gather_bytes<0x0073>(x[3], x[2], x[1], x[0]);
@@ -106,6 +152,7 @@ __device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& di
                              __float_as_uint(d[6]) ^ __float_as_uint(d[7]));
     const bool odd0 = (pw & 1u) != 0u;
     const bool odd1 = ((pw ^ (pd >> 31)) & 1u) != 0u;
+    ok = ok && (u < 1.5f || !odd1);  // without a flip of coset 1 its minimum is not used
     // flip costs: 1 -+ 2 m0 for the integer coset, 1 -+ 2 (1/2 - mn) for the half-integer coset
     const float m0s = __uint_as_float(__float_as_uint(m0) ^ (away0 & 0x80000000u));
     const float c0 = __fmaf_rn(-2.0f, m0s, 1.0f);
@@ -120,14 +167,13 @@ __device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& di
     const uint32_t up = half ? up1 : up0;
     const uint32_t row = (half ? sel1 : sel0) ^ 3u;  // coordinate index of the flip
     const uint32_t stp = odd ? (up ? 1u : 0xffffffffu) : 0u;  // +1 when the rule moves up, -1 otherwise
-    // digit words from the chosen coset's rounded integers fs = f - half * g (coordinate 0 keeps its magic)
+    // digit words from the chosen coset's rounded integers fs = f - half * g
     float fs[8];
-    fs[0] = __fmaf_rn(nhf, g[0], w[0]);
 #pragma unroll
-    for (int i = 1; i < 8; ++i) fs[i] = __fmaf_rn(nhf, g[i], f[i]);
+    for (int i = 0; i < 4; ++i) split2(fma2(pair2(nhf, nhf), g2[i], f2[i]), fs[2 * i], fs[2 * i + 1]);
     const float t56 = __fadd_rn(fs[5], fs[6]), t46 = __fadd_rn(fs[4], t56), t36 = __fadd_rn(fs[3], t46);
     const float t26 = __fadd_rn(fs[2], t36), t16 = __fadd_rn(fs[1], t26), t06 = __fadd_rn(fs[0], t16);
-    const float A = __fmaf_rn(fs[7], 513.0f, __fmaf_rn(t46, 512.0f, t06));
+    const float A = __fmaf_rn(fs[7], 513.0f, __fmaf_rn(t46, 512.0f, __fadd_rn(t06, kMagicA)));
     const float B = __fmaf_rn(fs[7], 4112.0f, __fmaf_rn(t56, 2048.0f, __fmaf_rn(t16, 8.0f, kMagicB)));
     const float C = __fmaf_rn(fs[7], 24672.0f, __fmaf_rn(fs[6], 8192.0f, __fmaf_rn(t26, 32.0f, kMagicC)));
     const float D = __fmaf_rn(hf, 32768.0f, __fmaf_rn(fs[7], 66048.0f, __fmaf_rn(t36, 128.0f, kMagicD)));
