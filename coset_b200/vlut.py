@@ -13,7 +13,6 @@ weights) plus the scales beta, and applied from the codes:
 The math is the reference's one-sided vLUT inner product (coset/legacy/quant/vlut.py:72-117) in
 the layer's scale convention W_q = decode(codes) / beta (coset/core/layers.py:453-460).
 """
-import operator
 from typing import Optional
 
 import torch
@@ -189,18 +188,22 @@ class E8CodeLinear(nn.Module):
         later call may come from another stream or thread, and none of these may still read the one it replaces.  Inside a
         graph capture it is recorded with the call and not kept: nothing is computed before the replay."""
         entry = self._kept.get(name)
+        if entry is not None and entry[1] == settings:
+            for t, (kept, version, pointer) in zip(sources, entry[2]):
+                if t is not kept or t._version != version or t.data_ptr() != pointer:
+                    break
+            else:
+                return entry[0]
         if any(t.is_inference() for t in sources):  # no version counter: a write would go unseen
             return make()
-        versions = [(t._version, t.data_ptr()) for t in sources]
-        if entry is not None and entry[1] == versions and entry[2] == settings and all(map(operator.is_, entry[3], sources)):
-            return entry[0]
+        state = [(t, t._version, t.data_ptr()) for t in sources]
         value = make()
         if not torch.cuda.is_current_stream_capturing():
             if entry is not None:
                 torch.cuda.synchronize(value.device)
             else:
                 torch.cuda.current_stream(value.device).synchronize()
-            self._kept[name] = (value, versions, settings, sources)
+            self._kept[name] = (value, settings, state)
         return value
 
     @property
@@ -212,20 +215,28 @@ class E8CodeLinear(nn.Module):
         read the codes themselves: under capture, for a graph is replayed on whatever the codes then hold, and for codes
         without a version counter."""
         codes = self._buffers["codes"]
-        if torch.cuda.is_current_stream_capturing() or codes.is_inference():
+        if torch._C._cuda_isCurrentStreamCapturing() or codes.is_inference():
             return None
-        return self._keep("layout", (codes,), None, lambda: _lib.native().vlut_layout(codes))
+        return self._keep("layout", (codes,), None, self._make_layout)
+
+    def _make_layout(self):
+        return _lib.native().vlut_layout(self._buffers["codes"])
 
     def _dense_bf16(self):
         buf = self._buffers
-        return self._keep("dense", (buf["codes"], buf["beta"]), (self.weight_clip_value, self.blocks_per_tile),
-                          lambda: self.dense_weight(torch.bfloat16))
+        return self._keep("dense", (buf["codes"], buf["beta"]), (self.weight_clip_value, self.blocks_per_tile), self._make_dense)
+
+    def _make_dense(self):
+        return self.dense_weight(torch.bfloat16)
 
     def _bias_bf16(self):
         bias = self._buffers["bias"]
         if bias is None or bias.dtype == torch.bfloat16:
             return bias
-        return self._keep("bias", (bias,), None, lambda: bias.to(torch.bfloat16))
+        return self._keep("bias", (bias,), None, self._make_bias)
+
+    def _make_bias(self):
+        return self._buffers["bias"].to(torch.bfloat16)
 
     def check(self):
         """Synchronises and raises if a bounded barrier wait expired inside one of the tensor-core kernels since
