@@ -407,7 +407,7 @@ struct FakeQuant : torch::autograd::Function<FakeQuant> {
 // y = x W_q^T + bias as ONE autograd node: the forward quantises and multiplies, the backward forms dx, dW, dtheta
 // and dbias.  An eager step of a small layer is bound by the host; one node instead of five (cast, quantise,
 // transpose, product, bias) and native code on both sides took the step of the [3072, 768] layer with 4096
-// tokens from 312 us to the time of its kernels.
+// tokens from 330 to 171 us, 80 of them on the device.
 struct QatLinear : torch::autograd::Function<QatLinear> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& theta, const Tensor& bias,
                           const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip) {

@@ -97,6 +97,7 @@ class E8CodeLinear(nn.Module):
     the tokens in between, where decoding the whole weight per call costs more than the product itself.
     Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 5.5-10 us for 1-16
     tokens and a 4096 x 4096 weight; "tcgen05" keeps nothing and stays on the code-domain kernels (9.7-23 us).
+    A call under graph capture reads the codes themselves, so that a replay follows writes to them.
     small_t_max defaults to 16 ("auto", "cublas") or 48 ("tcgen05"): measured on a 4096 x 4096 layer the
     code-domain kernels take 9.7 / 23 / 44 / 86 us for 1 / 16 / 32 / 64 tokens (they re-read and re-decode the
     codes for every 16 tokens), the library on the cached copy 7-13 us, the fused kernel 64 us.
