@@ -41,6 +41,7 @@ const Tensor& cuda_arg(PyObject* o, const char* name) {
     return t;
 }
 Tensor optional_arg(PyObject* o, const char* name) { return o == Py_None ? Tensor() : tensor_arg(o, name); }
+std::optional<Tensor> maybe_arg(PyObject* o, const char* name) { return o == Py_None ? std::nullopt : std::optional<Tensor>(tensor_arg(o, name)); }
 
 int64_t int_arg(PyObject* o) {
     const long long v = PyLong_AsLongLong(o);
@@ -409,10 +410,11 @@ struct FakeQuant : torch::autograd::Function<FakeQuant> {
 // transpose, product, bias) and native code on both sides took the step of the [3072, 768] layer with 4096
 // tokens from 330 to 171 us, 80 of them on the device.
 struct QatLinear : torch::autograd::Function<QatLinear> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& theta, const Tensor& bias,
+    // the bias is optional, not undefined: an undefined tensor is an input of the node like any other and has no device
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& theta, const std::optional<Tensor>& bias,
                           const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip) {
         const Tensor w = contiguous(weight);
-        Tensor wq, codes, beta, b = bias, b16;
+        Tensor wq, codes, beta, b = bias ? *bias : Tensor(), b16;
         if (b.defined() && x.scalar_type() == at::kBFloat16) {
             if (b.scalar_type() == at::kFloat && b.is_contiguous() && b.device() == w.device()) b16 = empty(b.sizes(), at::kBFloat16, w);
             else b = b.to(at::kBFloat16);
@@ -426,7 +428,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         ctx->saved_data["bpt"] = bpt;
         ctx->saved_data["q"] = q;
         ctx->saved_data["clip"] = clip;
-        if (bias.defined()) ctx->saved_data["bias_type"] = (int64_t)bias.scalar_type();
+        if (bias) ctx->saved_data["bias_type"] = (int64_t)bias->scalar_type();
         return y;
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -450,8 +452,9 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
             out[1] = r.first;
             out[2] = r.second;
         }
-        if (ctx->needs_input_grad(3)) {
-            const auto type = (at::ScalarType)ctx->saved_data["bias_type"].toInt();
+        const auto bias_type = ctx->saved_data.find("bias_type");  // absent with the bias, which then is no input and has no edge
+        if (bias_type != ctx->saved_data.end() && ctx->needs_input_grad(3)) {
+            const auto type = (at::ScalarType)bias_type->second.toInt();
             const bool own = g2.is_contiguous() && (type == at::kFloat || type == at::kBFloat16) && (g2.scalar_type() == at::kFloat || g2.scalar_type() == at::kBFloat16)
                              && !at::GradMode::is_enabled();
             if (own) {
@@ -490,7 +493,7 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check_weight(w);
     cuda_arg(a[1], "weight");
     c10::cuda::CUDAGuard guard(w.device());
-    return THPVariable_Wrap(QatLinear::apply(x, w, tensor_arg(a[2], "theta"), optional_arg(a[3], "bias"), tensor_arg(a[4], "beta_min"),
+    return THPVariable_Wrap(QatLinear::apply(x, w, tensor_arg(a[2], "theta"), maybe_arg(a[3], "bias"), tensor_arg(a[4], "beta_min"),
                                              tensor_arg(a[5], "beta_range"), int_arg(a[6]), int_arg(a[7]), float_arg(a[8])));
     END_HANDLE_TH_ERRORS
 }

@@ -306,3 +306,29 @@ def test_bias_gradient_of_any_layout(grad):
         gy = torch.ones_like(y)
         y.sum().backward()
     torch.testing.assert_close(layer.bias.grad, gy.sum((0, 1)), rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("tiling", ["row", "block"])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 1e-2)])
+@pytest.mark.parametrize("made", ["without", "removed"])
+def test_layer_without_a_bias(made, tiling, dtype, tol):
+    """bias=False, and a bias taken away later, against the composed path: no_grad, backward and the gradient of a gradient."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    results = []
+    for diagnostics in (False, True):
+        layer = create_e8_hnlq_linear(72, 40, device="cuda", tiling=tiling, init_method="zeros", bias=made == "removed", enable_diagnostics=diagnostics)
+        layer.bias = None
+        g = torch.Generator(device="cuda").manual_seed(4)
+        with torch.no_grad():
+            layer.weight.copy_(torch.randn(40, 72, device="cuda", generator=g) * 20.0)
+        x = torch.randn(3, 11, 72, device="cuda", generator=g).to(dtype).requires_grad_()
+        with torch.no_grad():
+            still = layer(x)
+        y = layer(x)
+        gx, = torch.autograd.grad((y.float() ** 2).sum(), x, create_graph=True)
+        (y.float().sum() + (gx.float() ** 2).sum()).backward()
+        assert torch.equal(still, y)
+        results.append((y.detach(), gx.detach(), x.grad, layer.weight.grad, layer.theta_beta.grad))
+    for one, composed in zip(*results):
+        assert one.shape == composed.shape and one.dtype == composed.dtype
+        assert rel(one.float().cpu().numpy(), composed.float().cpu().numpy()) < tol
