@@ -296,10 +296,11 @@ class HNLQLinearQAT(nn.Module):
         The bounds depend only on the two statistics buffers, which change once every 256 quantised
         forwards, so they are kept until one of the buffers is written (in place or replaced) or a
         hyper-parameter changes; the arithmetic and its order are the reference's."""
-        state = self.__dict__
-        sigma, xmax = state["_buffers"]["sigma_ema"], state["_buffers"]["xmax_ema"]
-        key = (sigma._version, xmax._version, sigma.data_ptr(), xmax.data_ptr(), state["Delta0"], state["eta"], state["q"], state["M"])
-        if state.get("_bounds_key") != key:
+        buffers = self.__dict__["_buffers"]
+        sigma = buffers["sigma_ema"] if "sigma_ema" in buffers else self.sigma_ema
+        xmax = buffers["xmax_ema"] if "xmax_ema" in buffers else self.xmax_ema
+        key = (sigma._version, xmax._version, sigma.data_ptr(), xmax.data_ptr(), self.Delta0, self.eta, self.q, self.M)
+        if self.__dict__.get("_bounds_key") != key:
             with torch.no_grad():
                 qM = float(self.q ** self.M)
                 ginv = self._gamma_inv_host
@@ -384,13 +385,14 @@ class HNLQLinearQAT(nn.Module):
     def _one_node(self, x, low):
         """Whether the whole product can run as one native autograd node: the plain case of a quantised E8 layer
         on the GPU.  Warm-up, diagnostics (which look at the quantised weights), autocast, forward-mode derivatives (the
-        node has none), parametrised weights and a quantize_fn of the caller's own take the composed path."""
+        node has none), parametrised or pruned parameters and a quantize_fn of the caller's own take the composed path."""
         state = self.__dict__
         params = state["_parameters"]
         return (state["_fused"] and state["quantization_enabled"] and not state["enable_diagnostics"] and x.is_cuda
                 and (low or x.dtype == torch.float32) and not torch.is_autocast_enabled("cuda")
                 and forward_ad._current_level < 0
-                and "weight" in params and ("theta_beta" in params or not state["theta_trainable"]) and params["weight"].is_cuda)
+                and "weight" in params and "bias" in params and "theta_beta" in (params if state["theta_trainable"] else state["_buffers"])
+                and params["weight"].is_cuda)
 
     def forward(self, x):
         low = x.dtype == torch.bfloat16

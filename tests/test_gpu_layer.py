@@ -332,3 +332,32 @@ def test_layer_without_a_bias(made, tiling, dtype, tol):
     for one, composed in zip(*results):
         assert one.shape == composed.shape and one.dtype == composed.dtype
         assert rel(one.float().cpu().numpy(), composed.float().cpu().numpy()) < tol
+
+
+@pytest.mark.parametrize("how", ["parametrised", "pruned", "plain attribute"])
+def test_bias_that_is_no_plain_parameter(how):
+    """The layer reads its bias as an attribute: one that a parametrisation computes, a pruned one, a plain tensor."""
+    from torch.nn.utils import parametrize, prune
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 32, device="cuda")
+    with torch.no_grad():
+        layer.bias.copy_(torch.randn(32))
+    x = torch.randn(8, 64, device="cuda")
+    y, bias = layer(x).detach(), layer.bias.detach().clone()
+    if how == "parametrised":
+        class Double(torch.nn.Module):
+            def forward(self, b):
+                return 2 * b
+        parametrize.register_parametrization(layer, "bias", Double())
+    elif how == "pruned":
+        prune.l1_unstructured(layer, "bias", 0.5)
+    else:
+        del layer._parameters["bias"]
+        layer.bias = torch.ones(32, device="cuda")
+    steps = layer._step_host
+    got = layer(x)
+    torch.testing.assert_close(got.detach(), y - bias + layer.bias.detach(), rtol=1e-5, atol=1e-4)
+    assert layer._step_host == steps + 1
+    if how == "parametrised":
+        got.sum().backward()
+        torch.testing.assert_close(layer.parametrizations.bias.original.grad, torch.full((32,), 16.0, device="cuda"))
