@@ -50,6 +50,7 @@ SIGNATURES = {
     "coset_e8_vlut_layout_bytes": [_i32, _i32],
     "coset_e8_vlut_layout": [_vp, _i32, _i32, _vp, _vp],
     "coset_e8_vlut_product": [_vp, _vp, _i64, _i32, _i32, _vp, _i32, _i64, _i32, _vp, _vp, _i32, _i32, _i64, _f32, _vp],
+    "coset_e8_vlut_product_checked": [_vp, _vp, _vp, _i64, _i32, _i32, _vp, _i32, _i64, _i32, _vp, _vp, _i32, _i32, _i64, _f32, _vp],
     "coset_e8_quant_stats_scratch_bytes": [_i64],
     "coset_e8_quant_stats": [_vp, _i32, _vp, _i32, _i64, _i64, _vp, _i64, _vp, _vp],
     "coset_e8_quant_stats_static_max_blocks": [],

@@ -12,7 +12,7 @@
 //     clamped weights are exact too.
 // Bound: 1 byte per weight (+ 4 per 8 weights of per-block scales), 2.6-3.9 us of HBM traffic for 4096 x 4096.  Measured
 // there (graph replay, before -> now), one scale per row with a clamp: 14.4 -> 5.5 us for one token, 22.4 -> 9.5 for 16;
-// one per block: 9.9 -> 6.9, 22.8 -> 10.3; float32 tokens with a scale per row: 15.2 -> 9.7, 118 -> 20.6.  8192 x 8192, one
+// one per block: 9.9 -> 6.9, 22.8 -> 10.3 (before the codes were read too, see below); float32 tokens with a scale per row: 15.2 -> 9.7, 118 -> 20.6.  8192 x 8192, one
 // token, scale per row: 48 -> 16 us (4.2 TB/s).  What is left at 16 tokens is latency: two warps' worth of shared-memory
 // round trips per unit at 16 warps per SM (staging the activations once per CTA, deeper cp.async rings with the weights in
 // them and two-stage rings at higher occupancy were measured within 10 % of this form, and slower for few tokens).
@@ -23,7 +23,19 @@
 // Layout: [groups of 16 rows][units of 8 blocks][2][32 lanes] of 16 bytes; a lane's 32 bytes are eight words, word b =
 // coordinates 2c, 2c + 1 of block b of the unit for row g | the same for row g + 8, with g = lane / 4, c = lane % 4: the A
 // fragment of one m16n8k8 step, and two neighbouring words that of one m16n8k16 step.
+// Behind the tiles, one 64-bit hash of the codes for every group and every residue of the unit modulo 16.
+//
+// The copy must never answer for codes that have changed since: the host sees neither a write through another alias of the
+// codes nor one by a collective or a replayed graph.  So a warp of the product reads the codes of its units beside their
+// bytes, hashes them, and where the hash is not the kept one does its units again with words made from the codes, as the
+// layout kernel makes them.  The hash is a sum of the codes times odd keys modulo 2^64: one changed code always shows, other
+// changes go unseen once in about 2^64.  Price (4096 x 4096, one scale per row with a clamp, 12 weights in turn): 6.1 -> 8.6 us for
+one token, 10.8 -> 13.0 for 16.  Comparing every unit with a copy of its codes cost more (11.6, 12.9), and so did hashing inside
+the loop over the units, from registers (11.0) or through cp.async (8.8, 13.0): the loop has no registers to spare, which is
+also why the second time round is a copy of it.
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "e8_fast.cuh"
@@ -114,13 +126,12 @@ __device__ __forceinline__ uint2 code_bytes_of(const uint2* table, uint32_t code
     return make_uint2(t0.x + 4u * t1.x + shift, t0.y + 4u * t1.y + shift);
 }
 
-__global__ void __launch_bounds__(256)
-k_vlut_layout(const uint32_t* __restrict__ codes, int n_out, int kb, int units, int64_t tiles, const uint2* __restrict__ table, uint4* __restrict__ out) {
-    const int64_t tile = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (tile >= tiles) return;
+struct TileWords {
+    uint4 lo, hi;
+};
+// The eight words of this lane from the codes; the whole warp calls it.
+__device__ __forceinline__ TileWords tile_words(const uint32_t* __restrict__ codes, int n_out, int kb, int64_t group, int unit, const uint2* __restrict__ table) {
     const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
-    const int64_t group = tile / units;
-    const int unit = (int)(tile - group * units);
     uint2 b[2][2];  // [row g, g + 8][block 2c, 2c + 1]
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -139,13 +150,54 @@ k_vlut_layout(const uint32_t* __restrict__ codes, int n_out, int kb, int units, 
         const uint32_t hx = __shfl_sync(0xffffffffu, b[1][k & 1].x, src), hy = __shfl_sync(0xffffffffu, b[1][k & 1].y, src);
         w[k] = __byte_perm(c < 2 ? gx : gy, c < 2 ? hx : hy, c & 1 ? 0x7632 : 0x5410);
     }
-    out[tile * 64 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
-    out[tile * 64 + 32 + lane] = make_uint4(w[4], w[5], w[6], w[7]);
+    return {make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7])};
+}
+// The hash takes the codes of a group of 16 rows as the one array that they are, in parts of 128 codes (four per lane), one part
+// per unit, so that the reads are coalesced.  A lane's four codes, zero beyond the array; WIDE: it is 16-byte aligned.
+template <bool WIDE>
+__device__ __forceinline__ uint4 group_codes(const uint32_t* __restrict__ codes, int n_out, int kb, int64_t group, int part) {
+    const int64_t at = (int64_t)part * 128 + 4 * (threadIdx.x & 31);
+    const int64_t rows = n_out - group * 16 < 16 ? n_out - group * 16 : 16, left = rows * kb - at;
+    const uint32_t* p = codes + group * 16 * kb + at;
+    if (WIDE && left >= 4) return __ldcs(reinterpret_cast<const uint4*>(p));
+    return make_uint4(left > 0 ? __ldcs(p) : 0u, left > 1 ? __ldcs(p + 1) : 0u, left > 2 ? __ldcs(p + 2) : 0u, left > 3 ? __ldcs(p + 3) : 0u);
+}
+__device__ __forceinline__ unsigned long long hash_codes(const uint4& c, int part) {
+    const unsigned long long x = (unsigned long long)((uint32_t)part * 32u + (threadIdx.x & 31)) * 0x9e3779b97f4a7c15ull;
+    const unsigned long long key = ((x ^ (x >> 32)) * 0xd1b54a32d192ed03ull) | 1ull;
+    return key * ((unsigned long long)c.x * 0x85ebca6bu + (unsigned long long)c.y * 0xc2b2ae35u + (unsigned long long)c.z * 0x27d4eb2fu + (unsigned long long)c.w * 0x165667b1u);
+}
+// Hashes are added in two halves, each modulo 2^32.
+__device__ __forceinline__ void add_hash(uint2& sum, unsigned long long h) {
+    sum.x += (uint32_t)h;
+    sum.y += (uint32_t)(h >> 32);
+}
+__device__ __forceinline__ uint2 warp_sum(uint2 h) { return make_uint2(__reduce_add_sync(0xffffffffu, h.x), __reduce_add_sync(0xffffffffu, h.y)); }
+constexpr int kHashClasses = 16;  // the most warps that share a row group
+
+__global__ void __launch_bounds__(256)
+k_vlut_layout(const uint32_t* __restrict__ codes, int n_out, int kb, int units, int64_t tiles, const uint2* __restrict__ table, uint4* __restrict__ out) {
+    const int64_t tile = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (tile >= tiles) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t group = tile / units;
+    const int unit = (int)(tile - group * units);
+    const TileWords w = tile_words(codes, n_out, kb, group, unit, table);
+    out[tile * 64 + lane] = w.lo;
+    out[tile * 64 + 32 + lane] = w.hi;
+    uint2 h = make_uint2(0u, 0u);
+    add_hash(h, hash_codes(group_codes<false>(codes, n_out, kb, group, unit), unit));
+    h = warp_sum(h);
+    if (lane < 2) atomicAdd(reinterpret_cast<uint32_t*>(out + tiles * 64) + 2 * (group * kHashClasses + unit % kHashClasses) + lane, lane ? h.y : h.x);
 }
 
 // ---------------------------------------------------------------------------------------------
 struct Product {
     const uint4* w;
+    const uint2* hash;
+    const uint32_t* codes;  // null: the caller vouches for the layout
+    int wide_codes;
+    const uint2* table;
     const float* beta;
     int rows_per_scale;   // rows kernel: rows that share a scale
     e8::TileDiv td;       // blocks kernel: block index -> scale
@@ -158,11 +210,31 @@ struct Product {
     Targets out;
 };
 
+// Whether this warp's parts of the codes are others than those the layout was made from.
+template <bool WIDE>
+__device__ __forceinline__ bool codes_changed(const Product& a, int64_t group, int first, int kw) {
+    uint2 sum = make_uint2(0u, 0u);
+    if ((threadIdx.x & 31) == 0)
+        for (int k = first; k < kHashClasses; k += kw) {
+            const uint2 h = __ldg(a.hash + group * kHashClasses + k);
+            sum.x -= h.x;
+            sum.y -= h.y;
+        }
+    for (int u = first; u < a.units; u += 4 * kw) {
+        uint4 c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] = u + k * kw < a.units ? group_codes<WIDE>(a.codes, a.n_out, a.kb, group, u + k * kw) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) add_hash(sum, hash_codes(c[k], u + k * kw));
+    }
+    sum = warp_sum(sum);
+    return (sum.x | sum.y) != 0u;
+}
+
 // Adds the KW partial tiles of every row group of this CTA in a fixed order and stores the results.
 template <int NT, int WARPS>
 __device__ __forceinline__ void reduce_and_store(const float (*part)[16][8 * NT + 1], const Product& a, int t0) {
     const int rw = WARPS >> a.kw_log2, kw = 1 << a.kw_log2;
-    __syncthreads();
     for (int e = threadIdx.x; e < rw * 16 * 8 * NT; e += WARPS * 32) {
         const int r = e & 15, t = (e >> 4) & (8 * NT - 1), group = (e >> 4) / (8 * NT);  // consecutive threads: consecutive rows of one token
         const int row = (blockIdx.x * rw + group) * 16 + r;
@@ -196,8 +268,12 @@ __device__ __forceinline__ void load_matrices(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
+// CTAs per SM of bf16 tokens: what the loop over the layout needs; the loop over the codes spills instead.
+template <int NT, int P, int WARPS>
+constexpr int kProductCtas = P == 3 ? (NT == 1 ? 2 : 1) : (WARPS == 16 ? 2 : (NT == 1 ? 4 : 3));
+
 template <int NT, int P, bool CLIP, int SCALE, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
+__global__ void __launch_bounds__(WARPS * 32, kProductCtas<NT, P, WARPS>)
 k_product(const __grid_constant__ Product a) {
     typedef WarpSmem<NT, P, SCALE> Smem;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -213,10 +289,13 @@ k_product(const __grid_constant__ Product a) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[n][i] = sign_acc[n][i] = 0.0f;
     float row_scale[2] = {0.5f, 0.5f};
-    if (group * 16 < a.n_out) {
+    bool changed = false;
+    // This warp's units; DECODE: with words from the codes instead of the layout.
+    auto run_units = [&](auto from_codes) {
+        constexpr bool DECODE = decltype(from_codes)::value;
         const uint4* wp = a.w + ((int64_t)group * a.units + first) * 64 + lane;
         uint4 next[2];
-        if (first < a.units) { next[0] = __ldcs(wp); next[1] = __ldcs(wp + 32); }
+        if (!DECODE && first < a.units) { next[0] = __ldcs(wp); next[1] = __ldcs(wp + 32); }
 
         // Activations of unit u.  bf16: asynchronous 16-byte copies, eight lanes per token; float32: through registers (8
         // floats per lane and step), split into three planes.  Tokens beyond T are not written (their columns of the result
@@ -278,10 +357,15 @@ k_product(const __grid_constant__ Product a) {
         bool bind = CLIP && SCALE == kPerRow && __any_sync(0xffffffffu, kMaxTwice * fmaxf(fabsf(row_scale[0]), fabsf(row_scale[1])) > a.clip);
         int buffer = 0;
         for (int u = first; u < a.units; u += kw) {
+            if (DECODE) {
+                const TileWords t = tile_words(a.codes, a.n_out, a.kb, group, u, a.table);
+                next[0] = t.lo;
+                next[1] = t.hi;
+            }
             const uint32_t w[8] = {next[0].x, next[0].y, next[0].z, next[0].w, next[1].x, next[1].y, next[1].z, next[1].w};
             const bool more = u + kw < a.units;
             wp += 64 * kw;
-            if (more) { next[0] = __ldcs(wp); next[1] = __ldcs(wp + 32); }
+            if (!DECODE && more) { next[0] = __ldcs(wp); next[1] = __ldcs(wp + 32); }
             if constexpr (P == 3) {
 #pragma unroll
                 for (int i = 0; i < STEPS; ++i) {
@@ -382,19 +466,32 @@ k_product(const __grid_constant__ Product a) {
             __syncwarp();  // the next unit overwrites what this one read
             buffer ^= 1;
         }
+    };
+    if (group * 16 < a.n_out) {
+        if (a.codes) changed = a.wide_codes ? codes_changed<true>(a, group, first, kw) : codes_changed<false>(a, group, first, kw);
+        run_units(std::false_type());
     }
     // accumulator layout: [0], [1] = (row g, tokens 2c, 2c + 1); [2], [3] = (row g + 8, same tokens)
+    auto put_part = [&]() {
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float v = acc[n][i];
-            if (SCALE == kPerRow) {
-                v *= row_scale[i >> 1];
-                if (CLIP) v = __fmaf_rn(sign_acc[n][i], copysignf(a.clip, row_scale[i >> 1]), v);
+            for (int i = 0; i < 4; ++i) {
+                float v = acc[n][i];
+                if (SCALE == kPerRow) {
+                    v *= row_scale[i >> 1];
+                    if (CLIP) v = __fmaf_rn(sign_acc[n][i], copysignf(a.clip, row_scale[i >> 1]), v);
+                }
+                part[warp][g + 8 * (i >> 1)][8 * n + 2 * c + (i & 1)] = v;
+                acc[n][i] = sign_acc[n][i] = 0.0f;
             }
-            part[warp][g + 8 * (i >> 1)][8 * n + 2 * c + (i & 1)] = v;
-        }
+    };
+    put_part();
+    if (__syncthreads_or(changed)) {
+        if (group * 16 < a.n_out) run_units(std::true_type());
+        put_part();
+        __syncthreads();
+    }
     reduce_and_store<NT, WARPS>(part, a, t0);
 }
 
@@ -439,7 +536,7 @@ int launch_tokens(const Product& a, int scale, cudaStream_t st) {
 
 extern "C" int64_t coset_e8_vlut_layout_bytes(int n_out, int n_in) {
     if (n_out < 0 || n_in < 0) return 0;
-    return (((int64_t)n_out + 15) / 16) * (((int64_t)n_in + 63) / 64) * 1024;
+    return (((int64_t)n_out + 15) / 16) * (((int64_t)n_in + 63) / 64) * 1024 + (((int64_t)n_out + 15) / 16) * kHashClasses * 8;
 }
 
 extern "C" int coset_e8_vlut_layout(const void* codes, int n_out, int n_in, void* layout, void* stream) {
@@ -453,13 +550,14 @@ extern "C" int coset_e8_vlut_layout(const void* codes, int n_out, int n_in, void
     const int kb = n_in / 8, units = (kb + 7) / 8;
     const int64_t tiles = (((int64_t)n_out + 15) / 16) * units;
     const unsigned grid = (unsigned)((tiles + 7) / 8);
+    const int64_t groups = tiles / units;
+    if (int e = check_cuda(cudaMemsetAsync((uint8_t*)layout + tiles * 1024, 0, groups * kHashClasses * 8, st), "e8_vlut_layout")) return e;
     k_vlut_layout<<<grid, 256, 0, st>>>((const uint32_t*)codes, n_out, kb, units, tiles, table, (uint4*)layout);
     return check_launch("e8_vlut_layout");
 }
 
-extern "C" int coset_e8_vlut_product(const void* layout, const float* beta, int64_t blocks_per_tile, int n_out, int n_in, const void* x, int x_dtype,
-                                     int64_t ldx, int T, const float* bias, void* const* y_targets, int n_targets, int y_dtype, int64_t ldy,
-                                     float clip, void* stream) {
+static int vlut_product(const void* codes, const void* layout, const float* beta, int64_t blocks_per_tile, int n_out, int n_in, const void* x, int x_dtype,
+                        int64_t ldx, int T, const float* bias, void* const* y_targets, int n_targets, int y_dtype, int64_t ldy, float clip, void* stream) {
     if (n_out < 0 || n_in < 0 || T < 0 || (n_in % 8) != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
     if (n_targets < 1 || n_targets > kMaxTargets || !y_targets) return fail(COSET_E_BADARG, "need 1..16 result buffers");
     if (n_out == 0 || T == 0) return 0;
@@ -469,13 +567,19 @@ extern "C" int coset_e8_vlut_product(const void* layout, const float* beta, int6
     if (ldx < n_in || ldy < n_out) return fail(COSET_E_BADARG, "leading dimension too small");
     if (!aligned(x, 16) || ((ldx * (x_dtype == COSET_DTYPE_F32 ? 4 : 2)) % 16) != 0 || !aligned(layout, 16))
         return fail(COSET_E_ALIGN, "the layout and the rows of x must be 16-byte aligned");
+    if (!aligned(codes, 4)) return fail(COSET_E_ALIGN, "codes must be 4-byte aligned");
     if (beta && blocks_per_tile < 1) return fail(COSET_E_BADARG, "blocks_per_tile must be >= 1");
     if (!(clip == clip)) return fail(COSET_E_BADARG, "clip is not a number");
     const int kb = n_in / 8;
     Product a = {};
+    a.units = (kb + 7) / 8;
     a.w = (const uint4*)layout;
+    a.hash = (const uint2*)((const uint8_t*)layout + (((int64_t)n_out + 15) / 16) * a.units * 1024);
+    a.codes = (const uint32_t*)codes;
+    a.wide_codes = aligned(codes, 16);
+    if (codes && !(a.table = residual_table_q4((cudaStream_t)stream))) return COSET_E_STATE;
     a.beta = beta;
-    a.n_out = n_out; a.kb = kb; a.units = (kb + 7) / 8; a.T = T;
+    a.n_out = n_out; a.kb = kb; a.T = T;
     a.x = x; a.ldx = ldx; a.ldy = ldy; a.bias = bias; a.clip = clip > 0.0f ? clip : 0.0f;
     for (int k = 0; k < n_targets; ++k) {
         if (!y_targets[k]) return fail(COSET_E_BADARG, "result buffer %d is null", k);
@@ -489,4 +593,17 @@ extern "C" int coset_e8_vlut_product(const void* layout, const float* beta, int6
     cudaStream_t st = (cudaStream_t)stream;
     const int scale_kind = rows ? kPerRow : (one ? kPerBlock : kPerTile);
     return x_dtype == COSET_DTYPE_BF16 ? launch_tokens<1>(a, scale_kind, st) : launch_tokens<3>(a, scale_kind, st);
+}
+
+extern "C" int coset_e8_vlut_product(const void* layout, const float* beta, int64_t blocks_per_tile, int n_out, int n_in, const void* x, int x_dtype,
+                                     int64_t ldx, int T, const float* bias, void* const* y_targets, int n_targets, int y_dtype, int64_t ldy,
+                                     float clip, void* stream) {
+    return vlut_product(nullptr, layout, beta, blocks_per_tile, n_out, n_in, x, x_dtype, ldx, T, bias, y_targets, n_targets, y_dtype, ldy, clip, stream);
+}
+
+extern "C" int coset_e8_vlut_product_checked(const void* codes, const void* layout, const float* beta, int64_t blocks_per_tile, int n_out, int n_in,
+                                             const void* x, int x_dtype, int64_t ldx, int T, const float* bias, void* const* y_targets, int n_targets,
+                                             int y_dtype, int64_t ldy, float clip, void* stream) {
+    if (!codes && n_out > 0 && T > 0 && n_in > 0) return fail(COSET_E_BADARG, "null pointer");
+    return vlut_product(codes, layout, beta, blocks_per_tile, n_out, n_in, x, x_dtype, ldx, T, bias, y_targets, n_targets, y_dtype, ldy, clip, stream);
 }

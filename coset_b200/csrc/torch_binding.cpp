@@ -294,26 +294,46 @@ PyObject* vlut_layout(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// The product from a layout; `codes` undefined: the layout is trusted.
+Tensor layout_product(const Tensor& x, const Tensor& codes, const Tensor& layout, int64_t n_out, int64_t n_in, const Tensor& beta_arg, int64_t bpt,
+                      const Tensor& bias_arg, double clip, int y_code) {
+    TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in, "x must be [T, ", n_in, "], got ", x.sizes());
+    TORCH_CHECK_VALUE(layout.device() == x.device(), "the weight is on ", layout.device(), ", x on ", x.device());
+    TORCH_CHECK_VALUE((int64_t)layout.nbytes() == coset_e8_vlut_layout_bytes((int)n_out, (int)n_in), "the layout is not one of a [", n_out, ", ", n_in, "] weight");
+    c10::cuda::CUDAGuard guard(x.device());
+    c10::SmallVector<int64_t, 6> shape;
+    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
+    const Tensor beta = as_f32(beta_arg), bias = as_f32(bias_arg);
+    const int x_code = dtype_code(x2, "x");
+    Tensor y = empty(shape, scalar_type(y_code), x);
+    void* target = data(y);
+    if (target && codes.defined())
+        check_rc(coset_e8_vlut_product_checked(data(codes), data(layout), fdata(beta), bpt, (int)n_out, (int)n_in, data(x2), x_code, n_in,
+                                               (int)x2.size(0), fdata(bias), &target, 1, y_code, n_out, (float)clip, stream_of(x)), "coset_e8_vlut_product_checked");
+    else if (target)
+        check_rc(coset_e8_vlut_product(data(layout), fdata(beta), bpt, (int)n_out, (int)n_in, data(x2), x_code, n_in,
+                                       (int)x2.size(0), fdata(bias), &target, 1, y_code, n_out, (float)clip, stream_of(x)), "coset_e8_vlut_product");
+    return y;
+}
+
 // vlut_product(x [..., n_in], layout, n_out, n_in, beta or None, blocks_per_tile, bias or None, clip, out_dtype_code)
 PyObject* vlut_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     nargs_are(n, 9);
-    const Tensor &x = cuda_arg(a[0], "x"), &layout = tensor_arg(a[1], "layout");
-    const int64_t n_out = int_arg(a[2]), n_in = int_arg(a[3]);
-    TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in, "x must be [T, ", n_in, "], got ", x.sizes());
-    TORCH_CHECK_VALUE(layout.device() == x.device(), "the weight is on ", layout.device(), ", x on ", x.device());
-    c10::cuda::CUDAGuard guard(x.device());
-    c10::SmallVector<int64_t, 6> shape;
-    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
-    const Tensor beta = as_f32(optional_arg(a[4], "beta")), bias = as_f32(optional_arg(a[6], "bias"));
-    const int y_code = (int)int_arg(a[8]), x_code = dtype_code(x2, "x");
-    Tensor y = empty(shape, scalar_type(y_code), x);
-    void* target = data(y);
-    if (target)
-        check_rc(coset_e8_vlut_product(data(layout), fdata(beta), int_arg(a[5]), (int)n_out, (int)n_in, data(x2), x_code, n_in,
-                                       (int)x2.size(0), fdata(bias), &target, 1, y_code, n_out, (float)float_arg(a[7]), stream_of(x)),
-                 "coset_e8_vlut_product");
-    return THPVariable_Wrap(y);
+    return THPVariable_Wrap(layout_product(cuda_arg(a[0], "x"), Tensor(), tensor_arg(a[1], "layout"), int_arg(a[2]), int_arg(a[3]), optional_arg(a[4], "beta"),
+                                           int_arg(a[5]), optional_arg(a[6], "bias"), float_arg(a[7]), (int)int_arg(a[8])));
+    END_HANDLE_TH_ERRORS
+}
+
+// vlut_product_checked(x [..., n_in], codes, layout, beta or None, blocks_per_tile, bias or None, clip, out_dtype_code)
+PyObject* vlut_product_checked(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 8);
+    const Tensor &x = cuda_arg(a[0], "x"), &codes = cuda_arg(a[1], "codes");
+    check_codes(codes);
+    TORCH_CHECK_VALUE(codes.device() == x.device(), "the weight is on ", codes.device(), ", x on ", x.device());
+    return THPVariable_Wrap(layout_product(x, codes, tensor_arg(a[2], "layout"), codes.size(0), codes.size(1) * 8, optional_arg(a[3], "beta"),
+                                           int_arg(a[4]), optional_arg(a[5], "bias"), float_arg(a[6]), (int)int_arg(a[7])));
     END_HANDLE_TH_ERRORS
 }
 
@@ -501,8 +521,8 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define COSET_METHOD(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     COSET_METHOD(encode_packed), COSET_METHOD(decode_packed), COSET_METHOD(encode_digits), COSET_METHOD(decode_digits), COSET_METHOD(quantize),
-    COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(vlut_layout), COSET_METHOD(vlut_product), COSET_METHOD(decode_gemm),
-    COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
+    COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(vlut_layout), COSET_METHOD(vlut_product), COSET_METHOD(vlut_product_checked),
+    COSET_METHOD(decode_gemm), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_coset_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -4,8 +4,9 @@ The weight of a trained HNLQLinearQAT layer is exported as packed q=4, M=2 codes
 weights) plus the scales beta, and applied from the codes:
 
   * few tokens  (T <= small_t_max): by default a decode-ready copy of the codes, one byte per weight in tensor-core order
-    (coset_e8_vlut_layout, kept like the dense copy below), and coset_e8_vlut_product; `large_t_path="tcgen05"` keeps no
-    copy of any kind and reads the code stream (coset_e8_vlut_gemv);
+    (coset_e8_vlut_layout), and coset_e8_vlut_product_checked, which compares the copy with the codes as it reads it, so that
+    the result is that of the codes however they were written; `large_t_path="tcgen05"` keeps no copy of any kind and
+    reads the code stream (coset_e8_vlut_gemv);
   * many tokens (from 2048 by default): the weight is decoded into a transient bf16 buffer and multiplied by
     this library's tcgen05 GEMM (coset_e8_decode_gemm); nothing dense survives the call;
   * in between, by default, the library GEMM on a cached dense bf16 copy (`large_t_path` chooses).
@@ -95,8 +96,9 @@ class E8CodeLinear(nn.Module):
     cta_group::2 GEMM from 1024 tokens, the single-launch fused kernel below; "cublas" -- a cached dense bf16 copy
     and the library GEMM; "auto" (default) -- the own kernels from PAIR_GEMM_MIN_T tokens, the library path for
     the tokens in between, where decoding the whole weight per call costs more than the product itself.
-    Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 5.5-10 us for 1-16
-    tokens and a 4096 x 4096 weight; "tcgen05" keeps nothing and stays on the code-domain kernels (9.7-23 us).
+    Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 9-13 us for 1-16
+    tokens and a 4096 x 4096 weight; the kernel checks the copy against the codes in every call.  "tcgen05" keeps nothing and
+    stays on the code-domain kernels (9.7-23 us).
     A call under graph capture reads the codes themselves, so that a replay follows writes to them.
     small_t_max defaults to 16 ("auto", "cublas") or 48 ("tcgen05"): measured on a 4096 x 4096 layer the
     code-domain kernels take 9.7 / 23 / 44 / 86 us for 1 / 16 / 32 / 64 tokens (they re-read and re-decode the
@@ -253,8 +255,8 @@ class E8CodeLinear(nn.Module):
         if T <= self.small_t_max:
             layout = self._product_layout() if self.large_t_path != "tcgen05" and n_in else None
             if layout is not None:
-                return _lib.native().vlut_product(x, layout, self.out_features, n_in, buf["beta"], self.blocks_per_tile, buf["bias"],
-                                                  self.weight_clip_value, _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
+                return _lib.native().vlut_product_checked(x, buf["codes"], layout, buf["beta"], self.blocks_per_tile, buf["bias"],
+                                                          self.weight_clip_value, _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
             return _lib.native().vlut_linear(x, buf["codes"], buf["beta"], self.blocks_per_tile, buf["bias"], self.weight_clip_value,
                                              _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
         if dtype is torch.bfloat16:
@@ -361,8 +363,8 @@ class ColumnParallelE8CodeLinear(nn.Module):
             bias = _lib.ptr(bias32) if bias32 is not None else None
             layout = loc._product_layout() if loc.large_t_path != "tcgen05" and loc.in_features else None
             if layout is not None:  # the kernel of the unsharded layer, so that the results are the same bits
-                rc = _lib.lib().coset_e8_vlut_product(
-                    _lib.ptr(layout), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
+                rc = _lib.lib().coset_e8_vlut_product_checked(
+                    _lib.ptr(loc.codes), _lib.ptr(layout), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,
                     _lib.ptr(x2), _lib.dtype_code(x2, "x"), x2.stride(0), T, bias, ctypes.cast(targets, ctypes.c_void_p), self.world,
                     _lib.DTYPE_F32, self.out_features, float(loc.weight_clip_value), _lib.stream())
             else:

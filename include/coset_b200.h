@@ -269,17 +269,22 @@ int coset_e8_vlut_gemv_scatter(const void* codes, const float* beta, int64_t blo
 
 /*
  * The same product from a decode-ready copy of the weight: 2 x_hat + 64 as one byte per weight, in the order the
- * tensor cores want it (8 bytes per block beside its 4-byte code), for callers that multiply the same weight many
- * times.  coset_e8_vlut_layout writes it once (layout: coset_e8_vlut_layout_bytes(n_out, n_in) bytes, 16-byte aligned);
- * coset_e8_vlut_product multiplies: y = x * clamp(decode / beta)^T + bias, x float32 or bf16 with 16-byte aligned
- * rows, one or more result buffers of y_dtype that all receive every result (see coset_e8_vlut_gemv_scatter).
- * All products are exact; sums are float32.  A row's result does not depend on n_out.
+ * tensor cores want it (8 bytes per block beside its 4-byte code), and a hash of the codes, for callers that
+ * multiply the same weight many times.  coset_e8_vlut_layout writes it once (layout: coset_e8_vlut_layout_bytes(n_out, n_in)
+ * bytes, 16-byte aligned); the products multiply: y = x * clamp(decode / beta)^T + bias, x float32 or bf16 with
+ * 16-byte aligned rows, one or more result buffers of y_dtype that all receive every result (see
+ * coset_e8_vlut_gemv_scatter).  _checked reads the codes too and multiplies by what they hold at the call, whatever has been
+ * written to them since the layout was made; the other form trusts the layout.  All products are exact; sums are float32.
+ * A row's result does not depend on n_out.
  */
 int64_t coset_e8_vlut_layout_bytes(int n_out, int n_in);
 int coset_e8_vlut_layout(const void* codes, int n_out, int n_in, void* layout, void* stream);
 int coset_e8_vlut_product(const void* layout, const float* beta, int64_t blocks_per_tile, int n_out, int n_in,
                           const void* x, int x_dtype, int64_t ldx, int T, const float* bias, void* const* y_targets,
                           int n_targets, int y_dtype, int64_t ldy, float clip, void* stream);
+int coset_e8_vlut_product_checked(const void* codes, const void* layout, const float* beta, int64_t blocks_per_tile,
+                                  int n_out, int n_in, const void* x, int x_dtype, int64_t ldx, int T, const float* bias,
+                                  void* const* y_targets, int n_targets, int y_dtype, int64_t ldy, float clip, void* stream);
 
 /*
  * Quantisation statistics of the q=4, M=2 codec over a tensor (one pass, deterministic):

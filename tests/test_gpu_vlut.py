@@ -374,3 +374,57 @@ def test_few_tokens_refuse_other_types_at_any_count():
     for T in (0, 3):
         with pytest.raises(TypeError):
             lin(x[:T].half())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n_out,n_in", [(1, 8), (17, 72), (200, 1032), (64, 4096)])
+@pytest.mark.parametrize("T,clip,row", [(1, 0.0, True), (3, 0.05, False), (16, 0.05, True)])
+def test_few_tokens_follow_writes_that_no_version_shows(n_out, n_in, T, clip, row, dtype):
+    """All codes, one code and the last code written through `.data`, the codes written by a replayed graph and by the encoder's
+    `out`: the product is that of the codes, to the bit that a fresh layer returns, and of the old codes once they are back."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_encode_packed
+    from coset_b200.vlut import E8CodeLinear
+    g = torch.Generator(device="cuda").manual_seed(n_out + T)
+    kb = n_in // 8
+    bpt = kb if row else 1
+    beta = 25.0 * (0.75 + 0.5 * torch.rand(n_out * kb // bpt, device="cuda", generator=g))
+    weights = [torch.randn(n_out * kb, 8, device="cuda", generator=g) * s for s in (0.02, 0.03)]
+    encode = lambda w, **kw: e8_encode_packed(w, scale=beta, scale_mode=_lib.SCALE_MUL_TILE, blocks_per_tile=bpt, **kw)
+    old, new = (encode(w).view(torch.int32).view(n_out, kb) for w in weights)
+    x = torch.randn(T, n_in, device="cuda", generator=g).to(dtype)
+    fresh = lambda codes: E8CodeLinear(codes.clone(), beta, bpt, None, weight_clip_value=clip)(x)
+    layer = E8CodeLinear(old.clone(), beta, bpt, None, weight_clip_value=clip)
+    assert torch.equal(layer(x), fresh(old))
+    version = layer.codes._version
+    for what in ("all", "one", "last"):
+        codes = old.clone()
+        if what == "all":
+            codes.copy_(new)
+        else:
+            at = (n_out // 2, kb // 2) if what == "one" else (n_out - 1, kb - 1)
+            codes[at] = codes[at] ^ 0x1234
+        layer.codes.data.copy_(codes)
+        assert layer.codes._version == version
+        assert torch.equal(layer(x), fresh(codes)), what
+    layer.codes.data.copy_(old)
+    assert torch.equal(layer(x), fresh(old))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer.codes.copy_(new)
+    assert torch.equal(layer(x), fresh(old))
+    graph.replay()
+    assert torch.equal(layer(x), fresh(new))
+    encode(weights[0], out=layer.codes)
+    assert torch.equal(layer(x), fresh(old))
+
+
+@pytest.mark.parametrize("n_out,n_in,T", [(17, 72, 1), (64, 4096, 3), (16, 8192, 16)])
+def test_few_tokens_read_the_layout_while_the_codes_are_those_it_was_made_from(n_out, n_in, T):
+    """A layout whose bytes are zeroed behind the layer's back (its hash is not) gives a product of zeros: the units are taken from
+    the layout and not made anew."""
+    layer, _ = _kept_copy_layer(n_out, n_in)
+    x = torch.randn(T, n_in, device="cuda").to(torch.bfloat16)
+    assert bool((layer(x) != 0).any())
+    layer._product_layout()[:((n_out + 15) // 16) * ((n_in + 63) // 64) * 1024] = 64
+    assert not bool((layer(x) != 0).any())
