@@ -30,9 +30,9 @@
 // bytes, hashes them, and where the hash is not the kept one does its units again with words made from the codes, as the
 // layout kernel makes them.  The hash is a sum of the codes times odd keys modulo 2^64: one changed code always shows, other
 // changes go unseen once in about 2^64.  Price (4096 x 4096, one scale per row with a clamp, 12 weights in turn): 6.1 -> 8.6 us for
-one token, 10.8 -> 13.0 for 16.  Comparing every unit with a copy of its codes cost more (11.6, 12.9), and so did hashing inside
-the loop over the units, from registers (11.0) or through cp.async (8.8, 13.0): the loop has no registers to spare, which is
-also why the second time round is a copy of it.
+// one token, 10.8 -> 13.0 for 16.  Comparing every unit with a copy of its codes cost more (11.6, 12.9), and so did hashing inside
+// the loop over the units, from registers (11.0) or through cp.async (8.8, 13.0): the loop has no registers to spare, which is
+// also why the second time round is a copy of it.
 #include <cuda_bf16.h>
 
 #include <type_traits>
