@@ -7,7 +7,9 @@
 // bf16x2 subtraction leaves t exactly, and mma.sync multiplies it UNSCALED with the activations; the scale is applied to
 // the float32 inner products -- once per row when a scale covers whole rows, once per block otherwise (m16n8k8 then
 // spans exactly one block).  Every product is exact, nothing is rounded to bf16 but the result.
-//   * float32 activations are the exact sum of three bf16 terms and take three products;
+//   * float32 activations are the exact sum of three bf16 terms and take three products, summed so that the error against 64 bits
+//     is no larger than that of a chain of fused multiply-adds (8e-8 of the result at any K; one accumulator for all three
+//     gave 2.2e-7; time for 4096 x 4096 float32, one scale per row with a clamp: 11.5 -> 12.5 us for one token, 24.8 -> 26.3 for 16);
 //   * a clamp that can bind (|t| > clip 2 beta for some possible t) is a second product of the clamped signs, so the
 //     clamped weights are exact too.
 // Bound: 1 byte per weight (+ 4 per 8 weights of per-block scales), 2.6-3.9 us of HBM traffic for 4096 x 4096.  Measured
@@ -101,10 +103,19 @@ __device__ __forceinline__ uint32_t clamp_limit(float clip, float scale) {
     const __nv_bfloat162 h = __float2bfloat162_rn(fminf(floorf(__fdividef(clip, fabsf(scale))), 64.0f));
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// 1 / v: rounded to nearest for float32 tokens, to about an ulp for bf16 ones
+template <bool EXACT>
 __device__ __forceinline__ float reciprocal(float v) {
+    if (EXACT) return __frcp_rn(v);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
+}
+// s += v, and what the rounded sum lacks to e (Knuth's two-sum)
+__device__ __forceinline__ void add_exactly(float& s, float& e, float v) {
+    const float t = s + v, z = t - s;
+    e += (s - (t - z)) + (v - z);
+    s = t;
 }
 // The exact three-term bf16 split of two floats, packed: out[p] = (p-th term of a, p-th term of b).
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&out)[3]) {
@@ -283,11 +294,11 @@ k_product(const __grid_constant__ Product a) {
     const int kw = 1 << a.kw_log2, rw = WARPS >> a.kw_log2, first = warp & (kw - 1), t0 = blockIdx.y * (8 * NT);
     const int group = blockIdx.x * rw + (warp >> a.kw_log2);
     const int tokens = a.T - t0 < 8 * NT ? a.T - t0 : 8 * NT;
-    float acc[NT][4], sign_acc[NT][4];
+    float acc[NT][4], sign_acc[NT][4], lost[NT][4];  // lost: what rounding took from acc, float32 tokens only
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] = sign_acc[n][i] = 0.0f;
+        for (int i = 0; i < 4; ++i) acc[n][i] = sign_acc[n][i] = lost[n][i] = 0.0f;
     float row_scale[2] = {0.5f, 0.5f};
     bool changed = false;
     // This warp's units; DECODE: with words from the codes instead of the layout.
@@ -351,7 +362,7 @@ k_product(const __grid_constant__ Product a) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int row = group * 16 + g + 8 * h;
-                row_scale[h] = 0.5f * reciprocal(__ldg(a.beta + (row < a.n_out ? row : a.n_out - 1) / a.rows_per_scale));
+                row_scale[h] = 0.5f * reciprocal<P == 3>(__ldg(a.beta + (row < a.n_out ? row : a.n_out - 1) / a.rows_per_scale));
             }
         }
         bool bind = CLIP && SCALE == kPerRow && __any_sync(0xffffffffu, kMaxTwice * fmaxf(fabsf(row_scale[0]), fabsf(row_scale[1])) > a.clip);
@@ -381,7 +392,7 @@ k_product(const __grid_constant__ Product a) {
                 }
             }
             if (SCALE != kPerRow) {
-                const float4 r = make_float4(reciprocal(2.0f * next_scale.x), reciprocal(2.0f * next_scale.y), reciprocal(2.0f * next_scale.z), reciprocal(2.0f * next_scale.w));
+                const float4 r = make_float4(reciprocal<P == 3>(2.0f * next_scale.x), reciprocal<P == 3>(2.0f * next_scale.y), reciprocal<P == 3>(2.0f * next_scale.z), reciprocal<P == 3>(2.0f * next_scale.w));
                 *reinterpret_cast<float4*>(mem.scale + (lane & 1) * 64 + (lane >> 1) * 4) = r;
                 if (CLIP) bind = __any_sync(0xffffffffu, kMaxTwice * fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w))) > a.clip);
                 if (more) request_scales(u + kw);
@@ -392,7 +403,14 @@ k_product(const __grid_constant__ Product a) {
                 else asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
             __syncwarp();
-            float d[NT][4], ds[NT][4];
+            // float32 tokens: the products of the lower planes are summed apart and a unit's blocks before they join the others',
+            // for the tensor cores truncate where they add a small term to a large one and a long chain of additions rounds more
+            float d[NT][4], ds[NT][4], low[NT][4], low_s[NT][4], unit_acc[NT][4];
+            float(&into)[NT][4] = P == 3 ? unit_acc : acc;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) unit_acc[n][i] = 0.0f;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {  // blocks 4 half .. + 3
                 float scale[2][4];
@@ -424,11 +442,13 @@ k_product(const __grid_constant__ Product a) {
                         if (SCALE == kPerRow) {
 #pragma unroll
                             for (int p = 0; p < P; ++p) {
-                                if (b0 == 0 && p == 0) mma_16816<true>(d[n], t, b[n][p][k], b[n][p][k + 1]);
-                                else mma_16816<false>(d[n], t, b[n][p][k], b[n][p][k + 1]);
+                                float(&dp)[4] = p == 0 ? d[n] : low[n];
+                                float(&dsp)[4] = p == 0 ? ds[n] : low_s[n];
+                                if (b0 == 0 && p < 2) mma_16816<true>(dp, t, b[n][p][k], b[n][p][k + 1]);
+                                else mma_16816<false>(dp, t, b[n][p][k], b[n][p][k + 1]);
                                 if (CLIP && bind) {
-                                    if (b0 == 0 && p == 0) mma_16816<true>(ds[n], sign, b[n][p][k], b[n][p][k + 1]);
-                                    else mma_16816<false>(ds[n], sign, b[n][p][k], b[n][p][k + 1]);
+                                    if (b0 == 0 && p < 2) mma_16816<true>(dsp, sign, b[n][p][k], b[n][p][k + 1]);
+                                    else mma_16816<false>(dsp, sign, b[n][p][k], b[n][p][k + 1]);
                                 }
                             }
                         } else {
@@ -436,17 +456,25 @@ k_product(const __grid_constant__ Product a) {
                             for (int q = 0; q < 2; ++q) {
                                 const uint32_t tq[2] = {t[2 * q], t[2 * q + 1]};
                                 mma_1688<true>(d[n], tq, b[n][0][k + q]);
+                                if constexpr (P == 3) {
+                                    mma_1688<true>(low[n], tq, b[n][1][k + q]);
+                                    mma_1688<false>(low[n], tq, b[n][2][k + q]);
 #pragma unroll
-                                for (int p = 1; p < P; ++p) mma_1688<false>(d[n], tq, b[n][p][k + q]);
+                                    for (int i = 0; i < 4; ++i) d[n][i] += low[n][i];
+                                }
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) acc[n][i] = __fmaf_rn(d[n][i], scale[i >> 1][k + q], acc[n][i]);
+                                for (int i = 0; i < 4; ++i) into[n][i] = __fmaf_rn(d[n][i], scale[i >> 1][k + q], into[n][i]);
                                 if (CLIP && bind) {
                                     const uint32_t sq[2] = {sign[2 * q], sign[2 * q + 1]};
                                     mma_1688<true>(ds[n], sq, b[n][0][k + q]);
+                                    if constexpr (P == 3) {
+                                        mma_1688<true>(low_s[n], sq, b[n][1][k + q]);
+                                        mma_1688<false>(low_s[n], sq, b[n][2][k + q]);
 #pragma unroll
-                                    for (int p = 1; p < P; ++p) mma_1688<false>(ds[n], sq, b[n][p][k + q]);
+                                        for (int i = 0; i < 4; ++i) ds[n][i] += low_s[n][i];
+                                    }
 #pragma unroll
-                                    for (int i = 0; i < 4; ++i) acc[n][i] = __fmaf_rn(ds[n][i], copysignf(a.clip, scale[i >> 1][k + q]), acc[n][i]);
+                                    for (int i = 0; i < 4; ++i) into[n][i] = __fmaf_rn(ds[n][i], copysignf(a.clip, scale[i >> 1][k + q]), into[n][i]);
                                 }
                             }
                         }
@@ -459,9 +487,15 @@ k_product(const __grid_constant__ Product a) {
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        acc[n][i] += d[n][i];
-                        if (CLIP && bind) sign_acc[n][i] += ds[n][i];
+                        if (P == 3) add_exactly(acc[n][i], lost[n][i], d[n][i] + low[n][i]);
+                        else acc[n][i] += d[n][i];
+                        if (CLIP && bind) sign_acc[n][i] += P == 3 ? ds[n][i] + low_s[n][i] : ds[n][i];
                     }
+            } else if (P == 3) {
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) add_exactly(acc[n][i], lost[n][i], unit_acc[n][i]);
             }
             __syncwarp();  // the next unit overwrites what this one read
             buffer ^= 1;
@@ -478,12 +512,13 @@ k_product(const __grid_constant__ Product a) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float v = acc[n][i];
+                if (P == 3 && lost[n][i] == lost[n][i]) v += lost[n][i];
                 if (SCALE == kPerRow) {
                     v *= row_scale[i >> 1];
                     if (CLIP) v = __fmaf_rn(sign_acc[n][i], copysignf(a.clip, row_scale[i >> 1]), v);
                 }
                 part[warp][g + 8 * (i >> 1)][8 * n + 2 * c + (i & 1)] = v;
-                acc[n][i] = sign_acc[n][i] = 0.0f;
+                acc[n][i] = sign_acc[n][i] = lost[n][i] = 0.0f;
             }
     };
     put_part();

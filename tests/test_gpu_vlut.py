@@ -428,3 +428,23 @@ def test_few_tokens_read_the_layout_while_the_codes_are_those_it_was_made_from(n
     assert bool((layer(x) != 0).any())
     layer._product_layout()[:((n_out + 15) // 16) * ((n_in + 63) // 64) * 1024] = 64
     assert not bool((layer(x) != 0).any())
+
+
+@pytest.mark.parametrize("row,clip", [(True, 0.0), (True, 0.05), (False, 0.0), (False, 0.05)])
+@pytest.mark.parametrize("T,n_out,n_in", [(1, 320, 64), (8, 384, 256), (16, 320, 7424)])
+def test_few_float32_tokens_keep_float32_precision(T, n_out, n_in, row, clip):
+    """The root mean square of the error against 64 bits stays below 2^-23 of the results' at any K: two roundings of the scales
+    (reciprocal, product) and one of the result at 2^-24 at most each, and sums whose own error does not grow with K."""
+    from coset_b200.core.e8 import e8_decode_packed
+    layer, _ = _kept_copy_layer(n_out, n_in, seed=n_in)
+    if not row:
+        from coset_b200.vlut import E8CodeLinear
+        g = torch.Generator(device="cuda").manual_seed(T)
+        beta = 25.0 * (0.8 + 0.4 * torch.rand(n_out * n_in // 8, device="cuda", generator=g))
+        layer = E8CodeLinear(layer.codes, beta, 1, None)
+    layer.weight_clip_value = clip
+    x = torch.randn(T, n_in, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T))
+    w = e8_decode_packed(layer.codes.view(-1)).double().view(layer.beta.numel(), -1) / layer.beta.double().view(-1, 1)
+    w = w.view(n_out, n_in).clamp(-clip, clip) if clip else w.view(n_out, n_in)
+    want = x.double() @ w.T
+    assert float((layer(x).double() - want).norm() / want.norm()) < 2.0 ** -23
