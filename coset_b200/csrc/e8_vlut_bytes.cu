@@ -37,6 +37,8 @@
 // also why the second time round is a copy of it.
 #include <cuda_bf16.h>
 
+#include <math.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -210,7 +212,8 @@ struct Product {
     int wide_codes;
     const uint2* table;
     const float* beta;
-    int rows_per_scale;   // rows kernel: rows that share a scale
+    int per_row;          // one scale covers whole rows: rows_per_scale of them
+    int rows_per_scale;
     e8::TileDiv td;       // blocks kernel: block index -> scale
     int n_out, kb, units, T;
     const void* x;
@@ -242,18 +245,59 @@ __device__ __forceinline__ bool codes_changed(const Product& a, int64_t group, i
     return (sum.x | sum.y) != 0u;
 }
 
+// One result from weights that are scaled and clamped first, by a whole warp.  The kernel multiplies unscaled, so its sums can
+// overflow where the product does not, and it takes a clamp apart into two products, which turns an infinite activation or a
+// scale of zero into 0 * inf: a result that is not finite is taken from here instead.
+template <int P>
+__device__ __noinline__ float scaled_product(const Product& a, int row, int t) {
+    const int lane = threadIdx.x & 31, r = row & 15;
+    const uint8_t* tile = reinterpret_cast<const uint8_t*>(a.w) + (int64_t)(row >> 4) * a.units * 1024 + (r & 7) * 64 + (r >> 3) * 2;
+    float sum = 0.0f;
+    for (int first = 0; first < a.kb; first += 32) {
+        const int blk = first + lane;
+        if (blk < a.kb) {
+            const int64_t at = (int64_t)row * a.kb + blk;
+            uint32_t bytes[4];  // coordinates 2 c, 2 c + 1
+            if (a.codes) {
+                const uint2 b = code_bytes_of(a.table, __ldg(a.codes + at));
+                bytes[0] = b.x; bytes[1] = b.x >> 16; bytes[2] = b.y; bytes[3] = b.y >> 16;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    bytes[c] = __ldg(reinterpret_cast<const uint16_t*>(tile + (int64_t)(blk >> 3) * 1024 + ((blk >> 2) & 1) * 512 + c * 16 + (blk & 3) * 4));
+            }
+            const float scale = a.beta ? __ldg(a.beta + (a.per_row ? row / a.rows_per_scale : e8::tile_of(a.td, at))) : 1.0f;
+            const char* x = reinterpret_cast<const char*>(a.x) + ((int64_t)t * a.ldx + blk * 8) * (P == 1 ? 2 : 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float w = __fdiv_rn(0.5f * (float)((int)((bytes[i >> 1] >> (8 * (i & 1))) & 0xffu) - kByteBias), scale);
+                if (a.clip > 0.0f) w = fminf(fmaxf(w, -a.clip), a.clip);
+                sum = __fmaf_rn(w, P == 1 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i]) : reinterpret_cast<const float*>(x)[i], sum);
+            }
+        }
+        if (__any_sync(0xffffffffu, sum != sum)) return NAN;  // and nothing makes it a number again
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
 // Adds the KW partial tiles of every row group of this CTA in a fixed order and stores the results.
-template <int NT, int WARPS>
+template <int NT, int P, int WARPS>
 __device__ __forceinline__ void reduce_and_store(const float (*part)[16][8 * NT + 1], const Product& a, int t0) {
     const int rw = WARPS >> a.kw_log2, kw = 1 << a.kw_log2;
-    for (int e = threadIdx.x; e < rw * 16 * 8 * NT; e += WARPS * 32) {
+    for (int e = threadIdx.x; e < rw * 16 * 8 * NT; e += WARPS * 32) {  // the bound is a multiple of 32: whole warps
         const int r = e & 15, t = (e >> 4) & (8 * NT - 1), group = (e >> 4) / (8 * NT);  // consecutive threads: consecutive rows of one token
         const int row = (blockIdx.x * rw + group) * 16 + r;
-        if (row < a.n_out && t0 + t < a.T) {
-            float v = part[group << a.kw_log2][r][t];
-            for (int w = 1; w < kw; ++w) v += part[(group << a.kw_log2) + w][r][t];
-            store_result(a.out, (int64_t)(t0 + t) * a.ldy + row, v + (a.bias ? __ldg(a.bias + row) : 0.0f));
+        const bool mine = row < a.n_out && t0 + t < a.T;
+        float v = part[group << a.kw_log2][r][t];
+        for (int w = 1; w < kw; ++w) v += part[(group << a.kw_log2) + w][r][t];
+        for (uint32_t todo = __ballot_sync(0xffffffffu, mine && !(fabsf(v) < INFINITY)); todo; todo &= todo - 1) {  // rare
+            const int src = __ffs(todo) - 1;
+            const float again = scaled_product<P>(a, __shfl_sync(0xffffffffu, row, src), __shfl_sync(0xffffffffu, t0 + t, src));
+            if ((int)(threadIdx.x & 31) == src) v = again;
         }
+        if (mine) store_result(a.out, (int64_t)(t0 + t) * a.ldy + row, v + (a.bias ? __ldg(a.bias + row) : 0.0f));
     }
 }
 
@@ -527,7 +571,7 @@ k_product(const __grid_constant__ Product a) {
         put_part();
         __syncthreads();
     }
-    reduce_and_store<NT, WARPS>(part, a, t0);
+    reduce_and_store<NT, P, WARPS>(part, a, t0);
 }
 
 // Whether one scale covers whole rows.
@@ -615,7 +659,7 @@ static int vlut_product(const void* codes, const void* layout, const float* beta
     if (codes && !(a.table = residual_table_q4((cudaStream_t)stream))) return COSET_E_STATE;
     a.beta = beta;
     a.n_out = n_out; a.kb = kb; a.T = T;
-    a.x = x; a.ldx = ldx; a.ldy = ldy; a.bias = bias; a.clip = clip > 0.0f ? clip : 0.0f;
+    a.x = x; a.ldx = ldx; a.ldy = ldy; a.bias = bias; a.clip = clip > 0.0f && clip < INFINITY ? clip : 0.0f;  // an infinite clamp is none
     for (int k = 0; k < n_targets; ++k) {
         if (!y_targets[k]) return fail(COSET_E_BADARG, "result buffer %d is null", k);
         a.out.y[k] = y_targets[k];
@@ -623,6 +667,7 @@ static int vlut_product(const void* codes, const void* layout, const float* beta
     a.out.n = n_targets;
     a.out.bf16 = y_dtype == COSET_DTYPE_BF16 ? 1 : 0;
     const bool rows = scale_per_row(beta, blocks_per_tile, kb), one = blocks_per_tile == 1 && (kb % 8) == 0 && aligned(beta, 16);
+    a.per_row = rows;
     a.rows_per_scale = rows && beta && kb > 0 ? (int)(blocks_per_tile / kb) : 1;
     if (!rows) a.td = e8::make_tile_div(blocks_per_tile, (int64_t)n_out * kb);
     cudaStream_t st = (cudaStream_t)stream;

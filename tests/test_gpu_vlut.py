@@ -448,3 +448,55 @@ def test_few_float32_tokens_keep_float32_precision(T, n_out, n_in, row, clip):
     w = w.view(n_out, n_in).clamp(-clip, clip) if clip else w.view(n_out, n_in)
     want = x.double() @ w.T
     assert float((layer(x).double() - want).norm() / want.norm()) < 2.0 ** -23
+
+
+def _awkward(kind, T, n_in):
+    x = torch.randn(T, n_in, device="cuda", generator=torch.Generator(device="cuda").manual_seed(7))
+    if kind == "infinity":
+        x[0, 3], x[T - 1, n_in - 1] = float("inf"), float("-inf")
+    elif kind == "nan":
+        x[T // 2, 5] = float("nan")
+    elif kind == "large":
+        x = x.clamp(-3, 3) * 3e36
+    return x
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 1e-2), (torch.float32, 1e-5)])
+@pytest.mark.parametrize("row", [True, False])
+@pytest.mark.parametrize("clip", [0.0, 0.05, 2.0, float("inf")])
+@pytest.mark.parametrize("kind", ["plain", "infinity", "nan", "large"])
+@pytest.mark.parametrize("T,n_in", [(1, 256), (3, 1032), (16, 4096)])
+def test_few_tokens_with_awkward_values(T, n_in, kind, clip, row, dtype, tol):
+    """Infinities, NaN, activations whose unscaled sums overflow and an infinite clamp, against the sum in 64 bits: the same
+    results are finite, infinite and NaN, from the layout and from the codes."""
+    from coset_b200 import _lib
+    from coset_b200.vlut import E8CodeLinear
+    layer, _ = _kept_copy_layer(40, n_in)
+    bpt = n_in // 8 if row else 1
+    layer = E8CodeLinear(layer.codes, torch.full((40 * n_in // 8 // bpt,), 25.0, device="cuda"), bpt, torch.randn(40, device="cuda"), weight_clip_value=clip)
+    x = _awkward(kind, T, n_in).to(dtype)
+    w = layer.dense_weight().double()
+    want = (x.double().unsqueeze(1) * w).sum(2) + layer.bias.double()  # not matmul: 0 * inf must count
+    trusted = _lib.native().vlut_product(x, layer._product_layout(), 40, n_in, layer.beta, bpt, layer.bias, clip, _lib.DTYPE_F32)
+    for got in (layer(x).double(), trusted.double()):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        assert torch.equal(got[got.isinf()], want[want.isinf()])
+        assert rel(got[got.isfinite()].cpu().numpy(), want[want.isfinite()].cpu().numpy()) < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("row", [True, False])
+@pytest.mark.parametrize("scale", [0.0, 1e-39, float("inf"), float("nan")])
+def test_few_tokens_with_awkward_scales_and_a_clamp(scale, row, dtype):
+    """A scale of zero or NaN: the weights are the clamped values that a minimum and a maximum make of them, as in the kernels
+    that read the codes."""
+    from coset_b200.vlut import E8CodeLinear, e8_vlut_matmul
+    layer, _ = _kept_copy_layer(40, 256)
+    bpt = 32 if row else 1
+    beta = torch.full((40 * 32 // bpt,), 25.0, device="cuda")
+    beta[::3] = scale
+    layer = E8CodeLinear(layer.codes, beta, bpt, None, weight_clip_value=0.5)
+    x = torch.randn(2, 256, device="cuda").to(dtype)
+    want = e8_vlut_matmul(layer.codes, beta, bpt, x, None, 0.5, dtype)
+    assert bool(want.isfinite().all())
+    torch.testing.assert_close(layer(x), want, rtol=1e-2 if dtype == torch.bfloat16 else 1e-5, atol=1e-4)
