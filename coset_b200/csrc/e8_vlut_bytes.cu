@@ -668,7 +668,7 @@ static int vlut_product(const void* codes, const void* layout, const float* beta
     a.out.bf16 = y_dtype == COSET_DTYPE_BF16 ? 1 : 0;
     const bool rows = scale_per_row(beta, blocks_per_tile, kb), one = blocks_per_tile == 1 && (kb % 8) == 0 && aligned(beta, 16);
     a.per_row = rows;
-    a.rows_per_scale = rows && beta && kb > 0 ? (int)(blocks_per_tile / kb) : 1;
+    a.rows_per_scale = rows && beta && kb > 0 ? (int)(blocks_per_tile / kb < n_out ? blocks_per_tile / kb : n_out) : 1;
     if (!rows) a.td = e8::make_tile_div(blocks_per_tile, (int64_t)n_out * kb);
     cudaStream_t st = (cudaStream_t)stream;
     const int scale_kind = rows ? kPerRow : (one ? kPerBlock : kPerTile);

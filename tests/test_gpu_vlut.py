@@ -500,3 +500,13 @@ def test_few_tokens_with_awkward_scales_and_a_clamp(scale, row, dtype):
     want = e8_vlut_matmul(layer.codes, beta, bpt, x, None, 0.5, dtype)
     assert bool(want.isfinite().all())
     torch.testing.assert_close(layer(x), want, rtol=1e-2 if dtype == torch.bfloat16 else 1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("rows", [64, 1 << 20, 1 << 31, 1 << 32, (1 << 32) + 1])
+def test_one_scale_for_more_rows_than_there_are(rows):
+    """A scale tile may be larger than the weight, by any factor: the kernel's row count per scale is no wider than an int."""
+    from coset_b200.vlut import E8CodeLinear
+    layer, x = _kept_copy_layer(64, 256)
+    want = x.double() @ layer.dense_weight().double().T
+    got = E8CodeLinear(layer.codes, torch.full((1,), 25.0, device="cuda"), rows * 32, None)(x)
+    assert rel(got.cpu().numpy(), want.cpu().numpy()) < 1e-5
