@@ -99,7 +99,9 @@ class E8CodeLinear(nn.Module):
     Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 9-13 us for 1-16
     tokens and a 4096 x 4096 weight; the kernel checks the copy against the codes in every call.  "tcgen05" keeps nothing and
     stays on the code-domain kernels (9.7-23 us).
-    A call under graph capture reads the codes themselves, so that a replay follows writes to them.
+    A call under graph capture reads the codes, scales and bias themselves (it decodes the weight where it would use the dense
+    copy), so that a replay follows writes to them and reads nothing that a later call gives back.  The dense copy follows
+    writes that PyTorch's version counters show; see forget_copies for the others.
     small_t_max defaults to 16 ("auto", "cublas") or 48 ("tcgen05"): measured on a 4096 x 4096 layer the
     code-domain kernels take 9.7 / 23 / 44 / 86 us for 1 / 16 / 32 / 64 tokens (they re-read and re-decode the
     codes for every 16 tokens), the library on the cached copy 7-13 us, the fused kernel 64 us.
@@ -186,28 +188,42 @@ class E8CodeLinear(nn.Module):
         return w.view(self.out_features, self.in_features)
 
     def _keep(self, name, sources, settings, make):
-        """`make()`, kept until one of the buffers it was made from is written or replaced (the entry holds the buffers, so
-        their identity cannot be taken over by another tensor).  It is complete on the device before it is published, for a
-        later call may come from another stream or thread, and none of these may still read the one it replaces.  Inside a
-        graph capture it is recorded with the call and not kept: nothing is computed before the replay."""
+        """`make()`, kept until one of the buffers it was made from is seen to be written or replaced (the entry holds the buffers,
+        so their identity cannot be taken over by another tensor).  A call on another stream than the one that made it waits there
+        for the copy and marks it as used, so that it may be replaced or dropped at any time.  Inside a graph capture it is made
+        in the call and not kept: a replay follows its sources, and reads no memory that a later call gives back."""
+        if torch._C._cuda_isCurrentStreamCapturing():
+            return make()
+        device = sources[0].get_device()
+        stream = torch._C._cuda_getCurrentRawStream(device)
         entry = self._kept.get(name)
         if entry is not None and entry[1] == settings:
             for t, (kept, version, pointer) in zip(sources, entry[2]):
                 if t is not kept or t._version != version or t.data_ptr() != pointer:
                     break
             else:
+                if entry[3] != stream:
+                    here = torch.cuda.current_stream(device)
+                    here.wait_event(entry[4])
+                    entry[0].record_stream(here)
                 return entry[0]
         if any(t.is_inference() for t in sources):  # no version counter: a write would go unseen
             return make()
         state = [(t, t._version, t.data_ptr()) for t in sources]
         value = make()
-        if not torch.cuda.is_current_stream_capturing():
-            if entry is not None:
-                torch.cuda.synchronize(value.device)
-            else:
-                torch.cuda.current_stream(value.device).synchronize()
-            self._kept[name] = (value, settings, state)
+        made = torch.cuda.current_stream(device).record_event()
+        self._kept[name] = (value, settings, state, stream, made)
         return value
+
+    def forget_copies(self):
+        """Drops the copies of the weight in other forms; the next call makes them again.  The dense copy of the library path
+        follows writes that the buffers' version counters show; a write to the codes or scales by `.data`, a collective or a
+        replayed graph shows in none, and wants this call behind it.  Few tokens do not need it: their kernel checks its copy."""
+        self._kept = {}
+
+    def _apply(self, fn, *args, **kwargs):
+        self._kept = {}  # neither the copies nor the buffers they were made from outlive a move
+        return super()._apply(fn, *args, **kwargs)
 
     @property
     def _dense(self):
@@ -231,15 +247,6 @@ class E8CodeLinear(nn.Module):
 
     def _make_dense(self):
         return self.dense_weight(torch.bfloat16)
-
-    def _bias_bf16(self):
-        bias = self._buffers["bias"]
-        if bias is None or bias.dtype == torch.bfloat16:
-            return bias
-        return self._keep("bias", (bias,), None, self._make_bias)
-
-    def _make_bias(self):
-        return self._buffers["bias"].to(torch.bfloat16)
 
     def check(self):
         """Synchronises and raises if a bounded barrier wait expired inside one of the tensor-core kernels since
@@ -269,7 +276,6 @@ class E8CodeLinear(nn.Module):
                 y = e8_dequant_gemm(buf["codes"], buf["beta"], self.blocks_per_tile, x.reshape(-1, n_in), buf["bias"],
                                     clip=self.weight_clip_value, status=self._status).to(dtype)
                 return y.reshape(*x.shape[:-1], self.out_features)
-            return torch.nn.functional.linear(x, self._dense_bf16(), self._bias_bf16())
         if dtype is torch.float32:
             return torch.nn.functional.linear(x, self.dense_weight(torch.float32), buf["bias"])
         b = buf["bias"].to(dtype) if buf["bias"] is not None else None

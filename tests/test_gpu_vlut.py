@@ -510,3 +510,67 @@ def test_one_scale_for_more_rows_than_there_are(rows):
     want = x.double() @ layer.dense_weight().double().T
     got = E8CodeLinear(layer.codes, torch.full((1,), 25.0, device="cuda"), rows * 32, None)(x)
     assert rel(got.cpu().numpy(), want.cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("clip", [0.0, 0.05])
+@pytest.mark.parametrize("T", [3, 64])
+def test_capture_after_an_eager_call_follows_every_buffer(T, clip):
+    """An eager call first, as a warm-up does, then a capture: its replay follows in-place writes to codes, scales and bias, before
+    and after an eager call has replaced the copies that the layer keeps."""
+    import gc
+    layer, _ = _kept_copy_layer(64, 256, weight_clip_value=clip)
+    layer.bias = torch.randn(64, device="cuda")
+    other, _ = _kept_copy_layer(64, 256, seed=6)
+    x = torch.randn(T, 256, device="cuda").to(torch.bfloat16)
+    want = lambda: x.double() @ layer.dense_weight().double().T + layer.bias.double()
+    layer(x)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        y = layer(x)
+    same = lambda got: rel(got.float().cpu().numpy(), want().cpu().numpy()) < 1e-2
+    for write in (lambda: None, lambda: layer.bias.add_(3.0), lambda: layer.bias.data.mul_(-2.0), lambda: layer.codes.copy_(other.codes), lambda: layer.beta.mul_(0.5)):
+        write()
+        graph.replay()
+        assert same(y)
+        assert same(layer(x))
+        gc.collect()
+        filler = [torch.full((1 << 16,), 3e38, device="cuda") for _ in range(64)]  # into whatever the eager call gave back
+        graph.replay()
+        assert same(y)
+        del filler
+
+
+@pytest.mark.parametrize("T", [3, 64])
+def test_kept_copies_do_not_outlive_a_move_and_can_be_dropped(T):
+    layer, _ = _kept_copy_layer(64, 256)
+    x = torch.randn(T, 256, device="cuda").to(torch.bfloat16)
+    y = layer(x)
+    assert layer._kept
+    layer.cpu()
+    assert not layer._kept
+    layer.cuda()
+    assert torch.equal(layer(x), y)
+    other, _ = _kept_copy_layer(64, 256, seed=6)
+    layer.codes.data.copy_(other.codes)
+    layer.forget_copies()
+    assert torch.equal(layer(x), other(x))
+
+
+def test_kept_copy_replaced_while_another_stream_reads_it():
+    """A copy that another stream still reads is not given back to the allocator when a write replaces it."""
+    side = torch.cuda.Stream()
+    layer, _ = _kept_copy_layer(2048, 2048)
+    x = torch.randn(64, 2048, device="cuda").to(torch.bfloat16)
+    other, _ = _kept_copy_layer(2048, 2048, seed=6)
+    want = layer(x)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+        y = layer(x)
+    layer.codes = other.codes
+    layer(x)
+    filler = [torch.full((2048, 2048), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    del filler
