@@ -74,6 +74,10 @@ Tensor as_f32(const Tensor& t) {
     Tensor f = t.scalar_type() == at::kFloat ? t : t.to(at::kFloat);
     return f.is_contiguous() ? f : f.contiguous();
 }
+// A kernel has written through the tensor's pointer: what was saved or made from it has to be seen as out of date.
+void written(const Tensor& t) {
+    if (!t.is_inference()) t.unsafeGetTensorImpl()->bump_version();
+}
 Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 
 // rows of 8: a vector is one row
@@ -139,6 +143,7 @@ PyObject* encode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     check_rc(coset_e8_encode(data(x), dtype_code(x, "x"), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, (int)int_arg(a[7]), data(out),
                              stream_of(x)), "coset_e8_encode");
+    if (a[6] != Py_None) written(out);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
 }
@@ -164,6 +169,7 @@ PyObject* decode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     check_rc(coset_e8_decode(data(codes), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, COSET_SEM_CORE, data(out), dtype_code(out, "out"),
                              stream_of(codes)), "coset_e8_decode");
+    if (a[7] != Py_None) written(out);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
 }
@@ -230,6 +236,7 @@ PyObject* grad_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     c10::cuda::CUDAGuard guard(x.device());
     check_rc(coset_e8_encode(data(x), dtype_code(x, "grad"), fdata(s), COSET_SCALE_MUL_TILE, nb, nb > 0 ? nb : 1, 4, 2,
                              (int)int_arg(a[3]), data(out), stream_of(x)), "coset_e8_encode");
+    written(out);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
 }
@@ -242,6 +249,7 @@ PyObject* decode_mean(PyObject*, PyObject* const* a, Py_ssize_t n) {
     c10::cuda::CUDAGuard guard(codes.device());
     check_rc(coset_e8_decode_mean(data(codes), (int)int_arg(a[1]), int_arg(a[2]), codes.size(1), (float)float_arg(a[3]), data(out),
                                   dtype_code(out, "out"), stream_of(codes)), "coset_e8_decode_mean");
+    written(out);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
 }

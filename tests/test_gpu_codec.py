@@ -393,3 +393,24 @@ def test_round_trip_and_digits_around_the_row_count_switch(e8, cfgcls, n, spread
     assert torch.equal(digits, (words & 3).float())
     assert torch.equal(e8.e8_quantize(x, 4), want)
     assert torch.equal(e8.e8_decode(digits, config), want)
+
+
+def test_out_shows_that_it_was_written():
+    """Whoever watches the version counter of a tensor (autograd, a layer's copy of its weight) sees a write through `out`."""
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    from coset_b200.gradcomm import CudaCodec
+    x = torch.randn(64, 8, device="cuda")
+    codes, xh, mean = torch.empty(64, dtype=torch.int32, device="cuda"), torch.empty(64, 8, device="cuda"), torch.empty(64, 8, device="cuda")
+    codec = CudaCodec()
+    for out, write in ((codes, lambda: e8_encode_packed(x, out=codes)), (xh, lambda: e8_decode_packed(codes, out=xh)),
+                       (codes, lambda: codec.encode(x, 1.0, codes)), (mean, lambda: codec.decode_mean(codes.view(1, 64), 1, 64, 1.0, mean))):
+        version = out._version
+        write()
+        assert out._version == version + 1
+    weight = x.clone().requires_grad_()
+    y = (weight * xh).sum()
+    e8_decode_packed(codes, out=xh)
+    with pytest.raises(RuntimeError):  # xh was saved for the product's gradient
+        y.backward()
+    with torch.inference_mode():
+        e8_encode_packed(x, out=torch.empty(64, dtype=torch.int32, device="cuda"))
