@@ -109,7 +109,7 @@ Scale scale_arg(PyObject* o, int64_t mode, int64_t n_blocks, int64_t bpt, const 
         if (!number) throw python_error();
         const double value = PyFloat_AS_DOUBLE(number);
         Py_DECREF(number);
-        s.t = at::full({1}, value, x.options().dtype(at::kFloat));
+        s.t = at::full({1}, (double)(float)value, x.options().dtype(at::kFloat));  // beyond float32: an infinity
     }
     if (mode == COSET_SCALE_DIV_SCALAR) {
         TORCH_CHECK_VALUE(s.t.numel() == 1, "the codec (divide) convention takes one scalar beta");

@@ -414,3 +414,13 @@ def test_out_shows_that_it_was_written():
         y.backward()
     with torch.inference_mode():
         e8_encode_packed(x, out=torch.empty(64, dtype=torch.int32, device="cuda"))
+
+
+@pytest.mark.parametrize("value,same", [(1e60, float("inf")), (-1e60, float("-inf")), (1e-60, 0.0)])
+def test_scale_beyond_float32(value, same):
+    """A Python scale is taken as float32 takes it."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_encode_packed
+    x = torch.randn(64, 8, device="cuda")
+    got = e8_encode_packed(x, scale=value, scale_mode=_lib.SCALE_DIV_SCALAR)
+    assert torch.equal(got, e8_encode_packed(x, scale=torch.tensor(same, device="cuda"), scale_mode=_lib.SCALE_DIV_SCALAR))
