@@ -276,6 +276,8 @@ class E8CodeLinear(nn.Module):
                 y = e8_dequant_gemm(buf["codes"], buf["beta"], self.blocks_per_tile, x.reshape(-1, n_in), buf["bias"],
                                     clip=self.weight_clip_value, status=self._status).to(dtype)
                 return y.reshape(*x.shape[:-1], self.out_features)
+        if x.dim() != 2:  # with other shapes and strides the library may add the bias to the rounded product
+            return self.forward(x.reshape(-1, n_in)).reshape(*x.shape[:-1], self.out_features)
         if dtype is torch.float32:
             return torch.nn.functional.linear(x, self.dense_weight(torch.float32), buf["bias"])
         b = buf["bias"].to(dtype) if buf["bias"] is not None else None

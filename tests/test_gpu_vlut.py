@@ -574,3 +574,26 @@ def test_kept_copy_replaced_while_another_stream_reads_it():
     torch.cuda.synchronize()
     assert torch.equal(y, want)
     del filler
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", ["rows", "three", "four", "transposed", "strided", "expanded"])
+def test_library_path_rounds_once_for_every_shape(shape, dtype):
+    """The tokens of the library path, given in any number of dimensions and any strides, are those of the plain rows, to the bit."""
+    layer, _ = _kept_copy_layer(64, 256)
+    layer.bias = torch.randn(64, device="cuda") * 10
+    x = torch.randn(12, 16, 256, device="cuda").to(dtype)
+    want = layer(x.view(192, 256)).view(12, 16, 64)
+    if shape == "rows":
+        got = layer(torch.cat([x, x], 2).view(192, 512)[:, :256]).view(12, 16, 64)
+    elif shape == "three":
+        got = layer(x)
+    elif shape == "four":
+        got = layer(x.view(4, 3, 16, 256)).view(12, 16, 64)
+    elif shape == "transposed":
+        got = layer(x.transpose(0, 1).contiguous().transpose(0, 1))
+    elif shape == "strided":
+        got = layer(torch.cat([x, x], 2)[..., :256])
+    else:
+        got, want = layer(x[:1].expand(12, 16, 256)), want[:1].expand(12, 16, 64)
+    assert got.shape == want.shape and torch.equal(got, want)
