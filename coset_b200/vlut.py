@@ -129,6 +129,7 @@ class E8CodeLinear(nn.Module):
         self.blocks_per_tile = int(blocks_per_tile)
         self.weight_clip_value = float(weight_clip_value)
         self._kept = {}      # copies of the weight in other forms, see _keep
+        self._rows = self.out_features  # of the whole weight, where this layer holds a shard of its rows
         self._status = None  # device word the tensor-core kernels set when a bounded wait gave up
 
     def _load_from_state_dict(self, state_dict, prefix, *args, **kwargs):
@@ -143,6 +144,7 @@ class E8CodeLinear(nn.Module):
     def __setstate__(self, state):
         super().__setstate__({k: v for k, v in state.items() if k not in ("_dense", "_dense_key")})
         self.__dict__.setdefault("_kept", {})
+        self.__dict__.setdefault("_rows", self.out_features)
 
     @classmethod
     def from_weight(cls, weight: torch.Tensor, beta: torch.Tensor, blocks_per_tile: int, bias=None, **kw):
@@ -238,6 +240,19 @@ class E8CodeLinear(nn.Module):
             return None
         return self._keep("layout", (codes,), None, self._make_layout)
 
+    def _codes_are_faster(self, T, dtype):
+        """Whether the kernel that reads the codes beats the one that reads the layout: one or two float32 tokens, where the layout's
+        three products per weight cost more than one decoding unless many rows share the chip.  Codes against layout, us: scales
+        per block, 1024 x 8192 one token 7.5 / 23.6, two 8.7 / 23.6; 2048 x 4096 8.5 / 13.5, 10.4 / 13.5; 4096 x 4096 14.2 / 15.6,
+        15.9 / 15.5; 8192 x 8192 41 / 52, 53 / 52; but 8192 x 512 9.8 / 6.8; per row, 1024 x 8192 10.0 / 15.7, 2048 x 2048
+        8.0 / 6.3.  Below 2^22 weights the host takes longer than either.  The rule sees the whole weight, so that the
+        shards of a layer return its bits."""
+        if T > 2 or dtype is torch.bfloat16 or self._rows * self.in_features < 1 << 22:
+            return False
+        if self.blocks_per_tile % (self.in_features // 8) == 0:
+            return self._rows <= 1024
+        return self.in_features >= 1024 and (T == 1 or self._rows <= 2048)
+
     def _make_layout(self):
         return _lib.native().vlut_layout(self._buffers["codes"])
 
@@ -260,7 +275,7 @@ class E8CodeLinear(nn.Module):
         buf, n_in, dtype = self._buffers, self.in_features, x.dtype
         T = x.numel() // n_in
         if T <= self.small_t_max:
-            layout = self._product_layout() if self.large_t_path != "tcgen05" and n_in else None
+            layout = self._product_layout() if self.large_t_path != "tcgen05" and n_in and not self._codes_are_faster(T, dtype) else None
             if layout is not None:
                 return _lib.native().vlut_product_checked(x, buf["codes"], layout, buf["beta"], self.blocks_per_tile, buf["bias"],
                                                           self.weight_clip_value, _lib.DTYPE_BF16 if dtype is torch.bfloat16 else _lib.DTYPE_F32)
@@ -329,6 +344,7 @@ class ColumnParallelE8CodeLinear(nn.Module):
         lo, hi = out_feature_shard(out_features, self.world, self.rank)
         if local.out_features != hi - lo:
             raise ValueError(f"local shard has {local.out_features} rows, expected {hi - lo}")
+        local._rows = out_features
 
     @classmethod
     def from_weight(cls, weight: torch.Tensor, beta: torch.Tensor, blocks_per_tile: int, bias=None, group=None,
@@ -369,7 +385,8 @@ class ColumnParallelE8CodeLinear(nn.Module):
         bias32 = loc.bias.to(torch.float32).contiguous() if loc.bias is not None else None
         with torch.cuda.device(x2.device):
             bias = _lib.ptr(bias32) if bias32 is not None else None
-            layout = loc._product_layout() if loc.large_t_path != "tcgen05" and loc.in_features else None
+            layout = (loc._product_layout() if loc.large_t_path != "tcgen05" and loc.in_features and not loc._codes_are_faster(T, x2.dtype)
+                      else None)
             if layout is not None:  # the kernel of the unsharded layer, so that the results are the same bits
                 rc = _lib.lib().coset_e8_vlut_product_checked(
                     _lib.ptr(loc.codes), _lib.ptr(layout), _lib.ptr(loc.beta), loc.blocks_per_tile, loc.out_features, loc.in_features,

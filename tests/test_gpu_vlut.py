@@ -597,3 +597,26 @@ def test_library_path_rounds_once_for_every_shape(shape, dtype):
     else:
         got, want = layer(x[:1].expand(12, 16, 256)), want[:1].expand(12, 16, 64)
     assert got.shape == want.shape and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n_out,n_in,row,T,dtype,codes", [
+    (512, 8192, False, 1, torch.float32, True), (512, 8192, False, 2, torch.float32, True), (512, 8192, False, 3, torch.float32, False),
+    (512, 8184, False, 1, torch.float32, False), (1024, 4096, True, 1, torch.float32, True), (1032, 4096, True, 1, torch.float32, False),
+    (4104, 1024, False, 1, torch.float32, True), (4104, 1024, False, 2, torch.float32, False), (4608, 1016, False, 1, torch.float32, False),
+    (1024, 4096, False, 1, torch.bfloat16, False)])
+def test_one_or_two_float32_tokens_read_the_codes(n_out, n_in, row, T, dtype, codes):
+    """The line between the two kernels, a shard that keeps to the rule of the whole weight, and the same result from both."""
+    from coset_b200 import _lib
+    from coset_b200.vlut import E8CodeLinear, e8_vlut_matmul
+    layer, _ = _kept_copy_layer(n_out, n_in)
+    bpt = n_in // 8 if row else 1
+    beta = torch.full((n_out * n_in // 8 // bpt,), 25.0, device="cuda")
+    layer = E8CodeLinear(layer.codes, beta, bpt, None)
+    x = torch.randn(T, n_in, device="cuda").to(dtype)
+    from_codes = e8_vlut_matmul(layer.codes, beta, bpt, x, None, 0.0, dtype)
+    from_layout = _lib.native().vlut_product(x, layer._product_layout(), n_out, n_in, beta, bpt, None, 0.0, _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_F32)
+    assert torch.equal(layer(x), from_codes if codes else from_layout)
+    assert rel(from_layout.float().cpu().numpy(), from_codes.float().cpu().numpy()) < (1e-2 if dtype == torch.bfloat16 else 1e-6)
+    shard = E8CodeLinear(layer.codes[:n_out // 2], beta[:beta.numel() // 2], bpt, None)
+    shard._rows = n_out
+    assert torch.equal(shard(x), layer(x)[:, :n_out // 2])
