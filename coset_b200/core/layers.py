@@ -97,6 +97,57 @@ class _E8FakeQuant(torch.autograd.Function):
         return grad_w, (grad_beta.view(beta_shape) if need_beta else None), None, None, None, None
 
 
+class _E8LayerFakeQuant(torch.autograd.Function):
+    """The layer's weight path as a Python node, for torch.jit.trace: a trace records it as an operator that runs again, where the
+    native node (layer_fake_quant) would leave it the weights of the traced call as constants."""
+
+    @staticmethod
+    def forward(ctx, weight, theta, beta_min, beta_range, blocks_per_tile, q, clip, out_dtype):
+        _lib.require_float32(weight, "weight")
+        _lib.require_cuda(weight, "weight")
+        w = weight.contiguous()
+        th = theta.detach().to(torch.float32).contiguous().view(-1)
+        n_blocks = w.numel() // 8
+        lib = _lib.lib()
+        code_bytes = lib.coset_e8_code_bytes(q, 2)
+        if code_bytes == 0:
+            raise ValueError(f"unsupported q={q} for the fused E8 weight quantiser (2 <= q <= 16)")
+        codes = torch.empty((n_blocks, code_bytes), dtype=torch.uint8, device=w.device)
+        out = torch.empty(w.shape, dtype=out_dtype, device=w.device)
+        beta = torch.empty_like(th)
+        with torch.cuda.device(w.device):
+            rc = lib.coset_e8_layer_fake_quant_fwd(_lib.ptr(w), _lib.ptr(th), _lib.ptr(beta_min), _lib.ptr(beta_range), n_blocks,
+                                                   blocks_per_tile, q, float(clip), _lib.ptr(out), _lib.dtype_code(out, "out"),
+                                                   _lib.ptr(codes), _lib.ptr(beta), _lib.stream())
+        _lib.check(rc, "coset_e8_layer_fake_quant_fwd")
+        ctx.save_for_backward(w, th, beta, codes)
+        # the bounds tensors are refreshed in place once every stat_update_interval steps (so that a captured
+        # graph keeps reading them); kept outside save_for_backward, whose version check would turn a refresh
+        # between this forward and its backward into an error
+        ctx.beta_range = beta_range
+        ctx.meta = (blocks_per_tile, q, float(clip), theta.shape)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        w, th, beta, codes = ctx.saved_tensors
+        beta_range = ctx.beta_range
+        blocks_per_tile, q, clip, theta_shape = ctx.meta
+        g = grad_out.contiguous()
+        if g.dtype not in (torch.float32, torch.bfloat16):
+            g = g.float()
+        grad_w = torch.empty_like(w)
+        need_theta = ctx.needs_input_grad[1]
+        grad_theta = torch.empty_like(th) if need_theta else None
+        with torch.cuda.device(w.device):
+            rc = _lib.lib().coset_e8_layer_fake_quant_bwd(_lib.ptr(g), _lib.dtype_code(g, "grad"), _lib.ptr(w), _lib.ptr(codes),
+                                                          _lib.ptr(beta), _lib.ptr(th), _lib.ptr(beta_range), w.numel() // 8,
+                                                          blocks_per_tile, q, clip, _lib.ptr(grad_w), _lib.ptr(grad_theta),
+                                                          _lib.stream())
+        _lib.check(rc, "coset_e8_layer_fake_quant_bwd")
+        return grad_w, (grad_theta.view(theta_shape) if need_theta else None), None, None, None, None, None, None
+
+
 def e8_fake_quantize(weight, beta, blocks_per_tile, q=4, clip=2.0, out_dtype=torch.float32):
     """Differentiable fused weight quantiser used by HNLQLinearQAT (see _E8FakeQuant)."""
     return _E8FakeQuant.apply(weight, beta, int(blocks_per_tile), int(q), float(clip), out_dtype)
@@ -358,9 +409,13 @@ class HNLQLinearQAT(nn.Module):
         bpt = self.blocks_per_row if self.tiling == "row" else 1
         if self._fused and W.is_cuda:
             beta_min, _ = self._bounds()
-            W_q = _lib.native().layer_fake_quant(W, self.theta_beta, beta_min, self._bounds_cache[2], bpt, int(self.q),
-                                                 float(self.weight_clip_value),
-                                                 _lib.DTYPE_BF16 if out_dtype == torch.bfloat16 else _lib.DTYPE_F32)
+            if torch._C._get_tracing_state() is not None:
+                W_q = _E8LayerFakeQuant.apply(W, self.theta_beta, beta_min, self._bounds_cache[2], bpt, int(self.q),
+                                              float(self.weight_clip_value), out_dtype)
+            else:
+                W_q = _lib.native().layer_fake_quant(W, self.theta_beta, beta_min, self._bounds_cache[2], bpt, int(self.q),
+                                                     float(self.weight_clip_value),
+                                                     _lib.DTYPE_BF16 if out_dtype == torch.bfloat16 else _lib.DTYPE_F32)
         elif self._fused_d4 and W.is_cuda:
             from .d4.layers import d4_fake_quantize
             W_q = d4_fake_quantize(W, self._beta(), bpt, self.weight_clip_value, out_dtype)
@@ -385,10 +440,12 @@ class HNLQLinearQAT(nn.Module):
     def _one_node(self, x, low):
         """Whether the whole product can run as one native autograd node: the plain case of a quantised E8 layer
         on the GPU.  Warm-up, diagnostics (which look at the quantised weights), autocast, forward-mode derivatives (the
-        node has none), parametrised or pruned parameters and a quantize_fn of the caller's own take the composed path."""
+        node has none), parametrised or pruned parameters, a quantize_fn of the caller's own, and whoever looks at the torch
+        calls (a trace, a torch-function mode, a tensor subclass) take the composed path."""
         state = self.__dict__
         params = state["_parameters"]
         return (state["_fused"] and state["quantization_enabled"] and not state["enable_diagnostics"] and x.is_cuda
+                and type(x) is torch.Tensor and torch._C._get_tracing_state() is None and not torch._C._len_torch_function_stack()
                 and (low or x.dtype == torch.float32) and not torch.is_autocast_enabled("cuda")
                 and forward_ad._current_level < 0
                 and "weight" in params and "bias" in params and "theta_beta" in (params if state["theta_trainable"] else state["_buffers"])

@@ -361,3 +361,49 @@ def test_bias_that_is_no_plain_parameter(how):
     if how == "parametrised":
         got.sum().backward()
         torch.testing.assert_close(layer.parametrizations.bias.original.grad, torch.full((32,), 16.0, device="cuda"))
+
+
+@pytest.mark.parametrize("tiling", ["row", "block"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_traced_layer_follows_its_weights(tiling, dtype):
+    """A trace quantises the weights it finds when it runs, and its gradients reach weight, scale and bias."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 32, device="cuda", tiling=tiling)
+    with torch.no_grad():
+        layer.weight.copy_(torch.randn(32, 64) * 20.0)
+        layer.bias.copy_(torch.randn(32))
+    x = torch.randn(8, 64, device="cuda").to(dtype)
+    traced = torch.jit.trace(layer, x, check_trace=False)
+    with torch.no_grad():
+        layer.weight.mul_(1.5)
+        layer.bias.add_(1.0)
+    y = traced(x)
+    assert torch.equal(y, layer(x))
+    y.float().sum().backward()
+    got = [p.grad.clone() for p in (layer.weight, layer.theta_beta, layer.bias)]
+    layer.zero_grad()
+    layer(x).float().sum().backward()
+    for a, b in zip(got, (layer.weight.grad, layer.theta_beta.grad, layer.bias.grad)):
+        torch.testing.assert_close(a, b, rtol=1e-2 if dtype == torch.bfloat16 else 1e-5, atol=1e-3)
+
+
+def test_subclasses_and_function_modes_see_the_product():
+    from torch.overrides import TorchFunctionMode
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+
+    class Marked(torch.Tensor):
+        pass
+
+    class Names(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", ""))
+            return func(*args, **(kwargs or {}))
+
+    seen = []
+    layer = create_e8_hnlq_linear(64, 32, device="cuda")
+    x = torch.randn(8, 64, device="cuda")
+    want = layer(x)
+    assert type(layer(x.as_subclass(Marked))) is Marked
+    with Names():
+        y = layer(x)
+    assert "linear" in seen and torch.equal(y, want)
