@@ -32,4 +32,11 @@ const uint16_t* residual_table_q4_compact(cudaStream_t stream);
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
+// s += v, and what the rounded sum lacks to e (Knuth's two-sum)
+__device__ __forceinline__ void add_exactly(float& s, float& e, float v) {
+    const float t = s + v, z = t - s;
+    e += (s - (t - z)) + (v - z);
+    s = t;
+}
+
 }  // namespace coset

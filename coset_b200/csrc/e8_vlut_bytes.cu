@@ -113,12 +113,6 @@ __device__ __forceinline__ float reciprocal(float v) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
-// s += v, and what the rounded sum lacks to e (Knuth's two-sum)
-__device__ __forceinline__ void add_exactly(float& s, float& e, float v) {
-    const float t = s + v, z = t - s;
-    e += (s - (t - z)) + (v - z);
-    s = t;
-}
 // The exact three-term bf16 split of two floats, packed: out[p] = (p-th term of a, p-th term of b).
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&out)[3]) {
 #pragma unroll

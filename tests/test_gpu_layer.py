@@ -407,3 +407,22 @@ def test_subclasses_and_function_modes_see_the_product():
     with Names():
         y = layer(x)
     assert "linear" in seen and torch.equal(y, want)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (32, 128), (128, 768), (333, 1001), (8192, 256)])
+def test_column_sum_of_float32_is_rounded_once(rows, cols):
+    """The sum keeps what rounding takes from it: what is left is the rounding of the result and, at 2^-48 a term, that of the
+    corrections.  An infinite sum stays infinite."""
+    from coset_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, device="cuda", generator=g) * 10.0 ** torch.randint(-3, 4, (rows, cols), device="cuda", generator=g)
+    x[rows // 2, 3] = float("inf")
+    x[rows - 1, 5] = float("nan")
+    y = torch.empty(cols, device="cuda")
+    rc = _lib.lib().coset_column_sum(x.data_ptr(), _lib.DTYPE_F32, rows, cols, _lib.ptr(y), _lib.DTYPE_F32, _lib.stream())
+    _lib.check(rc, "coset_column_sum")
+    want, size = x.double().sum(0), x.double().abs().sum(0)
+    assert y[3] == float("inf") and y[5].isnan()
+    fine = want.isfinite()
+    bound = want.abs() * 2.0 ** -24 + size * rows * 2.0 ** -47
+    assert bool(((y.double() - want).abs() <= bound)[fine].all())
