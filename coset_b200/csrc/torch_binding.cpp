@@ -23,6 +23,14 @@ namespace {
 using at::Tensor;
 
 // ---------------------------------------------------------------- small helpers
+// Lets other Python threads run while this one allocates and launches (the first use of the decoder's table also waits for its
+// stream), as ctypes and PyTorch's own functions do.  Nothing inside its scope touches a Python object.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    NoGil() = default;
+    NoGil(const NoGil&) = delete;
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
 void* stream_of(const Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 void* data(const Tensor& t) { return t.defined() && t.numel() > 0 ? t.data_ptr() : nullptr; }
 float* fdata(const Tensor& t) { return (float*)data(t); }
@@ -141,8 +149,11 @@ PyObject* encode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
         TORCH_CHECK_VALUE((int64_t)out.nbytes() == nb * bytes && out.is_contiguous() && out.device() == x.device(),
                           "out has the wrong size, layout or device");
     }
-    check_rc(coset_e8_encode(data(x), dtype_code(x, "x"), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, (int)int_arg(a[7]), data(out),
-                             stream_of(x)), "coset_e8_encode");
+    const int sem = (int)int_arg(a[7]);
+    {
+        NoGil no_gil;
+        check_rc(coset_e8_encode(data(x), dtype_code(x, "x"), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, sem, data(out), stream_of(x)), "coset_e8_encode");
+    }
     if (a[6] != Py_None) written(out);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
@@ -167,8 +178,11 @@ PyObject* decode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
         TORCH_CHECK_VALUE(out.dim() == 2 && out.size(0) == nb && out.size(1) == 8 && out.is_contiguous() && out.device() == codes.device(),
                           "out has the wrong shape, layout or device");
     }
-    check_rc(coset_e8_decode(data(codes), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, COSET_SEM_CORE, data(out), dtype_code(out, "out"),
-                             stream_of(codes)), "coset_e8_decode");
+    {
+        NoGil no_gil;
+        check_rc(coset_e8_decode(data(codes), fdata(s.t), s.mode, nb, s.bpt, (int)q, (int)M, COSET_SEM_CORE, data(out), dtype_code(out, "out"),
+                                 stream_of(codes)), "coset_e8_decode");
+    }
     if (a[7] != Py_None) written(out);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
@@ -185,9 +199,13 @@ PyObject* encode_digits(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t q = int_arg(a[1]), M = int_arg(a[2]);
     code_bytes(q, M);
     c10::cuda::CUDAGuard guard(x.device());
-    Tensor digits = squeeze ? empty({M, 8}, at::kFloat, x) : empty({x.size(0), M, 8}, at::kFloat, x);
-    check_rc(coset_e8_encode_digits_f32(fdata(x), (float)float_arg(a[3]), x.size(0), (int)q, (int)M, fdata(digits), stream_of(x)),
-             "coset_e8_encode_digits_f32");
+    const float beta = (float)float_arg(a[3]);
+    Tensor digits;
+    {
+        NoGil no_gil;
+        digits = squeeze ? empty({M, 8}, at::kFloat, x) : empty({x.size(0), M, 8}, at::kFloat, x);
+        check_rc(coset_e8_encode_digits_f32(fdata(x), beta, x.size(0), (int)q, (int)M, fdata(digits), stream_of(x)), "coset_e8_encode_digits_f32");
+    }
     return THPVariable_Wrap(digits);
     END_HANDLE_TH_ERRORS
 }
@@ -202,10 +220,14 @@ PyObject* decode_digits(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t q = int_arg(a[1]), M = b.size(-2), nb = squeeze ? 1 : b.size(0);
     code_bytes(q, M);
     c10::cuda::CUDAGuard guard(b.device());
-    const Tensor digits = as_f32(b);
-    Tensor out = squeeze ? empty({8}, at::kFloat, b) : empty({nb, 8}, at::kFloat, b);
-    check_rc(coset_e8_decode_digits_f32(fdata(digits), (float)float_arg(a[2]), nb, (int)q, (int)M, fdata(out), stream_of(b)),
-             "coset_e8_decode_digits_f32");
+    const float beta = (float)float_arg(a[2]);
+    Tensor out;
+    {
+        NoGil no_gil;
+        const Tensor digits = as_f32(b);
+        out = squeeze ? empty({8}, at::kFloat, b) : empty({nb, 8}, at::kFloat, b);
+        check_rc(coset_e8_decode_digits_f32(fdata(digits), beta, nb, (int)q, (int)M, fdata(out), stream_of(b)), "coset_e8_decode_digits_f32");
+    }
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
 }
@@ -219,9 +241,13 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t q = int_arg(a[1]);
     code_bytes(q, 2);
     c10::cuda::CUDAGuard guard(x.device());
-    Tensor out = squeeze ? empty({8}, at::kFloat, x) : empty({x.size(0), 8}, at::kFloat, x);
-    check_rc(coset_e8_quantize(data(x), dtype_code(x, "x"), nullptr, COSET_SCALE_NONE, x.size(0), 1, (int)q, 2, 0.0f, data(out),
-                               COSET_DTYPE_F32, nullptr, stream_of(x)), "coset_e8_quantize");
+    Tensor out;
+    {
+        NoGil no_gil;
+        out = squeeze ? empty({8}, at::kFloat, x) : empty({x.size(0), 8}, at::kFloat, x);
+        check_rc(coset_e8_quantize(data(x), dtype_code(x, "x"), nullptr, COSET_SCALE_NONE, x.size(0), 1, (int)q, 2, 0.0f, data(out),
+                                   COSET_DTYPE_F32, nullptr, stream_of(x)), "coset_e8_quantize");
+    }
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
 }
@@ -233,9 +259,13 @@ PyObject* grad_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     nargs_are(n, 4);
     const Tensor &x = tensor_arg(a[0], "grad"), &s = tensor_arg(a[1], "scale"), &out = tensor_arg(a[2], "out");
     const int64_t nb = x.size(0);
-    c10::cuda::CUDAGuard guard(x.device());
-    check_rc(coset_e8_encode(data(x), dtype_code(x, "grad"), fdata(s), COSET_SCALE_MUL_TILE, nb, nb > 0 ? nb : 1, 4, 2,
-                             (int)int_arg(a[3]), data(out), stream_of(x)), "coset_e8_encode");
+    const int sem = (int)int_arg(a[3]);
+    {
+        NoGil no_gil;
+        c10::cuda::CUDAGuard guard(x.device());
+        check_rc(coset_e8_encode(data(x), dtype_code(x, "grad"), fdata(s), COSET_SCALE_MUL_TILE, nb, nb > 0 ? nb : 1, 4, 2, sem, data(out), stream_of(x)),
+                 "coset_e8_encode");
+    }
     written(out);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
@@ -246,9 +276,14 @@ PyObject* decode_mean(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     nargs_are(n, 5);
     const Tensor &codes = tensor_arg(a[0], "codes"), &out = tensor_arg(a[4], "out");
-    c10::cuda::CUDAGuard guard(codes.device());
-    check_rc(coset_e8_decode_mean(data(codes), (int)int_arg(a[1]), int_arg(a[2]), codes.size(1), (float)float_arg(a[3]), data(out),
-                                  dtype_code(out, "out"), stream_of(codes)), "coset_e8_decode_mean");
+    const int64_t world = int_arg(a[1]), nb = int_arg(a[2]);
+    const float scale = (float)float_arg(a[3]);
+    {
+        NoGil no_gil;
+        c10::cuda::CUDAGuard guard(codes.device());
+        check_rc(coset_e8_decode_mean(data(codes), (int)world, nb, codes.size(1), scale, data(out), dtype_code(out, "out"), stream_of(codes)),
+                 "coset_e8_decode_mean");
+    }
     written(out);
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS
@@ -275,15 +310,20 @@ PyObject* vlut_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check_codes(codes);
     const int64_t n_out = codes.size(0), n_in = codes.size(1) * 8;
     TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in, "x must be [T, ", n_in, "], got ", x.sizes());
-    c10::cuda::CUDAGuard guard(x.device());
-    c10::SmallVector<int64_t, 6> shape;
-    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
-    const Tensor beta = as_f32(optional_arg(a[2], "beta")), bias = as_f32(optional_arg(a[4], "bias"));
+    const Tensor beta_arg = optional_arg(a[2], "beta"), bias_arg = optional_arg(a[4], "bias");
+    const int64_t bpt = int_arg(a[3]);
+    const float clip = (float)float_arg(a[5]);
     const int y_code = (int)int_arg(a[6]);
-    Tensor y = empty(shape, scalar_type(y_code), x);
-    check_rc(coset_e8_vlut_gemv(data(codes), fdata(beta), int_arg(a[3]), (int)n_out, (int)n_in, data(x2), dtype_code(x2, "x"), n_in,
-                                (int)x2.size(0), fdata(bias), data(y), y_code, n_out, (float)float_arg(a[5]), stream_of(x)),
-             "coset_e8_vlut_gemv");
+    Tensor y;
+    {
+        NoGil no_gil;
+        c10::cuda::CUDAGuard guard(x.device());
+        c10::SmallVector<int64_t, 6> shape;
+        const Tensor x2 = token_rows(x, n_in, n_out, &shape), beta = as_f32(beta_arg), bias = as_f32(bias_arg);
+        y = empty(shape, scalar_type(y_code), x);
+        check_rc(coset_e8_vlut_gemv(data(codes), fdata(beta), bpt, (int)n_out, (int)n_in, data(x2), dtype_code(x2, "x"), n_in, (int)x2.size(0), fdata(bias),
+                                    data(y), y_code, n_out, clip, stream_of(x)), "coset_e8_vlut_gemv");
+    }
     return THPVariable_Wrap(y);
     END_HANDLE_TH_ERRORS
 }
@@ -296,8 +336,12 @@ PyObject* vlut_layout(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check_codes(codes);
     const int n_out = (int)codes.size(0), n_in = (int)codes.size(1) * 8;
     c10::cuda::CUDAGuard guard(codes.device());
-    Tensor layout = empty({coset_e8_vlut_layout_bytes(n_out, n_in)}, at::kByte, codes);
-    check_rc(coset_e8_vlut_layout(data(codes), n_out, n_in, data(layout), stream_of(codes)), "coset_e8_vlut_layout");
+    Tensor layout;
+    {
+        NoGil no_gil;
+        layout = empty({coset_e8_vlut_layout_bytes(n_out, n_in)}, at::kByte, codes);
+        check_rc(coset_e8_vlut_layout(data(codes), n_out, n_in, data(layout), stream_of(codes)), "coset_e8_vlut_layout");
+    }
     return THPVariable_Wrap(layout);
     END_HANDLE_TH_ERRORS
 }
@@ -305,6 +349,7 @@ PyObject* vlut_layout(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // The product from a layout; `codes` undefined: the layout is trusted.
 Tensor layout_product(const Tensor& x, const Tensor& codes, const Tensor& layout, int64_t n_out, int64_t n_in, const Tensor& beta_arg, int64_t bpt,
                       const Tensor& bias_arg, double clip, int y_code) {
+    NoGil no_gil;
     TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in, "x must be [T, ", n_in, "], got ", x.sizes());
     TORCH_CHECK_VALUE(layout.device() == x.device(), "the weight is on ", layout.device(), ", x on ", x.device());
     TORCH_CHECK_VALUE((int64_t)layout.nbytes() == coset_e8_vlut_layout_bytes((int)n_out, (int)n_in), "the layout is not one of a [", n_out, ", ", n_in, "] weight");
@@ -355,22 +400,26 @@ PyObject* decode_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     check_codes(codes);
     const int64_t n_out = codes.size(0), n_in = codes.size(1) * 8;
     TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == n_in && n_in % 64 == 0, "x must be [T, ", n_in, "] with n_in a multiple of 64, got ", x.sizes());
-    c10::cuda::CUDAGuard guard(x.device());
-    c10::SmallVector<int64_t, 6> shape;
-    const Tensor x2 = token_rows(x, n_in, n_out, &shape);
-    Tensor scratch = optional_arg(a[6], "scratch");
-    if (!scratch.defined()) scratch = empty({n_out * n_in}, at::kBFloat16, x);
-    else
-        TORCH_CHECK_VALUE(scratch.scalar_type() == at::kBFloat16 && scratch.numel() >= n_out * n_in && scratch.is_contiguous() && scratch.device() == x.device(),
-                          "scratch must be a contiguous bfloat16 tensor of at least ", n_out * n_in, " values on ", x.device());
+    Tensor scratch = optional_arg(a[6], "scratch"), status = optional_arg(a[8], "status"), y;
+    const Tensor beta_arg = optional_arg(a[2], "beta"), bias_arg = optional_arg(a[4], "bias");
+    const int64_t bpt = int_arg(a[3]);
+    const float clip = (float)float_arg(a[5]);
     const int y_code = (int)int_arg(a[7]);
-    Tensor y = empty(shape, scalar_type(y_code), x);
-    Tensor status = optional_arg(a[8], "status");
-    if (!status.defined()) status = at::zeros({1}, x.options().dtype(at::kInt));
-    const Tensor beta = as_f32(optional_arg(a[2], "beta")), bias = as_f32(optional_arg(a[4], "bias"));
-    check_rc(coset_e8_decode_gemm(data(codes), fdata(beta), int_arg(a[3]), (int)n_out, (int)n_in, data(x2), n_in, (int)x2.size(0),
-                                  fdata(bias), data(y), y_code, n_out, (float)float_arg(a[5]), data(scratch), (int64_t)scratch.nbytes(),
-                                  (int*)data(status), stream_of(x)), "coset_e8_decode_gemm");
+    {
+        NoGil no_gil;
+        c10::cuda::CUDAGuard guard(x.device());
+        c10::SmallVector<int64_t, 6> shape;
+        const Tensor x2 = token_rows(x, n_in, n_out, &shape);
+        if (!scratch.defined()) scratch = empty({n_out * n_in}, at::kBFloat16, x);
+        else
+            TORCH_CHECK_VALUE(scratch.scalar_type() == at::kBFloat16 && scratch.numel() >= n_out * n_in && scratch.is_contiguous() && scratch.device() == x.device(),
+                              "scratch must be a contiguous bfloat16 tensor of at least ", n_out * n_in, " values on ", x.device());
+        y = empty(shape, scalar_type(y_code), x);
+        if (!status.defined()) status = at::zeros({1}, x.options().dtype(at::kInt));
+        const Tensor beta = as_f32(beta_arg), bias = as_f32(bias_arg);
+        check_rc(coset_e8_decode_gemm(data(codes), fdata(beta), bpt, (int)n_out, (int)n_in, data(x2), n_in, (int)x2.size(0), fdata(bias), data(y), y_code, n_out,
+                                      clip, data(scratch), (int64_t)scratch.nbytes(), (int*)data(status), stream_of(x)), "coset_e8_decode_gemm");
+    }
     return Py_BuildValue("NN", THPVariable_Wrap(y), THPVariable_Wrap(status));
     END_HANDLE_TH_ERRORS
 }
@@ -507,9 +556,16 @@ PyObject* layer_fake_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor& w = tensor_arg(a[0], "weight");
     check_weight(w);
     cuda_arg(a[0], "weight");
-    c10::cuda::CUDAGuard guard(w.device());
-    return THPVariable_Wrap(FakeQuant::apply(w, tensor_arg(a[1], "theta"), tensor_arg(a[2], "beta_min"), tensor_arg(a[3], "beta_range"),
-                                             int_arg(a[4]), int_arg(a[5]), float_arg(a[6]), int_arg(a[7])));
+    const Tensor &theta = tensor_arg(a[1], "theta"), &beta_min = tensor_arg(a[2], "beta_min"), &beta_range = tensor_arg(a[3], "beta_range");
+    const int64_t bpt = int_arg(a[4]), q = int_arg(a[5]), out_code = int_arg(a[7]);
+    const double clip = float_arg(a[6]);
+    Tensor wq;
+    {
+        NoGil no_gil;
+        c10::cuda::CUDAGuard guard(w.device());
+        wq = FakeQuant::apply(w, theta, beta_min, beta_range, bpt, q, clip, out_code);
+    }
+    return THPVariable_Wrap(wq);
     END_HANDLE_TH_ERRORS
 }
 
@@ -520,9 +576,17 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor &x = tensor_arg(a[0], "x"), &w = tensor_arg(a[1], "weight");
     check_weight(w);
     cuda_arg(a[1], "weight");
-    c10::cuda::CUDAGuard guard(w.device());
-    return THPVariable_Wrap(QatLinear::apply(x, w, tensor_arg(a[2], "theta"), maybe_arg(a[3], "bias"), tensor_arg(a[4], "beta_min"),
-                                             tensor_arg(a[5], "beta_range"), int_arg(a[6]), int_arg(a[7]), float_arg(a[8])));
+    const Tensor &theta = tensor_arg(a[2], "theta"), &beta_min = tensor_arg(a[4], "beta_min"), &beta_range = tensor_arg(a[5], "beta_range");
+    const std::optional<Tensor> bias = maybe_arg(a[3], "bias");
+    const int64_t bpt = int_arg(a[6]), q = int_arg(a[7]);
+    const double clip = float_arg(a[8]);
+    Tensor y;
+    {
+        NoGil no_gil;
+        c10::cuda::CUDAGuard guard(w.device());
+        y = QatLinear::apply(x, w, theta, bias, beta_min, beta_range, bpt, q, clip);
+    }
+    return THPVariable_Wrap(y);
     END_HANDLE_TH_ERRORS
 }
 

@@ -424,3 +424,32 @@ def test_scale_beyond_float32(value, same):
     x = torch.randn(64, 8, device="cuda")
     got = e8_encode_packed(x, scale=value, scale_mode=_lib.SCALE_DIV_SCALAR)
     assert torch.equal(got, e8_encode_packed(x, scale=torch.tensor(same, device="cuda"), scale_mode=_lib.SCALE_DIV_SCALAR))
+
+
+def test_other_threads_run_while_a_call_waits_for_the_device(e8):
+    """A launch that waits for room in the device's queue holds no Python lock: another thread keeps ticking meanwhile."""
+    import threading
+    import time
+    x = torch.randn(8, device="cuda")
+    e8.e8_quantize(x, 4)
+    torch.cuda.synchronize()
+    ticks, done = [time.monotonic()], threading.Event()
+
+    def tick():
+        while not done.is_set():
+            time.sleep(0.002)
+            ticks.append(time.monotonic())
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    torch.cuda._sleep(1_200_000_000)  # 0.6 s and more
+    begin = time.monotonic()
+    for _ in range(4000):
+        e8.e8_quantize(x, 4)
+    waited = time.monotonic() - begin
+    done.set()
+    thread.join()
+    torch.cuda.synchronize()
+    if waited < 0.4:
+        pytest.skip("the device's queue took all launches")
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.5 * waited
