@@ -32,7 +32,7 @@
 // bytes, hashes them, and where the hash is not the kept one does its units again with words made from the codes, as the
 // layout kernel makes them.  The hash is a sum of the codes times odd keys modulo 2^64: one changed code always shows, other
 // changes go unseen once in about 2^64.  Price (4096 x 4096, one scale per row with a clamp, 12 weights in turn): 6.1 -> 8.6 us for
-// one token, 10.8 -> 13.0 for 16.  Comparing every unit with a copy of its codes cost more (11.6, 12.9), and so did hashing inside
+// one token, 10.8 -> 12.6 for 16.  Comparing every unit with a copy of its codes cost more (11.6, 12.9), and so did hashing inside
 // the loop over the units, from registers (11.0) or through cp.async (8.8, 13.0): the loop has no registers to spare, which is
 // also why the second time round is a copy of it.
 #include <cuda_bf16.h>
@@ -219,7 +219,7 @@ struct Product {
 };
 
 // Whether this warp's parts of the codes are others than those the layout was made from.
-template <bool WIDE>
+template <bool WIDE, int BATCH>
 __device__ __forceinline__ bool codes_changed(const Product& a, int64_t group, int first, int kw) {
     uint2 sum = make_uint2(0u, 0u);
     if ((threadIdx.x & 31) == 0)
@@ -228,12 +228,12 @@ __device__ __forceinline__ bool codes_changed(const Product& a, int64_t group, i
             sum.x -= h.x;
             sum.y -= h.y;
         }
-    for (int u = first; u < a.units; u += 4 * kw) {
-        uint4 c[4];
+    for (int u = first; u < a.units; u += BATCH * kw) {
+        uint4 c[BATCH];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c[k] = u + k * kw < a.units ? group_codes<WIDE>(a.codes, a.n_out, a.kb, group, u + k * kw) : make_uint4(0u, 0u, 0u, 0u);
+        for (int k = 0; k < BATCH; ++k) c[k] = u + k * kw < a.units ? group_codes<WIDE>(a.codes, a.n_out, a.kb, group, u + k * kw) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) add_hash(sum, hash_codes(c[k], u + k * kw));
+        for (int k = 0; k < BATCH; ++k) add_hash(sum, hash_codes(c[k], u + k * kw));
     }
     sum = warp_sum(sum);
     return (sum.x | sum.y) != 0u;
@@ -319,7 +319,7 @@ __device__ __forceinline__ void load_matrices(uint32_t addr, uint32_t (&r)[4]) {
 
 // CTAs per SM of bf16 tokens: what the loop over the layout needs; the loop over the codes spills instead.
 template <int NT, int P, int WARPS>
-constexpr int kProductCtas = P == 3 ? (NT == 1 ? 2 : 1) : (WARPS == 16 ? 2 : (NT == 1 ? 4 : 3));
+constexpr int kProductCtas = P == 3 ? (NT == 1 ? 2 : 1) : (WARPS == 16 ? 2 : (NT == 1 ? 4 : 2));
 
 template <int NT, int P, bool CLIP, int SCALE, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, kProductCtas<NT, P, WARPS>)
@@ -540,7 +540,7 @@ k_product(const __grid_constant__ Product a) {
         }
     };
     if (group * 16 < a.n_out) {
-        if (a.codes) changed = a.wide_codes ? codes_changed<true>(a, group, first, kw) : codes_changed<false>(a, group, first, kw);
+        if (a.codes) changed = a.wide_codes ? codes_changed<true, NT == 1 ? 4 : 8>(a, group, first, kw) : codes_changed<false, NT == 1 ? 4 : 8>(a, group, first, kw);
         run_units(std::false_type());
     }
     // accumulator layout: [0], [1] = (row g, tokens 2c, 2c + 1); [2], [3] = (row g + 8, same tokens)
