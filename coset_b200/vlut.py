@@ -295,8 +295,11 @@ class E8CodeLinear(nn.Module):
             return self.forward(x.reshape(-1, n_in)).reshape(*x.shape[:-1], self.out_features)
         if dtype is torch.float32:
             return torch.nn.functional.linear(x, self.dense_weight(torch.float32), buf["bias"])
-        b = buf["bias"].to(dtype) if buf["bias"] is not None else None
-        return torch.nn.functional.linear(x, self._dense_bf16().to(dtype), b)
+        b, w = buf["bias"], self._dense_bf16()
+        if (b is not None and dtype is torch.bfloat16 and type(x) is torch.Tensor and torch._C._get_tracing_state() is None
+                and not torch._C._len_torch_function_stack()):
+            return _lib.native().linear_cast_bias(x, w, b)
+        return torch.nn.functional.linear(x, w.to(dtype), b.to(dtype) if b is not None else None)
 
 
 def out_feature_shard(n_out: int, world: int, rank: int):

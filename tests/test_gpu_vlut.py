@@ -620,3 +620,19 @@ def test_one_or_two_float32_tokens_read_the_codes(n_out, n_in, row, T, dtype, co
     shard = E8CodeLinear(layer.codes[:n_out // 2], beta[:beta.numel() // 2], bpt, None)
     shard._rows = n_out
     assert torch.equal(shard(x), layer(x)[:, :n_out // 2])
+
+
+@pytest.mark.parametrize("bias_dtype", [torch.float32, torch.bfloat16, torch.float64])
+def test_library_path_with_biases_of_other_types_and_gradients(bias_dtype):
+    """The bias is rounded to bf16 in the call, whatever it is; the product stays differentiable in the activations, under vmap too."""
+    layer, _ = _kept_copy_layer(64, 256)
+    x = torch.randn(32, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+    layer.bias = torch.randn(128, device="cuda").to(bias_dtype)[::2]
+    dense, doubled = layer.dense_weight(torch.bfloat16), x.detach().view(2, 32, 128).repeat(1, 1, 2)
+    for bias in (layer.bias, layer.bias.contiguous()):
+        layer.bias = bias
+        plain = lambda v: torch.nn.functional.linear(v, dense, bias.to(torch.bfloat16))
+        y, want = layer(x), plain(x)
+        assert torch.equal(y, want)
+        assert torch.equal(torch.autograd.grad(y.float().sum(), x)[0], torch.autograd.grad(want.float().sum(), x)[0])
+        assert torch.equal(torch.vmap(layer)(doubled), torch.vmap(plain)(doubled))
