@@ -19,6 +19,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libcoset_b200.so")
 TORCH_PATH = os.path.join(LIB_DIR, "_coset_torch.so")
 TORCH_SOURCE = "torch_binding.cpp"
+TORCH_STAMP = os.path.join(LIB_DIR, "_coset_torch.version")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = [
@@ -61,6 +62,20 @@ def _run(cmd, verbose):
     subprocess.check_call(cmd)
 
 
+def _torch_stamp():
+    """What the PyTorch module is bound to besides its source: its ABI follows the version of torch and of Python."""
+    import torch
+    return f"torch {torch.__version__}, Python {sys.version.split()[0]}\n"
+
+
+def _stamp_is(text):
+    try:
+        with open(TORCH_STAMP) as f:
+            return f.read() == text
+    except OSError:
+        return False
+
+
 def _build_torch_module(verbose):
     import torch
     from torch.utils import cpp_extension
@@ -91,8 +106,11 @@ def build(force=False, verbose=False):
     if force or not _newer(LIB_PATH, objs):
         _run([_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"], verbose)
     # the module finds the library's functions at load time: only its own source and the header matter to it
-    if force or not _newer(TORCH_PATH, [os.path.join(CSRC, TORCH_SOURCE), header, __file__]):
+    stamp = _torch_stamp()
+    if force or not _stamp_is(stamp) or not _newer(TORCH_PATH, [os.path.join(CSRC, TORCH_SOURCE), header, __file__]):
         _build_torch_module(verbose)
+        with open(TORCH_STAMP, "w") as f:
+            f.write(stamp)
     return LIB_PATH
 
 

@@ -137,3 +137,17 @@ def test_low_precision_parameters_are_refused_before_any_launch(dtype):
         d4_fake_quantize(w8, beta, 4)
     with pytest.raises(TypeError, match="float32"):
         d4_quantize(torch.zeros(4, 4, dtype=dtype))
+
+
+def test_torch_module_is_built_again_for_another_torch(monkeypatch, tmp_path):
+    """The module's ABI follows the installed torch and Python: a module of another version counts as out of date, one of this not."""
+    from coset_b200 import build
+    build.build()
+    built = []
+    monkeypatch.setattr(build, "TORCH_STAMP", str(tmp_path / "version"))
+    monkeypatch.setattr(build, "_build_torch_module", built.append)
+    (tmp_path / "version").write_text("torch 1.0\n")
+    build.build()
+    assert built == [False]
+    build.build()
+    assert built == [False]
