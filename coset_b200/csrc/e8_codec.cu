@@ -218,7 +218,7 @@ k_encode_q4m2(const void* __restrict__ x, const float* __restrict__ scale, e8::T
     __stcs(codes + b, e8::encode_q4m2<LITERAL>(v));
 }
 
-// Queued encoder (the production path for q=4, M=2).
+// Queued encoder: the fused round trip and the digits of q=4, M=2 (codes alone: k_encode_q4m2_listed below).
 //
 // Warps are persistent; one loop iteration of a warp covers ROWS * 32 consecutive blocks,
 // one row per lane and sub-step.  Every lane runs the cheapest tier (level_fast2_q4: one rounding
@@ -233,11 +233,7 @@ k_encode_q4m2(const void* __restrict__ x, const float* __restrict__ scale, e8::T
 // round trip per 32 deferred blocks -- and encodes it from scratch with the always-valid tiers.
 // This also serves an overloaded quantiser, where most blocks need the top level: the queue then
 // fills every iteration and is drained by full warps.
-// SAT: every scaled coordinate is first clamped to +-kSaturate, which keeps the two-level code from
-// wrapping around (the top level stays the origin); only deferred blocks can exceed the bound, so the
-// clamp costs nothing on the common path.
 constexpr int kEncWarps = kThreads / 32;
-constexpr float kSaturate = 3.9f;  // 8 * 3.9 / 4 < 7.96 and 3.9 / 4 < 1.96: level 1 of a clamped block is the origin
 
 // Rows per lane and iteration of the encoders: three keep the loads of the later rows behind the arithmetic of the
 // earlier ones (four at 85 registers and 3 CTAs per SM were 5 % slower); one where three would leave resident CTAs of the
@@ -266,7 +262,7 @@ __device__ __forceinline__ void store_digits(float* __restrict__ digits, int64_t
     e8::Row8<0>::store(digits, row, f);
 }
 
-template <int DT, int MODE, int KIND, int DTO, bool SAT, int ROWS>
+template <int DT, int MODE, int KIND, int DTO, int ROWS>
 __global__ void __launch_bounds__(kThreads, 4)
 k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n,
                      uint32_t* __restrict__ codes, const uint2* __restrict__ table, void* __restrict__ out, float value) {
@@ -303,10 +299,7 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
             e8::Row8<DT>::load(x, b, v);
             const float s = scale_of(b);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                v[i] = scale_in<MODE>(v[i], s);
-                if (SAT) v[i] = fminf(fmaxf(v[i], -kSaturate), kSaturate);  // NaN -> -kSaturate: finite, harmless
-            }
+            for (int i = 0; i < 8; ++i) v[i] = scale_in<MODE>(v[i], s);
             emit(b, e8::finish_block_q4(v, 0u, 0), s);
         }
         count -= take;
@@ -397,7 +390,11 @@ __device__ __forceinline__ uint32_t level_any_q4(const float (&x)[8], float amax
     return e8::level_slow_q4(x, s1 == s1 && s1 - s1 == 0.0f ? amax : __int_as_float(0x7fc00000));
 }
 
-// ROWS: rows per lane and iteration.
+// ROWS: rows per lane and iteration.  SAT: every scaled coordinate is first clamped to +-kSaturate, which keeps the two-level
+// code from wrapping around (the top level stays the origin); only deferred blocks can exceed the bound, so the clamp costs
+// nothing on the common path.
+constexpr float kSaturate = 3.9f;  // 8 * 3.9 / 4 < 7.96 and 3.9 / 4 < 1.96: level 1 of a clamped block is the origin
+
 template <int DT, int MODE, bool SAT, int ROWS>
 __global__ void __launch_bounds__(kThreads, 4)
 k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n, uint32_t* codes) {
@@ -867,7 +864,7 @@ int coset_e8_quantize(const void* x, int x_dtype, const float* scale, int scale_
         if (!table) return COSET_E_STATE;
         int rows;
         const unsigned qgrid = encoder_grid(n_blocks, &rows);
-        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (rows == 3 ? (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, false, 3><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)) : (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, false, 1><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip))))))
+        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (rows == 3 ? (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, 3><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)) : (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, 1><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip))))))
     } else if (q <= 4) {
         DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_quantize_generic<DTI, DTO, MODE, 2><<<grid, kThreads, 0, st>>>(x, scale, td, n_blocks, q, M, clip, out, codes_out)))))
     } else {
@@ -906,7 +903,7 @@ int coset_e8_encode_digits_f32(const float* x, float beta, int64_t n_blocks, int
         int rows;
         const unsigned grid = encoder_grid(n_blocks, &rows);
         // two rows where the rule says three: with three, 104 bytes of registers spill (2^20 blocks 60 -> 54 us, both calls)
-#define DIGITS_AS(MODE, ROWS) k_encode_q4m2_queued<0, MODE, kDigits, 0, false, ROWS><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, beta)
+#define DIGITS_AS(MODE, ROWS) k_encode_q4m2_queued<0, MODE, kDigits, 0, ROWS><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, beta)
         if (beta == 1.0f) {  // x / 1 is x
             if (rows == 3) DIGITS_AS(COSET_SCALE_NONE, 2); else DIGITS_AS(COSET_SCALE_NONE, 1);
         } else {
