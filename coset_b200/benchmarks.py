@@ -159,8 +159,8 @@ def iter_vlut(tilings=("block", "row")):
             flops = 2.0 * T * n * n
             rec = {"bench": "vlut_matmul", "tiling": tiling, "T": T, "shape": [n, n], "ms": ms,
                    "tokens_per_s": T / (ms * 1e-3),
-                   "path": ("E8CodeLinear default: code-domain kernel" if T <= 64 else
-                            "E8CodeLinear default: cached dense bf16 copy + library GEMM" if T < lin.PAIR_GEMM_MIN_T else
+                   "path": ("E8CodeLinear under capture: code-domain kernel" if T <= 64 else
+                            "E8CodeLinear under capture: the weight decoded with the call + library GEMM" if T < lin.PAIR_GEMM_MIN_T else
                             "E8CodeLinear default: decode + tcgen05 cta_group::2 GEMM, bf16 result"),
                    "timing": "CUDA graph replay" if T <= 256 else "CUDA events over eager calls",
                    "peaks": src}
@@ -170,6 +170,12 @@ def iter_vlut(tilings=("block", "row")):
             else:
                 rec.update({"bound": "tensor", "TFLOPs": flops / (ms * 1e-3) / 1e12, "frac": flops / (ms * 1e-3) / 1e12 / tf})
             yield rec
+            if T < lin.PAIR_GEMM_MIN_T:  # eager calls take the copies that the layer keeps
+                mse = cuda_time(lambda: lin(x), iters=200)
+                yield {"bench": "vlut_matmul", "tiling": tiling, "T": T, "shape": [n, n], "ms": mse, "tokens_per_s": T / (mse * 1e-3),
+                       "path": ("E8CodeLinear default: byte layout checked against the codes" if T <= 64 else
+                                "E8CodeLinear default: cached dense bf16 copy + library GEMM"),
+                       "timing": "CUDA events over eager calls", "peaks": src}
             if T >= lin.PAIR_GEMM_MIN_T:  # the library path beside it
                 dense = lin._dense_bf16()
                 msl = cuda_time(lambda: torch.nn.functional.linear(x, dense), iters=10)
