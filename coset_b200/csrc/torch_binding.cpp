@@ -520,7 +520,10 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         FakeQuant::launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, x.scalar_type(), wq, codes, beta, b, b16);
         if (b16.defined()) b = b16;
         Tensor y = at::linear(x, wq, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
-        ctx->save_for_backward({x, w, theta, beta, codes, wq});
+        // x serves the gradients of the weight and its scale, wq that of x: a frozen layer does not hold on to its input
+        const bool weights = weight.requires_grad() || theta.requires_grad();
+        ctx->save_for_backward({weights ? x : Tensor(), w, theta, beta, codes, x.requires_grad() ? wq : Tensor()});
+        ctx->saved_data["x_type"] = (int64_t)x.scalar_type();
         ctx->saved_data["range"] = beta_range;
         ctx->saved_data["min"] = beta_min;
         ctx->saved_data["bpt"] = bpt;
@@ -532,21 +535,25 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const auto saved = ctx->get_saved_variables();
         const Tensor &x = saved[0], &w = saved[1], &theta = saved[2], &beta = saved[3], &codes = saved[4];
-        c10::cuda::CUDAGuard guard(x.device());
+        c10::cuda::CUDAGuard guard(w.device());
         const int64_t bpt = ctx->saved_data["bpt"].toInt(), q = ctx->saved_data["q"].toInt();
         const double clip = ctx->saved_data["clip"].toDouble();
         const Tensor range = ctx->saved_data["range"].toTensor();
         Tensor wq = saved[5];
         // create_graph: the gradient of x has to depend on the weight, so the weight is quantised again under autograd
-        if (at::GradMode::is_enabled())
+        if (at::GradMode::is_enabled() && ctx->needs_input_grad(0))
             wq = FakeQuant::apply(w, theta, ctx->saved_data["min"].toTensor(), range, bpt, q, clip,
-                                  (int64_t)(x.scalar_type() == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16));
-        const Tensor g2 = grads[0].reshape({-1, w.size(0)}), x2 = x.reshape({-1, w.size(1)});
+                                  (int64_t)((at::ScalarType)ctx->saved_data["x_type"].toInt() == at::kFloat ? COSET_DTYPE_F32 : COSET_DTYPE_BF16));
+        const Tensor g2 = grads[0].reshape({-1, w.size(0)});
         variable_list out(9);
-        if (ctx->needs_input_grad(0)) out[0] = at::mm(g2, wq).view(x.sizes());
+        if (ctx->needs_input_grad(0)) {
+            c10::SmallVector<int64_t, 6> x_shape(grads[0].sizes().begin(), grads[0].sizes().end());
+            x_shape.back() = w.size(1);
+            out[0] = at::mm(g2, wq).view(x_shape);
+        }
         const bool need_theta = ctx->needs_input_grad(2);
         if (ctx->needs_input_grad(1) || need_theta) {
-            auto r = FakeQuant::backward_launch(at::mm(g2.t(), x2), w, theta, beta, codes, range, bpt, q, clip, need_theta);
+            auto r = FakeQuant::backward_launch(at::mm(g2.t(), x.reshape({-1, w.size(1)})), w, theta, beta, codes, range, bpt, q, clip, need_theta);
             out[1] = r.first;
             out[2] = r.second;
         }

@@ -426,3 +426,27 @@ def test_column_sum_of_float32_is_rounded_once(rows, cols):
     fine = want.isfinite()
     bound = want.abs() * 2.0 ** -24 + size * rows * 2.0 ** -47
     assert bool(((y.double() - want).abs() <= bound)[fine].all())
+
+
+@pytest.mark.parametrize("frozen,kept", [(True, False), (False, True)])
+def test_frozen_layer_does_not_hold_on_to_its_input(frozen, kept):
+    """The input serves the gradients of the weight and its scale alone: with both frozen it is free after the forward pass, and
+    the gradients of the bias and of what came before are what they are with a trained weight."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(256, 64, device="cuda")
+    with torch.no_grad():
+        layer.weight.copy_(torch.randn(64, 256) * 20.0)
+    layer.weight.requires_grad_(not frozen)
+    layer.theta_beta.requires_grad_(not frozen)
+    x = torch.randn(4096, 256, device="cuda").requires_grad_()
+    layer(x * 2).sum().backward()
+    want, bias = x.grad.clone(), layer.bias.grad.clone()
+    x.grad = layer.bias.grad = None
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    y = layer(x * 2)
+    held = torch.cuda.memory_allocated() - before - y.numel() * 4
+    assert (held >= x.numel() * 4) == kept, held
+    y.sum().backward()
+    assert torch.equal(x.grad, want) and torch.equal(layer.bias.grad, bias)
+    assert (layer.weight.grad is None) == frozen
