@@ -183,8 +183,10 @@ class E8CodeLinear(nn.Module):
 
     def dense_weight(self, dtype=torch.float32) -> torch.Tensor:
         """Wq = clamp(decode(codes) / beta) as a dense [n_out, n_in] tensor."""
+        # rounding to bf16 keeps the order, so the clamp of the rounded weights is the rounded clamp
+        first = torch.float32 if self.weight_clip_value > 0 and dtype is not torch.bfloat16 else dtype
         w = e8_decode_packed(self.codes.view(-1), 4, 2, scale=self.beta, scale_mode=_lib.SCALE_MUL_TILE,
-                             blocks_per_tile=self.blocks_per_tile, dtype=torch.float32 if self.weight_clip_value > 0 else dtype)
+                             blocks_per_tile=self.blocks_per_tile, dtype=first)
         if self.weight_clip_value > 0:
             w = w.clamp_(-self.weight_clip_value, self.weight_clip_value).to(dtype)
         return w.view(self.out_features, self.in_features)

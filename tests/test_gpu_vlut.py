@@ -636,3 +636,11 @@ def test_library_path_with_biases_of_other_types_and_gradients(bias_dtype):
         assert torch.equal(y, want)
         assert torch.equal(torch.autograd.grad(y.float().sum(), x)[0], torch.autograd.grad(want.float().sum(), x)[0])
         assert torch.equal(torch.vmap(layer)(doubled), torch.vmap(plain)(doubled))
+
+
+@pytest.mark.parametrize("clip", [0.05, 0.02, 0.0625, 1e-3, 2.0, float("inf")])
+def test_dense_bf16_weight_is_the_rounded_clamp(clip):
+    layer, _ = _kept_copy_layer(64, 4096, weight_clip_value=clip)
+    beta = layer.beta.clone()
+    layer.beta.copy_(beta * (0.5 + torch.rand_like(beta)))
+    assert torch.equal(layer.dense_weight(torch.bfloat16), layer.dense_weight(torch.float32).to(torch.bfloat16))
