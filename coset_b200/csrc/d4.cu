@@ -104,7 +104,7 @@ __device__ __forceinline__ void d4_fake_quant_block(const float (&w)[4], float b
     d4_projection(xs, p);
     if (SCALED) {
         // p / beta: for integer numerators up to 64 the sequence q0 = p r, q = fma(fma(-q0, beta, p), r, q0)
-        // with r = RN(1 / beta) is the correctly rounded quotient for every float32 significand of
+        // with r = RN(1 / beta) (P. Markstein, IBM J. Res. Dev. 34, 1990) is the correctly rounded quotient for every float32 significand of
         // beta (checked exhaustively on the CPU) while beta stays far from the exponent limits;
         // anything else takes the IEEE division.
         float amax = fmaxf(fmaxf(fabsf(p[0]), fabsf(p[1])), fmaxf(fabsf(p[2]), fabsf(p[3])));

@@ -323,7 +323,7 @@ __device__ __forceinline__ void twice_from_packed(uint32_t e0, uint32_t e1, floa
 //   MODE 1: x_hat * s                  (coset/core/e8/codecs.py:175)   = RN(v2 * (s/2))
 //   MODE 2: x_hat / s                  (coset/core/layers.py:455-460)  = RN(v2 / (2 s))
 // For MODE 2 the quotient is formed as q0 = v2*r, q = fma(fma(-q0, 2s, v2), r, q0) with
-// r = RN(1/(2s)); for the integer numerators that occur (|v2| <= 55) this equals the correctly
+// r = RN(1/(2s)) (P. Markstein, IBM J. Res. Dev. 34, 1990); for the integer numerators that occur (|v2| <= 55) this equals the correctly
 // rounded IEEE quotient for every float32 significand of s (checked exhaustively on the CPU),
 // as long as s is far from the exponent limits -- outside that range the IEEE division is used.
 template <int MODE>

@@ -127,7 +127,7 @@ k_decode_mean(const uint32_t* __restrict__ codes, PeerStreams peers, int world, 
 // entries another, and sums of up to four such pairs stay inside 4-bit lanes (4 x 3 = 12), of eight inside bytes.
 // Streams beyond `world` are all-zero codes, whose residual is 0.  A block with a non-zero top-level word or a marked
 // entry in any stream is summed by the general routine.  The quotient v / (2 d) is formed with one corrected
-// multiplication: q0 = v r, q = q0 + r (v - 2 d q0) with r = RN(1 / 2 d) equals the IEEE quotient for every float32
+// multiplication (P. Markstein, IBM J. Res. Dev. 34, 1990): q0 = v r, q = q0 + r (v - 2 d q0) with r = RN(1 / 2 d) equals the IEEE quotient for every float32
 // significand and every integer |v| <= 1024 (exhaustive check on the CPU), and |v| <= 16 * 55 here.
 constexpr int kCompactThreads = 1024;
 constexpr int kCompactMaxWorld = 16;
