@@ -101,7 +101,9 @@ class E8CodeLinear(nn.Module):
     stays on the code-domain kernels (9.7-23 us).
     A call under graph capture reads the codes, scales and bias themselves (it decodes the weight where it would use the dense
     copy), so that a replay follows writes to them and reads nothing that a later call gives back.  The dense copy follows
-    writes that PyTorch's version counters show; see forget_copies for the others.
+    writes that PyTorch's version counters show; see forget_copies for the others.  The kernels of the two routes add up in
+    different orders (and for 3-16 bf16 tokens the one that reads the codes rounds the scaled weights to bf16), so a call and its
+    replay agree to the precision of the type, not to the bit.
     small_t_max defaults to 16 ("auto", "cublas") or 48 ("tcgen05"): measured on a 4096 x 4096 layer the
     code-domain kernels take 9.7 / 23 / 44 / 86 us for 1 / 16 / 32 / 64 tokens (they re-read and re-decode the
     codes for every 16 tokens), the library on the cached copy 7-13 us, the fused kernel 64 us.
