@@ -172,10 +172,13 @@ def iter_vlut(tilings=("block", "row")):
             yield rec
             if T < lin.PAIR_GEMM_MIN_T:  # eager calls take the copies that the layer keeps
                 mse = cuda_time(lambda: lin(x), iters=200)
+                by = wbytes + n * n + T * n * 4  # codes, scales, layout, activations and result
                 yield {"bench": "vlut_matmul", "tiling": tiling, "T": T, "shape": [n, n], "ms": mse, "tokens_per_s": T / (mse * 1e-3),
                        "path": ("E8CodeLinear default: byte layout checked against the codes" if T <= 64 else
                                 "E8CodeLinear default: cached dense bf16 copy + library GEMM"),
-                       "timing": "CUDA events over eager calls", "peaks": src}
+                       "timing": "CUDA events over eager calls", "peaks": src,
+                       **({"bound": "hbm", "GBps": by / (mse * 1e-3) / 1e9, "frac": by / (mse * 1e-3) / 1e9 / hbm} if T <= 64 else
+                          {"bound": "tensor", "TFLOPs": flops / (mse * 1e-3) / 1e12, "frac": flops / (mse * 1e-3) / 1e12 / tf})}
             if T >= lin.PAIR_GEMM_MIN_T:  # the library path beside it
                 dense = lin._dense_bf16()
                 msl = cuda_time(lambda: torch.nn.functional.linear(x, dense), iters=10)
