@@ -5,8 +5,7 @@
 // (32 MiB for a 4096 x 4096 layer against 126 MiB of L2), and nothing of it has to survive the call, so the
 // layer keeps 4 bits per weight in HBM.  Against the single-launch kernel of e8_dequant_gemm.cu this moves the
 // decode out of the GEMM's K loop: no producer warps, both operands arrive by TMA, and the results are the same
-// bits.  Measured on a 4096 x 4096 layer: 1.30 PFLOP/s at 8192 tokens and 1.47 at 16384 (decode included),
-// against 0.91 / 1.04 for the single-launch kernel.
+// bits.  Measured on a 4096 x 4096 layer (graph replays, decode included): 101 us at 4096 tokens and 192 at 8192.
 //
 // The GEMM runs on pairs of CTAs (a cluster of two on the two SMs of a TPC) that share one instruction
 // stream of tcgen05.mma.cta_group::2: M = 256 tokens x N = 256 features x K = 16 per instruction.  CTA r of
@@ -23,10 +22,13 @@
 // per stage round trip held the K loop at 1900 cycles per step against 1049 of tensor work:
 //   "full"  lives in rank 0 alone and counts the bytes of BOTH CTAs' tiles: rank 1's loads are cta_group::2 TMA
 //           copies that land in rank 1's shared memory and complete on rank 0's barrier;
-//   "empty" (and "done") are signalled by two tcgen05.commit, one onto each CTA's barrier (the operand is a
-//           shared::cluster address, rank 1's comes from mapa).
+//   "empty" (and "done") are signalled by one tcgen05.commit that arrives on the barrier of either CTA.
+//   The issuing code sits behind elect.sync and on values that a shuffle has made uniform: behind a comparison of the lane's number a
+//   K step's four instructions and its commits took 450 cycles to issue, now 200, and the K loop runs at the tensor cores' rate
+//   (1060 cycles a step instead of about 1400); one multicast commit releases the stage in both CTAs.  With the epilogue below
+//   (16-byte stores) 4096 tokens took 88 us instead of 94 in short runs; in long ones the 1000 W limit lowers the clock and 1-2 % are left.
 // Every wait is bounded in time; on expiry the kernel sets the status word, skips its stores, frees its tensor
-// memory and returns.  No multicast of any kind: every TMA load lands in the CTA that issued it.
+// memory and returns.  Every TMA load lands in the CTA that issued it.
 // Measured and not kept: persistent clusters walking over tiles, (a) with 256-token tiles and the two accumulators
 // alternating so that the epilogue runs under the next tile's main loop -- 0.232 / 0.444 ms at 8192 / 16384 tokens
 // against 0.207 / 0.365 here (a third more operand bytes per flop through L2), though faster below 2048 tokens,
@@ -75,73 +77,19 @@ constexpr int PAIR_N = 256;    // features per pair = N of one instruction
 constexpr int HALF_N = 128;    // weight rows held by one CTA
 constexpr int STAGES = 4;
 constexpr int STAGE_BYTES = MSUB * TILE_BYTES + HALF_N * BK * 2;  // 48 KiB
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 128 /*barriers, tmem slot*/;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 128 /*barriers, tmem slot*/ + PAIR_N * 4 /*bias*/;
 constexpr int EPI_WARPS = 16, TMA_WARP = 16, MMA_WARP = 17;
 constexpr int THREADS = 18 * 32;
 constexpr uint32_t TMEM_COLS = MSUB * PAIR_N;  // 512: the whole tensor memory of the SM
 // kind::f16 instruction descriptor: fp32 accumulate, bf16 x bf16, both K-major, N = 256, M = 256 over the pair
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PAIR_N >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
-static_assert(EPI_WARPS * 32 * 33 * 4 <= STAGES * STAGE_BYTES, "epilogue scratch inside the idle stages");
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// Address of this CTA's shared-memory location `addr` in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// TMA tile load whose completion is counted on a barrier of the pair's OTHER CTA (allowed with cta_group::2);
-// the tile itself lands in this CTA.  No multicast.
-__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap* map, int k0, int row, uint32_t pair_bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(map), "r"(k0), "r"(row), "r"(pair_bar) : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The bounded wait with cluster-scope acquire, for phases that the other CTA of the pair completes.
-// SLEEP: nanoseconds between polls, for warps that wait through the whole main loop.
-template <int SLEEP = 0>
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint64_t t0 = 0;
-    for (int it = 0; it < (1 << 24); ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-        if (SLEEP > 0) __nanosleep(SLEEP);
-        if ((it & 63) == 63) {
-            uint64_t now;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > 200000000ull) return false;
-        }
-    }
-    return false;
-}
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
+static_assert(EPI_WARPS * 32 * 128 <= STAGES * STAGE_BYTES, "epilogue scratch inside the idle stages");
 
 template <typename YT>  // float or __nv_bfloat16 result
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 k_gemm_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, int N, int K, int T,
-            const float* __restrict__ bias, YT* __restrict__ y, int64_t ldy, int* __restrict__ status) {
+            const float* __restrict__ bias, YT* __restrict__ y, int64_t ldy, int vector_rows, int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // the same offset in both CTAs: same kernel, same dynamic size
@@ -151,10 +99,9 @@ k_gemm_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
     const uint32_t full_base = bar_base + 8 * STAGES, done_bar = bar_base + 16 * STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + STAGES * STAGE_BYTES + 16 * STAGES + 8);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t crank = cluster_rank();
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // the shuffle makes the role uniform for the compiler
+    const uint32_t crank = __shfl_sync(0xffffffffu, cluster_rank(), 0);
     const bool leader = crank == 0;
-    const uint32_t other_base = peer_smem(base, crank ^ 1u);  // the partner's `base`; offsets carry over
     const uint32_t leader_full = peer_smem(base, 0u) + (full_base - base);
     const int tile_n = blockIdx.x >> 1, tile_m = blockIdx.y;
     const int tok0 = tile_m * (2 * MSUB * BM) + (int)crank * (MSUB * BM);  // this CTA's 2 x 128 tokens
@@ -176,15 +123,17 @@ k_gemm_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
     __syncthreads();
     cluster_sync();  // the partner's barriers exist before anything arrives on them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_d = *tmem_slot;
+    const uint32_t tmem_d = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
+    float* bias_s = reinterpret_cast<float*>(gen + STAGES * STAGE_BYTES + 128);
+    if (bias && tid < PAIR_N) bias_s[tid] = tile_n * PAIR_N + tid < N ? __ldg(bias + tile_n * PAIR_N + tid) : 0.0f;
 
     const int KT = K / BK;
     if (warp == TMA_WARP) {
         for (int kt = 0; kt < KT; ++kt) {
             const int s = kt % STAGES;
             if (kt >= STAGES) ok = ok && mbar_wait_cluster(bar_base + 8 * s, (uint32_t)((kt / STAGES - 1) & 1));
-            if (lane == 0) {  // rows beyond T or N arrive as zeros
+            if (elect_one()) {  // rows beyond T or N arrive as zeros
                 const uint32_t stage_addr = base + s * STAGE_BYTES;
                 const uint32_t bar = leader_full + 8 * s;  // rank 0's barrier, from either CTA
                 if (leader) mbar_arrive_expect_tx(full_base + 8 * s, (uint32_t)(2 * STAGE_BYTES));
@@ -202,7 +151,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
             const int s = kt % STAGES;
             ok = ok && mbar_wait_cluster(full_base + 8 * s, (uint32_t)((kt / STAGES) & 1));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t a_lo = desc_lo0 + (uint32_t)(s * (STAGE_BYTES >> 4)), b_lo = a_lo + (uint32_t)((MSUB * TILE_BYTES) >> 4);
                 const uint32_t first = kt > 0 ? 1u : 0u;
 #pragma unroll
@@ -212,43 +161,73 @@ k_gemm_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                         umma_f16_pair(tmem_d + (uint32_t)(a * PAIR_N), make_desc(a_lo + (uint32_t)(a * (TILE_BYTES >> 4) + k * 2), desc_hi),
                                       make_desc(b_lo + (uint32_t)(k * 2), desc_hi), IDESC, k > 0 ? 1u : first);
                 }
-                // both CTAs' stage s may be overwritten once these MMAs retire: one commit per CTA's barrier
-                umma_commit_pair(bar_base + 8 * s);
-                umma_commit_pair(other_base + (bar_base - base) + 8 * s);
-                if (kt == KT - 1) {  // ... and the accumulators of both CTAs are complete
-                    umma_commit_pair(done_bar);
-                    umma_commit_pair(other_base + (done_bar - base));
-                }
+                umma_commit_pair(bar_base + 8 * s, 3);             // both CTAs' stage s may be overwritten once these MMAs retire
+                if (kt == KT - 1) umma_commit_pair(done_bar, 3);  // ... and the accumulators of both CTAs are complete
             }
             __syncwarp();
         }
     }
     if (!ok && status) atomicExch(status, 1);
     // always: the MMAs must have retired before the tensor memory is read or freed
-    ok = mbar_wait_cluster<128>(done_bar, 0u) && ok;
+    ok = __all_sync(0xffffffffu, mbar_wait_cluster<128>(done_bar, 0u) && ok);
+    __syncthreads();  // the bias is in shared memory
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // epilogue: warp w reads tensor-memory lanes 32*(w%4).. of both accumulators, 32 columns at a time (one
-    // thread = one token row, 32 consecutive features), and transposes each 32 x 32 piece through shared memory
-    // (the stages are idle by now) so that every global store instruction writes 128 contiguous bytes of one row
+    // epilogue: warp w reads tensor-memory lanes 32*(w%4).. of both accumulators, 128 bytes of result at a time (one
+    // thread = one token row, 32 or 64 consecutive features), and transposes each piece through shared memory (the stages are
+    // idle by now) in 16-byte chunks, the chunk's place exclusive-ored with the row so that neither side meets bank
+    // conflicts: eight lanes then store the 128 bytes of one row.  Results whose rows are not made of 16-byte chunks are stored one by one.
     if (warp < EPI_WARPS) {
+        constexpr int COLS = 128 / (int)sizeof(YT);
         const int q = warp & 3, grp = warp >> 2;
-        float* scr = reinterpret_cast<float*>(gen) + warp * (32 * 33);
+        uint4* scr = reinterpret_cast<uint4*>(gen) + warp * (32 * 8);
         for (int a = 0; a < MSUB; ++a) {
             const int tok_first = tok0 + a * BM + q * 32;
             if (tok_first >= T) continue;  // warp-uniform
-            for (int col0 = grp * 32; col0 < PAIR_N; col0 += 4 * 32) {
-                uint32_t r[32];
-                tmem_ld32(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * PAIR_N + col0), r);
+            const int rows = T - tok_first < 32 ? T - tok_first : 32;
+            for (int col0 = grp * COLS; col0 < PAIR_N; col0 += 4 * COLS) {
+                const int n0 = tile_n * PAIR_N + col0;
+                if (n0 >= N) break;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) scr[lane * 33 + j] = __uint_as_float(r[j]);
+                for (int part = 0; part < COLS / 32; ++part) {
+                    uint32_t r[32];
+                    tmem_ld32(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * PAIR_N + col0 + 32 * part), r);
+                    if (bias) {
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4) {
+                            const float4 b = *reinterpret_cast<const float4*>(bias_s + col0 + 32 * part + j);
+                            r[j] = __float_as_uint(__uint_as_float(r[j]) + b.x); r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + b.y);
+                            r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + b.z); r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + b.w);
+                        }
+                    }
+                    if constexpr (sizeof(YT) == 4) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) scr[lane * 8 + (j ^ (lane & 7))] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                    } else {
+                        uint32_t h[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) h[j] = pack_bf16x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) scr[lane * 8 + ((4 * part + j) ^ (lane & 7))] = make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
+                    }
+                }
                 __syncwarp();
-                const int n = tile_n * PAIR_N + col0 + lane;
-                const float bv = (bias && n < N) ? __ldg(bias + n) : 0.0f;
-                if (ok && n < N) {
-                    YT* dst = y + (int64_t)tok_first * ldy + n;
-                    const int rows = T - tok_first < 32 ? T - tok_first : 32;
-                    for (int rr = 0; rr < rows; ++rr) dst[(int64_t)rr * ldy] = (YT)(scr[rr * 33 + lane] + bv);
+                if (ok && vector_rows) {
+                    const int chunk = lane & 7, n = n0 + chunk * (16 / (int)sizeof(YT));
+                    if (n < N) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int rr = 4 * i + (lane >> 3);
+                            if (rr < rows) *reinterpret_cast<uint4*>(y + (int64_t)(tok_first + rr) * ldy + n) = scr[rr * 8 + (chunk ^ (rr & 7))];
+                        }
+                    }
+                } else if (ok) {
+                    for (int rr = 0; rr < rows; ++rr)
+#pragma unroll
+                        for (int part = 0; part < COLS / 32; ++part) {
+                            const int at = 32 * part + lane, chunk = at / (16 / (int)sizeof(YT));
+                            if (n0 + at < N) y[(int64_t)(tok_first + rr) * ldy + n0 + at] = reinterpret_cast<const YT*>(scr + rr * 8 + (chunk ^ (rr & 7)))[at % (16 / (int)sizeof(YT))];
+                        }
                 }
                 __syncwarp();
             }
@@ -299,13 +278,14 @@ extern "C" int coset_e8_decode_gemm(const void* codes, const float* beta, int64_
     if (beta) k_decode_weights_bf16<2><<<dgrid, 256, 0, st>>>((const uint32_t*)codes, beta, td, n_blocks, table, c, (uint4*)scratch);
     else k_decode_weights_bf16<0><<<dgrid, 256, 0, st>>>((const uint32_t*)codes, nullptr, td, n_blocks, table, c, (uint4*)scratch);
     if (int e = check_launch("e8_decode_gemm (weights)")) return e;
+    const int elem = y_dtype == COSET_DTYPE_F32 ? 4 : 2, vector_rows = aligned(y, 16) && (ldy * elem) % 16 == 0 && (n_out * (int64_t)elem) % 16 == 0;
     dim3 grid(2 * ((n_out + PAIR_N - 1) / PAIR_N), (unsigned)tiles_m);
     if (y_dtype == COSET_DTYPE_F32) {
         if (int e = check_cuda(cudaFuncSetAttribute(k_gemm_pair<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES), "cudaFuncSetAttribute")) return e;
-        k_gemm_pair<float><<<grid, THREADS, SMEM_BYTES, st>>>(x_map, w_map, n_out, n_in, T, bias, (float*)y, ldy, status);
+        k_gemm_pair<float><<<grid, THREADS, SMEM_BYTES, st>>>(x_map, w_map, n_out, n_in, T, bias, (float*)y, ldy, vector_rows, status);
     } else {
         if (int e = check_cuda(cudaFuncSetAttribute(k_gemm_pair<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES), "cudaFuncSetAttribute")) return e;
-        k_gemm_pair<__nv_bfloat16><<<grid, THREADS, SMEM_BYTES, st>>>(x_map, w_map, n_out, n_in, T, bias, (__nv_bfloat16*)y, ldy, status);
+        k_gemm_pair<__nv_bfloat16><<<grid, THREADS, SMEM_BYTES, st>>>(x_map, w_map, n_out, n_in, T, bias, (__nv_bfloat16*)y, ldy, vector_rows, status);
     }
     return check_launch("e8_decode_gemm");
 }

@@ -133,6 +133,22 @@ def test_tcgen05_dequant_gemm(T, n_out, n_in, tiling, form):
         assert torch.equal(got16.cpu(), torch.from_numpy(got).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,n_out", [(1, 1), (31, 203), (545, 204), (513, 264), (1030, 520)])
+def test_pair_gemm_result_rows(T, n_out, out_dtype):
+    """Result rows that are made of 16-byte chunks and rows that are not, tails of every tile, with a bias."""
+    from coset_b200.vlut import E8CodeLinear, e8_decode_gemm
+    W, beta, bpt, _, w_hat = make(n_out, 192, "row")
+    bias = torch.randn(n_out)
+    lin = E8CodeLinear.from_weight(W.cuda(), beta.cuda(), bpt, bias.cuda())
+    x = torch.randn(T, 192).to(torch.bfloat16)
+    wb = torch.from_numpy(w_hat).to(torch.bfloat16).double().numpy()
+    want = x.double().numpy() @ wb.T + bias.double().numpy()
+    got = e8_decode_gemm(lin.codes, lin.beta, bpt, x.cuda(), lin.bias, check=True, out_dtype=out_dtype).double().cpu().numpy()
+    # float32 sums of 192 exact products; the bf16 result (8 significant bits) is rounded once, to 2^-8 of itself at most
+    assert got.shape == want.shape and rel(got, want) < (1e-5 if out_dtype == torch.float32 else 2.0 ** -8)
+
+
 @pytest.mark.parametrize("path", ["auto", "tcgen05", "cublas"])
 def test_layer_dispatch_for_many_tokens(path):
     """Every large_t_path of E8CodeLinear at token counts on both sides of its thresholds (64 / 1024 / 2048):
