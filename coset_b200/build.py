@@ -33,6 +33,7 @@ SOURCES = [
     "e8_ref.cu",
     "e8_dequant_gemm.cu",
     "e8_decode_gemm.cu",
+    "e8_dense_gemm.cu",
     "d4.cu",
 ]
 

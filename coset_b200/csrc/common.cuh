@@ -39,4 +39,11 @@ __device__ __forceinline__ void add_exactly(float& s, float& e, float v) {
     s = t;
 }
 
+// Programmatic dependent launch.  A kernel launched with the attribute may start while the kernel before it in the stream still
+// runs; grid_wait returns once that kernel (and with it every earlier one) has finished and its writes are visible, and grid_trigger
+// lets the next such kernel start.  A kernel calls grid_wait before its first access to memory that others write, and grid_trigger
+// only behind it, so that a kernel that has started early knows all but its direct predecessor to be complete.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 }  // namespace coset

@@ -1,0 +1,327 @@
+// Product of the layer's kept dense weight with a batch of tokens that is neither a few nor thousands:
+//     y[T, N] = x[T, K] (bf16) * W[N, K]^T (bf16) + bias (float32), float32 sums, one rounding of the result.
+//
+// Between 17 and 2047 tokens a 4096 x 4096 layer has 32 MB of weights to stream and 0.6 to 69 GFLOP to do: the tiles must be large
+// in features (so that the tokens are not read over and over) and there must be enough of them for 148 SMs.  So a pair of CTAs
+// owns 256 features (tcgen05.mma.cta_group::2, M = 256: features are the rows, tokens the N of the instruction, 32 to 256 of them, so
+// that no tensor work is done for tokens that are not there), and where feature and token tiles leave SMs idle, K is split
+// over the 2 or 4 pairs of one cluster.  The pairs then add their sums through distributed shared memory in the order of K: every pair
+// owns a part of the tokens, receives the others' sums for it and stores it.  No scratch memory, no second launch, same bits in
+// every run.  The bias joins the float32 sums.
+//
+// Roles of the warps and the barriers of a pair are those of k_gemm_pair (e8_decode_gemm.cu); every wait is bounded in time.  What bounds
+// a small product is latency: 2.3 thousand cycles until the first load, 1.2 until it arrives, 105 ns per K step of 64 with 32 or 64 tokens (the issue
+// of its four instructions and one wait; stages of two steps below 160 tokens share the wait), 2 to 7 thousand cycles for the sums.  The kernel is
+// launched as a programmatic dependent, which hides about 2 us of that behind the kernel before it.
+// Measured, 4096 x 4096 with a bias, torch's product and its bias cast against this kernel (graph replays, three weights in turn): 64 tokens 8.9 + 2.9
+// against 10.7 us, 256 tokens 11.1 + 2.9 against 14.1, 1024 tokens 25.2 + 2.9 against 26.9; a call of the layer with 256 tokens 20.7 -> 14.5 us, for
+// the host was what bounded it.
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include "common.cuh"
+#include "umma.cuh"
+
+using namespace coset;
+using namespace coset::umma;
+
+namespace {
+
+constexpr int kRows = 128;           // weight rows of one CTA
+constexpr int kMaxStages = 8;
+constexpr int kEpilogueWarps = 16, kTmaWarp = 16, kMmaWarp = 17;
+constexpr int kThreads = 18 * 32;
+constexpr int kSmemBudget = 226 * 1024;  // 227 KB less the alignment
+constexpr int kBarrierBytes = 16 * kMaxStages + 16;
+constexpr int kScratchRow = 40;       // 32 features and a pad, in values
+constexpr int kScratchBytes = kEpilogueWarps * 32 * kScratchRow * 2;
+
+struct Plan {
+    int tokens;  // N of the instruction: tokens of one pair, a multiple of 32 up to 256
+    int split;   // pairs that share K: 1, 2 or 4
+    int stages;
+    int sub;     // 64-wide K steps of a stage
+};
+
+struct Shape {
+    int N, K, T;
+    Plan plan;
+    const float* bias;
+    __nv_bfloat16* y;
+    int64_t ldy;
+    int vector_rows;  // rows of y are made of 16-byte chunks
+    int* status;
+};
+
+// what a pair receives of the others' sums: apart from the stages, which a slower pair may still be using when a faster one sends
+__host__ __device__ constexpr int sums_bytes(int tokens, int split) { return (split - 1) * (tokens / split) * kRows * 4; }
+__host__ __device__ constexpr int stage_bytes(int tokens, int sub) { return sub * (kRows + tokens / 2) * BK * 2; }
+
+// Columns (tokens) of this CTA's accumulator that other pairs own, W at a time, into their reduction buffers [slot][token][row].
+template <int W>
+__device__ __forceinline__ void send_columns(const Shape& s, uint32_t tmem, uint32_t base, int pair, int half, int row, int group) {
+    const int own = s.plan.tokens / s.plan.split;
+    for (int c = group * W; c < s.plan.tokens; c += (kEpilogueWarps / 4) * W) {
+        const int to = c / own;  // W divides own
+        if (to == pair) continue;
+        uint32_t r[W];
+        tmem_ld(tmem + (uint32_t)c, r);
+        const int slot = pair < to ? pair : pair - 1;
+        const uint32_t dst = peer_smem(base, (uint32_t)(2 * to + half)) + (uint32_t)(((slot * own + c - to * own) * kRows + row) * 4);
+#pragma unroll
+        for (int j = 0; j < W; ++j) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * kRows * 4)), "r"(r[j]) : "memory");
+    }
+}
+// The columns this pair owns: summed with what the others sent, plus bias, rounded and stored.  A lane holds one feature and W tokens;
+// a scratch of the warp turns them into rows of 32 features, so that four lanes store the 64 bytes of a token.
+template <int W>
+__device__ __forceinline__ void store_columns(const Shape& s, uint32_t tmem, const float* sums, __nv_bfloat16* scratch, int pair, int row, int group, int feature0,
+                                              int token0) {
+    const int own = s.plan.tokens / s.plan.split, lane = threadIdx.x & 31;
+    const float bias = s.bias && feature0 + lane < s.N ? __ldg(s.bias + feature0 + lane) : 0.0f;
+    for (int c = group * W; c < own; c += (kEpilogueWarps / 4) * W) {
+        const int t = token0 + pair * own + c;
+        if (t >= s.T || feature0 >= s.N) break;
+        uint32_t r[W];
+        tmem_ld(tmem + (uint32_t)(pair * own + c), r);
+        float v[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) v[j] = 0.0f;
+        for (int p = 0; p < s.plan.split; ++p) {  // in the order of K
+            if (p == pair) {
+#pragma unroll
+                for (int j = 0; j < W; ++j) v[j] += __uint_as_float(r[j]);
+            } else {
+                const float* from = sums + ((p < pair ? p : p - 1) * own + c) * kRows + row;
+#pragma unroll
+                for (int j = 0; j < W; ++j) v[j] += from[j * kRows];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < W; ++j) scratch[j * kScratchRow + lane] = __float2bfloat16_rn(v[j] + bias);
+        __syncwarp();
+        const int count = s.T - t < W ? s.T - t : W;
+        if (s.vector_rows) {
+            const int chunk = lane & 3;
+            __nv_bfloat16* y = s.y + (int64_t)(t + (lane >> 2)) * s.ldy + feature0 + 8 * chunk;
+            if (feature0 + 8 * chunk < s.N) {
+#pragma unroll
+                for (int j = 0; j < W; j += 8, y += 8 * s.ldy)
+                    if (j + (lane >> 2) < count) *reinterpret_cast<uint4*>(y) = *reinterpret_cast<const uint4*>(scratch + (j + (lane >> 2)) * kScratchRow + 8 * chunk);
+            }
+        } else if (feature0 + lane < s.N) {
+            for (int j = 0; j < count; ++j) s.y[(int64_t)(t + j) * s.ldy + feature0 + lane] = scratch[j * kScratchRow + lane];
+        }
+        __syncwarp();
+    }
+}
+
+template <int kSub>
+__global__ void __launch_bounds__(kThreads, 1)
+k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ Shape s) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;  // the same offset in all CTAs of the cluster
+    uint8_t* gen = smem_raw + (base - raw);
+    const int bytes = stage_bytes(s.plan.tokens, kSub), stages = s.plan.stages;
+    const uint32_t bar_base = base + (uint32_t)(stages * bytes);
+    const uint32_t full_base = bar_base + 8 * kMaxStages, done_bar = bar_base + 16 * kMaxStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + stages * bytes + 16 * kMaxStages + 8);
+
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t crank = __shfl_sync(0xffffffffu, cluster_rank(), 0);
+    const int half = (int)(crank & 1u), pair = (int)(crank >> 1);
+    const bool leader = half == 0;
+    const uint16_t both = (uint16_t)(3u << (crank & ~1u));
+    const uint32_t leader_full = peer_smem(base, crank & ~1u) + (full_base - base);
+    const int row0 = (int)(blockIdx.x / (2 * s.plan.split)) * 2 * kRows + half * kRows;  // this CTA's features
+    const int token0 = (int)blockIdx.y * s.plan.tokens;                                  // this pair's tokens
+    uint32_t columns = 32;
+    while ((int)columns < s.plan.tokens) columns *= 2;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(columns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    if (tid == kTmaWarp * 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&w_map) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&x_map) : "memory");
+        for (int i = 0; i < stages; ++i) {
+            mbar_init(bar_base + 8 * i, 1);   // empty: one commit
+            mbar_init(full_base + 8 * i, 1);  // full (used in the leader): its arrive + both CTAs' bytes
+        }
+        mbar_init(done_bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();  // the partner's barriers exist before anything arrives on them
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    bool ok = true;
+    grid_wait();
+    grid_trigger();
+
+    const int steps = (s.K + BK - 1) / BK, split_log2 = s.plan.split >> 1;  // 1, 2, 4
+    const int first = steps * pair >> split_log2, last = steps * (pair + 1) >> split_log2;
+    const uint32_t x_at = kSub * kRows * BK * 2, x_bytes = (uint32_t)(s.plan.tokens * BK);
+    if (warp == kTmaWarp) {
+        int stage = 0;
+        uint32_t phase = 1;  // of the round before
+        for (int k = first, n = 0; k < last; k += kSub, ++n) {
+            if (n >= stages && !mbar_wait_warp(bar_base + 8 * stage, phase)) { ok = false; break; }
+            if (elect_one()) {  // rows beyond N or T and columns beyond K arrive as zeros
+                const uint32_t at = base + (uint32_t)(stage * bytes), bar = leader_full + 8 * stage;
+                const int subs = last - k < kSub ? last - k : kSub;
+                if (leader) mbar_arrive_expect_tx(full_base + 8 * stage, (uint32_t)(2 * subs) * (kRows * BK * 2 + x_bytes));
+#pragma unroll
+                for (int i = 0; i < kSub; ++i)
+                    if (i < subs) {
+                        tma_load_pair(at + i * (kRows * BK * 2), &w_map, (k + i) * BK, row0, bar);
+                        tma_load_pair(at + x_at + i * x_bytes, &x_map, (k + i) * BK, token0 + half * (s.plan.tokens / 2), bar);
+                    }
+            }
+            __syncwarp();
+            if (++stage == stages) { stage = 0; phase ^= 1u; }
+        }
+    } else if (warp == kMmaWarp && leader) {
+        const uint64_t desc0 = umma_desc(base);
+        const uint32_t desc_hi = (uint32_t)(desc0 >> 32), desc_lo0 = (uint32_t)desc0;
+        // kind::f16: float32 sums, bf16 x bf16, both K-major, M = 256 over the pair
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(s.plan.tokens >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+        int stage = 0;
+        uint32_t phase = 0;
+        for (int k = first; k < last; k += kSub) {
+            if (!mbar_wait_warp(full_base + 8 * stage, phase)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+                const uint32_t a_lo = desc_lo0 + (uint32_t)(stage * (bytes >> 4)), b_lo = a_lo + (x_at >> 4);
+#pragma unroll
+                for (int i = 0; i < kSub; ++i)
+                    if (i == 0 || k + i < last) {
+#pragma unroll
+                        for (int j = 0; j < BK / 16; ++j)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle row
+                            umma_f16_pair(tmem, make_desc(a_lo + (uint32_t)(i * (kRows * BK * 2 >> 4) + j * 2), desc_hi),
+                                          make_desc(b_lo + (uint32_t)i * (x_bytes >> 4) + (uint32_t)(j * 2), desc_hi), idesc, i + j > 0 || k > first ? 1u : 0u);
+                    }
+                umma_commit_pair(bar_base + 8 * stage, both);
+                if (k + kSub >= last) umma_commit_pair(done_bar, both);
+            }
+            __syncwarp();
+            if (++stage == stages) { stage = 0; phase ^= 1u; }
+        }
+    }
+    __syncwarp();
+    if (!ok && s.status) atomicExch(s.status, 1);
+    ok = __all_sync(0xffffffffu, mbar_wait_cluster<32>(done_bar, 0u) && ok);  // always: the products must have retired before tensor memory is read or freed
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;  // a warp reads lanes 32 (warp % 4) .. + 31
+    const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+    const int own = s.plan.tokens / s.plan.split;
+    if (s.plan.split > 1) {
+        if (warp < kEpilogueWarps) {
+            if (own >= 64) send_columns<16>(s, lanes, bar_base + kBarrierBytes, pair, half, row, group);
+            else send_columns<8>(s, lanes, bar_base + kBarrierBytes, pair, half, row, group);
+        }
+        cluster_sync();  // ... and the sums have arrived
+    }
+    if (warp < kEpilogueWarps && ok) {
+        const float* sums = reinterpret_cast<const float*>(gen + stages * bytes + kBarrierBytes);
+        __nv_bfloat16* scratch = reinterpret_cast<__nv_bfloat16*>(gen) + warp * 32 * kScratchRow;
+        const int feature0 = row0 + quarter * 32;
+        if (own >= 128) store_columns<32>(s, lanes, sums, scratch, pair, row, group, feature0, token0);
+        else if (own >= 64) store_columns<16>(s, lanes, sums, scratch, pair, row, group, feature0, token0);
+        else store_columns<8>(s, lanes, sums, scratch, pair, row, group, feature0, token0);
+    }
+    if (!ok) {
+        if (s.status) atomicExch(s.status, 1);
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);  // a wait gave up: leave copies still in flight time to land
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();  // neither CTA frees tensor memory or leaves while the pair's work could still touch it
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(columns) : "memory");
+}
+
+// Stages: what fits, no more than there is work for, and room for the epilogue's scratch.
+Plan with_stages(int tokens, int split, int steps) {
+    Plan p = {tokens, split, 1, tokens <= 128 ? 2 : 1};
+    const int bytes = stage_bytes(tokens, p.sub), need = ((steps + split - 1) / split + p.sub - 1) / p.sub, least = (kScratchBytes + bytes - 1) / bytes;
+    p.stages = (kSmemBudget - kBarrierBytes - sums_bytes(tokens, split)) / bytes;
+    if (p.stages > kMaxStages) p.stages = kMaxStages;
+    if (p.stages > need) p.stages = need;
+    if (p.stages < least) p.stages = least;
+    return p;
+}
+
+// Clusters of 2 * split CTAs that the device runs at once.  148 SMs hold 74 pairs, but the GPCs' sizes leave fewer places for larger
+// clusters (14 of eight CTAs: 16 took two waves).
+int clusters_at_once(int split) { return split == 1 ? sm_count() / 2 : split == 2 ? sm_count() * 35 / 148 : sm_count() * 13 / 148; }
+
+// The plan of the least estimated time in ns.  Measured over 14 shapes from [17, 4096] x [4096, 4096] to [1000, 768] x [768, 3072]: a K step
+// of 64 takes 132 ns with 32 tokens and 361 with 256 (the loads of the weights, then the tensor cores), the exchange of the
+// sums 1.7 us with 32 tokens and two pairs and 4 us with 256.  The plan taken was within 2 % of the best one on average, 18 % at worst
+// ([256, 4096] x [4096, 4096]: 128 tokens, two pairs 14.1 us, against 17.3 with one pair and 23.7 with 256 tokens).
+Plan make_plan(int N, int K, int T) {
+    const int steps = (K + BK - 1) / BK;
+    Plan best = with_stages(32, 1, steps);
+    double least = 0.0;
+    for (int tokens = 32; tokens <= 256 && tokens < T + 32; tokens += 32)
+        for (int split = 1; split <= 4 && split <= steps; split *= 2) {
+            const int64_t clusters = (int64_t)((N + 2 * kRows - 1) / (2 * kRows)) * ((T + tokens - 1) / tokens);
+            const int64_t at_once = clusters_at_once(split), waves = (clusters + at_once - 1) / at_once, pairs = clusters * split < 74 ? clusters * split : 74;
+            const double exchange = split == 1 ? 0.0 : split == 2 ? 1300.0 + 12.0 * tokens : 1800.0 + 16.0 * tokens;
+            const double time = (double)waves * ((double)((steps + split - 1) / split) * (100.0 + 1.02 * tokens) + exchange + 1500.0) + 30.0 * (double)pairs;
+            if (least == 0.0 || time < least) {
+                least = time;
+                best = with_stages(tokens, split, steps);
+            }
+        }
+    return best;
+}
+
+template <int kSub>
+int launch_linear(const CUtensorMap& x_map, const CUtensorMap& w_map, const Shape& s, cudaStream_t st) {
+    const int smem = 1024 /* alignment */ + s.plan.stages * stage_bytes(s.plan.tokens, kSub) + kBarrierBytes + sums_bytes(s.plan.tokens, s.plan.split);
+    if (int e = check_cuda(cudaFuncSetAttribute(k_linear_pair<kSub>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((s.N + 2 * kRows - 1) / (2 * kRows) * 2 * s.plan.split), (unsigned)((s.T + s.plan.tokens - 1) / s.plan.tokens));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)(2 * s.plan.split);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+    if (int e = check_cuda(cudaLaunchKernelEx(&cfg, k_linear_pair<kSub>, x_map, w_map, s), "e8_dense_linear")) return e;
+    return check_launch("e8_dense_linear");
+}
+
+int dense_linear(const void* w, int n_out, int n_in, const void* x, int64_t ldx, int T, const float* bias, void* y, int64_t ldy,
+                 int* status, const Plan* given, void* stream) {
+    if (n_out < 0 || n_in < 0 || T < 0 || (n_in % 8) != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
+    if (n_out == 0 || T == 0) return 0;
+    if (n_in == 0) return fail(COSET_E_BADARG, "n_in is 0");
+    if (!w || !x || !y) return fail(COSET_E_BADARG, "null pointer");
+    if (ldx < n_in || ldy < n_out || (ldx % 8) != 0) return fail(COSET_E_BADARG, "leading dimensions: ldx >= n_in and a multiple of 8, ldy >= n_out");
+    if (!aligned(x, 16) || !aligned(w, 16)) return fail(COSET_E_ALIGN, "x and the weight must be 16-byte aligned");
+    const int vector_rows = aligned(y, 16) && ldy % 8 == 0 && n_out % 8 == 0;
+    Shape s = {n_out, n_in, T, given ? *given : make_plan(n_out, n_in, T), bias, (__nv_bfloat16*)y, ldy, vector_rows, status};
+    if ((T + s.plan.tokens - 1) / s.plan.tokens > 65535) return fail(COSET_E_UNSUPPORTED, "T too large");
+    CUtensorMap x_map, w_map;
+    if (int e = make_bf16_map(&x_map, x, n_in, T, ldx, s.plan.tokens / 2)) return e;
+    if (int e = make_bf16_map(&w_map, w, n_in, n_out, n_in, kRows)) return e;
+    return s.plan.sub == 2 ? launch_linear<2>(x_map, w_map, s, (cudaStream_t)stream) : launch_linear<1>(x_map, w_map, s, (cudaStream_t)stream);
+}
+
+}  // namespace
+
+extern "C" int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, void* y,
+                                     int64_t ldy, int* status, void* stream) {
+    return dense_linear(w_bf16, n_out, n_in, x_bf16, ldx, T, bias, y, ldy, status, nullptr, stream);
+}

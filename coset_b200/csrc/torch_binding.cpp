@@ -9,7 +9,9 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -424,22 +426,47 @@ PyObject* decode_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// linear_cast_bias(x bf16, w bf16, bias): the library's product with the bias rounded to bf16 in the call (9 us less host time than the
-// two torch calls from Python).
-PyObject* linear_cast_bias(PyObject*, PyObject* const* a, Py_ssize_t n) {
+// A tensor that is nothing but memory on the GPU: no batch of a transform, no lazy negation, no tangent, not recorded.
+bool plain(const Tensor& t) {
+    if (!t.defined()) return true;
+    static const c10::DispatchKeySet known = c10::DispatchKeySet(c10::DispatchKey::CUDA) | c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA) |
+                                             c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) | c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA);
+    return (t.key_set().raw_repr() & ~known.raw_repr()) == 0 && !(at::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined();
+}
+
+// dense_linear(x [T, n_in] bf16, w [n_out, n_in] bf16, bias or None, status or None, own): x w^T + bias as bf16.  `own`: by the library's own
+// kernel, which adds the float32 bias to the float32 sums; else, and for whoever looks at the torch call (autograd, autocast, transforms,
+// dispatch modes), by torch's product with the bias rounded to bf16 first.
+PyObject* dense_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    nargs_are(n, 3);
-    const Tensor &x = cuda_arg(a[0], "x"), &w = cuda_arg(a[1], "w"), &bias = tensor_arg(a[2], "bias");
+    nargs_are(n, 5);
+    const Tensor &x = cuda_arg(a[0], "x"), &w = cuda_arg(a[1], "w");
+    const Tensor bias = optional_arg(a[2], "bias"), status = optional_arg(a[3], "status");
+    bool own = a[4] == Py_True;
     Tensor y;
     {
         NoGil no_gil;
         c10::cuda::CUDAGuard guard(x.device());
-        Tensor b;
-        if (bias.scalar_type() == at::kFloat && bias.device() == x.device() && bias.has_storage() && bias.is_contiguous() && !bias.requires_grad()) {
-            b = empty(bias.sizes(), at::kBFloat16, bias);
-            check_rc(coset_layer_beta_bias(nullptr, nullptr, nullptr, 0, nullptr, fdata(bias), bias.numel(), data(b), stream_of(x)), "coset_layer_beta_bias");
-        } else b = bias.to(at::kBFloat16);
-        y = at::linear(x, w, b);
+        own = own && x.dim() == 2 && w.dim() == 2 && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.size(1) == w.size(1) && x.size(1) > 0 &&
+              x.size(1) % 8 == 0 && w.is_contiguous() && (uintptr_t)w.const_data_ptr() % 16 == 0 && w.device() == x.device() && plain(x) && plain(w) && plain(bias) &&
+              (!bias.defined() || (bias.device() == x.device() && bias.dim() == 1 && bias.size(0) == w.size(0))) &&
+              !at::autocast::is_autocast_enabled(at::kCUDA) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
+        if (own) {
+            const bool rows = x.stride(1) == 1 && x.stride(0) >= x.size(1) && x.stride(0) % 8 == 0 && (uintptr_t)x.const_data_ptr() % 16 == 0;
+            const Tensor x2 = rows ? x : x.clone(at::MemoryFormat::Contiguous), b = as_f32(bias);
+            y = empty({x.size(0), w.size(0)}, at::kBFloat16, x);
+            check_rc(coset_e8_dense_linear(data(w), (int)w.size(0), (int)w.size(1), data(x2), x2.stride(0), (int)x2.size(0), fdata(b), data(y), y.size(1),
+                                           (int*)data(status), stream_of(x)), "coset_e8_dense_linear");
+        } else {
+            Tensor b = bias;
+            if (b.defined()) {
+                if (b.scalar_type() == at::kFloat && b.device() == x.device() && b.has_storage() && b.is_contiguous() && !b.requires_grad()) {
+                    b = empty(bias.sizes(), at::kBFloat16, bias);
+                    check_rc(coset_layer_beta_bias(nullptr, nullptr, nullptr, 0, nullptr, fdata(bias), bias.numel(), data(b), stream_of(x)), "coset_layer_beta_bias");
+                } else b = bias.to(at::kBFloat16);
+            }
+            y = at::linear(x, w, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
+        }
     }
     return THPVariable_Wrap(y);
     END_HANDLE_TH_ERRORS
@@ -622,7 +649,7 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef kMethods[] = {
     COSET_METHOD(encode_packed), COSET_METHOD(decode_packed), COSET_METHOD(encode_digits), COSET_METHOD(decode_digits), COSET_METHOD(quantize),
     COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(vlut_layout), COSET_METHOD(vlut_product), COSET_METHOD(vlut_product_checked),
-    COSET_METHOD(decode_gemm), COSET_METHOD(linear_cast_bias), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
+    COSET_METHOD(decode_gemm), COSET_METHOD(dense_linear), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_coset_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

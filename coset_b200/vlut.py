@@ -9,7 +9,8 @@ weights) plus the scales beta, and applied from the codes:
     reads the code stream (coset_e8_vlut_gemv);
   * many tokens (from 2048 by default): the weight is decoded into a transient bf16 buffer and multiplied by
     this library's tcgen05 GEMM (coset_e8_decode_gemm); nothing dense survives the call;
-  * in between, by default, the library GEMM on a cached dense bf16 copy (`large_t_path` chooses).
+  * in between, by default, this library's product with a kept dense bf16 copy (coset_e8_dense_linear) up to 2^34 multiply-adds and
+    torch's beyond (`large_t_path` chooses).
 
 The math is the reference's one-sided vLUT inner product (coset/legacy/quant/vlut.py:72-117) in
 the layer's scale convention W_q = decode(codes) / beta (coset/core/layers.py:453-460).
@@ -94,8 +95,9 @@ class E8CodeLinear(nn.Module):
     Up to small_t_max tokens go to the code-domain kernels; more bf16 tokens go to (large_t_path): "tcgen05" --
     this library's tensor-core kernels, which keep no dense weight: decode to a transient bf16 buffer + TMA-fed
     cta_group::2 GEMM from 1024 tokens, the single-launch fused kernel below; "cublas" -- a cached dense bf16 copy
-    and the library GEMM; "auto" (default) -- the own kernels from PAIR_GEMM_MIN_T tokens, the library path for
-    the tokens in between, where decoding the whole weight per call costs more than the product itself.
+    and the library GEMM; "auto" (default) -- the own kernels from PAIR_GEMM_MIN_T tokens, the kept dense copy for
+    the tokens in between, where decoding the whole weight per call costs more than the product itself (multiplied by this library's kernel
+    up to DENSE_OWN_MAX multiply-adds).
     Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 9-13 us for 1-16
     tokens and a 4096 x 4096 weight; the kernel checks the copy against the codes in every call.  "tcgen05" keeps nothing and
     stays on the code-domain kernels (9.7-23 us).
@@ -110,6 +112,10 @@ class E8CodeLinear(nn.Module):
     weight_clip_value > 0: the weights are clamp(decode(codes) / beta, +-clip), the clamp the training
     layer applies after de-scaling (coset/core/layers.py:463); 0 disables it."""
 
+    # Up to here (in multiply-adds) the library's own product with the kept dense copy is as fast on the device as torch's product and its
+    # cast of the bias (4096 x 4096: 256 tokens 14.1 us against 11.1 + 3, 1024 tokens 26.9 against 25.2 + 3; 2047 tokens 52 against 47 + 3), and it
+    # costs the host one launch instead of two library calls (10 us), which is what bounds such a call.
+    DENSE_OWN_MAX = 1 << 34
     PAIR_GEMM_MIN_T = 2048  # from here on the decode + cta_group::2 GEMM is within 10-25 % of the library on a dense copy
 
     def __init__(self, codes: torch.Tensor, beta: torch.Tensor, blocks_per_tile: int,
@@ -300,9 +306,12 @@ class E8CodeLinear(nn.Module):
         if dtype is torch.float32:
             return torch.nn.functional.linear(x, self.dense_weight(torch.float32), buf["bias"])
         b, w = buf["bias"], self._dense_bf16()
-        if (b is not None and dtype is torch.bfloat16 and type(x) is torch.Tensor and torch._C._get_tracing_state() is None
-                and not torch._C._len_torch_function_stack()):
-            return _lib.native().linear_cast_bias(x, w, b)
+        if dtype is torch.bfloat16 and type(x) is torch.Tensor and torch._C._get_tracing_state() is None and not torch._C._len_torch_function_stack():
+            own = self.large_t_path == "auto" and T < self.PAIR_GEMM_MIN_T and T * n_in * self.out_features <= self.DENSE_OWN_MAX
+            status = self._status
+            if own and (status is None or status.device != x.device):  # not inside a capture, whose memory is the graph's
+                status = self._status = None if torch._C._cuda_isCurrentStreamCapturing() else torch.zeros(1, dtype=torch.int32, device=x.device)
+            return _lib.native().dense_linear(x, w, b, status, own)
         return torch.nn.functional.linear(x, w.to(dtype), b.to(dtype) if b is not None else None)
 
 

@@ -404,6 +404,15 @@ int coset_e8_decode_gemm(const void* codes, const float* beta, int64_t blocks_pe
                          const void* x_bf16, int64_t ldx, int T, const float* bias, void* y, int y_dtype,
                          int64_t ldy, float clip, void* scratch, int64_t scratch_bytes, int* status, void* stream);
 
+/* Product with a dense bf16 weight that the caller keeps, [n_out, n_in] contiguous and 16-byte aligned, for some tens to some
+ * thousand tokens: y[T, ldy] (bf16) = x[T, ldx] (bf16, rows 16-byte aligned) * W^T + bias (float32 or null), float32 sums, one
+ * rounding.  n_in is a multiple of 8.  One launch, no scratch memory.  status (device int, may be null) is set to 1 when a bounded wait
+ * inside the kernel gave up; the result is then incomplete.
+ * Replaces the dense-weight matmul after a one-off dequantisation, coset/legacy/quant/vlut.py:72-117.
+ */
+int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, void* y,
+                          int64_t ldy, int* status, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -660,3 +660,74 @@ def test_dense_bf16_weight_is_the_rounded_clamp(clip):
     beta = layer.beta.clone()
     layer.beta.copy_(beta * (0.5 + torch.rand_like(beta)))
     assert torch.equal(layer.dense_weight(torch.bfloat16), layer.dense_weight(torch.float32).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T,n_out,n_in", [(1, 1, 8), (17, 64, 8), (32, 256, 64), (33, 257, 72), (64, 4096, 128), (65, 264, 4104), (130, 136, 8192),
+                                          (257, 1000, 520), (300, 768, 3072), (600, 99, 192), (1030, 3080, 136)])
+@pytest.mark.parametrize("form", ["rows", "padded", "offset"])
+def test_product_with_the_kept_dense_weight(T, n_out, n_in, form):
+    """Every tile's edges, one to four pairs over K, ragged K, result rows with and without 16-byte chunks; tokens in rows, in padded
+    rows and at an address that is no multiple of 16."""
+    from coset_b200 import _lib
+    x = torch.randn(T, n_in, device="cuda").bfloat16()
+    w = (torch.randn(n_out, n_in, device="cuda") * 0.02).bfloat16()
+    bias = torch.randn(n_out, device="cuda")
+    if form == "padded":
+        x = torch.cat([x, torch.full((T, 16), float("nan"), device="cuda", dtype=torch.bfloat16)], 1)[:, :n_in]
+    elif form == "offset":
+        x = torch.cat([torch.zeros(1, device="cuda", dtype=torch.bfloat16), x.reshape(-1)])[1:].view(T, n_in)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for b in (bias, None):
+        got = _lib.native().dense_linear(x, w, b, status, True)
+        want = x.double() @ w.double().T + (b.double() if b is not None else 0.0)
+        # one rounding to 8 significant bits, and float32 sums of K exact products and the bias, each of which may round or truncate
+        # its part of a sum that is no larger than the sum of the magnitudes
+        bound = 2.0 ** -8 * want.abs() + 2.0 ** -22 * (x.double().abs() @ w.double().abs().T + (b.abs().double() if b is not None else 0.0))
+        assert got.dtype == torch.bfloat16 and bool(((got.double() - want).abs() <= bound).all())
+    assert int(status.item()) == 0
+
+
+def test_product_with_the_kept_dense_weight_refuses():
+    from coset_b200 import _lib
+    L = _lib.lib()
+    w, x, y = (torch.zeros(64, 64, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    call = lambda n_out=64, n_in=64, ldx=64, T=64, ldy=64, wp=w.data_ptr(), xp=x.data_ptr(): L.coset_e8_dense_linear(
+        wp, n_out, n_in, xp, ldx, T, None, y.data_ptr(), ldy, None, _lib.stream())
+    assert call() == 0 and call(T=0) == 0 and call(n_out=0) == 0
+    for bad in (dict(n_in=60), dict(n_in=0), dict(ldx=56), dict(ldx=68), dict(ldy=63), dict(wp=None), dict(xp=None), dict(wp=w.data_ptr() + 2), dict(xp=x.data_ptr() + 8), dict(T=-1)):
+        assert call(**bad) < 0, bad
+
+
+@pytest.mark.parametrize("how", ["autograd", "tangent", "autocast", "vmap", "mode"])
+def test_product_with_the_kept_dense_weight_is_torchs_for_who_looks_at_it(how):
+    from torch.utils._python_dispatch import TorchDispatchMode
+    layer, _ = _kept_copy_layer(64, 256)
+    layer.bias = torch.randn(64, device="cuda")
+    x = torch.randn(32, 256, device="cuda").bfloat16()
+    w = layer.dense_weight(torch.bfloat16)
+    if how == "autograd":
+        x.requires_grad_()
+        layer(x).sum().backward()
+        assert torch.allclose(x.grad.float(), w.float().sum(0).expand(32, 256), rtol=2.0 ** -6, atol=1e-3)
+    elif how == "tangent":
+        with torch.autograd.forward_ad.dual_level():
+            t = torch.autograd.forward_ad.unpack_dual(layer(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)))).tangent
+            assert t is not None and torch.allclose(t.float(), w.float().sum(1).expand(32, 64), rtol=2.0 ** -6, atol=1e-3)
+    elif how == "autocast":
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert layer(x).dtype == torch.float16
+    elif how == "vmap":
+        batch = torch.randn(3, 32, 256, device="cuda").bfloat16()
+        got = torch.func.vmap(layer)(batch)
+        assert torch.allclose(got.float(), torch.stack([layer(b) for b in batch]).float(), rtol=2.0 ** -6, atol=2.0 ** -6)
+    else:
+        class Seen(TorchDispatchMode):
+            calls = []
+
+            def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+                self.calls.append(str(func))
+                return func(*args, **(kwargs or {}))
+        layer(x)
+        with Seen() as seen:
+            layer(x)
+        assert any("mm" in c or "linear" in c for c in seen.calls)
