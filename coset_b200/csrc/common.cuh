@@ -45,5 +45,32 @@ __device__ __forceinline__ void add_exactly(float& s, float& e, float v) {
 // only behind it, so that a kernel that has started early knows all but its direct predecessor to be complete.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The same value, which the compiler knows only behind every volatile statement before: loads through the read-only path (__ldg, const
+// __restrict__) count as invariant and could otherwise be moved in front of grid_wait.  An address that is read depends on one, or the read is conditional on a bound.
+__device__ __forceinline__ int behind_wait(int v) {
+    asm volatile("" : "+r"(v) : : "memory");
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ T* behind_wait(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
+
+// Launches a kernel that calls grid_wait as a programmatic dependent of the one before it.
+template <typename... Params, typename... Args>
+int launch_dependent(const char* what, void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...), what);
+}
 
 }  // namespace coset

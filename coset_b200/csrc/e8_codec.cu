@@ -269,6 +269,11 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
     constexpr int kQueueSlots = 32 * (ROWS + 1);  // < 32 left after a drain + at most 32 per sub-step
     __shared__ uint32_t q_index[kEncWarps][2][kQueueSlots];  // block index lo / hi
     __shared__ int q_count[kEncWarps];
+    if ((threadIdx.x & 31) == 0) q_count[threadIdx.x >> 5] = 0;
+    __syncwarp();
+    grid_wait();
+    grid_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto emit = [&](int64_t b, uint32_t code, float s) {
         if constexpr (KIND == kDigits) {
             store_digits((float*)out, 2 * b, code & 0xffffu);
@@ -284,9 +289,6 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
         }
     };
     auto scale_of = [&](int64_t b) { return MODE == kScaleDivValue ? value : load_scale<MODE>(scale, td, b); };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) q_count[warp] = 0;
-    __syncwarp();
     int count = 0;  // warp-uniform copy of q_count[warp] as of the last look
 
     // Completes the last min(count, 32) queued blocks with all lanes busy.
@@ -405,6 +407,8 @@ k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale
     if (threadIdx.x < 8) flip_rows[threadIdx.x] = e8::kFlipRows[threadIdx.x];
     if (threadIdx.x == 0) listed = 0u;
     __syncthreads();
+    grid_wait();
+    grid_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t span = 32 * ROWS;
     const int64_t stride = (int64_t)gridDim.x * kEncWarps * span;
@@ -516,7 +520,10 @@ template <int DT, int MODE, typename TABLE>
 __global__ void __launch_bounds__(kThreads)
 k_decode_q4m2(const uint32_t* __restrict__ codes, const float* __restrict__ scale, e8::TileDiv td, int64_t n,
               const TABLE* __restrict__ table, void* __restrict__ out) {
-    int64_t base = (int64_t)blockIdx.x * (kThreads * kDecPerThread) + threadIdx.x;
+    grid_wait();
+    grid_trigger();
+    const int64_t base = (int64_t)blockIdx.x * (kThreads * kDecPerThread) + behind_wait((int)threadIdx.x);
+    if (MODE == COSET_SCALE_DIV_SCALAR) scale = behind_wait(scale);
     uint32_t code[kDecPerThread];
     float s[kDecPerThread];
 #pragma unroll
@@ -615,7 +622,9 @@ k_pack_f32(const float* __restrict__ digits, int64_t n_words, int q, void* __res
 // codes in between, without the packed array (4 launches and 72 bytes per block less for q = 4, M = 2).
 __global__ void __launch_bounds__(kThreads)
 k_encode_digits_generic(const float* __restrict__ x, float beta, int64_t n, int q, int M, float* __restrict__ digits) {
-    const int64_t b = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    grid_wait();
+    grid_trigger();
+    const int64_t b = (int64_t)blockIdx.x * kThreads + behind_wait((int)threadIdx.x);
     if (b >= n) return;
     float xl[8];
     e8::Row8<0>::load(x, b, xl);
@@ -640,7 +649,9 @@ k_encode_digits_generic(const float* __restrict__ x, float beta, int64_t n, int 
 template <bool Q4>
 __global__ void __launch_bounds__(kThreads)
 k_decode_digits(const float* __restrict__ digits, float beta, int64_t n, int q, int M, const uint2* __restrict__ table, float* __restrict__ out) {
-    const int64_t b = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    grid_wait();
+    grid_trigger();
+    const int64_t b = (int64_t)blockIdx.x * kThreads + behind_wait((int)threadIdx.x);
     if (b >= n) return;
     float xh[8];
 #pragma unroll
@@ -754,9 +765,7 @@ int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_
         const unsigned iterations = (grid + resident - 1) / resident;
         grid = (grid + iterations - 1) / iterations;
     }
-    if (rows == 3) k_encode_q4m2_listed<DT, MODE, SAT, 3><<<grid, kThreads, 0, st>>>(x, scale, td, n, codes);
-    else k_encode_q4m2_listed<DT, MODE, SAT, 1><<<grid, kThreads, 0, st>>>(x, scale, td, n, codes);
-    return check_launch("e8_encode");
+    return launch_dependent("e8_encode", rows == 3 ? k_encode_q4m2_listed<DT, MODE, SAT, 3> : k_encode_q4m2_listed<DT, MODE, SAT, 1>, grid, kThreads, 0, st, x, scale, td, n, codes);
 }
 
 }  // namespace
@@ -834,12 +843,14 @@ int coset_e8_decode(const void* codes, const float* scale, int scale_mode, int64
         const uint2* table = residual_table_q4(st);
         const uint32_t* packed = residual_table_q4_packed(st);
         if (!table || !packed) return COSET_E_STATE;
+        int rc = 0;
         unsigned grid2 = (unsigned)((n_blocks + kThreads * kDecPerThread - 1) / (kThreads * kDecPerThread));
         if (out_dtype == COSET_DTYPE_F32) {
-            DISPATCH_MODE(scale_mode, (k_decode_q4m2<0, MODE, uint32_t><<<grid2, kThreads, 0, st>>>((const uint32_t*)codes, scale, td, n_blocks, packed, out)))
+            DISPATCH_MODE(scale_mode, (rc = launch_dependent("e8_decode", k_decode_q4m2<0, MODE, uint32_t>, grid2, kThreads, 0, st, (const uint32_t*)codes, scale, td, n_blocks, packed, out)))
         } else {
-            DISPATCH_MODE(scale_mode, (k_decode_q4m2<1, MODE, uint2><<<grid2, kThreads, 0, st>>>((const uint32_t*)codes, scale, td, n_blocks, table, out)))
+            DISPATCH_MODE(scale_mode, (rc = launch_dependent("e8_decode", k_decode_q4m2<1, MODE, uint2>, grid2, kThreads, 0, st, (const uint32_t*)codes, scale, td, n_blocks, table, out)))
         }
+        return rc;
     } else if (q <= 4) {
         DISPATCH_DT(out_dtype, DT, DISPATCH_MODE(scale_mode, (k_decode_generic<DT, MODE, 2><<<grid, kThreads, 0, st>>>(codes, scale, td, n_blocks, q, M, out))))
     } else {
@@ -864,7 +875,9 @@ int coset_e8_quantize(const void* x, int x_dtype, const float* scale, int scale_
         if (!table) return COSET_E_STATE;
         int rows;
         const unsigned qgrid = encoder_grid(n_blocks, &rows);
-        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (rows == 3 ? (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, 3><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)) : (k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, 1><<<qgrid, kThreads, 0, st>>>(x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip))))))
+        int rc = 0;
+        DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (rc = launch_dependent("e8_quantize", rows == 3 ? k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, 3> : k_encode_q4m2_queued<DTI, MODE, kRecon, DTO, 1>, qgrid, kThreads, 0, st, x, scale, td, n_blocks, (uint32_t*)codes_out, table, out, clip)))))
+        return rc;
     } else if (q <= 4) {
         DISPATCH_DT(x_dtype, DTI, DISPATCH_DT(out_dtype, DTO, DISPATCH_MODE(scale_mode, (k_quantize_generic<DTI, DTO, MODE, 2><<<grid, kThreads, 0, st>>>(x, scale, td, n_blocks, q, M, clip, out, codes_out)))))
     } else {
@@ -903,17 +916,16 @@ int coset_e8_encode_digits_f32(const float* x, float beta, int64_t n_blocks, int
         int rows;
         const unsigned grid = encoder_grid(n_blocks, &rows);
         // two rows where the rule says three: with three, 104 bytes of registers spill (2^20 blocks 60 -> 54 us, both calls)
-#define DIGITS_AS(MODE, ROWS) k_encode_q4m2_queued<0, MODE, kDigits, 0, ROWS><<<grid, kThreads, 0, st>>>(x, nullptr, td, n_blocks, nullptr, nullptr, digits, beta)
+#define DIGITS_AS(MODE, ROWS) return launch_dependent("e8_encode_digits_f32", k_encode_q4m2_queued<0, MODE, kDigits, 0, ROWS>, grid, kThreads, 0, st, (const void*)x, (const float*)nullptr, td, n_blocks, (uint32_t*)nullptr, (const uint2*)nullptr, (void*)digits, beta)
         if (beta == 1.0f) {  // x / 1 is x
-            if (rows == 3) DIGITS_AS(COSET_SCALE_NONE, 2); else DIGITS_AS(COSET_SCALE_NONE, 1);
-        } else {
-            if (rows == 3) DIGITS_AS(kScaleDivValue, 2); else DIGITS_AS(kScaleDivValue, 1);
+            if (rows == 3) DIGITS_AS(COSET_SCALE_NONE, 2);
+            DIGITS_AS(COSET_SCALE_NONE, 1);
         }
+        if (rows == 3) DIGITS_AS(kScaleDivValue, 2);
+        DIGITS_AS(kScaleDivValue, 1);
 #undef DIGITS_AS
-    } else {
-        k_encode_digits_generic<<<grid_for(n_blocks), kThreads, 0, st>>>(x, beta, n_blocks, q, M, digits);
     }
-    return check_launch("e8_encode_digits_f32");
+    return launch_dependent("e8_encode_digits_f32", k_encode_digits_generic, grid_for(n_blocks), kThreads, 0, st, x, beta, n_blocks, q, M, digits);
 }
 
 int coset_e8_decode_digits_f32(const float* digits, float beta, int64_t n_blocks, int q, int M, float* out, void* stream) {
@@ -924,11 +936,9 @@ int coset_e8_decode_digits_f32(const float* digits, float beta, int64_t n_blocks
     if (q == 4) {
         const uint2* table = residual_table_q4(st);
         if (!table) return COSET_E_STATE;
-        k_decode_digits<true><<<grid_for(n_blocks), kThreads, 0, st>>>(digits, beta, n_blocks, q, M, table, out);
-    } else {
-        k_decode_digits<false><<<grid_for(n_blocks), kThreads, 0, st>>>(digits, beta, n_blocks, q, M, nullptr, out);
+        return launch_dependent("e8_decode_digits_f32", k_decode_digits<true>, grid_for(n_blocks), kThreads, 0, st, digits, beta, n_blocks, q, M, table, out);
     }
-    return check_launch("e8_decode_digits_f32");
+    return launch_dependent("e8_decode_digits_f32", k_decode_digits<false>, grid_for(n_blocks), kThreads, 0, st, digits, beta, n_blocks, q, M, (const uint2*)nullptr, out);
 }
 
 }  // extern "C"

@@ -78,7 +78,7 @@ template <int W>
 __device__ __forceinline__ void store_columns(const Shape& s, uint32_t tmem, const float* sums, __nv_bfloat16* scratch, int pair, int row, int group, int feature0,
                                               int token0) {
     const int own = s.plan.tokens / s.plan.split, lane = threadIdx.x & 31;
-    const float bias = s.bias && feature0 + lane < s.N ? __ldg(s.bias + feature0 + lane) : 0.0f;
+    const float bias = s.bias && feature0 + lane < s.N ? __ldg(behind_wait(s.bias) + feature0 + lane) : 0.0f;
     for (int c = group * W; c < own; c += (kEpilogueWarps / 4) * W) {
         const int t = token0 + pair * own + c;
         if (t >= s.T || feature0 >= s.N) break;

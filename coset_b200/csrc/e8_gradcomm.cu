@@ -139,10 +139,12 @@ k_decode_mean_compact(const uint32_t* __restrict__ codes, PeerStreams peers, int
                       float inverse, const uint16_t* __restrict__ compact, const uint2* __restrict__ table, void* __restrict__ out,
                       const int* __restrict__ status) {
     extern __shared__ uint16_t lut[];
-    if (PEERS && status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;  // see k_decode_mean
 #pragma unroll
     for (int k = 0; k < kTableBytes / 16 / kCompactThreads; ++k)
         reinterpret_cast<uint4*>(lut)[k * kCompactThreads + threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(compact) + k * kCompactThreads + threadIdx.x);
+    grid_wait();  // the table is there for good; the streams may come from the kernel before
+    grid_trigger();
+    if (PEERS && status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;  // see k_decode_mean
     const int64_t step = (int64_t)gridDim.x * kCompactThreads;
     uint32_t next[2 * PAIRS];
     auto fetch = [&](int64_t b) {
@@ -160,7 +162,7 @@ k_decode_mean_compact(const uint32_t* __restrict__ codes, PeerStreams peers, int
             }
         }
     };
-    int64_t b = (int64_t)blockIdx.x * kCompactThreads + threadIdx.x;
+    int64_t b = (int64_t)blockIdx.x * kCompactThreads + behind_wait((int)threadIdx.x);
     fetch(b);
     __syncthreads();
     for (; b < n; b += step) {
@@ -233,7 +235,7 @@ int launch_decode_mean(const uint32_t* codes, const PeerStreams& peers, int worl
 #define COMPACT_LAUNCH(PAIRS)                                                                                                       \
     do {                                                                                                                            \
         if (int e = check_cuda(cudaFuncSetAttribute(k_decode_mean_compact<DT, PEERS, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes), "cudaFuncSetAttribute")) return e; \
-        k_decode_mean_compact<DT, PEERS, PAIRS><<<sm_count(), kCompactThreads, kTableBytes, st>>>(codes, peers, world, n, stride, twice, inverse, compact, table, out, status); \
+        return launch_dependent("e8_decode_mean", k_decode_mean_compact<DT, PEERS, PAIRS>, sm_count(), kCompactThreads, kTableBytes, st, codes, peers, world, n, stride, twice, inverse, compact, table, out, status); \
     } while (0)
         if (world <= 2) COMPACT_LAUNCH(1);
         else if (world <= 4) COMPACT_LAUNCH(2);

@@ -326,7 +326,9 @@ __global__ void __launch_bounds__(WARPS * 32, kProductCtas<NT, P, WARPS>)
 k_product(const __grid_constant__ Product a) {
     typedef WarpSmem<NT, P, SCALE> Smem;
     extern __shared__ __align__(128) uint8_t smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+    grid_wait();
+    grid_trigger();
+    const int thread = behind_wait((int)threadIdx.x), warp = thread >> 5, lane = thread & 31, g = lane >> 2, c = lane & 3;
     Smem& mem = reinterpret_cast<Smem*>(smem)[warp];
     float(*part)[16][8 * NT + 1] = reinterpret_cast<float(*)[16][8 * NT + 1]>(smem + WARPS * sizeof(Smem));
     const int kw = 1 << a.kw_log2, rw = WARPS >> a.kw_log2, first = warp & (kw - 1), t0 = blockIdx.y * (8 * NT);
@@ -579,8 +581,7 @@ int launch_as(const Product& a, cudaStream_t st) {
     constexpr int smem = WARPS * (int)(sizeof(WarpSmem<NT, P, SCALE>) + 16 * (8 * NT + 1) * sizeof(float));
     if (smem > 48 * 1024)
         if (int e = check_cuda(cudaFuncSetAttribute(k_product<NT, P, CLIP, SCALE, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
-    k_product<NT, P, CLIP, SCALE, WARPS><<<grid, WARPS * 32, smem, st>>>(a);
-    return check_launch("e8_vlut_product");
+    return launch_dependent("e8_vlut_product", k_product<NT, P, CLIP, SCALE, WARPS>, grid, WARPS * 32, smem, st, a);
 }
 
 template <int NT, int P, bool CLIP>

@@ -453,3 +453,33 @@ def test_other_threads_run_while_a_call_waits_for_the_device(e8):
     if waited < 0.4:
         pytest.skip("the device's queue took all launches")
     assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.5 * waited
+
+
+@pytest.mark.parametrize("n", [1, 257, 4099, 300001])
+def test_chained_calls_read_what_the_call_before_wrote(n):
+    """Every launch starts while the one before it drains: a chain through the same buffers has the results of the calls one by one."""
+    from coset_b200.core.base import LatticeConfig
+    from coset_b200.core.e8 import e8_decode, e8_decode_packed, e8_encode, e8_encode_packed, e8_quantize
+    config = LatticeConfig(lattice_type="E8", q=4, M=2, beta=0.7)
+    xs = [torch.randn(n, 8, device="cuda") * s for s in (0.3, 1.0, 3.0, 9.0)]
+    codes, back, moved = torch.empty(n, 4, dtype=torch.uint8, device="cuda"), torch.empty(n, 8, device="cuda"), torch.empty(n, 8, device="cuda")
+
+    def passes(wait):
+        results = []
+        for x in xs + xs[::-1]:
+            moved.copy_(x)
+            wait()
+            e8_encode_packed(moved, out=codes)
+            wait()
+            e8_decode_packed(codes, out=back)
+            wait()
+            e8_encode_packed(back, out=codes)
+            wait()
+            digits, _ = e8_encode(moved, config)
+            wait()
+            results.append((e8_decode(digits, config), codes.clone(), e8_quantize(back, 4)))
+            wait()
+        return results
+
+    for a, b in zip(passes(torch.cuda.synchronize), passes(lambda: None)):
+        assert all(torch.equal(s, t) for s, t in zip(a, b))
