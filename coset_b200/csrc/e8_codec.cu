@@ -392,72 +392,137 @@ __device__ __forceinline__ uint32_t level_any_q4(const float (&x)[8], float amax
     return e8::level_slow_q4(x, s1 == s1 && s1 - s1 == 0.0f ? amax : __int_as_float(0x7fc00000));
 }
 
-// ROWS: rows per lane and iteration.  SAT: every scaled coordinate is first clamped to +-kSaturate, which keeps the two-level
-// code from wrapping around (the top level stays the origin); only deferred blocks can exceed the bound, so the clamp costs
-// nothing on the common path.
+// SAT: every scaled coordinate is first clamped to +-kSaturate, which keeps the two-level code from wrapping around (the top level
+// stays the origin); only deferred blocks can exceed the bound, so the clamp costs nothing on the common path.
 constexpr float kSaturate = 3.9f;  // 8 * 3.9 / 4 < 7.96 and 3.9 / 4 < 1.96: level 1 of a clamped block is the origin
 
-template <int DT, int MODE, bool SAT, int ROWS>
+// How a block's scale is found: any MODE by the general rule, one block per scale, or by a division that fits 32 bits.
+constexpr int kAnyScale = 0, kBlockScale = 1, kTileScale = 2;
+
+// kRing > 0: rows on their way to shared memory per thread (cp.async), so that the loop waits for no load and holds one row in
+// registers.  What bounds the loop is then the issue of instructions (80 % of the cycles, ALU pipe 70 %; before, with three rows per
+// iteration in registers, 73 %, and 62 % for bf16), hence offsets of 32 bits (n < 2^27 blocks, the caller cuts longer calls), a form
+// for each kind of scale, and the signs at the flip coordinates read from the row by index.  The two halves of a float32 row lie in the
+// order of bit 2 of the thread, so that eight lanes meet eight groups of banks; they come through L1, whose lines both halves share.
+// Measured against the form with registers: 2^25 float32 blocks with a scale each 298 -> 271 us, with one scale for 96 blocks 317 -> 290,
+// bf16 342 -> 291; 13.7 M blocks with one scale 136 -> 120; 10^6 bf16 blocks 18.9 -> 13.7.  Three rows under way were 2 % slower, five
+// CTAs per SM (48 registers) 3-4 %.
+// kRing = 0: straight from global memory, for calls in which a thread has a block or two (65536 blocks 4.2 us, through the ring 4.9).
+constexpr int kRowsUnderWay = 2;
+
+__device__ __forceinline__ void copy_async_if(bool go, uint32_t dst, const void* src) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p cp.async.ca.shared.global [%1], [%2], 16;\n\t}" ::"r"((uint32_t)go), "r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_if(bool go, uint32_t dst, uint32_t dst_next, const void* src) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p cp.async.ca.shared.global [%1], [%3], 16;\n\t@p cp.async.ca.shared.global [%2], [%3 + 16], 16;\n\t}"
+                 ::"r"((uint32_t)go), "r"(dst), "r"(dst_next), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_word_async_if(bool go, uint32_t dst, const void* src) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p cp.async.ca.shared.global [%1], [%2], 4;\n\t}" ::"r"((uint32_t)go), "r"(dst), "l"(src) : "memory");
+}
+
+// n < 2^27; scale: of block 0, which is block `skip` of its tile (kTileScale).
+template <int DT, int MODE, bool SAT, int SCALES, int kRing>
 __global__ void __launch_bounds__(kThreads, 4)
-k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, int64_t n, uint32_t* codes) {
+k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale, e8::TileDiv td, uint32_t skip, uint32_t n, uint32_t* codes) {
+    constexpr int kRowBytes = DT == 0 ? 32 : 16, kSlots = kRing > 0 ? kRing : 1;
+    __shared__ __align__(16) uint8_t ring[kSlots][kThreads][kRowBytes];
+    __shared__ float ring_scale[SCALES == kBlockScale ? kSlots : 1][kThreads];
     __shared__ uint4 flip_rows[8];
-    __shared__ int64_t list[kListCap];
-    __shared__ int64_t queue[kEncWarps][64];
+    __shared__ uint32_t list[kListCap];
     __shared__ uint32_t listed;
+    static_assert(sizeof(ring) >= kEncWarps * 64 * sizeof(uint32_t), "the sweep's queue fits the idle ring");
     if (threadIdx.x < 8) flip_rows[threadIdx.x] = e8::kFlipRows[threadIdx.x];
     if (threadIdx.x == 0) listed = 0u;
     __syncthreads();
     grid_wait();
     grid_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t span = 32 * ROWS;
-    const int64_t stride = (int64_t)gridDim.x * kEncWarps * span;
-    const int64_t first = ((int64_t)blockIdx.x * kEncWarps + warp) * span;
-    for (int64_t base = first; base < n; base += stride) {
-        float v[ROWS][8];
-        float sc[ROWS];
+    const uint32_t stride = gridDim.x * kThreads, first = blockIdx.x * kThreads + threadIdx.x;
+    auto scale_of = [&](uint32_t b) -> float {
+        if (SCALES == kBlockScale) return __ldcs(scale + b);
+        if (SCALES == kTileScale) return __ldg(scale + (__umulhi(skip + b, td.mul) >> td.shr));
+        return load_scale<MODE>(scale, td, b);
+    };
+    // The code of a block by the cheapest tier, or a place on the list; `between` runs once the block has been read.
+    auto encode = [&](uint32_t b, const float (&v)[8], auto fetch, auto between) {
+        float s1 = 0.0f;
 #pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
-            const int64_t b = base + j * 32 + lane;
-            sc[j] = 1.0f;
-            if (b < n) {
-                e8::Row8<DT>::load(x, b, v[j]);
-                sc[j] = load_scale<MODE>(scale, td, b);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[j][i] = 0.0f;
+        for (int i = 0; i < 8; ++i) s1 += fabsf(v[i]);
+        // max |x_i| as a tree of three-input maxima; a NaN is dropped by fmaxf but poisons s1
+        const float m0 = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fabsf(v[2]));
+        const float m1 = fmaxf(fmaxf(fabsf(v[3]), fabsf(v[4])), fabsf(v[5]));
+        const float amax = fmaxf(fmaxf(m0, m1), fmaxf(fabsf(v[6]), fabsf(v[7])));
+        const bool pre = amax <= 1.96f && s1 <= 7.96f;     // top level is the origin, tier applicable
+        const bool origin = amax <= 0.49f && s1 <= 1.99f;  // this level is the origin too: code 0
+        uint32_t code;
+        const bool proven = e8::level_fast2_q4(v, code, flip_rows, fetch);
+        between();
+        if (b < n) {
+            if (origin || (pre && proven)) {
+                __stcs(reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(codes) + (uint64_t)(b * 4u)), origin ? 0u : code);
+            } else {  // rare
+                const uint32_t pos = atomicAdd(&listed, 1u);
+                if (pos < (uint32_t)kListCap) list[pos] = b;
+                else codes[b] = kDeferredMark;
             }
         }
+    };
+    if constexpr (kRing > 0) {
+        const uint32_t row_at = (uint32_t)__cvta_generic_to_shared(&ring[0][threadIdx.x][0]), scale_at = (uint32_t)__cvta_generic_to_shared(&ring_scale[0][threadIdx.x]);
+        const uint32_t flip = DT == 0 ? (threadIdx.x & 4u) * 4u : 0u;  // 16: the halves change places
+        auto request = [&](uint32_t b, int slot) {
+            const uint8_t* src = reinterpret_cast<const uint8_t*>(x) + (uint64_t)(b * (uint32_t)kRowBytes);
+            const uint32_t dst = row_at + (uint32_t)(slot * kThreads * kRowBytes);
+            if (DT == 0) copy_async_if(b < n, dst + flip, dst + (flip ^ 16u), src);
+            else copy_async_if(b < n, dst, src);
+            if (SCALES == kBlockScale) copy_word_async_if(b < n, scale_at + (uint32_t)(slot * kThreads * 4), reinterpret_cast<const uint8_t*>(scale) + (uint64_t)(b * 4u));
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
 #pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
-            const int64_t b = base + j * 32 + lane;
-            float s1 = 0.0f;
-            scale_row<MODE>(v[j], sc[j]);
+        for (int k = 0; k < kRing; ++k) request(first + k * stride, k);
+        for (uint32_t base = first; base < n; base += kRing * stride) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s1 += fabsf(v[j][i]);
-            // max |x_i| as a tree of three-input maxima; a NaN is dropped by fmaxf but poisons s1
-            const float m0 = fmaxf(fmaxf(fabsf(v[j][0]), fabsf(v[j][1])), fabsf(v[j][2]));
-            const float m1 = fmaxf(fmaxf(fabsf(v[j][3]), fabsf(v[j][4])), fabsf(v[j][5]));
-            const float amax = fmaxf(fmaxf(m0, m1), fmaxf(fabsf(v[j][6]), fabsf(v[j][7])));
-            const bool pre = amax <= 1.96f && s1 <= 7.96f;     // top level is the origin, tier applicable
-            const bool origin = amax <= 0.49f && s1 <= 1.99f;  // this level is the origin too: code 0
-            uint32_t code;
-            const bool proven = e8::level_fast2_q4(v[j], code, flip_rows);
-            if (b < n) {
-                if (origin || (pre && proven)) {
-                    __stcs(codes + b, origin ? 0u : code);
-                } else {  // rare
-                    const uint32_t pos = atomicAdd(&listed, 1u);
-                    if (pos < (uint32_t)kListCap) list[pos] = b;
-                    else codes[b] = kDeferredMark;
+            for (int k = 0; k < kRing; ++k) {
+                const uint32_t b = base + k * stride;
+                const float direct = SCALES != kBlockScale && b < n ? scale_of(b) : 1.0f;
+                asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
+                const uint8_t* row = &ring[k][threadIdx.x][0];
+                float v[8];
+                if (DT == 0) {
+                    const float4 lo = *reinterpret_cast<const float4*>(row + flip), hi = *reinterpret_cast<const float4*>(row + (flip ^ 16u));
+                    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+                } else {
+                    const uint4 r = *reinterpret_cast<const uint4*>(row);
+                    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        v[2 * i] = __uint_as_float(w[i] << 16);
+                        v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                    }
                 }
+                const float sc = SCALES == kBlockScale ? ring_scale[k][threadIdx.x] : direct;
+                scale_row<MODE>(v, sc);
+                const auto coordinate = [&](uint32_t i) {
+                    const float r = DT == 0 ? *reinterpret_cast<const float*>(row + ((i * 4u) ^ flip))
+                                            : __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(row + i * 2u) << 16);
+                    return scale_in<MODE>(r, sc);
+                };
+                encode(b, v, coordinate, [&]() { request(b + kRing * stride, k); });
             }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        for (uint32_t b = first; b < n; b += stride) {
+            float v[8];
+            e8::Row8<DT>::load(x, b, v);
+            scale_row<MODE>(v, scale_of(b));
+            encode(b, v, e8::NoFetch(), []() {});
         }
     }
-    auto finish = [&](int64_t b) {
+    auto finish = [&](uint32_t b) {
         float v[8];
         e8::Row8<DT>::load(x, b, v);
-        const float s = load_scale<MODE>(scale, td, b);
+        const float s = scale_of(b);
         float amax = 0.0f, s1 = 0.0f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -485,23 +550,22 @@ k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale
         // be the marker is finished twice, with the same result; the sweep is over before the list is worked off, whose
         // results may equal the marker.
         int count = 0;
+        const int lane = threadIdx.x & 31;
+        uint32_t* queue = reinterpret_cast<uint32_t*>(&ring[0][0][0]) + (threadIdx.x >> 5) * 64;
         auto drain = [&](int take) {
-            if (lane < take) finish(queue[warp][count - take + lane]);
+            if (lane < take) finish(queue[count - take + lane]);
             count -= take;
             __syncwarp();
         };
-        for (int64_t base = first; base < n; base += stride) {
-#pragma unroll 1
-            for (int j = 0; j < ROWS; ++j) {
-                const int64_t b = base + j * 32 + lane;
-                const bool marked = b < n && codes[b] == kDeferredMark;
-                const uint32_t bal = __ballot_sync(0xffffffffu, marked);
-                if (bal) {
-                    if (marked) queue[warp][count + __popc(bal & ((1u << lane) - 1u))] = b;
-                    count += __popc(bal);
-                    __syncwarp();
-                    if (count >= 32) drain(32);
-                }
+        for (uint32_t base = first - lane; base < n; base += stride) {
+            const uint32_t b = base + lane;
+            const bool marked = b < n && codes[b] == kDeferredMark;
+            const uint32_t bal = __ballot_sync(0xffffffffu, marked);
+            if (bal) {
+                if (marked) queue[count + __popc(bal & ((1u << lane) - 1u))] = b;
+                count += __popc(bal);
+                __syncwarp();
+                if (count >= 32) drain(32);
             }
         }
         if (count > 0) drain(count);
@@ -756,16 +820,41 @@ namespace {
 
 template <int DT, int MODE, bool SAT>
 int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_t n, uint32_t* codes, cudaStream_t st) {
-    int rows;
-    unsigned grid = encoder_grid(n, &rows);
-    // Up to kEncCtasPerSm one-iteration CTAs per SM would each pay for a pass over their list: the resident ones take two or
-    // three iterations, evenly (10^6 bf16 blocks 20.4 -> 18.6 us; beyond that size it costs 1 %: all finish at once).
-    const unsigned resident = 4u * (unsigned)sm_count();
-    if (rows == 3 && grid < kEncCtasPerSm * (unsigned)sm_count()) {
-        const unsigned iterations = (grid + resident - 1) / resident;
-        grid = (grid + iterations - 1) / iterations;
+    const int64_t resident = 4 * (int64_t)sm_count();
+    if (n < 3 * resident * kThreads) {  // a thread has at most three blocks
+        const int64_t need = (n + kThreads - 1) / kThreads;
+        return launch_dependent("e8_encode", k_encode_q4m2_listed<DT, MODE, SAT, kAnyScale, 0>, (unsigned)(need < resident ? need : resident), kThreads, 0, st,
+                                x, scale, td, 0u, (uint32_t)n, codes);
     }
-    return launch_dependent("e8_encode", rows == 3 ? k_encode_q4m2_listed<DT, MODE, SAT, 3> : k_encode_q4m2_listed<DT, MODE, SAT, 1>, grid, kThreads, 0, st, x, scale, td, n, codes);
+    constexpr int64_t kMost = 1 << 26, kLongTile = 1 << 30;
+    const int64_t tile = MODE == COSET_SCALE_MUL_TILE ? td.divisor : 1;
+    for (int64_t at = 0; at < n;) {
+        int64_t count = n - at < kMost ? n - at : kMost;
+        const int64_t skip = at % tile;
+        const float* s = scale;
+        e8::TileDiv part = {};
+        if (MODE == COSET_SCALE_MUL_TILE) {
+            s += at / tile;
+            if (tile > kLongTile) count = count < tile - skip ? count : tile - skip;  // one tile: the quotient of the empty division is 0
+            else if (tile > 1) part = e8::make_tile_div(tile, kLongTile + kMost);
+        }
+        const uint32_t within = tile > kLongTile ? 0u : (uint32_t)skip;
+        // Up to 32 blocks per thread of the resident CTAs, these alone, each with one pass over its list; beyond, three CTAs follow one another, so that
+        // the lists of the first are worked off while others are in their loops (4.2 M blocks 47 us against 52, 13.7 M 124 against 120).
+        const int64_t need = (count + kThreads - 1) / kThreads, cap = need <= 32 * resident ? resident : 3 * resident;
+        const unsigned grid = (unsigned)(need < cap ? need : cap);
+        const void* xs = (const uint8_t*)x + at * (DT == 0 ? 32 : 16);
+        int rc;
+        if (MODE != COSET_SCALE_MUL_TILE)
+            rc = launch_dependent("e8_encode", k_encode_q4m2_listed<DT, MODE, SAT, kAnyScale, kRowsUnderWay>, grid, kThreads, 0, st, xs, s, part, within, (uint32_t)count, codes + at);
+        else if (tile == 1)
+            rc = launch_dependent("e8_encode", k_encode_q4m2_listed<DT, COSET_SCALE_MUL_TILE, SAT, kBlockScale, kRowsUnderWay>, grid, kThreads, 0, st, xs, s, part, within, (uint32_t)count, codes + at);
+        else
+            rc = launch_dependent("e8_encode", k_encode_q4m2_listed<DT, COSET_SCALE_MUL_TILE, SAT, kTileScale, kRowsUnderWay>, grid, kThreads, 0, st, xs, s, part, within, (uint32_t)count, codes + at);
+        if (rc) return rc;
+        at += count;
+    }
+    return 0;
 }
 
 }  // namespace

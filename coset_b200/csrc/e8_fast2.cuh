@@ -26,6 +26,7 @@
 // 317 -> 307 us.  With the uniqueness of the minimum asked for only where it is used, which halves the deferred blocks of data
 // with equal magnitudes: 300 us, bf16 362 -> 351.
 #pragma once
+#include <type_traits>
 #include "e8_fast.cuh"
 
 namespace e8 {
@@ -98,7 +99,12 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 // 16-bit level word, or false when a guard refuses.
 // rows: the eight kFlipRows entries, in shared memory when the caller has a copy there (lanes index it
 // with different values; constant memory would serialise those reads), else kFlipRows itself.
-__device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& digits, const uint4* rows = kFlipRows) {
+struct NoFetch {};
+// fetch(i): coordinate i of the scaled block by a run-time index, from wherever the caller has the block in memory; without it the
+// signs at the flip coordinates come out of gathered sign bytes (20 more instructions for the ALU pipe).
+template <typename Fetch = NoFetch>
+__device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& digits, const uint4* rows = kFlipRows, Fetch fetch = Fetch()) {
+    constexpr bool kFetch = !std::is_same<Fetch, NoFetch>::value;
     const float kTie = 2.96f * 4.76837158203125e-07f;
     // Rounding, remainder and g = [d < 0] in pairs: g is rint - floor, for x is away from the integers (guarded).
     float w[8], d[8];
@@ -135,28 +141,32 @@ __device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& di
     float u, u_hi;
     split2(add2(add2(u2[0], u2[1]), add2(u2[2], u2[3])), u, u_hi);
     u = __fadd_rn(u, u_hi);
-    // sign bytes of d and of x, one byte per coordinate in key-lane order
-    const uint32_t sA = gather_bytes<0x0073>(d[7], d[6], d[5], d[4]), sB = gather_bytes<0x0073>(d[3], d[2], d[1], d[0]);
-    const uint32_t xA = gather_bytes<0x0073>(x[7], x[6], x[5], x[4]), xB = gather_bytes<0x0073>(x[3], x[2], x[1], x[0]);
     const uint32_t sel0 = (key0 & 3u) | (low0 ? 0u : 4u), sel1 = (key1 & 3u) | (low1 ? 0u : 4u);
-    const uint32_t rep0 = (sel0 | 8u) * 0x1111u, rep1 = (sel1 | 8u) * 0x1111u;  // sign-replicating selectors
-    const uint32_t dneg0 = prmt(sB, sA, rep0), xneg0 = prmt(xB, xA, rep0);  // 0 or ~0
-    const uint32_t dneg1 = prmt(sB, sA, rep1), xneg1 = prmt(xB, xA, rep1);
-    const uint32_t away0 = ~dneg0 & xneg0, up0 = ~(dneg0 | xneg0);
-    const uint32_t away1 = dneg1 & xneg1, up1 = dneg1 & ~xneg1;
-    // parities: sum f odd?  sum f' odd? (one more flip per negative d)
-    const uint32_t pw = xor3(xor3(__float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2])),
-                             xor3(__float_as_uint(w[3]), __float_as_uint(w[4]), __float_as_uint(w[5])),
-                             __float_as_uint(w[6]) ^ __float_as_uint(w[7]));
-    const uint32_t pd = xor3(xor3(__float_as_uint(d[0]), __float_as_uint(d[1]), __float_as_uint(d[2])),
-                             xor3(__float_as_uint(d[3]), __float_as_uint(d[4]), __float_as_uint(d[5])),
-                             __float_as_uint(d[6]) ^ __float_as_uint(d[7]));
-    const bool odd0 = (pw & 1u) != 0u;
-    const bool odd1 = ((pw ^ (pd >> 31)) & 1u) != 0u;
+    bool away0, up0, away1, up1;  // the signs of d and of x at the flip coordinates
+    if constexpr (kFetch) {
+        const float x0 = fetch(sel0 ^ 3u), x1 = fetch(sel1 ^ 3u);
+        const float d0 = __fsub_rn(x0, __fsub_rn(__fadd_rn(x0, kMagic), kMagic)), d1 = __fsub_rn(x1, __fsub_rn(__fadd_rn(x1, kMagic), kMagic));
+        away0 = d0 > 0.0f && x0 < 0.0f; up0 = d0 > 0.0f && !(x0 < 0.0f);
+        away1 = d1 < 0.0f && x1 < 0.0f; up1 = d1 < 0.0f && !(x1 < 0.0f);
+    } else {  // sign bytes of d and of x, one byte per coordinate in key-lane order
+        const uint32_t sA = gather_bytes<0x0073>(d[7], d[6], d[5], d[4]), sB = gather_bytes<0x0073>(d[3], d[2], d[1], d[0]);
+        const uint32_t xA = gather_bytes<0x0073>(x[7], x[6], x[5], x[4]), xB = gather_bytes<0x0073>(x[3], x[2], x[1], x[0]);
+        const uint32_t rep0 = (sel0 | 8u) * 0x1111u, rep1 = (sel1 | 8u) * 0x1111u;  // sign-replicating selectors
+        const uint32_t dneg0 = prmt(sB, sA, rep0), xneg0 = prmt(xB, xA, rep0);  // 0 or ~0
+        const uint32_t dneg1 = prmt(sB, sA, rep1), xneg1 = prmt(xB, xA, rep1);
+        away0 = (~dneg0 & xneg0) != 0u; up0 = (~(dneg0 | xneg0)) != 0u;
+        away1 = (dneg1 & xneg1) != 0u; up1 = (dneg1 & ~xneg1) != 0u;
+    }
+    // parities: sum f odd?  sum f' odd? (one more flip per negative d).  Sums of floats on the FMA pipe instead of exclusive-or trees.
+    const F2 F = add2(add2(f2[0], f2[1]), add2(f2[2], f2[3])), G = add2(add2(g2[0], g2[1]), add2(g2[2], g2[3]));
+    float f_lo, f_hi, g_lo, g_hi;
+    split2(F, f_lo, f_hi);
+    split2(G, g_lo, g_hi);
+    const float p0 = __fadd_rn(__fadd_rn(f_lo, kMagic), f_hi), p1 = __fsub_rn(__fsub_rn(p0, g_lo), g_hi);
+    const bool odd0 = (__float_as_uint(p0) & 1u) != 0u, odd1 = (__float_as_uint(p1) & 1u) != 0u;
     ok = ok && (u < 1.5f || !odd1);  // without a flip of coset 1 its minimum is not used
     // flip costs: 1 -+ 2 m0 for the integer coset, 1 -+ 2 (1/2 - mn) for the half-integer coset
-    const float m0s = __uint_as_float(__float_as_uint(m0) ^ (away0 & 0x80000000u));
-    const float c0 = __fmaf_rn(-2.0f, m0s, 1.0f);
+    const float c0 = __fmaf_rn(away0 ? 2.0f : -2.0f, m0, 1.0f);
     const float c1 = away1 ? __fmaf_rn(-2.0f, mn, 2.0f) : __fmul_rn(2.0f, mn);
     float delta = __fsub_rn(2.0f, l1);  // dist1 - dist0 (the shared sum d^2 cancels)
     if (odd1) delta = __fadd_rn(delta, c1);
@@ -165,7 +175,7 @@ __device__ __forceinline__ bool level_fast2_q4(const float (&x)[8], uint32_t& di
     const bool half = delta < 0.0f;
     const float hf = half ? 1.0f : 0.0f, nhf = half ? -1.0f : 0.0f;
     const bool odd = half ? odd1 : odd0;
-    const uint32_t up = half ? up1 : up0;
+    const bool up = half ? up1 : up0;
     const uint32_t row = (half ? sel1 : sel0) ^ 3u;  // coordinate index of the flip
     const uint32_t stp = odd ? (up ? 1u : 0xffffffffu) : 0u;  // +1 when the rule moves up, -1 otherwise
     // digit words from the chosen coset's rounded integers fs = f - half * g
