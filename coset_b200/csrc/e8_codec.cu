@@ -384,12 +384,16 @@ k_encode_q4m2_queued(const void* __restrict__ x, const float* __restrict__ scale
 constexpr uint32_t kDeferredMark = 0x80000000u;
 constexpr int kListCap = 1024;  // the benchmark data defers 1 % of the 19000 blocks of a CTA
 
+// One level by the tiers that accept every block.  amax, s1: max and sum of |x_i|.
+__device__ __forceinline__ uint32_t level_exact_q4(const float (&x)[8], float amax, float s1) {
+    return e8::level_slow_q4(x, s1 == s1 && s1 - s1 == 0.0f ? amax : __int_as_float(0x7fc00000));
+}
 // One level of a deferred block: the cheapest tier when it applies, then the exact-rounding tier, then the
-// literal search.  amax, s1: max and sum of |x_i|.
+// literal search.
 __device__ __forceinline__ uint32_t level_any_q4(const float (&x)[8], float amax, float s1, const uint4* rows) {
     uint32_t digits;
     if (amax <= 1.96f && s1 <= 7.96f && e8::level_fast2_q4(x, digits, rows)) return digits;
-    return e8::level_slow_q4(x, s1 == s1 && s1 - s1 == 0.0f ? amax : __int_as_float(0x7fc00000));
+    return level_exact_q4(x, amax, s1);
 }
 
 // SAT: every scaled coordinate is first clamped to +-kSaturate, which keeps the two-level code from wrapping around (the top level
@@ -535,7 +539,8 @@ k_encode_q4m2_listed(const void* __restrict__ x, const float* __restrict__ scale
 #pragma unroll 1
         for (int m = 0; m < 2; ++m) {
             const bool origin = amax <= 0.49f && s1 <= 1.99f;
-            if (!origin) code |= level_any_q4(v, amax, s1, flip_rows) << (16 * m);
+            // the cheapest tier has refused level 0 as it is
+            if (!origin) code |= (m > 0 ? level_any_q4(v, amax, s1, flip_rows) : level_exact_q4(v, amax, s1)) << (16 * m);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(v[i], 0.25f);
             amax *= 0.25f;
