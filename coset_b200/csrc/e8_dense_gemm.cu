@@ -1,5 +1,7 @@
-// Product of the layer's kept dense weight with a batch of tokens that is neither a few nor thousands:
-//     y[T, N] = x[T, K] (bf16) * W[N, K]^T (bf16) + bias (float32), float32 sums, one rounding of the result.
+// Dense products of medium size in bf16, float32 sums, one rounding of the result:
+//     y[T, N] = x[T, K] W[N, K]^T + bias (float32)    a layer's kept dense weight with some tens to some thousand tokens
+//     dx[T, K] = g[T, N] W[N, K]                       and the two products of a training layer's backward pass: the same kernel, with one
+//     dw[N, K] = g[T, N]^T x[T, K]                     or both operands read along the other dimension (MN-major tiles)
 //
 // Between 17 and 2047 tokens a 4096 x 4096 layer has 32 MB of weights to stream and 0.6 to 69 GFLOP to do: the tiles must be large
 // in features (so that the tokens are not read over and over) and there must be enough of them for 148 SMs.  So a pair of CTAs
@@ -13,11 +15,14 @@
 // a small product is latency: 2.3 thousand cycles until the first load, 1.2 until it arrives, 105 ns per K step of 64 with 32 or 64 tokens (the issue
 // of its four instructions and one wait; stages of two steps below 160 tokens share the wait), 2 to 7 thousand cycles for the sums.  The kernel is
 // launched as a programmatic dependent, which hides about 2 us of that behind the kernel before it.
+// Two CTAs fit an SM (ten warps, at most 112 KB of stages) where there are more tiles than SMs.
 // Measured, 4096 x 4096 with a bias, torch's product and its bias cast against this kernel (graph replays, three weights in turn): 64 tokens 8.9 + 2.9
-// against 10.7 us, 256 tokens 11.1 + 2.9 against 14.1, 1024 tokens 25.2 + 2.9 against 26.9; a call of the layer with 256 tokens 20.7 -> 14.5 us, for
-// the host was what bounded it.
+// against 8.8 us, 256 tokens 11.1 + 2.9 against 12.6, 1024 tokens 25.2 + 2.9 against 25.5; a call of the layer with 256 tokens 20.7 -> 13.3 us, for
+// the host was what bounded it.  The products of a training step of a [3072, 768] layer with 4096 tokens: 22.7 + 16.3 + 15.1 us against 18.0 + 15.3 + 13.8 for
+// torch's, but 15 us of host time instead of 42, and the host bounds the step.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <math.h>
 
 #include "common.cuh"
 #include "umma.cuh"
@@ -29,9 +34,10 @@ namespace {
 
 constexpr int kRows = 128;           // weight rows of one CTA
 constexpr int kMaxStages = 8;
-constexpr int kEpilogueWarps = 16, kTmaWarp = 16, kMmaWarp = 17;
-constexpr int kThreads = 18 * 32;
+constexpr int kEpilogueWarps = 8, kTmaWarp = 8, kMmaWarp = 9;
+constexpr int kThreads = 10 * 32;
 constexpr int kSmemBudget = 226 * 1024;  // 227 KB less the alignment
+constexpr int kSmemOfTwo = 112 * 1024;   // two CTAs on an SM (228 KB, 1 KB of which each CTA takes)
 constexpr int kBarrierBytes = 16 * kMaxStages + 16;
 constexpr int kScratchRow = 40;       // 32 features and a pad, in values
 constexpr int kScratchBytes = kEpilogueWarps * 32 * kScratchRow * 2;
@@ -47,6 +53,7 @@ struct Shape {
     int N, K, T;
     Plan plan;
     const float* bias;
+    int round_bias;   // to bf16 before it is added, as torch does
     __nv_bfloat16* y;
     int64_t ldy;
     int vector_rows;  // rows of y are made of 16-byte chunks
@@ -75,10 +82,11 @@ __device__ __forceinline__ void send_columns(const Shape& s, uint32_t tmem, uint
 // The columns this pair owns: summed with what the others sent, plus bias, rounded and stored.  A lane holds one feature and W tokens;
 // a scratch of the warp turns them into rows of 32 features, so that four lanes store the 64 bytes of a token.
 template <int W>
-__device__ __forceinline__ void store_columns(const Shape& s, uint32_t tmem, const float* sums, __nv_bfloat16* scratch, int pair, int row, int group, int feature0,
+__device__ __forceinline__ void store_columns(const Shape& s, bool ok, uint32_t tmem, const float* sums, __nv_bfloat16* scratch, int pair, int row, int group, int feature0,
                                               int token0) {
     const int own = s.plan.tokens / s.plan.split, lane = threadIdx.x & 31;
-    const float bias = s.bias && feature0 + lane < s.N ? __ldg(behind_wait(s.bias) + feature0 + lane) : 0.0f;
+    float bias = !ok ? NAN : s.bias && feature0 + lane < s.N ? __ldg(behind_wait(s.bias) + feature0 + lane) : 0.0f;  // a wait gave up: no number
+    if (s.round_bias) bias = __bfloat162float(__float2bfloat16_rn(bias));
     for (int c = group * W; c < own; c += (kEpilogueWarps / 4) * W) {
         const int t = token0 + pair * own + c;
         if (t >= s.T || feature0 >= s.N) break;
@@ -116,8 +124,17 @@ __device__ __forceinline__ void store_columns(const Shape& s, uint32_t tmem, con
     }
 }
 
-template <int kSub>
-__global__ void __launch_bounds__(kThreads, 1)
+// One K step of 64 of an operand's `rows` rows from `row0` on into `dst`.
+template <bool MN>
+__device__ __forceinline__ void load_operand(uint32_t dst, const CUtensorMap* map, int rows, int row0, int k0, uint32_t bar) {
+    if (!MN) tma_load_pair(dst, map, k0, row0, bar);
+    else
+        for (int r = 0; r < rows; r += 64) tma_load_pair(dst + (uint32_t)(r * BK * 2), map, row0 + r, k0, bar);
+}
+
+// W_MN, X_MN: the operand lies in memory with K as its slow dimension.
+template <int kSub, bool W_MN, bool X_MN>
+__global__ void __launch_bounds__(kThreads, 2)
 k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ Shape s) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -177,32 +194,34 @@ k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
 #pragma unroll
                 for (int i = 0; i < kSub; ++i)
                     if (i < subs) {
-                        tma_load_pair(at + i * (kRows * BK * 2), &w_map, (k + i) * BK, row0, bar);
-                        tma_load_pair(at + x_at + i * x_bytes, &x_map, (k + i) * BK, token0 + half * (s.plan.tokens / 2), bar);
+                        load_operand<W_MN>(at + i * (kRows * BK * 2), &w_map, kRows, row0, (k + i) * BK, bar);
+                        load_operand<X_MN>(at + x_at + i * x_bytes, &x_map, s.plan.tokens / 2, token0 + half * (s.plan.tokens / 2), (k + i) * BK, bar);
                     }
             }
             __syncwarp();
             if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
     } else if (warp == kMmaWarp && leader) {
-        const uint64_t desc0 = umma_desc(base);
-        const uint32_t desc_hi = (uint32_t)(desc0 >> 32), desc_lo0 = (uint32_t)desc0;
-        // kind::f16: float32 sums, bf16 x bf16, both K-major, M = 256 over the pair
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(s.plan.tokens >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+        // the descriptors of all tiles differ in the 14-bit address field alone (units of 16 bytes)
+        const uint64_t w0 = W_MN ? umma_desc_mn(base) : umma_desc(base), x0 = X_MN ? umma_desc_mn(base) : umma_desc(base);
+        const uint32_t w_hi = (uint32_t)(w0 >> 32), w_lo = (uint32_t)w0, x_hi = (uint32_t)(x0 >> 32), x_lo = (uint32_t)x0;
+        constexpr uint32_t kWStep = W_MN ? 128 : 2, kXStep = X_MN ? 128 : 2;  // 16 of K: two groups of eight rows, or 32 bytes inside the swizzle row
+        // kind::f16: float32 sums, bf16 x bf16, M = 256 over the pair
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((W_MN ? 1u : 0u) << 15) | ((X_MN ? 1u : 0u) << 16) | ((uint32_t)(s.plan.tokens >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
         int stage = 0;
         uint32_t phase = 0;
         for (int k = first; k < last; k += kSub) {
             if (!mbar_wait_warp(full_base + 8 * stage, phase)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (elect_one()) {
-                const uint32_t a_lo = desc_lo0 + (uint32_t)(stage * (bytes >> 4)), b_lo = a_lo + (x_at >> 4);
+                const uint32_t a_lo = w_lo + (uint32_t)(stage * (bytes >> 4)), b_lo = x_lo + (uint32_t)(stage * (bytes >> 4)) + (x_at >> 4);
 #pragma unroll
                 for (int i = 0; i < kSub; ++i)
                     if (i == 0 || k + i < last) {
 #pragma unroll
-                        for (int j = 0; j < BK / 16; ++j)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle row
-                            umma_f16_pair(tmem, make_desc(a_lo + (uint32_t)(i * (kRows * BK * 2 >> 4) + j * 2), desc_hi),
-                                          make_desc(b_lo + (uint32_t)i * (x_bytes >> 4) + (uint32_t)(j * 2), desc_hi), idesc, i + j > 0 || k > first ? 1u : 0u);
+                        for (int j = 0; j < BK / 16; ++j)
+                            umma_f16_pair(tmem, make_desc(a_lo + (uint32_t)(i * (kRows * BK * 2 >> 4)) + (uint32_t)j * kWStep, w_hi),
+                                          make_desc(b_lo + (uint32_t)i * (x_bytes >> 4) + (uint32_t)j * kXStep, x_hi), idesc, i + j > 0 || k > first ? 1u : 0u);
                     }
                 umma_commit_pair(bar_base + 8 * stage, both);
                 if (k + kSub >= last) umma_commit_pair(done_bar, both);
@@ -226,13 +245,13 @@ k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
         }
         cluster_sync();  // ... and the sums have arrived
     }
-    if (warp < kEpilogueWarps && ok) {
+    if (warp < kEpilogueWarps) {
         const float* sums = reinterpret_cast<const float*>(gen + stages * bytes + kBarrierBytes);
         __nv_bfloat16* scratch = reinterpret_cast<__nv_bfloat16*>(gen) + warp * 32 * kScratchRow;
         const int feature0 = row0 + quarter * 32;
-        if (own >= 128) store_columns<32>(s, lanes, sums, scratch, pair, row, group, feature0, token0);
-        else if (own >= 64) store_columns<16>(s, lanes, sums, scratch, pair, row, group, feature0, token0);
-        else store_columns<8>(s, lanes, sums, scratch, pair, row, group, feature0, token0);
+        if (own >= 128) store_columns<32>(s, ok, lanes, sums, scratch, pair, row, group, feature0, token0);
+        else if (own >= 64) store_columns<16>(s, ok, lanes, sums, scratch, pair, row, group, feature0, token0);
+        else store_columns<8>(s, ok, lanes, sums, scratch, pair, row, group, feature0, token0);
     }
     if (!ok) {
         if (s.status) atomicExch(s.status, 1);
@@ -245,10 +264,10 @@ k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
 }
 
 // Stages: what fits, no more than there is work for, and room for the epilogue's scratch.
-Plan with_stages(int tokens, int split, int steps) {
+Plan with_stages(int tokens, int split, int steps, bool two = false) {
     Plan p = {tokens, split, 1, tokens <= 128 ? 2 : 1};
     const int bytes = stage_bytes(tokens, p.sub), need = ((steps + split - 1) / split + p.sub - 1) / p.sub, least = (kScratchBytes + bytes - 1) / bytes;
-    p.stages = (kSmemBudget - kBarrierBytes - sums_bytes(tokens, split)) / bytes;
+    p.stages = ((two ? kSmemOfTwo : kSmemBudget) - kBarrierBytes - sums_bytes(tokens, split)) / bytes;
     if (p.stages > kMaxStages) p.stages = kMaxStages;
     if (p.stages > need) p.stages = need;
     if (p.stages < least) p.stages = least;
@@ -259,32 +278,36 @@ Plan with_stages(int tokens, int split, int steps) {
 // clusters (14 of eight CTAs: 16 took two waves).
 int clusters_at_once(int split) { return split == 1 ? sm_count() / 2 : split == 2 ? sm_count() * 35 / 148 : sm_count() * 13 / 148; }
 
-// The plan of the least estimated time in ns.  Measured over 14 shapes from [17, 4096] x [4096, 4096] to [1000, 768] x [768, 3072]: a K step
-// of 64 takes 132 ns with 32 tokens and 361 with 256 (the loads of the weights, then the tensor cores), the exchange of the
-// sums 1.7 us with 32 tokens and two pairs and 4 us with 256.  The plan taken was within 2 % of the best one on average, 18 % at worst
-// ([256, 4096] x [4096, 4096]: 128 tokens, two pairs 14.1 us, against 17.3 with one pair and 23.7 with 256 tokens).
-Plan make_plan(int N, int K, int T) {
+// The plan of the least estimated time in ns.  Measured over 41 products from [17, 4096] x [4096, 4096] to [4096, 2048] x [2048, 2048] in all three
+// forms: a K step of 64 takes 110 ns with 16 pairs at work and 155 with 74 (the loads), or 1.4 ns a token (the tensor cores, from 110
+// tokens on); the exchange of the sums 1.7 us with 32 tokens and two pairs and 4.4 with 256; every further round of clusters 2 to 4 us where a CTA has
+// an SM to itself, and half of that where two share one and each one's loads and stores run under the other's products ([4096, 2048] x [2048, 2048]
+// 30.3 -> 26.8 us).  The plan taken was within 3 % of the best one on average, 15 % at worst.
+Plan make_plan(int N, int K, int T, int unit) {  // unit: tokens come in multiples of it
     const int steps = (K + BK - 1) / BK;
-    Plan best = with_stages(32, 1, steps);
+    Plan best = with_stages(unit, 1, steps);
     double least = 0.0;
-    for (int tokens = 32; tokens <= 256 && tokens < T + 32; tokens += 32)
+    for (int tokens = unit; tokens <= 256 && tokens < T + unit; tokens += unit)
         for (int split = 1; split <= 4 && split <= steps; split *= 2) {
             const int64_t clusters = (int64_t)((N + 2 * kRows - 1) / (2 * kRows)) * ((T + tokens - 1) / tokens);
-            const int64_t at_once = clusters_at_once(split), waves = (clusters + at_once - 1) / at_once, pairs = clusters * split < 74 ? clusters * split : 74;
+            const int64_t at_once = clusters_at_once(split), rounds = (clusters + at_once - 1) / at_once, pairs = clusters * split < 74 ? clusters * split : 74;
+            const bool two = rounds > 1 && split == 1;
+            const double loads = 100.0 + 0.75 * (double)pairs, products = 1.4 * tokens, step = loads > products ? loads : products;
             const double exchange = split == 1 ? 0.0 : split == 2 ? 1300.0 + 12.0 * tokens : 1800.0 + 16.0 * tokens;
-            const double time = (double)waves * ((double)((steps + split - 1) / split) * (100.0 + 1.02 * tokens) + exchange + 1500.0) + 30.0 * (double)pairs;
+            const double time = exchange + (double)rounds * ((steps + split - 1) / split) * step + (double)(rounds - 1) * (two ? 2200.0 : 4300.0);
             if (least == 0.0 || time < least) {
                 least = time;
-                best = with_stages(tokens, split, steps);
+                best = with_stages(tokens, split, steps, two);
             }
         }
     return best;
 }
 
-template <int kSub>
+template <int kSub, bool W_MN, bool X_MN>
 int launch_linear(const CUtensorMap& x_map, const CUtensorMap& w_map, const Shape& s, cudaStream_t st) {
     const int smem = 1024 /* alignment */ + s.plan.stages * stage_bytes(s.plan.tokens, kSub) + kBarrierBytes + sums_bytes(s.plan.tokens, s.plan.split);
-    if (int e = check_cuda(cudaFuncSetAttribute(k_linear_pair<kSub>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
+    const auto kernel = k_linear_pair<kSub, W_MN, X_MN>;
+    if (int e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((s.N + 2 * kRows - 1) / (2 * kRows) * 2 * s.plan.split), (unsigned)((s.T + s.plan.tokens - 1) / s.plan.tokens));
     cfg.blockDim = dim3(kThreads);
@@ -294,34 +317,43 @@ int launch_linear(const CUtensorMap& x_map, const CUtensorMap& w_map, const Shap
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)(2 * s.plan.split);
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
     cfg.numAttrs = 2;
-    if (int e = check_cuda(cudaLaunchKernelEx(&cfg, k_linear_pair<kSub>, x_map, w_map, s), "e8_dense_linear")) return e;
-    return check_launch("e8_dense_linear");
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, x_map, w_map, s), "dense product");
 }
 
-int dense_linear(const void* w, int n_out, int n_in, const void* x, int64_t ldx, int T, const float* bias, void* y, int64_t ldy,
-                 int* status, const Plan* given, void* stream) {
-    if (n_out < 0 || n_in < 0 || T < 0 || (n_in % 8) != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
-    if (n_out == 0 || T == 0) return 0;
-    if (n_in == 0) return fail(COSET_E_BADARG, "n_in is 0");
+template <bool W_MN, bool X_MN>
+int dense_product(const void* w, int64_t ldw, const void* x, int64_t ldx, int N, int T, int K, const float* bias, int round_bias, void* y, int64_t ldy,
+                  int* status, const Plan* given, void* stream) {
+    if (N < 0 || T < 0 || K < 0) return fail(COSET_E_BADARG, "negative size");
+    if (N == 0 || T == 0) return 0;
+    if (K == 0) return fail(COSET_E_BADARG, "nothing to sum over");
     if (!w || !x || !y) return fail(COSET_E_BADARG, "null pointer");
-    if (ldx < n_in || ldy < n_out || (ldx % 8) != 0) return fail(COSET_E_BADARG, "leading dimensions: ldx >= n_in and a multiple of 8, ldy >= n_out");
-    if (!aligned(x, 16) || !aligned(w, 16)) return fail(COSET_E_ALIGN, "x and the weight must be 16-byte aligned");
-    const int vector_rows = aligned(y, 16) && ldy % 8 == 0 && n_out % 8 == 0;
-    Shape s = {n_out, n_in, T, given ? *given : make_plan(n_out, n_in, T), bias, (__nv_bfloat16*)y, ldy, vector_rows, status};
-    if ((T + s.plan.tokens - 1) / s.plan.tokens > 65535) return fail(COSET_E_UNSUPPORTED, "T too large");
+    if (ldw < (W_MN ? N : K) || ldx < (X_MN ? T : K) || ldw % 8 != 0 || ldx % 8 != 0 || ldy < N)
+        return fail(COSET_E_BADARG, "leading dimensions: at least a row, and multiples of 8 for the operands");
+    if (!aligned(x, 16) || !aligned(w, 16)) return fail(COSET_E_ALIGN, "the operands must be 16-byte aligned");
+    Shape s = {N, K, T, given ? *given : make_plan(N, K, T, X_MN ? 128 : 32), bias, round_bias, (__nv_bfloat16*)y, ldy, aligned(y, 16) && ldy % 8 == 0 && N % 8 == 0, status};
+    if ((T + s.plan.tokens - 1) / s.plan.tokens > 65535) return fail(COSET_E_UNSUPPORTED, "too many columns");
     CUtensorMap x_map, w_map;
-    if (int e = make_bf16_map(&x_map, x, n_in, T, ldx, s.plan.tokens / 2)) return e;
-    if (int e = make_bf16_map(&w_map, w, n_in, n_out, n_in, kRows)) return e;
-    return s.plan.sub == 2 ? launch_linear<2>(x_map, w_map, s, (cudaStream_t)stream) : launch_linear<1>(x_map, w_map, s, (cudaStream_t)stream);
+    if (int e = X_MN ? make_bf16_map(&x_map, x, T, K, ldx, BK) : make_bf16_map(&x_map, x, K, T, ldx, s.plan.tokens / 2)) return e;
+    if (int e = W_MN ? make_bf16_map(&w_map, w, N, K, ldw, BK) : make_bf16_map(&w_map, w, K, N, ldw, kRows)) return e;
+    return s.plan.sub == 2 ? launch_linear<2, W_MN, X_MN>(x_map, w_map, s, (cudaStream_t)stream) : launch_linear<1, W_MN, X_MN>(x_map, w_map, s, (cudaStream_t)stream);
 }
 
 }  // namespace
 
-extern "C" int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, void* y,
-                                     int64_t ldy, int* status, void* stream) {
-    return dense_linear(w_bf16, n_out, n_in, x_bf16, ldx, T, bias, y, ldy, status, nullptr, stream);
+extern "C" int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, int round_bias,
+                                     void* y, int64_t ldy, int* status, void* stream) {
+    if (n_in % 8 != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
+    return dense_product<false, false>(w_bf16, n_in, x_bf16, ldx, n_out, T, n_in, bias, round_bias, y, ldy, status, nullptr, stream);
+}
+
+extern "C" int coset_dense_input_grad(const void* g_bf16, const void* w_bf16, int T, int n_out, int n_in, void* dx, int* status, void* stream) {
+    return dense_product<true, false>(w_bf16, n_in, g_bf16, n_out, n_in, T, n_out, nullptr, 0, dx, n_in, status, nullptr, stream);
+}
+
+extern "C" int coset_dense_weight_grad(const void* g_bf16, const void* x_bf16, int T, int n_out, int n_in, void* dw, int* status, void* stream) {
+    return dense_product<true, true>(x_bf16, n_in, g_bf16, n_out, n_in, n_out, T, nullptr, 0, dw, n_in, status, nullptr, stream);
 }

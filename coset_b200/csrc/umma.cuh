@@ -154,6 +154,12 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
     return d;
 }
 
+// MN-major, SWIZZLE_128B: the tile is made of blocks of 64 rows (128 bytes, contiguous along the rows) x 64 K, 8 KiB each; LBO = 8192 B between
+// blocks of rows, SBO = 1024 B between groups of eight K.
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr) {
+    return (umma_desc(smem_addr) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(8192 >> 4) << 16);
+}
+
 __device__ __forceinline__ uint64_t make_desc(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
 
 __device__ __forceinline__ uint32_t swizzled_chunk_offset(int row, int chunk) {
@@ -211,9 +217,17 @@ inline int make_bf16_map(CUtensorMap* map, const void* x, int K, int T, int64_t 
     const cuuint64_t strides[1] = {(cuuint64_t)ldx * 2};  // bytes between rows; a multiple of 16 (ldx % 8 == 0)
     const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, elem,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const auto make = [&]() {
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = make();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {  // a thread (autograd's, say) that has not used the runtime yet: bind its device
+        int device = 0;
+        if (int e = check_cuda(cudaGetDevice(&device), "cudaGetDevice")) return e;
+        if (int e = check_cuda(cudaSetDevice(device), "cudaSetDevice")) return e;
+        r = make();
+    }
     if (r != CUDA_SUCCESS) return fail(COSET_E_BADARG, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return 0;
 }

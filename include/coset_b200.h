@@ -405,13 +405,20 @@ int coset_e8_decode_gemm(const void* codes, const float* beta, int64_t blocks_pe
                          int64_t ldy, float clip, void* scratch, int64_t scratch_bytes, int* status, void* stream);
 
 /* Product with a dense bf16 weight that the caller keeps, [n_out, n_in] contiguous and 16-byte aligned, for some tens to some
- * thousand tokens: y[T, ldy] (bf16) = x[T, ldx] (bf16, rows 16-byte aligned) * W^T + bias (float32 or null), float32 sums, one
- * rounding.  n_in is a multiple of 8.  One launch, no scratch memory.  status (device int, may be null) is set to 1 when a bounded wait
- * inside the kernel gave up; the result is then incomplete.
+ * thousand tokens: y[T, ldy] (bf16) = x[T, ldx] (bf16, rows 16-byte aligned) * W^T + bias (float32 or null; round_bias: rounded to bf16
+ * first), float32 sums, one rounding.  n_in is a multiple of 8.  One launch, no scratch memory.  status (device int, may be null) is set to 1 when a bounded wait
+ * inside the kernel gave up; the results of its tile are then not a number.
  * Replaces the dense-weight matmul after a one-off dequantisation, coset/legacy/quant/vlut.py:72-117.
  */
-int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, void* y,
-                          int64_t ldy, int* status, void* stream);
+int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, int round_bias,
+                          void* y, int64_t ldy, int* status, void* stream);
+
+/* The two products of its backward pass, all bf16 with contiguous rows, 16-byte aligned, n_out and n_in multiples of 8, float32 sums and one
+ * rounding: dx[T, n_in] = g[T, n_out] W[n_out, n_in] and dw[n_out, n_in] = g^T x[T, n_in].  Replaces the matmuls of autograd's linear
+ * backward behind coset/core/layers.py:524-536.  Where a bounded wait gave up, results are not a number.
+ */
+int coset_dense_input_grad(const void* g_bf16, const void* w_bf16, int T, int n_out, int n_in, void* dx, int* status, void* stream);
+int coset_dense_weight_grad(const void* g_bf16, const void* x_bf16, int T, int n_out, int n_in, void* dw, int* status, void* stream);
 
 #ifdef __cplusplus
 }

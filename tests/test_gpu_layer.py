@@ -450,3 +450,55 @@ def test_frozen_layer_does_not_hold_on_to_its_input(frozen, kept):
     y.sum().backward()
     assert torch.equal(x.grad, want) and torch.equal(layer.bias.grad, bias)
     assert (layer.weight.grad is None) == frozen
+
+
+@pytest.mark.parametrize("tokens,n_out,n_in", [(1, 8, 8), (63, 72, 136), (128, 768, 768), (257, 264, 520), (1000, 1024, 64), (4096, 200, 328)])
+@pytest.mark.parametrize("bias", [True, False])
+def test_bf16_products_of_a_training_step(tokens, n_out, n_in, bias):
+    """The layer's own products, forward and backward: edges of the tiles, K in one part and in several, against 64 bits."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(n_in, n_out, device="cuda", tiling="row", bias=bias, init_method="zeros")
+    layer.load_weights(torch.randn(n_out, n_in, device="cuda") * 20.0, torch.randn(n_out, device="cuda") if bias else None)
+    x = torch.randn(tokens, n_in, device="cuda").bfloat16().requires_grad_()
+    g = torch.randn(tokens, n_out, device="cuda").bfloat16()
+    y = layer(x)
+    y.backward(g)
+    wq = layer._quantize_weights(torch.bfloat16).detach().double()
+    b = layer.bias.detach().bfloat16().double() if bias else torch.zeros(n_out, device="cuda", dtype=torch.float64)
+    xd, gd = x.detach().double(), g.double()
+    # one rounding to 8 significant bits, and float32 sums whose parts round or truncate relative to the sum of the magnitudes
+    for got, want, size in ((y.detach(), xd @ wq.T + b, xd.abs() @ wq.abs().T + b.abs()), (x.grad, gd @ wq, gd.abs() @ wq.abs())):
+        assert got.dtype == torch.bfloat16 and bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * size).all())
+    dw = torch.empty(n_out, n_in, dtype=torch.bfloat16, device="cuda")
+    assert _lib.lib().coset_dense_weight_grad(_lib.ptr(g), _lib.ptr(x), tokens, n_out, n_in, _lib.ptr(dw), None, _lib.stream()) == 0
+    want, size = gd.T @ xd, gd.abs().T @ xd.abs()
+    assert bool(((dw.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * size).all())
+
+
+@pytest.mark.parametrize("form", ["expanded", "strided", "offset", "three"])
+def test_bf16_products_with_awkward_tensors(form):
+    """Gradients and inputs that the own products cannot read, or read only as rows, give what plain ones give."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 32, device="cuda", tiling="row", init_method="zeros")
+    layer.load_weights(torch.randn(32, 64, device="cuda") * 20.0, torch.randn(32, device="cuda"))
+    x, g = torch.randn(24, 64, device="cuda").bfloat16(), torch.randn(24, 32, device="cuda").bfloat16()
+    if form == "expanded":
+        g = g[:1].expand(24, 32)
+
+    def step(x, g):
+        layer.zero_grad()
+        x = x.detach().requires_grad_()
+        y = layer(x)
+        y.backward(g)
+        return [t.reshape(-1).float() for t in (y.detach(), x.grad, layer.weight.grad, layer.theta_beta.grad, layer.bias.grad)]
+    want = step(x, g.contiguous())
+    if form == "strided":
+        x, g = torch.cat([x, x], 1)[:, :64], torch.cat([g, g], 1)[:, :32]
+    elif form == "offset":
+        x = torch.cat([x.new_zeros(1), x.reshape(-1)])[1:].view(24, 64)
+        g = torch.cat([g.new_zeros(1), g.reshape(-1)])[1:].view(24, 32)
+    elif form == "three":
+        x, g = x.view(4, 6, 64), g.view(4, 6, 32)
+    for a, b in zip(step(x, g), want):  # sums of at most 64 products in another order, then bf16
+        assert torch.allclose(a, b, rtol=2.0 ** -7, atol=2.0 ** -7 * float(b.abs().max()))

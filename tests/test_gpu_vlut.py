@@ -692,7 +692,7 @@ def test_product_with_the_kept_dense_weight_refuses():
     L = _lib.lib()
     w, x, y = (torch.zeros(64, 64, dtype=torch.bfloat16, device="cuda") for _ in range(3))
     call = lambda n_out=64, n_in=64, ldx=64, T=64, ldy=64, wp=w.data_ptr(), xp=x.data_ptr(): L.coset_e8_dense_linear(
-        wp, n_out, n_in, xp, ldx, T, None, y.data_ptr(), ldy, None, _lib.stream())
+        wp, n_out, n_in, xp, ldx, T, None, 0, y.data_ptr(), ldy, None, _lib.stream())
     assert call() == 0 and call(T=0) == 0 and call(n_out=0) == 0
     for bad in (dict(n_in=60), dict(n_in=0), dict(ldx=56), dict(ldx=68), dict(ldy=63), dict(wp=None), dict(xp=None), dict(wp=w.data_ptr() + 2), dict(xp=x.data_ptr() + 8), dict(T=-1)):
         assert call(**bad) < 0, bad
