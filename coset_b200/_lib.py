@@ -68,6 +68,9 @@ SIGNATURES = {
     "coset_e8_dense_linear": [_vp, _i32, _i32, _vp, _i64, _i32, _vp, _i32, _vp, _i64, _vp, _vp],
     "coset_dense_input_grad": [_vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp],
     "coset_dense_weight_grad": [_vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp],
+    "coset_f32_linear": [_vp, _vp, _vp, _i32, _i32, _i32, _vp, _vp],
+    "coset_f32_input_grad": [_vp, _vp, _i32, _i32, _i32, _vp, _vp],
+    "coset_f32_weight_grad": [_vp, _vp, _i32, _i32, _i32, _vp, _vp],
     "coset_layer_beta": [_vp, _vp, _vp, _i64, _vp, _vp],
     "coset_layer_beta_bias": [_vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _vp],
     "coset_column_sum": [_vp, _i32, _i64, _i64, _vp, _i32, _vp],

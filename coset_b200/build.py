@@ -34,6 +34,7 @@ SOURCES = [
     "e8_dequant_gemm.cu",
     "e8_decode_gemm.cu",
     "e8_dense_gemm.cu",
+    "f32_product.cu",
     "d4.cu",
 ]
 

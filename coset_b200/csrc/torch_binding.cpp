@@ -434,15 +434,20 @@ bool plain(const Tensor& t) {
     return (t.key_set().raw_repr() & ~known.raw_repr()) == 0 && !(at::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined();
 }
 
-// Whether the library's own kernels may multiply bf16 matrices of these rows: contiguous, aligned, and nobody looks at the torch calls.
+// Whether the library's own kernels may multiply a matrix: contiguous (and in bf16 made of aligned 16-byte chunks), and nobody looks at the torch calls.
 bool own_rows(const Tensor& t) {
-    return t.dim() == 2 && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.size(0) > 0 && t.size(0) <= INT32_MAX && t.size(1) > 0 && t.size(1) % 8 == 0 &&
-           (uintptr_t)t.const_data_ptr() % 16 == 0 && plain(t) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
+    const bool f32 = t.scalar_type() == at::kFloat;
+    return t.dim() == 2 && (f32 || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0)) && t.is_contiguous() &&
+           t.size(0) > 0 && t.size(0) <= INT32_MAX && t.size(1) > 0 && plain(t) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
 }
-// Whether they should: a step of a layer of this size is bound by the host (117 us with them, 145 with torch's products), and
-// they cost the device up to 25 % more ([4096, 768] x [3072, 768] 22.7 us against 18.0).
-bool own_training_products(int64_t tokens, int64_t n_out, int64_t n_in) {
-    return n_out * n_in <= (int64_t)1 << 22 && tokens <= ((int64_t)1 << 34) / (n_out * n_in) && n_out % 8 == 0 && n_in % 8 == 0;
+// Whether they should: a step of a layer of this size is bound by the host (117 us with them, 145 with torch's products), and they cost the
+// device up to 25 % more in bf16 ([4096, 768] x [3072, 768] 22.7 us against 18.0) and, towards 2^28 multiply-adds, 30 % more in float32
+// (1024 x 512 x 512 61 us for the three against 55; 128 x 768 x 768 28 against 38).
+bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, int64_t n_in) {
+    if (tokens <= 0 || n_out <= 0 || n_in <= 0 || n_out * n_in > (int64_t)1 << 22) return false;
+    // the smallest float32 steps keep torch's product, whose bits a trace of the layer has
+    if (type == at::kFloat) return tokens <= ((int64_t)1 << 28) / (n_out * n_in) && tokens * n_out * n_in >= (int64_t)1 << 16;
+    return type == at::kBFloat16 && tokens <= ((int64_t)1 << 34) / (n_out * n_in) && n_out % 8 == 0 && n_in % 8 == 0;
 }
 
 // dense_linear(x [T, n_in] bf16, w [n_out, n_in] bf16, bias or None, status or None, own): x w^T + bias as bf16.  `own`: by the library's own
@@ -553,9 +558,9 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         Tensor wq, codes, beta, b = bias ? *bias : Tensor(), b16;
         const bool b_f32 = b.defined() && b.scalar_type() == at::kFloat && b.is_contiguous() && b.device() == w.device();
         Tensor x2;
-        if (x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() >= 1 && x.size(-1) == w.size(1) && w.numel() > 0 && (!b.defined() || (b_f32 && b.numel() == w.size(0))))
+        if (x.is_contiguous() && x.dim() >= 1 && x.size(-1) == w.size(1) && w.numel() > 0 && (!b.defined() || (b_f32 && b.numel() == w.size(0))))
             x2 = x.dim() == 2 ? x : x.view({-1, w.size(1)});
-        const bool own = x2.defined() && own_rows(x2) && own_training_products(x2.size(0), w.size(0), w.size(1));
+        const bool own = x2.defined() && own_rows(x2) && own_training_products(x.scalar_type(), x2.size(0), w.size(0), w.size(1));
         if (b.defined() && x.scalar_type() == at::kBFloat16 && !own) {
             if (b_f32) b16 = empty(b.sizes(), at::kBFloat16, w);
             else b = b.to(at::kBFloat16);
@@ -566,9 +571,10 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         if (own) {
             c10::SmallVector<int64_t, 6> y_shape(x.sizes().begin(), x.sizes().end());
             y_shape.back() = w.size(0);
-            y = empty(y_shape, at::kBFloat16, x);
-            check_rc(coset_e8_dense_linear(data(wq), (int)w.size(0), (int)w.size(1), data(x2), w.size(1), (int)x2.size(0), fdata(b), 1, data(y), w.size(0), nullptr, stream_of(x)),
-                     "coset_e8_dense_linear");
+            y = empty(y_shape, x.scalar_type(), x);
+            const int T = (int)x2.size(0), N = (int)w.size(0), K = (int)w.size(1);
+            check_rc(x.scalar_type() == at::kFloat ? coset_f32_linear(fdata(x2), fdata(wq), fdata(b), T, N, K, fdata(y), stream_of(x))
+                                                   : coset_e8_dense_linear(data(wq), N, K, data(x2), K, T, fdata(b), 1, data(y), N, nullptr, stream_of(x)), "the layer's product");
         } else {
             y = at::linear(x, wq, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
         }
@@ -599,22 +605,25 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         const Tensor g2 = grads[0].reshape({-1, w.size(0)});
         variable_list out(9);
         const int64_t T = g2.size(0), N = w.size(0), K = w.size(1);
-        const bool own = !at::GradMode::is_enabled() && own_training_products(T, N, K) && own_rows(g2);
+        const at::ScalarType type = g2.scalar_type();
+        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K) && own_rows(g2), f32 = type == at::kFloat;
         if (ctx->needs_input_grad(0)) {
             c10::SmallVector<int64_t, 6> x_shape(grads[0].sizes().begin(), grads[0].sizes().end());
             x_shape.back() = K;
-            if (own && own_rows(wq)) {
-                out[0] = empty(x_shape, at::kBFloat16, g2);
-                check_rc(coset_dense_input_grad(data(g2), data(wq), (int)T, (int)N, (int)K, data(out[0]), nullptr, stream_of(g2)), "coset_dense_input_grad");
+            if (own && own_rows(wq) && wq.scalar_type() == type) {
+                out[0] = empty(x_shape, type, g2);
+                check_rc(f32 ? coset_f32_input_grad(fdata(g2), fdata(wq), (int)T, (int)N, (int)K, fdata(out[0]), stream_of(g2))
+                             : coset_dense_input_grad(data(g2), data(wq), (int)T, (int)N, (int)K, data(out[0]), nullptr, stream_of(g2)), "the gradient of the input");
             } else out[0] = at::mm(g2, wq).view(x_shape);
         }
         const bool need_theta = ctx->needs_input_grad(2);
         if (ctx->needs_input_grad(1) || need_theta) {
             const Tensor x2 = x.reshape({-1, K});
             Tensor gw;
-            if (own && own_rows(x2) && x2.size(0) == T) {
-                gw = empty({N, K}, at::kBFloat16, g2);
-                check_rc(coset_dense_weight_grad(data(g2), data(x2), (int)T, (int)N, (int)K, data(gw), nullptr, stream_of(g2)), "coset_dense_weight_grad");
+            if (own && own_rows(x2) && x2.scalar_type() == type && x2.size(0) == T) {
+                gw = empty({N, K}, type, g2);
+                check_rc(f32 ? coset_f32_weight_grad(fdata(g2), fdata(x2), (int)T, (int)N, (int)K, fdata(gw), stream_of(g2))
+                             : coset_dense_weight_grad(data(g2), data(x2), (int)T, (int)N, (int)K, data(gw), nullptr, stream_of(g2)), "the gradient of the weight");
             } else gw = at::mm(g2.t(), x2);
             auto r = FakeQuant::backward_launch(gw, w, theta, beta, codes, range, bpt, q, clip, need_theta);
             out[1] = r.first;

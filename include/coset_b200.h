@@ -420,6 +420,14 @@ int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x
 int coset_dense_input_grad(const void* g_bf16, const void* w_bf16, int T, int n_out, int n_in, void* dx, int* status, void* stream);
 int coset_dense_weight_grad(const void* g_bf16, const void* x_bf16, int T, int n_out, int n_in, void* dw, int* status, void* stream);
 
+/* The three products of a training layer in float32 (full multiply-adds), contiguous rows of any length, for layers and batches so small that
+ * a library call is mostly overhead: y[T, n_out] = x W^T + bias (bias may be null), dx[T, n_in] = g W, dw[n_out, n_in] = g^T x.  One launch each,
+ * the same bits in every run.  Replaces F.linear and its backward, coset/core/layers.py:524-536.
+ */
+int coset_f32_linear(const float* x, const float* w, const float* bias, int T, int n_out, int n_in, float* y, void* stream);
+int coset_f32_input_grad(const float* g, const float* w, int T, int n_out, int n_in, float* dx, void* stream);
+int coset_f32_weight_grad(const float* g, const float* x, int T, int n_out, int n_in, float* dw, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -476,15 +476,34 @@ def test_bf16_products_of_a_training_step(tokens, n_out, n_in, bias):
     assert bool(((dw.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * size).all())
 
 
+@pytest.mark.parametrize("T,n_out,n_in", [(1, 1, 1), (3, 5, 7), (33, 65, 31), (32, 64, 128), (128, 96, 129), (70, 130, 1000), (257, 200, 64), (64, 1024, 2048)])
+def test_float32_products_of_a_training_step(T, n_out, n_in):
+    """Odd lengths and whole tiles, one to eight parts of K, against 64 bits and the library's error."""
+    from coset_b200 import _lib
+    L, st = _lib.lib(), _lib.stream()
+    x, w, b, g = (torch.randn(*s, device="cuda") for s in ((T, n_in), (n_out, n_in), (n_out,), (T, n_out)))
+    y, dx, dw = torch.empty(T, n_out, device="cuda"), torch.empty_like(x), torch.empty_like(w)
+    assert L.coset_f32_linear(_lib.ptr(x), _lib.ptr(w), _lib.ptr(b), T, n_out, n_in, _lib.ptr(y), st) == 0
+    assert L.coset_f32_input_grad(_lib.ptr(g), _lib.ptr(w), T, n_out, n_in, _lib.ptr(dx), st) == 0
+    assert L.coset_f32_weight_grad(_lib.ptr(g), _lib.ptr(x), T, n_out, n_in, _lib.ptr(dw), st) == 0
+    xd, wd, bd, gd = x.double(), w.double(), b.double(), g.double()
+    for got, want, size in ((y, xd @ wd.T + bd, xd.abs() @ wd.abs().T + bd.abs()), (dx, gd @ wd, gd.abs() @ wd.abs()), (dw, gd.T @ xd, gd.abs().T @ xd.abs())):
+        # chains of 128 roundings and at most 24 more additions, each within 2^-24 of the sum of the magnitudes
+        assert bool(((got.double() - want).abs() <= 152 * 2.0 ** -24 * size).all())
+    assert L.coset_f32_linear(_lib.ptr(x), _lib.ptr(w), None, T, n_out, n_in, _lib.ptr(dx) if T * n_in >= T * n_out else _lib.ptr(y), st) == 0
+    assert L.coset_f32_linear(_lib.ptr(x), None, None, T, n_out, n_in, _lib.ptr(y), st) < 0 and L.coset_f32_linear(_lib.ptr(x), _lib.ptr(w), None, T, n_out, 0, _lib.ptr(y), st) < 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("form", ["expanded", "strided", "offset", "three"])
-def test_bf16_products_with_awkward_tensors(form):
+def test_own_products_with_awkward_tensors(form, dtype):
     """Gradients and inputs that the own products cannot read, or read only as rows, give what plain ones give."""
     from coset_b200.core.e8 import create_e8_hnlq_linear
-    layer = create_e8_hnlq_linear(64, 32, device="cuda", tiling="row", init_method="zeros")
-    layer.load_weights(torch.randn(32, 64, device="cuda") * 20.0, torch.randn(32, device="cuda"))
-    x, g = torch.randn(24, 64, device="cuda").bfloat16(), torch.randn(24, 32, device="cuda").bfloat16()
+    layer = create_e8_hnlq_linear(64, 48, device="cuda", tiling="row", init_method="zeros")
+    layer.load_weights(torch.randn(48, 64, device="cuda") * 20.0, torch.randn(48, device="cuda"))
+    x, g = torch.randn(24, 64, device="cuda").to(dtype), torch.randn(24, 48, device="cuda").to(dtype)
     if form == "expanded":
-        g = g[:1].expand(24, 32)
+        g = g[:1].expand(24, 48)
 
     def step(x, g):
         layer.zero_grad()
@@ -494,11 +513,12 @@ def test_bf16_products_with_awkward_tensors(form):
         return [t.reshape(-1).float() for t in (y.detach(), x.grad, layer.weight.grad, layer.theta_beta.grad, layer.bias.grad)]
     want = step(x, g.contiguous())
     if form == "strided":
-        x, g = torch.cat([x, x], 1)[:, :64], torch.cat([g, g], 1)[:, :32]
+        x, g = torch.cat([x, x], 1)[:, :64], torch.cat([g, g], 1)[:, :48]
     elif form == "offset":
         x = torch.cat([x.new_zeros(1), x.reshape(-1)])[1:].view(24, 64)
-        g = torch.cat([g.new_zeros(1), g.reshape(-1)])[1:].view(24, 32)
+        g = torch.cat([g.new_zeros(1), g.reshape(-1)])[1:].view(24, 48)
     elif form == "three":
-        x, g = x.view(4, 6, 64), g.view(4, 6, 32)
-    for a, b in zip(step(x, g), want):  # sums of at most 64 products in another order, then bf16
-        assert torch.allclose(a, b, rtol=2.0 ** -7, atol=2.0 ** -7 * float(b.abs().max()))
+        x, g = x.view(4, 6, 64), g.view(4, 6, 48)
+    unit = 2.0 ** -7 if dtype == torch.bfloat16 else 64 * 2.0 ** -23  # sums of at most 64 products in another order, then the type's rounding
+    for a, b in zip(step(x, g), want):
+        assert torch.allclose(a, b, rtol=unit, atol=unit * float(b.abs().max()))
