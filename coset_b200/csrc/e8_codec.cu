@@ -613,6 +613,95 @@ k_decode_q4m2(const uint32_t* __restrict__ codes, const float* __restrict__ scal
     }
 }
 
+// Many blocks: the residual table in its compact form in shared memory, one CTA of 1024 threads per SM (see e8::compact_residues).
+//
+// What bounds the kernel above is the gathers, 27 cycles per warp for 32 lines of L1 and L2, the more so in bf16, whose rows are half as long.
+// A gather from shared memory costs the conflicts of 32 banks, both levels of a code share the arithmetic on 2-bit fields, and everything on
+// eight coordinates is done in pairs.  The table is loaded before grid_wait: it is there for good, and the kernel before still drains.
+// Rows requested ahead per thread: two float32 rows, next to each other across the CTA; four bf16 rows, far apart.  Measured, from the kernel above
+// (one scale per block): float32 400000 blocks 8.1 -> 6.2 us, 10^6 13.9 -> 9.8, 4 M 35.6 -> 28.4, 2^25 222 -> 217, but 200000 4.2 -> 4.4; bf16 10^6 6.9 -> 6.7 (one scale
+// for 96 blocks 7.7 -> 6.7, 2^25 160 -> 143), but 700000 4.8 -> 5.4.  Four float32 rows far apart took 267 us for 2^25, two bf16 rows 167.
+constexpr int kSharedThreads = 1024;
+template <int DT>
+constexpr int kSharedRows = DT == 0 ? 2 : 4;
+inline int64_t shared_decoder_from(int out_dtype) { return (out_dtype == COSET_DTYPE_F32 ? 2 : 6) * (int64_t)sm_count() * kSharedThreads; }
+constexpr int kSharedTableBytes = 65536 * 2;
+
+template <int MODE>
+__device__ __forceinline__ void scale_twice_pairs(const float (&v2)[8], float s, float (&out)[8]) {
+    const float a = fabsf(s);
+    if (MODE == COSET_SCALE_MUL_TILE && a > 1e-18f && a < 1e18f) {  // scale_twice, in pairs
+        const float s2 = __fmul_rn(s, 2.0f), r = __frcp_rn(s2);
+        const e8::F2 rr = e8::pair2(r, r), ss = e8::pair2(-s2, -s2);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const e8::F2 v = e8::pair2(v2[2 * i], v2[2 * i + 1]), q = e8::mul2(v, rr);
+            e8::split2(e8::fma2(e8::fma2(q, ss, v), rr, q), out[2 * i], out[2 * i + 1]);
+        }
+    } else {
+        e8::scale_twice<MODE>(v2, s, out);
+    }
+}
+
+template <int DT, int MODE, int SCALES>
+__global__ void __launch_bounds__(kSharedThreads, 1)
+k_decode_q4m2_shared(const uint32_t* __restrict__ codes, const float* __restrict__ scale, e8::TileDiv td, uint32_t skip, uint32_t n, const uint16_t* __restrict__ compact,
+                     const uint2* __restrict__ table, void* __restrict__ out) {
+    extern __shared__ __align__(16) uint16_t lut[];
+#pragma unroll
+    for (int k = 0; k < kSharedTableBytes / 16 / kSharedThreads; ++k)
+        reinterpret_cast<uint4*>(lut)[k * kSharedThreads + threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(compact) + k * kSharedThreads + threadIdx.x);
+    grid_wait();
+    grid_trigger();
+    constexpr int kRows = kSharedRows<DT>;
+    const uint32_t round = gridDim.x * kSharedThreads * kRows, stride = DT == 0 ? (uint32_t)kSharedThreads : gridDim.x * kSharedThreads;
+    const uint32_t first = blockIdx.x * kSharedThreads * (DT == 0 ? kRows : 1) + (uint32_t)behind_wait((int)threadIdx.x);
+    const float one = MODE == COSET_SCALE_DIV_SCALAR ? __ldg(behind_wait(scale)) : 1.0f;
+    uint32_t next[kRows];
+    float next_scale[kRows];
+    auto request = [&](uint32_t b, int j) {
+        next[j] = 0u;
+        next_scale[j] = one;
+        if (b < n) {
+            next[j] = __ldcs(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(codes) + (uint64_t)(b * 4u)));
+            if (SCALES == kBlockScale) next_scale[j] = __ldcs(reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(scale) + (uint64_t)(b * 4u)));
+            if (SCALES == kTileScale) next_scale[j] = __ldg(scale + (__umulhi(skip + b, td.mul) >> td.shr));
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) request(first + j * stride, j);
+    __syncthreads();
+    for (uint32_t base = first; base < n; base += round) {
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) {
+            const uint32_t b = base + j * stride;
+            const uint32_t code = next[j];
+            const float s = next_scale[j];
+            request(b + round, j);
+            if (b >= n) continue;
+            const uint32_t e = (uint32_t)lut[code & 0xffffu] | ((uint32_t)lut[code >> 16] << 16), r = e8::compact_residues(code);
+            float v2[8], xh[8];
+            if (e8::compact_marked(e) == 0u) {
+                // nibbles 4 m + s: coordinates 0, 2, 4, 6 and 1, 3, 5, 7 of level 0, and of level 1 in the upper half
+                const uint32_t even = ((e & 0x33333333u) << 2) | (r & 0x33333333u), odd = (e & 0xccccccccu) | ((r >> 2) & 0x33333333u);
+                auto levels = [](uint32_t t) { return t + 4u * (t >> 16); };  // bytes 0 and 1
+                const uint32_t t04 = levels(even & 0x0f0f0f0fu), t26 = levels((even >> 4) & 0x0f0f0f0fu);
+                const uint32_t t15 = levels(odd & 0x0f0f0f0fu), t37 = levels((odd >> 4) & 0x0f0f0f0fu);
+                const float off = -(12582912.0f + 5.0f * e8::kCompactBias), off7 = -(12582912.0f + 5.0f * e8::kCompactBias7);
+                const e8::F2 o = e8::pair2(off, off);
+                e8::split2(e8::add2(e8::pair2(e8::biased_byte_to_float<0>(t04), e8::biased_byte_to_float<0>(t15)), o), v2[0], v2[1]);
+                e8::split2(e8::add2(e8::pair2(e8::biased_byte_to_float<0>(t26), e8::biased_byte_to_float<0>(t37)), o), v2[2], v2[3]);
+                e8::split2(e8::add2(e8::pair2(e8::biased_byte_to_float<1>(t04), e8::biased_byte_to_float<1>(t15)), o), v2[4], v2[5]);
+                e8::split2(e8::add2(e8::pair2(e8::biased_byte_to_float<1>(t26), e8::biased_byte_to_float<1>(t37)), e8::pair2(off, off7)), v2[6], v2[7]);
+            } else {
+                e8::decode_q4m2_twice(code, table, v2);
+            }
+            scale_twice_pairs<MODE>(v2, s, xh);
+            e8::Row8<DT>::store(reinterpret_cast<uint8_t*>(out) + (uint64_t)(b * (DT == 0 ? 32u : 16u)), 0, xh);
+        }
+    }
+}
+
 // Residual table of the q=4 decoder, produced by the literal float32 decoder itself:
 // entry[w] = 2 * (G b - 4 Q(G b / 4)) + 7 for the 16-bit level word w, as 8 unsigned bytes.
 __global__ void k_build_table_q4(uint2* __restrict__ table, uint32_t* __restrict__ packed, uint16_t* __restrict__ compact, int* __restrict__ bad) {
@@ -823,6 +912,30 @@ const uint16_t* residual_table_q4_compact(cudaStream_t stream) {
 
 namespace {
 
+// A call in parts whose offsets fit 32 bits: fn(first block, blocks, scale of the first block, division of kTileScale, its place in its tile).
+template <int MODE, typename Fn>
+int in_parts(const float* scale, const e8::TileDiv& td, int64_t n, Fn fn) {
+    constexpr int64_t kMost = 1 << 26, kLongTile = 1 << 30;
+    const int64_t tile = MODE == COSET_SCALE_MUL_TILE ? td.divisor : 1;
+    for (int64_t at = 0; at < n;) {
+        int64_t count = n - at < kMost ? n - at : kMost, skip = at % tile;
+        const float* s = scale;
+        e8::TileDiv part = {};
+        if (MODE == COSET_SCALE_MUL_TILE) {
+            s += at / tile;
+            if (tile > kLongTile) {  // the part ends with its tile: the quotient of the empty division is 0
+                count = count < tile - skip ? count : tile - skip;
+                skip = 0;
+            } else if (tile > 1) {
+                part = e8::make_tile_div(tile, kLongTile + kMost);
+            }
+        }
+        if (int rc = fn(at, count, s, part, (uint32_t)skip)) return rc;
+        at += count;
+    }
+    return 0;
+}
+
 template <int DT, int MODE, bool SAT>
 int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_t n, uint32_t* codes, cudaStream_t st) {
     const int64_t resident = 4 * (int64_t)sm_count();
@@ -831,35 +944,30 @@ int launch_encode_q4m2(const void* x, const float* scale, e8::TileDiv td, int64_
         return launch_dependent("e8_encode", k_encode_q4m2_listed<DT, MODE, SAT, kAnyScale, 0>, (unsigned)(need < resident ? need : resident), kThreads, 0, st,
                                 x, scale, td, 0u, (uint32_t)n, codes);
     }
-    constexpr int64_t kMost = 1 << 26, kLongTile = 1 << 30;
-    const int64_t tile = MODE == COSET_SCALE_MUL_TILE ? td.divisor : 1;
-    for (int64_t at = 0; at < n;) {
-        int64_t count = n - at < kMost ? n - at : kMost;
-        const int64_t skip = at % tile;
-        const float* s = scale;
-        e8::TileDiv part = {};
-        if (MODE == COSET_SCALE_MUL_TILE) {
-            s += at / tile;
-            if (tile > kLongTile) count = count < tile - skip ? count : tile - skip;  // one tile: the quotient of the empty division is 0
-            else if (tile > 1) part = e8::make_tile_div(tile, kLongTile + kMost);
-        }
-        const uint32_t within = tile > kLongTile ? 0u : (uint32_t)skip;
+    return in_parts<MODE>(scale, td, n, [&](int64_t at, int64_t count, const float* s, e8::TileDiv part, uint32_t skip) {
         // Up to 32 blocks per thread of the resident CTAs, these alone, each with one pass over its list; beyond, three CTAs follow one another, so that
         // the lists of the first are worked off while others are in their loops (4.2 M blocks 47 us against 52, 13.7 M 124 against 120).
         const int64_t need = (count + kThreads - 1) / kThreads, cap = need <= 32 * resident ? resident : 3 * resident;
         const unsigned grid = (unsigned)(need < cap ? need : cap);
         const void* xs = (const uint8_t*)x + at * (DT == 0 ? 32 : 16);
-        int rc;
-        if (MODE != COSET_SCALE_MUL_TILE)
-            rc = launch_dependent("e8_encode", k_encode_q4m2_listed<DT, MODE, SAT, kAnyScale, kRowsUnderWay>, grid, kThreads, 0, st, xs, s, part, within, (uint32_t)count, codes + at);
-        else if (tile == 1)
-            rc = launch_dependent("e8_encode", k_encode_q4m2_listed<DT, COSET_SCALE_MUL_TILE, SAT, kBlockScale, kRowsUnderWay>, grid, kThreads, 0, st, xs, s, part, within, (uint32_t)count, codes + at);
-        else
-            rc = launch_dependent("e8_encode", k_encode_q4m2_listed<DT, COSET_SCALE_MUL_TILE, SAT, kTileScale, kRowsUnderWay>, grid, kThreads, 0, st, xs, s, part, within, (uint32_t)count, codes + at);
-        if (rc) return rc;
-        at += count;
-    }
-    return 0;
+        auto go = [&](auto kernel) { return launch_dependent("e8_encode", kernel, grid, kThreads, 0, st, xs, s, part, skip, (uint32_t)count, codes + at); };
+        if constexpr (MODE != COSET_SCALE_MUL_TILE) return go(k_encode_q4m2_listed<DT, MODE, SAT, kAnyScale, kRowsUnderWay>);
+        else return td.divisor == 1 ? go(k_encode_q4m2_listed<DT, MODE, SAT, kBlockScale, kRowsUnderWay>) : go(k_encode_q4m2_listed<DT, MODE, SAT, kTileScale, kRowsUnderWay>);
+    });
+}
+
+// The decoder with the table in shared memory.
+template <int DT, int MODE>
+int launch_decode_shared(const uint32_t* codes, const float* scale, e8::TileDiv td, int64_t n, const uint16_t* compact, const uint2* table, void* out, cudaStream_t st) {
+    return in_parts<MODE>(scale, td, n, [&](int64_t at, int64_t count, const float* s, e8::TileDiv part, uint32_t skip) {
+        auto go = [&](auto kernel) {
+            if (int e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedTableBytes), "cudaFuncSetAttribute")) return e;
+            return launch_dependent("e8_decode", kernel, (unsigned)sm_count(), kSharedThreads, kSharedTableBytes, st, codes + at, s, part, skip, (uint32_t)count, compact, table,
+                                    (void*)((uint8_t*)out + at * (DT == 0 ? 32 : 16)));
+        };
+        if constexpr (MODE != COSET_SCALE_MUL_TILE) return go(k_decode_q4m2_shared<DT, MODE, kAnyScale>);
+        else return td.divisor == 1 ? go(k_decode_q4m2_shared<DT, MODE, kBlockScale>) : go(k_decode_q4m2_shared<DT, MODE, kTileScale>);
+    });
 }
 
 }  // namespace
@@ -938,6 +1046,11 @@ int coset_e8_decode(const void* codes, const float* scale, int scale_mode, int64
         const uint32_t* packed = residual_table_q4_packed(st);
         if (!table || !packed) return COSET_E_STATE;
         int rc = 0;
+        if (n_blocks >= shared_decoder_from(out_dtype)) {
+            const uint16_t* compact = residual_table_q4_compact(st);
+            DISPATCH_DT(out_dtype, DT, DISPATCH_MODE(scale_mode, (rc = launch_decode_shared<DT, MODE>((const uint32_t*)codes, scale, td, n_blocks, compact, table, out, st))))
+            return rc;
+        }
         unsigned grid2 = (unsigned)((n_blocks + kThreads * kDecPerThread - 1) / (kThreads * kDecPerThread));
         if (out_dtype == COSET_DTYPE_F32) {
             DISPATCH_MODE(scale_mode, (rc = launch_dependent("e8_decode", k_decode_q4m2<0, MODE, uint32_t>, grid2, kThreads, 0, st, (const uint32_t*)codes, scale, td, n_blocks, packed, out)))

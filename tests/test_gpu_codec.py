@@ -483,3 +483,24 @@ def test_chained_calls_read_what_the_call_before_wrote(n):
 
     for a, b in zip(passes(torch.cuda.synchronize), passes(lambda: None)):
         assert all(torch.equal(s, t) for s, t in zip(a, b))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode,tile", [(0, 1), (1, 1), (2, 1), (2, 7), (2, 1 << 22)])
+def test_both_decoders_agree(dtype, mode, tile):
+    """The decoder with the table in shared memory, over every kind of code and scale, against the one that small calls use."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_decode_packed
+    n = 148 * 1024 * 6 + 1237
+    codes = torch.randint(-2**31, 2**31 - 1, (n,), device="cuda", dtype=torch.int32)
+    codes[::3] &= 0xffff  # top level zero
+    scale = None if mode == 0 else torch.rand((n + tile - 1) // tile if mode == 2 else 1, device="cuda") * 3 + 0.01
+    if mode == 2 and scale.numel() > 64:
+        scale[:4] = torch.tensor([1e-30, 1e30, -2.0, float("inf")], device="cuda")
+    whole = e8_decode_packed(codes, scale=scale, scale_mode=mode, blocks_per_tile=tile, dtype=dtype)
+    piece = 7 * 14000  # whole tiles, few enough blocks for the other kernel
+    for at in range(0, n, piece):
+        part = codes[at:at + piece].contiguous()
+        s = scale if mode < 2 or tile > piece else scale[at // tile:(at + part.numel() + tile - 1) // tile].contiguous()
+        got = e8_decode_packed(part, scale=s, scale_mode=mode, blocks_per_tile=tile, dtype=dtype)
+        assert torch.equal(got.view(torch.int16), whole[at:at + piece].contiguous().view(torch.int16)), at
