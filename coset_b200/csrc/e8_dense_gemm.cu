@@ -17,7 +17,7 @@
 // launched as a programmatic dependent, which hides about 2 us of that behind the kernel before it.
 // Two CTAs fit an SM (ten warps, at most 112 KB of stages) where there are more tiles than SMs.
 // Measured, 4096 x 4096 with a bias, torch's product and its bias cast against this kernel (graph replays, three weights in turn): 64 tokens 8.9 + 2.9
-// against 8.8 us, 256 tokens 11.1 + 2.9 against 12.6, 1024 tokens 25.2 + 2.9 against 25.5; a call of the layer with 256 tokens 20.7 -> 13.3 us, for
+// against 8.8 us, 256 tokens 11.1 + 2.9 against 12.6, 1024 tokens 25.2 + 2.9 against 25.5; a call of the layer with 256 tokens 20.7 -> 14.5 us, for
 // the host was what bounded it.  The products of a training step of a [3072, 768] layer with 4096 tokens: 22.7 + 16.3 + 15.1 us against 18.0 + 15.3 + 13.8 for
 // torch's, but 15 us of host time instead of 42, and the host bounds the step.
 #include <cuda.h>

@@ -504,3 +504,20 @@ def test_both_decoders_agree(dtype, mode, tile):
         s = scale if mode < 2 or tile > piece else scale[at // tile:(at + part.numel() + tile - 1) // tile].contiguous()
         got = e8_decode_packed(part, scale=s, scale_mode=mode, blocks_per_tile=tile, dtype=dtype)
         assert torch.equal(got.view(torch.int16), whole[at:at + piece].contiguous().view(torch.int16)), at
+
+
+@pytest.mark.parametrize("tile", [1, 96, (1 << 30) + 8])
+def test_calls_beyond_the_offsets_of_one_launch(tile):
+    """2^26 blocks and a few more are two launches: the codes and values of the second are those of a call of its own."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    n, cut = (1 << 26) + 777, (1 << 26) - (1 << 26) % 96
+    x = torch.empty(n, 8, device="cuda", dtype=torch.bfloat16).normal_(0.0, 0.02)
+    scale = torch.full(((n + tile - 1) // tile,), 25.0, device="cuda") * (0.8 + 0.4 * torch.rand((n + tile - 1) // tile, device="cuda"))
+    kw = dict(scale=scale, scale_mode=_lib.SCALE_MUL_TILE, blocks_per_tile=tile)
+    codes = e8_encode_packed(x, **kw)
+    back = e8_decode_packed(codes, dtype=torch.bfloat16, **kw)
+    for lo, hi in ((0, 960), (cut, n)):
+        part = dict(kw, scale=scale if tile > n else scale[lo // tile:(hi + tile - 1) // tile].contiguous())
+        assert torch.equal(e8_encode_packed(x[lo:hi].contiguous(), **part), codes[lo:hi])
+        assert torch.equal(e8_decode_packed(codes[lo:hi].contiguous(), dtype=torch.bfloat16, **part), back[lo:hi])
