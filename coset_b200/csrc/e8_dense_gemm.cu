@@ -36,7 +36,8 @@ constexpr int kRows = 128;           // weight rows of one CTA
 constexpr int kMaxStages = 8;
 constexpr int kEpilogueWarps = 8, kTmaWarp = 8, kMmaWarp = 9;
 constexpr int kThreads = 10 * 32;
-constexpr int kSmemBudget = 226 * 1024;  // 227 KB less the alignment
+constexpr int kAlignment = 1024;         // of the stages, which the base of the shared memory need not have
+constexpr int kSmemBudget = 227 * 1024 - kAlignment;
 constexpr int kSmemOfTwo = 112 * 1024;   // two CTAs on an SM (228 KB, 1 KB of which each CTA takes)
 constexpr int kBarrierBytes = 16 * kMaxStages + 16;
 constexpr int kScratchRow = 40;       // 32 features and a pad, in values
@@ -305,9 +306,10 @@ Plan make_plan(int N, int K, int T, int unit) {  // unit: tokens come in multipl
 
 template <int kSub, bool W_MN, bool X_MN>
 int launch_linear(const CUtensorMap& x_map, const CUtensorMap& w_map, const Shape& s, cudaStream_t st) {
-    const int smem = 1024 /* alignment */ + s.plan.stages * stage_bytes(s.plan.tokens, kSub) + kBarrierBytes + sums_bytes(s.plan.tokens, s.plan.split);
+    const int smem = kAlignment + s.plan.stages * stage_bytes(s.plan.tokens, kSub) + kBarrierBytes + sums_bytes(s.plan.tokens, s.plan.split);
     const auto kernel = k_linear_pair<kSub, W_MN, X_MN>;
-    if (int e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
+    // The bound belongs to the kernel, not to the call: what any plan may ask for, so that no thread lowers it between another's two calls.
+    if (int e = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlignment + kSmemBudget), "cudaFuncSetAttribute")) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((s.N + 2 * kRows - 1) / (2 * kRows) * 2 * s.plan.split), (unsigned)((s.T + s.plan.tokens - 1) / s.plan.tokens));
     cfg.blockDim = dim3(kThreads);

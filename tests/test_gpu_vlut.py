@@ -731,3 +731,31 @@ def test_product_with_the_kept_dense_weight_is_torchs_for_who_looks_at_it(how):
         with Seen() as seen:
             layer(x)
         assert any("mm" in c or "linear" in c for c in seen.calls)
+
+
+def test_products_of_different_plans_from_several_threads():
+    """The plans of these calls ask for different amounts of shared memory of the same kernels: no thread's call is refused for another's, and each has
+    the bits it has alone."""
+    import threading
+    from coset_b200 import _lib
+    calls = []
+    for T, n_out, n_in in ((32, 64, 64), (64, 4096, 4096), (256, 512, 256), (512, 1024, 1024)):
+        x, w = torch.randn(T, n_in, device="cuda").bfloat16(), torch.randn(n_out, n_in, device="cuda").bfloat16()
+        calls.append((x, w, _lib.native().dense_linear(x, w, None, None, True)))
+    torch.cuda.synchronize()
+    start, failures = threading.Barrier(len(calls)), []
+
+    def work(x, w, want):
+        try:
+            start.wait()
+            for _ in range(1500):
+                got = _lib.native().dense_linear(x, w, None, None, True)
+            assert torch.equal(got, want)
+        except Exception as e:  # noqa: BLE001 - reported by the test's own thread
+            failures.append(repr(e))
+    threads = [threading.Thread(target=work, args=c) for c in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
