@@ -449,6 +449,14 @@ bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, i
     if (type == at::kFloat) return tokens <= ((int64_t)1 << 28) / (n_out * n_in) && tokens * n_out * n_in >= (int64_t)1 << 16;
     return type == at::kBFloat16 && tokens <= ((int64_t)1 << 34) / (n_out * n_in) && n_out % 8 == 0 && n_in % 8 == 0;
 }
+// The rows of a layer's input where its product is the library's own, undefined where it is torch's (which refuses what does not fit together).
+Tensor own_layer_rows(const Tensor& x, const Tensor& w, const Tensor& bias) {
+    const int64_t n_out = w.size(0), n_in = w.size(1);
+    if (!x.is_contiguous() || x.dim() < 1 || x.size(-1) != n_in || w.numel() == 0 || x.device() != w.device()) return Tensor();
+    if (bias.defined() && !(bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.device() == w.device() && bias.numel() == n_out)) return Tensor();
+    const Tensor x2 = x.dim() == 2 ? x : x.view({-1, n_in});
+    return own_rows(x2) && own_training_products(x.scalar_type(), x2.size(0), n_out, n_in) ? x2 : Tensor();
+}
 
 // dense_linear(x [T, n_in] bf16, w [n_out, n_in] bf16, bias or None, status or None, own): x w^T + bias as bf16.  `own`: by the library's own
 // kernel, which adds the float32 bias to the float32 sums; else, and for whoever looks at the torch call (autograd, autocast, transforms,
@@ -556,13 +564,10 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
                           const Tensor& beta_min, const Tensor& beta_range, int64_t bpt, int64_t q, double clip) {
         const Tensor w = contiguous(weight);
         Tensor wq, codes, beta, b = bias ? *bias : Tensor(), b16;
-        const bool b_f32 = b.defined() && b.scalar_type() == at::kFloat && b.is_contiguous() && b.device() == w.device();
-        Tensor x2;
-        if (x.is_contiguous() && x.dim() >= 1 && x.size(-1) == w.size(1) && w.numel() > 0 && (!b.defined() || (b_f32 && b.numel() == w.size(0))))
-            x2 = x.dim() == 2 ? x : x.view({-1, w.size(1)});
-        const bool own = x2.defined() && own_rows(x2) && own_training_products(x.scalar_type(), x2.size(0), w.size(0), w.size(1));
+        const Tensor x2 = own_layer_rows(x, w, b);
+        const bool own = x2.defined();
         if (b.defined() && x.scalar_type() == at::kBFloat16 && !own) {
-            if (b_f32) b16 = empty(b.sizes(), at::kBFloat16, w);
+            if (b.scalar_type() == at::kFloat && b.is_contiguous() && b.device() == w.device()) b16 = empty(b.sizes(), at::kBFloat16, w);
             else b = b.to(at::kBFloat16);
         }
         FakeQuant::launch(w, as_f32(theta), beta_min, beta_range, bpt, q, clip, x.scalar_type(), wq, codes, beta, b, b16);
@@ -606,11 +611,11 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         variable_list out(9);
         const int64_t T = g2.size(0), N = w.size(0), K = w.size(1);
         const at::ScalarType type = g2.scalar_type();
-        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K) && own_rows(g2), f32 = type == at::kFloat;
+        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K) && own_rows(g2) && g2.device() == w.device(), f32 = type == at::kFloat;
         if (ctx->needs_input_grad(0)) {
             c10::SmallVector<int64_t, 6> x_shape(grads[0].sizes().begin(), grads[0].sizes().end());
             x_shape.back() = K;
-            if (own && own_rows(wq) && wq.scalar_type() == type) {
+            if (own && own_rows(wq) && wq.scalar_type() == type && wq.device() == w.device()) {
                 out[0] = empty(x_shape, type, g2);
                 check_rc(f32 ? coset_f32_input_grad(fdata(g2), fdata(wq), (int)T, (int)N, (int)K, fdata(out[0]), stream_of(g2))
                              : coset_dense_input_grad(data(g2), data(wq), (int)T, (int)N, (int)K, data(out[0]), nullptr, stream_of(g2)), "the gradient of the input");
@@ -620,7 +625,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         if (ctx->needs_input_grad(1) || need_theta) {
             const Tensor x2 = x.reshape({-1, K});
             Tensor gw;
-            if (own && own_rows(x2) && x2.scalar_type() == type && x2.size(0) == T) {
+            if (own && own_rows(x2) && x2.scalar_type() == type && x2.size(0) == T && x2.device() == w.device()) {
                 gw = empty({N, K}, type, g2);
                 check_rc(f32 ? coset_f32_weight_grad(fdata(g2), fdata(x2), (int)T, (int)N, (int)K, fdata(gw), stream_of(g2))
                              : coset_dense_weight_grad(data(g2), data(x2), (int)T, (int)N, (int)K, data(gw), nullptr, stream_of(g2)), "the gradient of the weight");
@@ -690,11 +695,21 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// own_product(x, weight, bias or None) -> whether qat_linear multiplies x by the library's own kernel; launches nothing
+PyObject* own_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 3);
+    const Tensor &x = tensor_arg(a[0], "x"), &w = tensor_arg(a[1], "weight");
+    at::AutoGradMode no_grad(false);  // as inside the node
+    return PyBool_FromLong(own_layer_rows(x, w, optional_arg(a[2], "bias")).defined());
+    END_HANDLE_TH_ERRORS
+}
+
 #define COSET_METHOD(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     COSET_METHOD(encode_packed), COSET_METHOD(decode_packed), COSET_METHOD(encode_digits), COSET_METHOD(decode_digits), COSET_METHOD(quantize),
     COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(vlut_layout), COSET_METHOD(vlut_product), COSET_METHOD(vlut_product_checked),
-    COSET_METHOD(decode_gemm), COSET_METHOD(dense_linear), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), {nullptr, nullptr, 0, nullptr}};
+    COSET_METHOD(decode_gemm), COSET_METHOD(dense_linear), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), COSET_METHOD(own_product), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_coset_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -522,3 +522,17 @@ def test_own_products_with_awkward_tensors(form, dtype):
     unit = 2.0 ** -7 if dtype == torch.bfloat16 else 64 * 2.0 ** -23  # sums of at most 64 products in another order, then the type's rounding
     for a, b in zip(step(x, g), want):
         assert torch.allclose(a, b, rtol=unit, atol=unit * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_own_products_are_for_tensors_of_one_device(dtype):
+    """A tensor elsewhere is torch's to refuse; the own kernels would read another device's memory."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    own = _lib.native().own_product
+    x, w, b = torch.randn(64, 128, device="cuda").to(dtype), torch.randn(96, 128, device="cuda"), torch.randn(96, device="cuda")
+    assert own(x, w, b) and own(x, w, None) and own(x.view(8, 8, 128), w, b)
+    assert not own(x, w.cpu(), None) and not own(x.cpu(), w, None) and not own(x, w, b.cpu())
+    if torch.cuda.device_count() > 1:
+        with pytest.raises(RuntimeError, match="device"):
+            create_e8_hnlq_linear(128, 96, device="cuda:0")(x.to("cuda:1"))
