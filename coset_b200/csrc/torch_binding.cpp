@@ -453,7 +453,7 @@ bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, i
 Tensor own_layer_rows(const Tensor& x, const Tensor& w, const Tensor& bias) {
     const int64_t n_out = w.size(0), n_in = w.size(1);
     if (!x.is_contiguous() || x.dim() < 1 || x.size(-1) != n_in || w.numel() == 0 || x.device() != w.device()) return Tensor();
-    if (bias.defined() && !(bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.device() == w.device() && bias.numel() == n_out)) return Tensor();
+    if (bias.defined() && !(bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.device() == w.device() && bias.dim() == 1 && bias.numel() == n_out)) return Tensor();
     const Tensor x2 = x.dim() == 2 ? x : x.view({-1, n_in});
     return own_rows(x2) && own_training_products(x.scalar_type(), x2.size(0), n_out, n_in) ? x2 : Tensor();
 }

@@ -536,3 +536,22 @@ def test_own_products_are_for_tensors_of_one_device(dtype):
     if torch.cuda.device_count() > 1:
         with pytest.raises(RuntimeError, match="device"):
             create_e8_hnlq_linear(128, 96, device="cuda:0")(x.to("cuda:1"))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_bias_that_is_no_row_is_torchs(dtype):
+    """A bias of another shape is broadcast, or refused, by torch's product; the own one would add it per feature."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(128, 96, device="cuda")
+    b = torch.randn(96, device="cuda")
+    x = torch.randn(96, 128, device="cuda").to(dtype)
+    without = create_e8_hnlq_linear(128, 96, device="cuda", bias=False)
+    without.load_state_dict({k: v for k, v in layer.state_dict().items() if k != "bias"})
+    unit = 2.0 ** -7 if dtype == torch.bfloat16 else 128 * 2.0 ** -23  # one more rounding of the result; sums of 128 products in another order
+    for shape in ((1, 96), (96, 1)):
+        layer.bias = torch.nn.Parameter(b.view(shape))
+        with torch.no_grad():
+            want = without(x).float() + b.to(dtype).float().view(shape)  # 96 tokens: a column is a value per token
+            assert torch.allclose(layer(x).float(), want, rtol=unit, atol=unit * float(want.abs().max()))
+    with pytest.raises(RuntimeError), torch.no_grad():
+        layer(x[:64])
