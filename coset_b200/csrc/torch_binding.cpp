@@ -440,14 +440,21 @@ bool own_rows(const Tensor& t) {
     return t.dim() == 2 && (f32 || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0)) && t.is_contiguous() &&
            t.size(0) > 0 && t.size(0) <= INT32_MAX && t.size(1) > 0 && plain(t) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
 }
-// Whether they should: a step of a layer of this size is bound by the host (117 us with them, 145 with torch's products), and they cost the
-// device up to 25 % more in bf16 ([4096, 768] x [3072, 768] 22.7 us against 18.0) and, towards 2^28 multiply-adds, 30 % more in float32
-// (1024 x 512 x 512 61 us for the three against 55; 128 x 768 x 768 28 against 38).
+// Whether they should multiply for a training step: where the host bounds it (110 us with them, 141 with torch's products) and the device, which they cost
+// more, does not.  Steps of a layer on this box, own / torch, us:
+//   bf16   the products take up to 40 % longer, most where rows are wide, and those of a wide input are read or written three times, of a wide
+//          output twice: T (n_out + 2 n_in) of 34 M values [8192 x 4096 x 64] 110 / 146, [8192 x 2048 x 1024] 126 / 141; 36 M [4096 x 8192 x 256]
+//          120 / 140; 42 M [8192 x 4096 x 512] 142 / 139; 50 M [16384 x 2048 x 512] 150 / 143; 68 M [4096 x 256 x 8192] 180 / 165; 101 M [8192 x 64 x 6144] 174 / 151.
+//   float32 up to 61 us of products at 2^28 multiply-adds ([1024 x 512 x 512]; 54 with torch's); tiles count whole ([4096 x 10 x 2048] 131 / 141).
+// The weight's gradient has few tiles in a narrow layer, and a cluster of eight CTAs at most sums over all tokens of one: bf16 [32768 x 64 x 64] 111 / 142 but
+// [262144 x 64 x 64] 442 / 180; float32 [16384 x 16 x 64] 109 / 143, [65536 x 64 x 64] 314 / 255, [2^20 x 8 x 8] 6195 / 993.
 bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, int64_t n_in) {
-    if (tokens <= 0 || n_out <= 0 || n_in <= 0 || n_out * n_in > (int64_t)1 << 22) return false;
-    // the smallest float32 steps keep torch's product, whose bits a trace of the layer has
-    if (type == at::kFloat) return tokens <= ((int64_t)1 << 28) / (n_out * n_in) && tokens * n_out * n_in >= (int64_t)1 << 16;
-    return type == at::kBFloat16 && tokens <= ((int64_t)1 << 34) / (n_out * n_in) && n_out % 8 == 0 && n_in % 8 == 0;
+    if (tokens <= 0 || tokens > 1 << 15 || n_out <= 0 || n_in <= 0 || n_out > ((int64_t)1 << 22) / n_in) return false;
+    const auto whole = [](int64_t v, int64_t tile) { return (v + tile - 1) / tile * tile; };
+    const int64_t products = tokens * n_out * n_in;
+    if (type == at::kFloat)  // the smallest steps keep torch's product, whose bits a trace of the layer has
+        return tokens <= 1 << 14 && products >= 1 << 16 && products <= 1 << 28 && whole(tokens, 32) * whole(n_out, 64) * whole(n_in, 64) <= 1 << 29;
+    return type == at::kBFloat16 && n_out % 8 == 0 && n_in % 8 == 0 && products <= (int64_t)1 << 34 && tokens * (n_out + 2 * n_in) <= 9 << 22;
 }
 // The rows of a layer's input where its product is the library's own, undefined where it is torch's (which refuses what does not fit together).
 Tensor own_layer_rows(const Tensor& x, const Tensor& w, const Tensor& bias) {
@@ -695,6 +702,14 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// own_product_sizes(dtype_code, tokens, n_out, n_in) -> whether a training step of these sizes is multiplied by the library's own kernels
+PyObject* own_product_sizes(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    nargs_are(n, 4);
+    return PyBool_FromLong(own_training_products(scalar_type((int)int_arg(a[0])), int_arg(a[1]), int_arg(a[2]), int_arg(a[3])));
+    END_HANDLE_TH_ERRORS
+}
+
 // own_product(x, weight, bias or None) -> whether qat_linear multiplies x by the library's own kernel; launches nothing
 PyObject* own_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -709,7 +724,7 @@ PyObject* own_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef kMethods[] = {
     COSET_METHOD(encode_packed), COSET_METHOD(decode_packed), COSET_METHOD(encode_digits), COSET_METHOD(decode_digits), COSET_METHOD(quantize),
     COSET_METHOD(grad_encode), COSET_METHOD(decode_mean), COSET_METHOD(vlut_linear), COSET_METHOD(vlut_layout), COSET_METHOD(vlut_product), COSET_METHOD(vlut_product_checked),
-    COSET_METHOD(decode_gemm), COSET_METHOD(dense_linear), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), COSET_METHOD(own_product), {nullptr, nullptr, 0, nullptr}};
+    COSET_METHOD(decode_gemm), COSET_METHOD(dense_linear), COSET_METHOD(layer_fake_quant), COSET_METHOD(qat_linear), COSET_METHOD(own_product), COSET_METHOD(own_product_sizes), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_coset_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -555,3 +555,16 @@ def test_bias_that_is_no_row_is_torchs(dtype):
             assert torch.allclose(layer(x).float(), want, rtol=unit, atol=unit * float(want.abs().max()))
     with pytest.raises(RuntimeError), torch.no_grad():
         layer(x[:64])
+
+
+@pytest.mark.parametrize("dtype,tokens", [(torch.float32, 65535 * 32 + 1), (torch.bfloat16, 65535 * 256 + 1)])
+def test_training_step_of_more_tokens_than_the_own_products_take(dtype, tokens):
+    """One tile of tokens more than a grid of the own kernels holds: torch's products, as for any long and narrow step."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(8, 8, device="cuda", tiling="row", init_method="zeros", bias=False)
+    layer.load_weights(torch.randn(8, 8, device="cuda") * 20.0)
+    x = torch.randn(tokens, 8, device="cuda").to(dtype).requires_grad_()
+    y = layer(x)
+    y.backward(x.detach())
+    wq = layer._quantize_weights(dtype).detach()
+    assert torch.equal(y, torch.nn.functional.linear(x, wq)) and torch.equal(x.grad, torch.mm(x.detach(), wq)) and layer.weight.grad is not None

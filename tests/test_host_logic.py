@@ -151,3 +151,25 @@ def test_torch_module_is_built_again_for_another_torch(monkeypatch, tmp_path):
     assert built == [False]
     build.build()
     assert built == [False]
+
+
+def test_sizes_of_the_training_layers_own_products():
+    """What the rule takes fits the kernels' grids, which refuse more than 65535 tiles of tokens; long and narrow steps, whose weight gradient
+    would run on a few CTAs, and wide ones, which the device bounds, stay with torch."""
+    from coset_b200 import _lib
+    own = _lib.native().own_product_sizes
+    f32, bf16 = _lib.DTYPE_F32, _lib.DTYPE_BF16
+    assert own(f32, 128, 768, 768) and own(f32, 16384, 16, 64) and own(f32, 1024, 512, 512) and own(f32, 8192, 10, 768)
+    assert own(bf16, 4096, 3072, 768) and own(bf16, 8192, 4096, 64) and own(bf16, 32768, 64, 64) and own(bf16, 1, 8, 8)
+    for tokens in (2097121, 1 << 22):  # 65536 tiles of 32 tokens and more, within 2^28 multiply-adds
+        assert not own(f32, tokens, 8, 8)
+    for tokens in (65535 * 256 + 1, 1 << 28):
+        assert not own(bf16, tokens, 8, 8)
+    for tokens, n_out, n_in in ((262144, 16, 64), (65536, 64, 64), (8192, 10, 3200), (0, 64, 64), (2048, 512, 512), (8, 32, 64), (64, 1 << 11, (1 << 11) + 8)):
+        assert not own(f32, tokens, n_out, n_in)
+    for tokens, n_out, n_in in ((262144, 64, 64), (8192, 64, 6144), (4096, 256, 8192), (64, 1 << 11, (1 << 11) + 8), (64, 60, 64), (64, 64, 60), (8192, 2048, 2048)):
+        assert not own(bf16, tokens, n_out, n_in)
+    assert not own(f32, 1 << 40, 8, 8) and not own(bf16, 64, 1 << 40, 1 << 40)  # no overflow on the way
+    for tokens in range(1, 1 << 25, 99991):
+        assert not own(f32, tokens, 8, 8) or tokens <= 65535 * 32
+        assert not own(bf16, tokens, 8, 8) or tokens <= 65535 * 32
