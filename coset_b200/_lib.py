@@ -66,6 +66,7 @@ SIGNATURES = {
     "coset_e8_decode_gemm_scratch_bytes": [_i32, _i32],
     "coset_e8_decode_gemm": [_vp, _vp, _i64, _i32, _i32, _vp, _i64, _i32, _vp, _vp, _i32, _i64, _f32, _vp, _i64, _vp, _vp],
     "coset_e8_dense_linear": [_vp, _i32, _i32, _vp, _i64, _i32, _vp, _i32, _vp, _i64, _vp, _vp],
+    "coset_e8_dense_linear_late": [_vp, _i32, _i32, _vp, _i32, _vp, _i32, _i32, _i32, _vp, _vp],
     "coset_dense_input_grad": [_vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp],
     "coset_dense_weight_grad": [_vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp],
     "coset_f32_linear": [_vp, _vp, _vp, _i32, _i32, _i32, _vp, _vp],

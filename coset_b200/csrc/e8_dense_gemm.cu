@@ -59,15 +59,17 @@ struct Shape {
     int64_t ldy;
     int vector_rows;  // rows of y are made of 16-byte chunks
     int* status;
+    int late;         // the pair of each cluster that takes its first wait for run out, -1: none (see coset_e8_dense_linear_late)
 };
 
 // what a pair receives of the others' sums: apart from the stages, which a slower pair may still be using when a faster one sends
 __host__ __device__ constexpr int sums_bytes(int tokens, int split) { return (split - 1) * (tokens / split) * kRows * 4; }
 __host__ __device__ constexpr int stage_bytes(int tokens, int sub) { return sub * (kRows + tokens / 2) * BK * 2; }
 
-// Columns (tokens) of this CTA's accumulator that other pairs own, W at a time, into their reduction buffers [slot][token][row].
+// Columns (tokens) of this CTA's accumulator that other pairs own, W at a time, into their reduction buffers [slot][token][row]; where a wait gave
+// up no numbers, so that the sums of no pair are taken for whole.
 template <int W>
-__device__ __forceinline__ void send_columns(const Shape& s, uint32_t tmem, uint32_t base, int pair, int half, int row, int group) {
+__device__ __forceinline__ void send_columns(const Shape& s, bool ok, uint32_t tmem, uint32_t base, int pair, int half, int row, int group) {
     const int own = s.plan.tokens / s.plan.split;
     for (int c = group * W; c < s.plan.tokens; c += (kEpilogueWarps / 4) * W) {
         const int to = c / own;  // W divides own
@@ -77,7 +79,7 @@ __device__ __forceinline__ void send_columns(const Shape& s, uint32_t tmem, uint
         const int slot = pair < to ? pair : pair - 1;
         const uint32_t dst = peer_smem(base, (uint32_t)(2 * to + half)) + (uint32_t)(((slot * own + c - to * own) * kRows + row) * 4);
 #pragma unroll
-        for (int j = 0; j < W; ++j) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * kRows * 4)), "r"(r[j]) : "memory");
+        for (int j = 0; j < W; ++j) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * kRows * 4)), "r"(ok ? r[j] : 0x7fffffffu) : "memory");
     }
 }
 // The columns this pair owns: summed with what the others sent, plus bias, rounded and stored.  A lane holds one feature and W tokens;
@@ -212,7 +214,7 @@ k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
         int stage = 0;
         uint32_t phase = 0;
         for (int k = first; k < last; k += kSub) {
-            if (!mbar_wait_warp(full_base + 8 * stage, phase)) { ok = false; break; }
+            if (pair == s.late || !mbar_wait_warp(full_base + 8 * stage, phase)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (elect_one()) {
                 const uint32_t a_lo = w_lo + (uint32_t)(stage * (bytes >> 4)), b_lo = x_lo + (uint32_t)(stage * (bytes >> 4)) + (x_at >> 4);
@@ -241,8 +243,8 @@ k_linear_pair(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
     const int own = s.plan.tokens / s.plan.split;
     if (s.plan.split > 1) {
         if (warp < kEpilogueWarps) {
-            if (own >= 64) send_columns<16>(s, lanes, bar_base + kBarrierBytes, pair, half, row, group);
-            else send_columns<8>(s, lanes, bar_base + kBarrierBytes, pair, half, row, group);
+            if (own >= 64) send_columns<16>(s, ok, lanes, bar_base + kBarrierBytes, pair, half, row, group);
+            else send_columns<8>(s, ok, lanes, bar_base + kBarrierBytes, pair, half, row, group);
         }
         cluster_sync();  // ... and the sums have arrived
     }
@@ -328,7 +330,7 @@ int launch_linear(const CUtensorMap& x_map, const CUtensorMap& w_map, const Shap
 
 template <bool W_MN, bool X_MN>
 int dense_product(const void* w, int64_t ldw, const void* x, int64_t ldx, int N, int T, int K, const float* bias, int round_bias, void* y, int64_t ldy,
-                  int* status, const Plan* given, void* stream) {
+                  int* status, void* stream, const Plan* given = nullptr, int late = -1) {
     if (N < 0 || T < 0 || K < 0) return fail(COSET_E_BADARG, "negative size");
     if (N == 0 || T == 0) return 0;
     if (K == 0) return fail(COSET_E_BADARG, "nothing to sum over");
@@ -336,7 +338,7 @@ int dense_product(const void* w, int64_t ldw, const void* x, int64_t ldx, int N,
     if (ldw < (W_MN ? N : K) || ldx < (X_MN ? T : K) || ldw % 8 != 0 || ldx % 8 != 0 || ldy < N)
         return fail(COSET_E_BADARG, "leading dimensions: at least a row, and multiples of 8 for the operands");
     if (!aligned(x, 16) || !aligned(w, 16)) return fail(COSET_E_ALIGN, "the operands must be 16-byte aligned");
-    Shape s = {N, K, T, given ? *given : make_plan(N, K, T, X_MN ? 128 : 32), bias, round_bias, (__nv_bfloat16*)y, ldy, aligned(y, 16) && ldy % 8 == 0 && N % 8 == 0, status};
+    Shape s = {N, K, T, given ? *given : make_plan(N, K, T, X_MN ? 128 : 32), bias, round_bias, (__nv_bfloat16*)y, ldy, aligned(y, 16) && ldy % 8 == 0 && N % 8 == 0, status, late};
     if ((T + s.plan.tokens - 1) / s.plan.tokens > 65535) return fail(COSET_E_UNSUPPORTED, "too many columns");
     CUtensorMap x_map, w_map;
     if (int e = X_MN ? make_bf16_map(&x_map, x, T, K, ldx, BK) : make_bf16_map(&x_map, x, K, T, ldx, s.plan.tokens / 2)) return e;
@@ -349,13 +351,21 @@ int dense_product(const void* w, int64_t ldw, const void* x, int64_t ldx, int N,
 extern "C" int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, int round_bias,
                                      void* y, int64_t ldy, int* status, void* stream) {
     if (n_in % 8 != 0) return fail(COSET_E_BADARG, "bad shape (n_in must be a multiple of 8)");
-    return dense_product<false, false>(w_bf16, n_in, x_bf16, ldx, n_out, T, n_in, bias, round_bias, y, ldy, status, nullptr, stream);
+    return dense_product<false, false>(w_bf16, n_in, x_bf16, ldx, n_out, T, n_in, bias, round_bias, y, ldy, status, stream);
+}
+
+extern "C" int coset_e8_dense_linear_late(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int T, void* y, int tokens, int split, int late, int* status, void* stream) {
+    const int steps = (n_in + BK - 1) / BK;
+    if (n_in <= 0 || n_in % 8 != 0 || tokens < 32 || tokens > 256 || tokens % 32 != 0 || (split != 1 && split != 2 && split != 4) || split > steps)
+        return fail(COSET_E_BADARG, "no such plan");
+    const Plan plan = with_stages(tokens, split, steps);
+    return dense_product<false, false>(w_bf16, n_in, x_bf16, n_in, n_out, T, n_in, nullptr, 0, y, n_out, status, stream, &plan, late);
 }
 
 extern "C" int coset_dense_input_grad(const void* g_bf16, const void* w_bf16, int T, int n_out, int n_in, void* dx, int* status, void* stream) {
-    return dense_product<true, false>(w_bf16, n_in, g_bf16, n_out, n_in, T, n_out, nullptr, 0, dx, n_in, status, nullptr, stream);
+    return dense_product<true, false>(w_bf16, n_in, g_bf16, n_out, n_in, T, n_out, nullptr, 0, dx, n_in, status, stream);
 }
 
 extern "C" int coset_dense_weight_grad(const void* g_bf16, const void* x_bf16, int T, int n_out, int n_in, void* dw, int* status, void* stream) {
-    return dense_product<true, true>(x_bf16, n_in, g_bf16, n_out, n_in, n_out, T, nullptr, 0, dw, n_in, status, nullptr, stream);
+    return dense_product<true, true>(x_bf16, n_in, g_bf16, n_out, n_in, n_out, T, nullptr, 0, dw, n_in, status, stream);
 }

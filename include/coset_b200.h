@@ -413,6 +413,13 @@ int coset_e8_decode_gemm(const void* codes, const float* beta, int64_t blocks_pe
 int coset_e8_dense_linear(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int64_t ldx, int T, const float* bias, int round_bias,
                           void* y, int64_t ldy, int* status, void* stream);
 
+/* The same by a given plan (tokens of a pair of CTAs: a multiple of 32 up to 256; pairs that share n_in: 1, 2 or 4), contiguous rows, no bias, in
+ * which pair `late` of every cluster takes its first wait for run out (-1: none): for tests of what such a wait leaves behind.  It returns after
+ * the 0.2 s that the waits behind it take.
+ */
+int coset_e8_dense_linear_late(const void* w_bf16, int n_out, int n_in, const void* x_bf16, int T, void* y, int tokens, int split, int late,
+                               int* status, void* stream);
+
 /* The two products of its backward pass, all bf16 with contiguous rows, 16-byte aligned, n_out and n_in multiples of 8, float32 sums and one
  * rounding: dx[T, n_in] = g[T, n_out] W[n_out, n_in] and dw[n_out, n_in] = g^T x[T, n_in].  Replaces the matmuls of autograd's linear
  * backward behind coset/core/layers.py:524-536.  Where a bounded wait gave up, results are not a number.

@@ -759,3 +759,21 @@ def test_products_of_different_plans_from_several_threads():
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+@pytest.mark.parametrize("tokens,split", [(32, 4), (64, 2), (128, 1), (256, 4), (224, 2)])
+def test_a_wait_that_gave_up_leaves_no_number(tokens, split):
+    """Each pair in turn takes its wait for run out: the results of every tile it has a part in are not a number, the status says so, and the
+    next call is as good as any."""
+    from coset_b200 import _lib
+    T, n_out, n_in = tokens + 5, 264, 520
+    x, w = torch.randn(T, n_in, device="cuda").bfloat16(), torch.randn(n_out, n_in, device="cuda").bfloat16()
+    want = x.double() @ w.double().T
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -22 * (x.double().abs() @ w.double().abs().T)
+    for late in (-1, *range(split), -1):
+        y, status = torch.zeros(T, n_out, device="cuda", dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32, device="cuda")
+        _lib.check(_lib.lib().coset_e8_dense_linear_late(_lib.ptr(w), n_out, n_in, _lib.ptr(x), T, _lib.ptr(y), tokens, split, late, _lib.ptr(status), _lib.stream()), "late")
+        if late < 0:
+            assert bool(((y.double() - want).abs() <= bound).all()) and int(status.item()) == 0
+        else:
+            assert bool(y.isnan().all()) and int(status.item()) == 1
