@@ -618,7 +618,8 @@ class GraphedTrainStep:
         loss = step(x, target)                                     # gradients are in p.grad afterwards
 
     The inputs of every call must have the shapes and dtypes of the examples.  Gradients are rewritten
-    (not accumulated) by every replay; read or apply them before the next call."""
+    (not accumulated) by every replay; read or apply them before the next call.  An eager step may multiply by other kernels than the graph
+    records, so the two agree to the rounding of the type."""
 
     def __init__(self, module: nn.Module, loss_fn, example_inputs, warmup: int = 3):
         self.module, self.loss_fn = module, loss_fn

@@ -12,6 +12,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -448,21 +449,27 @@ bool own_rows(const Tensor& t) {
 //   float32 up to 61 us of products at 2^28 multiply-adds ([1024 x 512 x 512]; 54 with torch's); tiles count whole ([4096 x 10 x 2048] 131 / 141).
 // The weight's gradient has few tiles in a narrow layer, and a cluster of eight CTAs at most sums over all tokens of one: bf16 [32768 x 64 x 64] 111 / 142 but
 // [262144 x 64 x 64] 442 / 180; float32 [16384 x 16 x 64] 109 / 143, [65536 x 64 x 64] 314 / 255, [2^20 x 8 x 8] 6195 / 993.
-bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, int64_t n_in) {
+// Under capture the host costs nothing, and what is quicker on the device is recorded: torch's in bf16 ([4096 x 3072 x 768] 105 us a replay against 115, [128 x 768 x 768]
+// 39 / 43), the own in float32 up to 2^27 ([128 x 768 x 768] 59 with torch's against 54, [4096 x 64 x 64] 78 / 51; beyond, [1024 x 512 x 512] 72 / 74), but for a few
+// tokens ([1 x 1024 x 1024] 36 / 45) and narrow layers with many ([16384 x 16 x 64] 55 / 112).
+bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, int64_t n_in, bool capturing) {
     if (tokens <= 0 || tokens > 1 << 15 || n_out <= 0 || n_in <= 0 || n_out > ((int64_t)1 << 22) / n_in) return false;
     const auto whole = [](int64_t v, int64_t tile) { return (v + tile - 1) / tile * tile; };
     const int64_t products = tokens * n_out * n_in;
-    if (type == at::kFloat)  // the smallest steps keep torch's product, whose bits a trace of the layer has
-        return tokens <= 1 << 14 && products >= 1 << 16 && products <= 1 << 28 && whole(tokens, 32) * whole(n_out, 64) * whole(n_in, 64) <= 1 << 29;
-    return type == at::kBFloat16 && n_out % 8 == 0 && n_in % 8 == 0 && products <= (int64_t)1 << 34 && tokens * (n_out + 2 * n_in) <= 9 << 22;
+    if (type == at::kFloat) {  // the smallest steps keep torch's product, whose bits a trace of the layer has
+        const int64_t of_tiles = whole(tokens, 32) * whole(n_out, 64) * whole(n_in, 64);
+        return tokens <= 1 << 14 && products >= 1 << 16 && products <= 1 << 28 && of_tiles <= 1 << 29 && !(capturing && (tokens < 16 || tokens > 4096 || of_tiles > 1 << 27));
+    }
+    return type == at::kBFloat16 && !capturing && n_out % 8 == 0 && n_in % 8 == 0 && products <= (int64_t)1 << 34 && tokens * (n_out + 2 * n_in) <= 9 << 22;
 }
+bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
 // The rows of a layer's input where its product is the library's own, undefined where it is torch's (which refuses what does not fit together).
 Tensor own_layer_rows(const Tensor& x, const Tensor& w, const Tensor& bias) {
     const int64_t n_out = w.size(0), n_in = w.size(1);
     if (!x.is_contiguous() || x.dim() < 1 || x.size(-1) != n_in || w.numel() == 0 || x.device() != w.device()) return Tensor();
     if (bias.defined() && !(bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.device() == w.device() && bias.dim() == 1 && bias.numel() == n_out)) return Tensor();
     const Tensor x2 = x.dim() == 2 ? x : x.view({-1, n_in});
-    return own_rows(x2) && own_training_products(x.scalar_type(), x2.size(0), n_out, n_in) ? x2 : Tensor();
+    return own_rows(x2) && own_training_products(x.scalar_type(), x2.size(0), n_out, n_in, capturing()) ? x2 : Tensor();
 }
 
 // dense_linear(x [T, n_in] bf16, w [n_out, n_in] bf16, bias or None, status or None, own): x w^T + bias as bf16.  `own`: by the library's own
@@ -618,7 +625,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         variable_list out(9);
         const int64_t T = g2.size(0), N = w.size(0), K = w.size(1);
         const at::ScalarType type = g2.scalar_type();
-        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K) && own_rows(g2) && g2.device() == w.device(), f32 = type == at::kFloat;
+        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K, capturing()) && own_rows(g2) && g2.device() == w.device(), f32 = type == at::kFloat;
         if (ctx->needs_input_grad(0)) {
             c10::SmallVector<int64_t, 6> x_shape(grads[0].sizes().begin(), grads[0].sizes().end());
             x_shape.back() = K;
@@ -702,11 +709,11 @@ PyObject* qat_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// own_product_sizes(dtype_code, tokens, n_out, n_in) -> whether a training step of these sizes is multiplied by the library's own kernels
+// own_product_sizes(dtype_code, tokens, n_out, n_in, capturing) -> whether a training step of these sizes is multiplied by the library's own kernels
 PyObject* own_product_sizes(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    nargs_are(n, 4);
-    return PyBool_FromLong(own_training_products(scalar_type((int)int_arg(a[0])), int_arg(a[1]), int_arg(a[2]), int_arg(a[3])));
+    nargs_are(n, 5);
+    return PyBool_FromLong(own_training_products(scalar_type((int)int_arg(a[0])), int_arg(a[1]), int_arg(a[2]), int_arg(a[3]), a[4] == Py_True));
     END_HANDLE_TH_ERRORS
 }
 
@@ -716,6 +723,7 @@ PyObject* own_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
     nargs_are(n, 3);
     const Tensor &x = tensor_arg(a[0], "x"), &w = tensor_arg(a[1], "weight");
     at::AutoGradMode no_grad(false);  // as inside the node
+    const c10::cuda::OptionalCUDAGuard guard(x.is_cuda() ? std::optional<c10::Device>(x.device()) : std::nullopt);
     return PyBool_FromLong(own_layer_rows(x, w, optional_arg(a[2], "bias")).defined());
     END_HANDLE_TH_ERRORS
 }

@@ -568,3 +568,34 @@ def test_training_step_of_more_tokens_than_the_own_products_take(dtype, tokens):
     y.backward(x.detach())
     wq = layer._quantize_weights(dtype).detach()
     assert torch.equal(y, torch.nn.functional.linear(x, wq)) and torch.equal(x.grad, torch.mm(x.detach(), wq)) and layer.weight.grad is not None
+
+
+@pytest.mark.parametrize("dtype,tokens,own", [(torch.bfloat16, 257, False), (torch.float32, 257, True), (torch.float32, 1601, False)])
+def test_captured_step_records_the_quicker_products(dtype, tokens, own):
+    """A captured step records torch's products where they are quicker on the device, bit for bit, and agrees with the eager step either way."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    from coset_b200.core.layers import GraphedTrainStep
+    layer = create_e8_hnlq_linear(520, 264, device="cuda", tiling="row", init_method="zeros")
+    layer.load_weights(torch.randn(264, 520, device="cuda") * 20.0, torch.randn(264, device="cuda"))
+    x, g = torch.randn(tokens, 520, device="cuda").to(dtype), torch.randn(tokens, 264, device="cuda").to(dtype)
+    seen = {}
+
+    def loss(y, g):
+        seen["y"] = y
+        if torch.cuda.is_current_stream_capturing():
+            seen["own"] = _lib.native().own_product(x, layer.weight, layer.bias)
+        return (y * g).sum()
+    step = GraphedTrainStep(layer, loss, (x, g))
+    step(x, g)
+    assert seen["own"] == own and _lib.native().own_product(x, layer.weight, layer.bias)
+    replayed = [seen["y"].detach().clone(), layer.weight.grad.clone(), layer.bias.grad.clone()]
+    wq, b = layer._quantize_weights(dtype).detach(), layer.bias.detach().to(dtype)
+    if not own:
+        assert torch.equal(replayed[0], torch.nn.functional.linear(x, wq, b))
+    layer.zero_grad()
+    y = layer(x)
+    (y * g).sum().backward()
+    unit = 2.0 ** -7 if dtype == torch.bfloat16 else 1601 * 2.0 ** -23  # the type's rounding; sums of at most 1601 products in another order
+    for a, b in zip(replayed, (y.detach(), layer.weight.grad, layer.bias.grad)):
+        assert torch.allclose(a.float(), b.float(), rtol=unit, atol=unit * float(b.abs().max()))

@@ -157,7 +157,7 @@ def test_sizes_of_the_training_layers_own_products():
     """What the rule takes fits the kernels' grids, which refuse more than 65535 tiles of tokens; long and narrow steps, whose weight gradient
     would run on a few CTAs, and wide ones, which the device bounds, stay with torch."""
     from coset_b200 import _lib
-    own = _lib.native().own_product_sizes
+    own = lambda *sizes, capturing=False: _lib.native().own_product_sizes(*sizes, capturing)
     f32, bf16 = _lib.DTYPE_F32, _lib.DTYPE_BF16
     assert own(f32, 128, 768, 768) and own(f32, 16384, 16, 64) and own(f32, 1024, 512, 512) and own(f32, 8192, 10, 768)
     assert own(bf16, 4096, 3072, 768) and own(bf16, 8192, 4096, 64) and own(bf16, 32768, 64, 64) and own(bf16, 1, 8, 8)
@@ -173,3 +173,9 @@ def test_sizes_of_the_training_layers_own_products():
     for tokens in range(1, 1 << 25, 99991):
         assert not own(f32, tokens, 8, 8) or tokens <= 65535 * 32
         assert not own(bf16, tokens, 8, 8) or tokens <= 65535 * 32
+    # a graph keeps what is quicker on the device
+    assert own(f32, 128, 768, 768, capturing=True) and own(f32, 32, 48, 64, capturing=True) and own(f32, 4096, 64, 64, capturing=True)
+    for tokens, n_out, n_in in ((1024, 512, 512), (8, 1024, 1024), (16384, 16, 64)):
+        assert own(f32, tokens, n_out, n_in) and not own(f32, tokens, n_out, n_in, capturing=True)
+    for tokens, n_out, n_in in ((4096, 3072, 768), (128, 768, 768), (8, 64, 64)):
+        assert own(bf16, tokens, n_out, n_in) and not own(bf16, tokens, n_out, n_in, capturing=True)
