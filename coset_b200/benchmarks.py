@@ -160,7 +160,7 @@ def iter_vlut(tilings=("block", "row")):
             rec = {"bench": "vlut_matmul", "tiling": tiling, "T": T, "shape": [n, n], "ms": ms,
                    "tokens_per_s": T / (ms * 1e-3),
                    "path": ("E8CodeLinear under capture: code-domain kernel" if T <= 64 else
-                            "E8CodeLinear under capture: the weight decoded with the call + coset_e8_dense_linear" if T < lin.PAIR_GEMM_MIN_T else
+                            "E8CodeLinear under capture: the weight decoded with the call + library GEMM" if T < lin.PAIR_GEMM_MIN_T else
                             "E8CodeLinear default: decode + tcgen05 cta_group::2 GEMM, bf16 result"),
                    "timing": "CUDA graph replay" if T <= 256 else "CUDA events over eager calls",
                    "peaks": src}

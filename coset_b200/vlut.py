@@ -10,7 +10,7 @@ weights) plus the scales beta, and applied from the codes:
   * many tokens (from 2048 by default): the weight is decoded into a transient bf16 buffer and multiplied by
     this library's tcgen05 GEMM (coset_e8_decode_gemm); nothing dense survives the call;
   * in between, by default, this library's product with a kept dense bf16 copy (coset_e8_dense_linear) up to 2^34 multiply-adds and
-    torch's beyond (`large_t_path` chooses).
+    torch's beyond, for very long rows and in graphs of small layers (`large_t_path` chooses).
 
 The math is the reference's one-sided vLUT inner product (coset/legacy/quant/vlut.py:72-117) in
 the layer's scale convention W_q = decode(codes) / beta (coset/core/layers.py:453-460).
@@ -97,7 +97,7 @@ class E8CodeLinear(nn.Module):
     cta_group::2 GEMM from 1024 tokens, the single-launch fused kernel below; "cublas" -- a cached dense bf16 copy
     and the library GEMM; "auto" (default) -- the own kernels from PAIR_GEMM_MIN_T tokens, the kept dense copy for
     the tokens in between, where decoding the whole weight per call costs more than the product itself (multiplied by this library's kernel
-    up to DENSE_OWN_MAX multiply-adds).
+    or by torch's, whichever is quicker; see DENSE_OWN_MAX).
     Few tokens use a one-byte-per-weight copy laid out on the first such call ("auto", "cublas"): 9-13 us for 1-16
     tokens and a 4096 x 4096 weight; the kernel checks the copy against the codes in every call.  "tcgen05" keeps nothing and
     stays on the code-domain kernels (9.7-23 us).
@@ -112,10 +112,15 @@ class E8CodeLinear(nn.Module):
     weight_clip_value > 0: the weights are clamp(decode(codes) / beta, +-clip), the clamp the training
     layer applies after de-scaling (coset/core/layers.py:463); 0 disables it."""
 
-    # Up to here (in multiply-adds) the library's own product with the kept dense copy is as fast on the device as torch's product and its
-    # cast of the bias (4096 x 4096: 256 tokens 14.1 us against 11.1 + 3, 1024 tokens 26.9 against 25.2 + 3; 2047 tokens 52 against 47 + 3), and it
-    # costs the host one launch instead of two library calls (10 us), which is what bounds such a call.
-    DENSE_OWN_MAX = 1 << 34
+    # The library's own product with the kept dense copy costs the host one launch where torch's costs a library call and, with a bias, its cast, and that bounds
+    # such a call: 4096 x 4096, own / torch with a bias / without, us a call: 17 tokens 8.5 / 19.2 / 14.9, 256 tokens 11.7 / 19.3 / 14.8, 1024 tokens
+    # 24.6 / 27.8 / 24.7; 8192 x 8192 and 256 tokens 35 / 37 / 33.5.  Beyond 2^34 multiply-adds torch's is quicker, and so it is where few CTAs sum over
+    # a long row ([64, 65536] with 17 tokens 29 / 21 / 17.5; [128, 32768] 16.6 / 21.5 / 17.4).
+    DENSE_OWN_MAX, DENSE_OWN_MAX_IN = 1 << 34, 1 << 15
+    # In a graph the host costs nothing: the own product pays where its start under the decoding before it counts, in large weights, the sooner with a
+    # bias to cast, and where torch's splits long rows (replays with 256 tokens, own / torch, us: 4096 x 4096 with a bias 23.0 / 23.1, without
+    # 22.9 / 21.8; 8192 x 8192 76 / 81, 76 / 79; 3072 x 768 without 9.6 / 8.1; 64 x 8192 10.4 / 16.6, 10.3 / 15.4).
+    DENSE_CAPTURED_MIN, DENSE_CAPTURED_MIN_NO_BIAS, DENSE_CAPTURED_LONG = 1 << 24, 1 << 25, 1 << 13
     PAIR_GEMM_MIN_T = 2048  # from here on the decode + cta_group::2 GEMM is within 10-25 % of the library on a dense copy
 
     def __init__(self, codes: torch.Tensor, beta: torch.Tensor, blocks_per_tile: int,
@@ -307,10 +312,13 @@ class E8CodeLinear(nn.Module):
             return torch.nn.functional.linear(x, self.dense_weight(torch.float32), buf["bias"])
         b, w = buf["bias"], self._dense_bf16()
         if dtype is torch.bfloat16 and type(x) is torch.Tensor and torch._C._get_tracing_state() is None and not torch._C._len_torch_function_stack():
-            own = self.large_t_path == "auto" and T < self.PAIR_GEMM_MIN_T and T * n_in * self.out_features <= self.DENSE_OWN_MAX
+            capturing = torch._C._cuda_isCurrentStreamCapturing()
+            weights = n_in * self.out_features
+            own = (self.large_t_path == "auto" and T < self.PAIR_GEMM_MIN_T and T * weights <= self.DENSE_OWN_MAX and n_in <= self.DENSE_OWN_MAX_IN
+                   and not (capturing and n_in < self.DENSE_CAPTURED_LONG and weights < (self.DENSE_CAPTURED_MIN if b is not None else self.DENSE_CAPTURED_MIN_NO_BIAS)))
             status = self._status
             if own and (status is None or status.device != x.device):  # not inside a capture, whose memory is the graph's
-                status = self._status = None if torch._C._cuda_isCurrentStreamCapturing() else torch.zeros(1, dtype=torch.int32, device=x.device)
+                status = self._status = None if capturing else torch.zeros(1, dtype=torch.int32, device=x.device)
             return _lib.native().dense_linear(x, w, b, status, own)
         return torch.nn.functional.linear(x, w.to(dtype), b.to(dtype) if b is not None else None)
 

@@ -777,3 +777,23 @@ def test_a_wait_that_gave_up_leaves_no_number(tokens, split):
             assert bool(((y.double() - want).abs() <= bound).all()) and int(status.item()) == 0
         else:
             assert bool(y.isnan().all()) and int(status.item()) == 1
+
+
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("how", ["captured", "long"])
+def test_kept_dense_weight_is_torchs_where_that_is_quicker(how, bias):
+    """In a graph, for a weight whose own product is the slower one, and for rows so long that few CTAs would sum over each: torch's bits."""
+    n_out, n_in = (256, 4096) if how == "captured" else (64, (1 << 15) + 8)
+    layer, _ = _kept_copy_layer(n_out, n_in)
+    layer.bias = torch.randn(n_out, device="cuda") if bias else None
+    x = torch.randn(64, n_in, device="cuda").bfloat16()
+    want = torch.nn.functional.linear(x, layer.dense_weight(torch.bfloat16), layer.bias.bfloat16() if bias else None)
+    if how == "long":
+        assert torch.equal(layer(x), want)
+        return
+    layer(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = layer(x)
+    graph.replay()
+    assert torch.equal(y, want)
