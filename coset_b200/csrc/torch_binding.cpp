@@ -9,6 +9,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/Context.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -435,10 +436,12 @@ bool plain(const Tensor& t) {
     return (t.key_set().raw_repr() & ~known.raw_repr()) == 0 && !(at::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined();
 }
 
+// The own float32 products multiply in float32: a caller who lets torch's use TF32 gets those.
+bool tf32_allowed() { return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32; }
 // Whether the library's own kernels may multiply a matrix: contiguous (and in bf16 made of aligned 16-byte chunks), and nobody looks at the torch calls.
 bool own_rows(const Tensor& t) {
     const bool f32 = t.scalar_type() == at::kFloat;
-    return t.dim() == 2 && (f32 || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0)) && t.is_contiguous() &&
+    return t.dim() == 2 && ((f32 && !tf32_allowed()) || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0)) && t.is_contiguous() &&
            t.size(0) > 0 && t.size(0) <= INT32_MAX && t.size(1) > 0 && plain(t) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
 }
 // Whether they should multiply for a training step: where the host bounds it (110 us with them, 141 with torch's products) and the device, which they cost

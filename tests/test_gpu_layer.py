@@ -599,3 +599,29 @@ def test_captured_step_records_the_quicker_products(dtype, tokens, own):
     unit = 2.0 ** -7 if dtype == torch.bfloat16 else 1601 * 2.0 ** -23  # the type's rounding; sums of at most 1601 products in another order
     for a, b in zip(replayed, (y.detach(), layer.weight.grad, layer.bias.grad)):
         assert torch.allclose(a.float(), b.float(), rtol=unit, atol=unit * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("how", ["allow_tf32", "high"])
+def test_float32_step_follows_the_callers_choice_of_tf32(how):
+    """Where torch may multiply in TF32 the layer's products are torch's, forward and backward; elsewhere the own ones, in float32."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(256, 192, device="cuda", tiling="row", init_method="zeros", bias=False)
+    layer.load_weights(torch.randn(192, 256, device="cuda") * 20.0)
+    x, g = torch.randn(128, 256, device="cuda").requires_grad_(), torch.randn(128, 192, device="cuda")
+    wq = layer._quantize_weights().detach()
+    assert _lib.native().own_product(x, layer.weight, None)
+    precision = torch.get_float32_matmul_precision()
+    try:
+        if how == "high":
+            torch.set_float32_matmul_precision("high")
+        else:
+            torch.backends.cuda.matmul.allow_tf32 = True
+        assert not _lib.native().own_product(x, layer.weight, None)
+        y = layer(x)
+        y.backward(g)
+        assert torch.equal(y, torch.nn.functional.linear(x, wq)) and torch.equal(x.grad, torch.mm(g, wq))
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = False
+        torch.set_float32_matmul_precision(precision)
+    assert _lib.native().own_product(x, layer.weight, None)
