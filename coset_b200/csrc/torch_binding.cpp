@@ -441,8 +441,8 @@ bool tf32_allowed() { return at::globalContext().float32Precision(at::Float32Bac
 // Whether the library's own kernels may multiply a matrix: contiguous (and in bf16 made of aligned 16-byte chunks), and nobody looks at the torch calls.
 bool own_rows(const Tensor& t) {
     const bool f32 = t.scalar_type() == at::kFloat;
-    return t.dim() == 2 && ((f32 && !tf32_allowed()) || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0)) && t.is_contiguous() &&
-           t.size(0) > 0 && t.size(0) <= INT32_MAX && t.size(1) > 0 && plain(t) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
+    return plain(t) && c10::impl::TorchDispatchModeTLS::stack_len() == 0 && t.dim() == 2 && t.is_contiguous() && t.size(0) > 0 && t.size(0) <= INT32_MAX && t.size(1) > 0 &&
+           ((f32 && !tf32_allowed()) || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0));
 }
 // Whether they should multiply for a training step: where the host bounds it (110 us with them, 141 with torch's products) and the device, which they cost
 // more, does not.  Steps of a layer on this box, own / torch, us:
@@ -489,7 +489,7 @@ PyObject* dense_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
         NoGil no_gil;
         c10::cuda::CUDAGuard guard(x.device());
         own = own && x.dim() == 2 && w.dim() == 2 && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && x.size(1) == w.size(1) && x.size(1) > 0 &&
-              x.size(1) % 8 == 0 && w.is_contiguous() && (uintptr_t)w.const_data_ptr() % 16 == 0 && w.device() == x.device() && plain(x) && plain(w) && plain(bias) &&
+              x.size(1) % 8 == 0 && plain(x) && plain(w) && plain(bias) && w.is_contiguous() && (uintptr_t)w.const_data_ptr() % 16 == 0 && w.device() == x.device() &&
               (!bias.defined() || (bias.device() == x.device() && bias.dim() == 1 && bias.size(0) == w.size(0))) &&
               !at::autocast::is_autocast_enabled(at::kCUDA) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
         if (own) {

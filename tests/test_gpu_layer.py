@@ -625,3 +625,17 @@ def test_float32_step_follows_the_callers_choice_of_tf32(how):
         torch.backends.cuda.matmul.allow_tf32 = False
         torch.set_float32_matmul_precision(precision)
     assert _lib.native().own_product(x, layer.weight, None)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gradients_of_a_batch_of_output_gradients(dtype):
+    """is_grads_batched: the backward pass gets a batch of a transform, which has no memory of its own to look at."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(256, 192, device="cuda", tiling="row", init_method="zeros")
+    layer.load_weights(torch.randn(192, 256, device="cuda") * 20.0)
+    x, g = torch.randn(64, 256, device="cuda").to(dtype).requires_grad_(), torch.randn(3, 64, 192, device="cuda").to(dtype)
+    got, = torch.autograd.grad(layer(x), x, g, is_grads_batched=True)
+    unit = 2.0 ** -7 if dtype == torch.bfloat16 else 192 * 2.0 ** -23  # the type's rounding; sums of 192 products in another order
+    for one, batch in zip(g, got):
+        want, = torch.autograd.grad(layer(x), x, one)
+        assert torch.allclose(batch.float(), want.float(), rtol=unit, atol=unit * float(want.abs().max()))
