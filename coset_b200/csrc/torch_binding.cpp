@@ -628,7 +628,8 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         variable_list out(9);
         const int64_t T = g2.size(0), N = w.size(0), K = w.size(1);
         const at::ScalarType type = g2.scalar_type();
-        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K, capturing()) && own_rows(g2) && g2.device() == w.device(), f32 = type == at::kFloat;
+        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K, capturing()) && own_rows(g2) && g2.device() == w.device() &&
+                         !at::autocast::is_autocast_enabled(at::kCUDA), f32 = type == at::kFloat;
         if (ctx->needs_input_grad(0)) {
             c10::SmallVector<int64_t, 6> x_shape(grads[0].sizes().begin(), grads[0].sizes().end());
             x_shape.back() = K;

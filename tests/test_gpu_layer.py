@@ -639,3 +639,17 @@ def test_gradients_of_a_batch_of_output_gradients(dtype):
     for one, batch in zip(g, got):
         want, = torch.autograd.grad(layer(x), x, one)
         assert torch.allclose(batch.float(), want.float(), rtol=unit, atol=unit * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("dtype,cast", [(torch.float32, torch.bfloat16), (torch.float32, torch.float16), (torch.bfloat16, torch.float16)])
+def test_backward_under_autocast_multiplies_in_its_type(dtype, cast):
+    """A backward pass inside an autocast region: its products are torch's, in the region's type, as in a composed layer."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(256, 192, device="cuda", tiling="row", init_method="zeros", bias=False)
+    layer.load_weights(torch.randn(192, 256, device="cuda") * 20.0)
+    x, g = torch.randn(64, 256, device="cuda").to(dtype).requires_grad_(), torch.randn(64, 192, device="cuda").to(dtype)
+    wq = layer._quantize_weights(dtype).detach()
+    y = layer(x)
+    with torch.autocast("cuda", dtype=cast):
+        y.backward(g)
+    assert torch.equal(x.grad, torch.mm(g.to(cast), wq.to(cast)).to(dtype))
