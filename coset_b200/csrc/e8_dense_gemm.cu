@@ -39,6 +39,7 @@ constexpr int kThreads = 10 * 32;
 constexpr int kAlignment = 1024;         // of the stages, which the base of the shared memory need not have
 constexpr int kSmemBudget = 227 * 1024 - kAlignment;
 constexpr int kSmemOfTwo = 112 * 1024;   // two CTAs on an SM (228 KB, 1 KB of which each CTA takes)
+constexpr int kMostSize = INT32_MAX - 512;
 constexpr int kBarrierBytes = 16 * kMaxStages + 16;
 constexpr int kScratchRow = 40;       // 32 features and a pad, in values
 constexpr int kScratchBytes = kEpilogueWarps * 32 * kScratchRow * 2;
@@ -332,6 +333,7 @@ template <bool W_MN, bool X_MN>
 int dense_product(const void* w, int64_t ldw, const void* x, int64_t ldx, int N, int T, int K, const float* bias, int round_bias, void* y, int64_t ldy,
                   int* status, void* stream, const Plan* given = nullptr, int late = -1) {
     if (N < 0 || T < 0 || K < 0) return fail(COSET_E_BADARG, "negative size");
+    if (N > kMostSize || T > kMostSize || K > kMostSize) return fail(COSET_E_UNSUPPORTED, "sizes are counted in 32 bits, with room for a tile");
     if (N == 0 || T == 0) return 0;
     if (K == 0) return fail(COSET_E_BADARG, "nothing to sum over");
     if (!w || !x || !y) return fail(COSET_E_BADARG, "null pointer");

@@ -18,6 +18,7 @@ namespace {
 
 constexpr int kM = 32, kN = 64, kK = 32, kThreads = 128;
 constexpr int kMostParts = 8;
+constexpr int kMostSize = INT32_MAX - 512;
 constexpr int kFlush = 4;  // steps of a chain of additions
 
 struct Operands {
@@ -192,6 +193,7 @@ k_f32_product(const __grid_constant__ Operands o) {
 template <bool A_K, bool B_K>
 int f32_product(const float* a, const float* b, const float* bias, int M, int N, int K, float* c, void* stream) {
     if (M < 0 || N < 0 || K < 0) return fail(COSET_E_BADARG, "negative size");
+    if (M > kMostSize || N > kMostSize || K > kMostSize) return fail(COSET_E_UNSUPPORTED, "sizes are counted in 32 bits, with room for a tile");
     if (M == 0 || N == 0) return 0;
     if (K == 0) return fail(COSET_E_BADARG, "nothing to sum over");
     if (!a || !b || !c) return fail(COSET_E_BADARG, "null pointer");

@@ -179,3 +179,21 @@ def test_sizes_of_the_training_layers_own_products():
         assert own(f32, tokens, n_out, n_in) and not own(f32, tokens, n_out, n_in, capturing=True)
     for tokens, n_out, n_in in ((4096, 3072, 768), (128, 768, 768), (8, 64, 64)):
         assert own(bf16, tokens, n_out, n_in) and not own(bf16, tokens, n_out, n_in, capturing=True)
+
+
+@pytest.mark.parametrize("size", [2 ** 31 - 1, 2 ** 31 - 8, 2 ** 31 - 512])
+def test_dense_products_refuse_sizes_that_their_counts_cannot_hold(size):
+    """Before anything is launched: with a tile added such a size wraps around (a count of -1 tiles is not more than the grid takes)."""
+    from coset_b200 import _lib
+    L = _lib.lib()
+    memory = torch.zeros(64, dtype=torch.float32)
+    p = (memory.data_ptr() + 127) // 128 * 128
+    wide = size // 8 * 8
+    if wide > 2 ** 31 - 513:
+        assert L.coset_e8_dense_linear(p, 64, wide, p, wide, 64, None, 0, p, 64, None, None) == -2
+        assert L.coset_dense_input_grad(p, p, 64, wide, 64, p, None, None) == -2 and L.coset_dense_weight_grad(p, p, 64, 64, wide, p, None, None) == -2
+    assert L.coset_e8_dense_linear(p, 64, 64, p, 64, size, None, 0, p, 64, None, None) == -2
+    assert L.coset_dense_weight_grad(p, p, size, 64, 64, p, None, None) == -2
+    for sizes in ((size, 64, 64), (64, size, 64), (64, 64, size)):
+        assert L.coset_f32_linear(p, p, None, *sizes, p, None) == -2
+        assert L.coset_f32_input_grad(p, p, *sizes, p, None) == -2 and L.coset_f32_weight_grad(p, p, *sizes, p, None) == -2
