@@ -40,11 +40,6 @@ __device__ __constant__ uint4 kFlipRows[8] = {
     {1u, 0u, 0u, 0u},     {1u, 8u, 0u, 0u},       {1u, 8u, 32u, 0u},       {1u, 8u, 32u, 128u},
     {513u, 8u, 32u, 128u}, {513u, 2056u, 32u, 128u}, {513u, 2056u, 8224u, 128u}, {513u, 4112u, 24672u, 66048u}};
 
-__device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-    return r;
-}
 // prmt.b32 with the full 4-bit selectors (bit 3 of a selector replicates the sign of the chosen byte)
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
     uint32_t r;
