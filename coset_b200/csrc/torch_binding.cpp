@@ -459,7 +459,9 @@ bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, i
     if (tokens <= 0 || tokens > 1 << 15 || n_out <= 0 || n_in <= 0 || n_out > ((int64_t)1 << 22) / n_in) return false;
     const auto whole = [](int64_t v, int64_t tile) { return (v + tile - 1) / tile * tile; };
     const int64_t products = tokens * n_out * n_in;
-    if (type == at::kFloat) {  // the smallest steps keep torch's product, whose bits a trace of the layer has
+    // A trace of the layer and a torch-function mode see torch's product, with which the own ones agree to the rounding of the type.  Float32 steps below 2^16 keep
+    // torch's, though it costs the host 25 us there as anywhere: a step that small is one that is compared to the bit with its trace.
+    if (type == at::kFloat) {
         const int64_t of_tiles = whole(tokens, 32) * whole(n_out, 64) * whole(n_in, 64);
         return tokens <= 1 << 14 && products >= 1 << 16 && products <= 1 << 28 && of_tiles <= 1 << 29 && !(capturing && (tokens < 16 || tokens > 4096 || of_tiles > 1 << 27));
     }

@@ -521,3 +521,54 @@ def test_calls_beyond_the_offsets_of_one_launch(tile):
         part = dict(kw, scale=scale if tile > n else scale[lo // tile:(hi + tile - 1) // tile].contiguous())
         assert torch.equal(e8_encode_packed(x[lo:hi].contiguous(), **part), codes[lo:hi])
         assert torch.equal(e8_decode_packed(codes[lo:hi].contiguous(), dtype=torch.bfloat16, **part), back[lo:hi])
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.float32, 500001), (torch.bfloat16, 1000003)])
+@pytest.mark.parametrize("tile", [1, 96])
+def test_chained_calls_of_many_blocks(dtype, n, tile):
+    """The encoder that has its rows in shared memory and the decoder that has its table there, through the same buffers: what a chain of calls
+    leaves is what the calls leave one by one."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    assert n >= 3 * 4 * 148 * 256 and n >= (2 if dtype == torch.float32 else 6) * 148 * 1024
+    scale = 0.5 + torch.rand((n + tile - 1) // tile, device="cuda")
+    kw = dict(scale=scale, scale_mode=_lib.SCALE_MUL_TILE, blocks_per_tile=tile)
+    xs = [(torch.randn(n, 8, device="cuda") * s).to(dtype) for s in (0.3, 1.0, 3.0)]
+    moved, codes, back = torch.empty(n, 8, device="cuda", dtype=dtype), torch.empty(n, 4, dtype=torch.uint8, device="cuda"), torch.empty(n, 8, device="cuda", dtype=dtype)
+
+    def passes(wait):
+        results = []
+        for x in xs + xs[::-1]:
+            for step in (lambda: moved.copy_(x), lambda: e8_encode_packed(moved, out=codes, **kw), lambda: e8_decode_packed(codes, out=back, dtype=dtype, **kw),
+                         lambda: e8_encode_packed(back, out=codes, **kw), lambda: e8_decode_packed(codes, out=moved, dtype=dtype, **kw)):
+                step()
+                wait()
+            results.append((codes.clone(), back.clone(), moved.clone()))
+            wait()
+        return results
+    for a, b in zip(passes(torch.cuda.synchronize), passes(lambda: None)):
+        assert all(torch.equal(s, t) for s, t in zip(a, b))
+
+
+@pytest.mark.parametrize("tile", [(1 << 30) - 8, (1 << 30) + 8])
+def test_boundary_of_a_long_tile_inside_a_call(tile):
+    """A second scale begins behind 2^30 blocks, in the 17th launch of the call: 17 GB of values, each side of the boundary as in a call of its own."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import e8_decode_packed, e8_encode_packed
+    n = tile + 1000
+    if torch.cuda.mem_get_info()[0] < 64 << 30:
+        pytest.skip("needs 40 GB of device memory")
+    pattern = torch.randn(1 << 20, 8, device="cuda").bfloat16()
+    x = torch.empty(n, 8, device="cuda", dtype=torch.bfloat16)
+    for at in range(0, n, 1 << 20):
+        x[at:at + (1 << 20)] = pattern[:n - at]
+    scale = torch.tensor([1.3, 0.4], device="cuda")
+    kw = dict(scale_mode=_lib.SCALE_MUL_TILE, blocks_per_tile=tile)
+    codes = e8_encode_packed(x, scale=scale, **kw)
+    back = e8_decode_packed(codes, scale=scale, dtype=torch.bfloat16, **kw)
+    for lo, hi, s in ((0, 3000, 0), ((1 << 26) - 1500, (1 << 26) + 1500, 0), (tile - 3000, tile, 0), (tile, n, 1)):
+        part = dict(scale=scale[s:s + 1].contiguous(), scale_mode=_lib.SCALE_MUL_TILE, blocks_per_tile=1 << 20)
+        assert torch.equal(e8_encode_packed(x[lo:hi].contiguous(), **part), codes[lo:hi]), lo
+        assert torch.equal(e8_decode_packed(codes[lo:hi].contiguous(), dtype=torch.bfloat16, **part), back[lo:hi]), lo
+    del x, codes, back
+    torch.cuda.empty_cache()

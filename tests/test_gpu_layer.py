@@ -653,3 +653,98 @@ def test_backward_under_autocast_multiplies_in_its_type(dtype, cast):
     with torch.autocast("cuda", dtype=cast):
         y.backward(g)
     assert torch.equal(x.grad, torch.mm(g.to(cast), wq.to(cast)).to(dtype))
+
+
+@pytest.mark.parametrize("dtype,tokens,n_out,n_in", [(torch.float32, 8, 64, 128), (torch.float32, 128, 768, 768), (torch.bfloat16, 8, 32, 64), (torch.bfloat16, 300, 264, 1032)])
+def test_traced_layer_agrees_to_the_rounding_of_the_type(dtype, tokens, n_out, n_in):
+    """A trace records torch's product; the eager layer's own one adds up in another order: the smallest own step in float32 and larger ones."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(n_in, n_out, device="cuda", tiling="row", init_method="zeros")
+    layer.load_weights(torch.randn(n_out, n_in, device="cuda") * 20.0, torch.randn(n_out, device="cuda"))
+    x = torch.randn(tokens, n_in, device="cuda").to(dtype)
+    assert _lib.native().own_product(x, layer.weight, layer.bias)
+    traced = torch.jit.trace(layer, x, check_trace=False)
+    with torch.no_grad():
+        y, t = layer(x).float(), traced(x).float()
+    wq, b = layer._quantize_weights(dtype).detach().float(), layer.bias.detach().to(dtype).float()
+    size = x.float().abs() @ wq.abs().T + b.abs()
+    # each side rounds to the type once (to half a unit); their float32 sums of n_in products differ by at most that many roundings each way
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    assert bool(((y - t).abs() <= unit * torch.maximum(y.abs(), t.abs()) + 2 * (n_in + 1) * 2.0 ** -24 * size).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,n_out,n_in", [(64, 128, 256), (200, 328, 520), (1000, 512, 264)])
+def test_chained_products_read_what_the_call_before_wrote(dtype, T, n_out, n_in):
+    """The products start while the one before them drains: a chain in which each overwrites what the one before has read leaves what the calls
+    leave one by one."""
+    from coset_b200 import _lib
+    L, P, f32 = _lib.lib(), _lib.ptr, dtype == torch.float32
+    g = torch.Generator(device="cuda").manual_seed(T)
+    first = [torch.randn(s, device="cuda", generator=g).to(dtype) for s in ((T, n_in), (n_out, n_in))]
+
+    def chain(wait):
+        x, w = (t.clone() for t in first)
+        y, left = torch.empty(T, n_out, device="cuda", dtype=dtype), []
+        for _ in range(12):
+            st = _lib.stream()
+            for call in ((lambda: L.coset_f32_linear(P(x), P(w), None, T, n_out, n_in, P(y), st)) if f32 else
+                         (lambda: L.coset_e8_dense_linear(P(w), n_out, n_in, P(x), n_in, T, None, 0, P(y), n_out, None, st)),
+                         (lambda: L.coset_f32_input_grad(P(y), P(w), T, n_out, n_in, P(x), st)) if f32 else
+                         (lambda: L.coset_dense_input_grad(P(y), P(w), T, n_out, n_in, P(x), None, st)),
+                         (lambda: L.coset_f32_weight_grad(P(y), P(x), T, n_out, n_in, P(w), st)) if f32 else
+                         (lambda: L.coset_dense_weight_grad(P(y), P(x), T, n_out, n_in, P(w), None, st))):
+                assert call() == 0
+                wait()
+            left.append([t.clone() for t in (x, w, y)])
+            for t in (x, w):  # back to the size of the start
+                t.div_(t.float().abs().amax().to(dtype) + 1e-6)
+        return left
+    for a, b in zip(chain(torch.cuda.synchronize), chain(lambda: None)):
+        assert all(torch.equal(s, t) and bool(s.isfinite().all()) for s, t in zip(a, b))
+
+
+def test_steps_and_products_from_two_threads():
+    """A training layer and a code layer each, on a stream of their own, in two threads: the results are those of one thread."""
+    import threading
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    from coset_b200.vlut import E8CodeLinear
+
+    def work(seed, results):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for dtype, tokens, n_out, n_in in ((torch.bfloat16, 300 + 256 * seed, 256, 512), (torch.float32, 64 + 64 * seed, 192, 256)):
+                layer = create_e8_hnlq_linear(n_in, n_out, device="cuda", tiling="row", init_method="zeros")
+                layer.load_weights(torch.randn(n_out, n_in, device="cuda", generator=g) * 20.0, torch.randn(n_out, device="cuda", generator=g))
+                code = E8CodeLinear.from_qat_layer(layer)
+                x = torch.randn(tokens, n_in, device="cuda", generator=g).to(dtype).requires_grad_()
+                up = torch.randn(tokens, n_out, device="cuda", generator=g).to(dtype)
+                for _ in range(200):
+                    layer.zero_grad(set_to_none=True)
+                    x.grad = None
+                    y = layer(x)
+                    y.backward(up)
+                    with torch.no_grad():
+                        z = code(x.detach())
+                results += [t.detach().clone() for t in (y, z, x.grad, layer.weight.grad, layer.theta_beta.grad, layer.bias.grad)]
+            torch.cuda.current_stream().synchronize()
+    alone, together, failures = ([], []), ([], []), []
+    for seed in (0, 1):
+        work(seed, alone[seed])
+
+    def guarded(seed):
+        try:
+            work(seed, together[seed])
+        except Exception as e:  # noqa: BLE001 - reported by the test's own thread
+            failures.append(repr(e))
+    threads = [threading.Thread(target=guarded, args=(seed,)) for seed in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+    for a, b in zip(alone, together):
+        assert len(a) == len(b) == 12
+        for s, t in zip(a, b):
+            assert torch.allclose(s.float(), t.float(), rtol=1e-6, atol=0) if s.dim() == 1 else torch.equal(s, t)
