@@ -5,7 +5,7 @@ exist, pyproject.toml:67).  One JSON line per measurement:
     python -m coset_b200.benchmarks vlut       # code-domain matmul, W [4096, 4096], T in {1, 16, 256, 4096}
     python -m torch.distributed.run --nproc-per-node N -m coset_b200.benchmarks gradcomm
                                                # E8-quantised gradient exchange, BERT-base-shaped gradient
-    python -m coset_b200.benchmarks profile-gemv | profile-gemv16 | profile-gemm | profile-gemm-pair
+    python -m coset_b200.benchmarks profile-gemv | profile-gemv16 | profile-gemm | profile-gemm-pair | profile-dense | profile-f32
                                                # small fixed cases of the matmul kernels for a profiler capture
 
 Timing: CUDA events on the current stream, warm-up first, inputs resident on the device.
@@ -353,15 +353,22 @@ def profile_case(which):
     """Small fixed cases for a profiler capture (W 4096 x 4096, per-block scales, bf16 tokens):
     `profile-gemv` / `profile-gemv16` run the few-token code-domain product five times at T = 1 / 16, `profile-gemm` the
     fused tcgen05 dequant-GEMM three times at T = 2048 and checks its status word, `profile-gemm-pair` the same with
-    the decode + cta_group::2 GEMM."""
+    the decode + cta_group::2 GEMM, `profile-dense` the product with the kept dense copy five times at T = 256, and `profile-f32` three
+    float32 training steps of a [768, 768] layer with 128 tokens."""
     from .vlut import E8CodeLinear, e8_decode_gemm, e8_dequant_gemm
     torch.manual_seed(0)
     n = 4096
     W = (torch.randn(n, n) * 0.02).cuda()
     beta = torch.full((n * n // 8,), 25.0, device="cuda")
     lin = E8CodeLinear.from_weight(W, beta, 1)
-    if which in ("profile-gemv", "profile-gemv16"):
-        x = torch.randn(1 if which == "profile-gemv" else 16, n, device="cuda").to(torch.bfloat16)
+    if which == "profile-f32":
+        from .core.e8 import create_e8_hnlq_linear
+        layer = create_e8_hnlq_linear(768, 768, device="cuda", tiling="row")
+        x, g = torch.randn(128, 768, device="cuda").requires_grad_(), torch.randn(128, 768, device="cuda")
+        for _ in range(3):
+            layer(x).backward(g)
+    elif which in ("profile-gemv", "profile-gemv16", "profile-dense"):
+        x = torch.randn({"profile-gemv": 1, "profile-gemv16": 16, "profile-dense": 256}[which], n, device="cuda").to(torch.bfloat16)
         for _ in range(5):
             lin(x)
     else:
@@ -376,7 +383,7 @@ def profile_case(which):
 def main(argv=None):
     argv = sys.argv[1:] if argv is None else argv
     which = argv[0] if argv else "all"
-    if which in ("profile-gemv", "profile-gemv16", "profile-gemm", "profile-gemm-pair"):
+    if which in ("profile-gemv", "profile-gemv16", "profile-gemm", "profile-gemm-pair", "profile-dense", "profile-f32"):
         profile_case(which)
         return
     if which in ("qat", "all"):

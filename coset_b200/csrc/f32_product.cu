@@ -3,11 +3,13 @@
 // At 128 tokens and 768 features a library product is 15 us of host time and a kernel of 24 to 96 tiles on 148 SMs, for 75 million
 // multiply-adds (2 us of the chip).  Here a CTA of 128 threads owns 32 x 64 results and a part of the sum: up to eight CTAs of a cluster
 // share K where tiles are few, and add their sums in the order of K through distributed shared memory, every CTA a part of the rows.
-// Chains of additions are 128 long and their sums are added apart, so the error against 64 bits is no larger than that of the library's
-// products (1.1e-7 to 2.2e-7 in 42 products; the library's 1.1e-7 to 8.1e-7).
+// Chains of additions are 64 long and their sums are added apart, so from 32 tokens on the error against 64 bits is no larger than that of the library's
+// products (1.0e-7 to 1.8e-7 over sums of 64 to 16384 products, the library's 1.0e-7 to 1.3e-6; chains of 128 had 2.1e-7, and 2.13e-7 against 2.02e-7 in
+// the weight gradient of 2048 x 10 x 768; chains of 32 slow the forward product by a fifth).  For fewer tokens the library splits its sums finer (one token,
+// 768 x 768: 1.24e-7 against 1.47e-7), and the training layer leaves them to it.
 // What bounds a small one is latency (three to six steps of a load from L2 and 32 x 32 x 64 products each), a larger one the two 16-byte reads
-// from shared memory per 16 multiply-adds: four rows by four columns per thread.  128 x 768 x 768, torch -> here: forward 17.0 -> 10.4 us, dx 14.5
-// -> 10.3, dW 6.1 -> 7.8; 1024 x 512 x 512 19.8 -> 20.8, 15.6 -> 20.3, 19.4 -> 20.4.  Twice as many parts gained nothing; rows read 32 bytes per lane
+// from shared memory per 16 multiply-adds: four rows by four columns per thread.  128 x 768 x 768, torch -> here: forward 17.0 -> 10.4 us, dx 14.6
+// -> 10.4, dW 6.1 -> 7.7; 1024 x 512 x 512 19.6 -> 20.8, 15.5 -> 20.5, 19.3 -> 20.5.  Twice as many parts gained nothing; rows read 32 bytes per lane
 // with K along the lanes' runs took 12.8 us.
 #include "common.cuh"
 #include "e8_fast2.cuh"
@@ -19,7 +21,7 @@ namespace {
 constexpr int kM = 32, kN = 64, kK = 32, kThreads = 128;
 constexpr int kMostParts = 8;
 constexpr int kMostSize = INT32_MAX - 512;
-constexpr int kFlush = 4;  // steps of a chain of additions
+constexpr int kFlush = 2;  // steps of a chain of additions
 
 struct Operands {
     const float* a;  // C[m][n] = sum over k of A(m, k) B(n, k)

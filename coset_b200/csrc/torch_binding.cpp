@@ -453,17 +453,19 @@ bool own_rows(const Tensor& t) {
 // The weight's gradient has few tiles in a narrow layer, and a cluster of eight CTAs at most sums over all tokens of one: bf16 [32768 x 64 x 64] 111 / 142 but
 // [262144 x 64 x 64] 442 / 180; float32 [16384 x 16 x 64] 109 / 143, [65536 x 64 x 64] 314 / 255, [2^20 x 8 x 8] 6195 / 993.
 // Under capture the host costs nothing, and what is quicker on the device is recorded: torch's in bf16 ([4096 x 3072 x 768] 105 us a replay against 115, [128 x 768 x 768]
-// 39 / 43), the own in float32 up to 2^27 ([128 x 768 x 768] 59 with torch's against 54, [4096 x 64 x 64] 78 / 51; beyond, [1024 x 512 x 512] 72 / 74), but for a few
-// tokens ([1 x 1024 x 1024] 36 / 45) and narrow layers with many ([16384 x 16 x 64] 55 / 112).
+// 39 / 43), the own in float32 up to 2^27 ([128 x 768 x 768] 59 with torch's against 54, [4096 x 64 x 64] 78 / 51; beyond, [1024 x 512 x 512] 72 / 74), but for narrow
+// layers with many tokens ([16384 x 16 x 64] 55 / 112).
 bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, int64_t n_in, bool capturing) {
     if (tokens <= 0 || tokens > 1 << 15 || n_out <= 0 || n_in <= 0 || n_out > ((int64_t)1 << 22) / n_in) return false;
     const auto whole = [](int64_t v, int64_t tile) { return (v + tile - 1) / tile * tile; };
     const int64_t products = tokens * n_out * n_in;
-    // A trace of the layer and a torch-function mode see torch's product, with which the own ones agree to the rounding of the type.  Float32 steps below 2^16 keep
-    // torch's, though it costs the host 25 us there as anywhere: a step that small is one that is compared to the bit with its trace.
+    // Below 32 tokens torch's float32 sums are the more precise ones (f32_product.cu).  A trace of the layer and a torch-function mode see torch's product, with which the
+    // own ones agree to the rounding of the type.  Float32 steps below 2^16 keep torch's, though it costs the host 25 us there as anywhere: a step that small is
+    // one that is compared to the bit with its trace.
     if (type == at::kFloat) {
         const int64_t of_tiles = whole(tokens, 32) * whole(n_out, 64) * whole(n_in, 64);
-        return tokens <= 1 << 14 && products >= 1 << 16 && products <= 1 << 28 && of_tiles <= 1 << 29 && !(capturing && (tokens < 16 || tokens > 4096 || of_tiles > 1 << 27));
+        return tokens >= 32 && tokens <= 1 << 14 && products >= 1 << 16 && products <= 1 << 28 && of_tiles <= 1 << 29 &&
+               !(capturing && (tokens > 4096 || of_tiles > 1 << 27));
     }
     return type == at::kBFloat16 && !capturing && n_out % 8 == 0 && n_in % 8 == 0 && products <= (int64_t)1 << 34 && tokens * (n_out + 2 * n_in) <= 9 << 22;
 }

@@ -655,7 +655,7 @@ def test_backward_under_autocast_multiplies_in_its_type(dtype, cast):
     assert torch.equal(x.grad, torch.mm(g.to(cast), wq.to(cast)).to(dtype))
 
 
-@pytest.mark.parametrize("dtype,tokens,n_out,n_in", [(torch.float32, 8, 64, 128), (torch.float32, 128, 768, 768), (torch.bfloat16, 8, 32, 64), (torch.bfloat16, 300, 264, 1032)])
+@pytest.mark.parametrize("dtype,tokens,n_out,n_in", [(torch.float32, 32, 32, 64), (torch.float32, 128, 768, 768), (torch.bfloat16, 8, 32, 64), (torch.bfloat16, 300, 264, 1032)])
 def test_traced_layer_agrees_to_the_rounding_of_the_type(dtype, tokens, n_out, n_in):
     """A trace records torch's product; the eager layer's own one adds up in another order: the smallest own step in float32 and larger ones."""
     from coset_b200 import _lib
@@ -748,3 +748,48 @@ def test_steps_and_products_from_two_threads():
         assert len(a) == len(b) == 12
         for s, t in zip(a, b):
             assert torch.allclose(s.float(), t.float(), rtol=1e-6, atol=0) if s.dim() == 1 else torch.equal(s, t)
+
+
+@pytest.mark.parametrize("tokens,n_out,n_in", [(1, 768, 768), (2, 512, 1024), (8, 256, 256), (16, 64, 64), (31, 128, 4096), (32, 256, 256), (48, 64, 2048), (128, 768, 768), (2048, 16, 768)])
+def test_float32_step_is_as_precise_as_torchs(tokens, n_out, n_in):
+    """Against 64 bits, forward and backward: no further off than torch's products of the same values (two such errors differ by a few percent of themselves)."""
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    g = torch.Generator(device="cuda").manual_seed(tokens + n_in)
+    layer = create_e8_hnlq_linear(n_in, n_out, device="cuda", tiling="row", init_method="zeros", bias=False)
+    layer.load_weights(torch.randn(n_out, n_in, device="cuda", generator=g) * 20.0)
+    x, up = torch.randn(tokens, n_in, device="cuda", generator=g).requires_grad_(), torch.randn(tokens, n_out, device="cuda", generator=g)
+    y = layer(x)
+    y.backward(up)
+    wq, xs = layer._quantize_weights().detach(), x.detach()
+    for got, torchs, exact in ((y.detach(), torch.nn.functional.linear(xs, wq), xs.double() @ wq.double().T), (x.grad, torch.mm(up, wq), up.double() @ wq.double())):
+        assert float((got.double() - exact).norm()) <= 1.1 * float((torchs.double() - exact).norm())
+
+
+@pytest.mark.parametrize("form", ["expanded", "strided", "offset", "three"])
+def test_own_float32_products_with_awkward_tensors(form):
+    """From 32 tokens on, where float32 steps take the own products: gradients and inputs that they cannot read, or read only as rows."""
+    from coset_b200 import _lib
+    from coset_b200.core.e8 import create_e8_hnlq_linear
+    layer = create_e8_hnlq_linear(64, 48, device="cuda", tiling="row", init_method="zeros")
+    layer.load_weights(torch.randn(48, 64, device="cuda") * 20.0, torch.randn(48, device="cuda"))
+    x, g = torch.randn(40, 64, device="cuda"), torch.randn(40, 48, device="cuda")
+    assert _lib.native().own_product(x, layer.weight, layer.bias)
+    if form == "expanded":
+        g = g[:1].expand(40, 48)
+
+    def step(x, g):
+        layer.zero_grad()
+        x = x.detach().requires_grad_()
+        y = layer(x)
+        y.backward(g)
+        return [t.reshape(-1) for t in (y.detach(), x.grad, layer.weight.grad, layer.theta_beta.grad, layer.bias.grad)]
+    want = step(x, g.contiguous())
+    if form == "strided":
+        x, g = torch.cat([x, x], 1)[:, :64], torch.cat([g, g], 1)[:, :48]
+    elif form == "offset":
+        x, g = torch.cat([x.new_zeros(1), x.reshape(-1)])[1:].view(40, 64), torch.cat([g.new_zeros(1), g.reshape(-1)])[1:].view(40, 48)
+    elif form == "three":
+        x, g = x.view(4, 10, 64), g.view(4, 10, 48)
+    unit = 64 * 2.0 ** -23  # sums of at most 64 products in another order
+    for a, b in zip(step(x, g), want):
+        assert torch.allclose(a, b, rtol=unit, atol=unit * float(b.abs().max()))

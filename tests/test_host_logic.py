@@ -165,7 +165,7 @@ def test_sizes_of_the_training_layers_own_products():
         assert not own(f32, tokens, 8, 8)
     for tokens in (65535 * 256 + 1, 1 << 28):
         assert not own(bf16, tokens, 8, 8)
-    for tokens, n_out, n_in in ((262144, 16, 64), (65536, 64, 64), (8192, 10, 3200), (0, 64, 64), (2048, 512, 512), (8, 32, 64), (64, 1 << 11, (1 << 11) + 8)):
+    for tokens, n_out, n_in in ((262144, 16, 64), (65536, 64, 64), (8192, 10, 3200), (0, 64, 64), (2048, 512, 512), (32, 24, 64), (31, 768, 768), (64, 1 << 11, (1 << 11) + 8)):
         assert not own(f32, tokens, n_out, n_in)
     for tokens, n_out, n_in in ((262144, 64, 64), (8192, 64, 6144), (4096, 256, 8192), (64, 1 << 11, (1 << 11) + 8), (64, 60, 64), (64, 64, 60), (8192, 2048, 2048)):
         assert not own(bf16, tokens, n_out, n_in)
@@ -175,7 +175,7 @@ def test_sizes_of_the_training_layers_own_products():
         assert not own(bf16, tokens, 8, 8) or tokens <= 65535 * 32
     # a graph keeps what is quicker on the device
     assert own(f32, 128, 768, 768, capturing=True) and own(f32, 32, 48, 64, capturing=True) and own(f32, 4096, 64, 64, capturing=True)
-    for tokens, n_out, n_in in ((1024, 512, 512), (8, 1024, 1024), (16384, 16, 64)):
+    for tokens, n_out, n_in in ((1024, 512, 512), (16384, 16, 64)):
         assert own(f32, tokens, n_out, n_in) and not own(f32, tokens, n_out, n_in, capturing=True)
     for tokens, n_out, n_in in ((4096, 3072, 768), (128, 768, 768), (8, 64, 64)):
         assert own(bf16, tokens, n_out, n_in) and not own(bf16, tokens, n_out, n_in, capturing=True)
