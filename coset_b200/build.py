@@ -86,7 +86,7 @@ def _build_torch_module(verbose):
     libs = [f for d in cpp_extension.library_paths() for f in ("-L", d)]
     _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc,
           os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_PATH, "-L", LIB_DIR, "-lcoset_b200", "-Wl,-rpath,$ORIGIN", *libs,
-          "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"], verbose)
+          "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"], verbose)
 
 
 def build(force=False, verbose=False):

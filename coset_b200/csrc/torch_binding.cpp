@@ -11,6 +11,7 @@
 #include <ATen/ATen.h>
 #include <ATen/Context.h>
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContextLight.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -436,6 +437,13 @@ bool plain(const Tensor& t) {
     return (t.key_set().raw_repr() & ~known.raw_repr()) == 0 && !(at::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined();
 }
 
+// Before torch's product in a capture: a thread's first one makes a cuBLAS handle, whose allocations a capture refuses unless the thread relaxes it.  The eager steps
+// before may have been the own kernels' and made none.
+void torch_product_in_capture() {
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    at::cuda::getCurrentCUDABlasHandle();
+}
+bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
 // The own float32 products multiply in float32: a caller who lets torch's use TF32 gets those.
 bool tf32_allowed() { return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32; }
 // Whether the library's own kernels may multiply a matrix: contiguous (and in bf16 made of aligned 16-byte chunks), and nobody looks at the torch calls.
@@ -469,7 +477,6 @@ bool own_training_products(at::ScalarType type, int64_t tokens, int64_t n_out, i
     }
     return type == at::kBFloat16 && !capturing && n_out % 8 == 0 && n_in % 8 == 0 && products <= (int64_t)1 << 34 && tokens * (n_out + 2 * n_in) <= 9 << 22;
 }
-bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
 // The rows of a layer's input where its product is the library's own, undefined where it is torch's (which refuses what does not fit together).
 Tensor own_layer_rows(const Tensor& x, const Tensor& w, const Tensor& bias) {
     const int64_t n_out = w.size(0), n_in = w.size(1);
@@ -510,6 +517,7 @@ PyObject* dense_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
                     check_rc(coset_layer_beta_bias(nullptr, nullptr, nullptr, 0, nullptr, fdata(bias), bias.numel(), data(b), stream_of(x)), "coset_layer_beta_bias");
                 } else b = bias.to(at::kBFloat16);
             }
+            if (capturing()) torch_product_in_capture();
             y = at::linear(x, w, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
         }
     }
@@ -602,6 +610,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
             check_rc(x.scalar_type() == at::kFloat ? coset_f32_linear(fdata(x2), fdata(wq), fdata(b), T, N, K, fdata(y), stream_of(x))
                                                    : coset_e8_dense_linear(data(wq), N, K, data(x2), K, T, fdata(b), 1, data(y), N, nullptr, stream_of(x)), "the layer's product");
         } else {
+            if (capturing()) torch_product_in_capture();
             y = at::linear(x, wq, b.defined() ? std::optional<Tensor>(b) : std::nullopt);
         }
         // x serves the gradients of the weight and its scale, wq that of x: a frozen layer does not hold on to its input
@@ -632,7 +641,12 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
         variable_list out(9);
         const int64_t T = g2.size(0), N = w.size(0), K = w.size(1);
         const at::ScalarType type = g2.scalar_type();
-        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K, capturing()) && own_rows(g2) && g2.device() == w.device() &&
+        const bool captured = capturing();
+        const auto torchs = [&](const Tensor& a, const Tensor& b) {
+            if (captured) torch_product_in_capture();
+            return at::mm(a, b);
+        };
+        const bool own = !at::GradMode::is_enabled() && own_training_products(type, T, N, K, captured) && own_rows(g2) && g2.device() == w.device() &&
                          !at::autocast::is_autocast_enabled(at::kCUDA), f32 = type == at::kFloat;
         if (ctx->needs_input_grad(0)) {
             c10::SmallVector<int64_t, 6> x_shape(grads[0].sizes().begin(), grads[0].sizes().end());
@@ -641,7 +655,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
                 out[0] = empty(x_shape, type, g2);
                 check_rc(f32 ? coset_f32_input_grad(fdata(g2), fdata(wq), (int)T, (int)N, (int)K, fdata(out[0]), stream_of(g2))
                              : coset_dense_input_grad(data(g2), data(wq), (int)T, (int)N, (int)K, data(out[0]), nullptr, stream_of(g2)), "the gradient of the input");
-            } else out[0] = at::mm(g2, wq).view(x_shape);
+            } else out[0] = torchs(g2, wq).view(x_shape);
         }
         const bool need_theta = ctx->needs_input_grad(2);
         if (ctx->needs_input_grad(1) || need_theta) {
@@ -651,7 +665,7 @@ struct QatLinear : torch::autograd::Function<QatLinear> {
                 gw = empty({N, K}, type, g2);
                 check_rc(f32 ? coset_f32_weight_grad(fdata(g2), fdata(x2), (int)T, (int)N, (int)K, fdata(gw), stream_of(g2))
                              : coset_dense_weight_grad(data(g2), data(x2), (int)T, (int)N, (int)K, data(gw), nullptr, stream_of(g2)), "the gradient of the weight");
-            } else gw = at::mm(g2.t(), x2);
+            } else gw = torchs(g2.t(), x2);
             auto r = FakeQuant::backward_launch(gw, w, theta, beta, codes, range, bpt, q, clip, need_theta);
             out[1] = r.first;
             out[2] = r.second;

@@ -793,3 +793,14 @@ def test_own_float32_products_with_awkward_tensors(form):
     unit = 64 * 2.0 ** -23  # sums of at most 64 products in another order
     for a, b in zip(step(x, g), want):
         assert torch.allclose(a, b, rtol=unit, atol=unit * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("what", ["bf16", "f32", "code"])
+def test_capture_behind_eager_steps_of_the_own_products(what):
+    """A graph may record torch's products where the eager steps before were the own kernels': in a process that has made no cuBLAS handle, the capture does."""
+    import os
+    import subprocess
+    import sys
+    child = os.path.join(os.path.dirname(os.path.abspath(__file__)), "capture_child.py")
+    done = subprocess.run([sys.executable, child, what], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and "ok" in done.stdout, done.stderr[-2000:]
