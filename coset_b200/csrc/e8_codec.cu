@@ -404,8 +404,8 @@ constexpr float kSaturate = 3.9f;  // 8 * 3.9 / 4 < 7.96 and 3.9 / 4 < 1.96: lev
 constexpr int kAnyScale = 0, kBlockScale = 1, kTileScale = 2;
 
 // kRing > 0: rows on their way to shared memory per thread (cp.async), so that the loop waits for no load and holds one row in
-// registers.  What bounds the loop is then the issue of instructions (80 % of the cycles, ALU pipe 70 %; before, with three rows per
-// iteration in registers, 73 %, and 62 % for bf16), hence offsets of 32 bits (n < 2^27 blocks, the caller cuts longer calls), a form
+// registers.  What bounds the loop is then the issue of instructions (82 % of the cycles, ALU pipe 63 %, FMA pipe 39 % over 2^24 blocks; with three rows
+// per iteration in registers 77, 72 and 33 % over 2^25), hence offsets of 32 bits (n < 2^27 blocks, the caller cuts longer calls), a form
 // for each kind of scale, and the signs at the flip coordinates read from the row by index.  The two halves of a float32 row lie in the
 // order of bit 2 of the thread, so that eight lanes meet eight groups of banks; they come through L1, whose lines both halves share.
 // Measured against the form with registers: 2^25 float32 blocks with a scale each 298 -> 271 us, with one scale for 96 blocks 317 -> 290,

@@ -5,7 +5,7 @@
 // (32 MiB for a 4096 x 4096 layer against 126 MiB of L2), and nothing of it has to survive the call, so the
 // layer keeps 4 bits per weight in HBM.  Against the single-launch kernel of e8_dequant_gemm.cu this moves the
 // decode out of the GEMM's K loop: no producer warps, both operands arrive by TMA, and the results are the same
-// bits.  Measured on a 4096 x 4096 layer (graph replays, decode included): 101 us at 4096 tokens and 192 at 8192.
+// bits.  Measured on a 4096 x 4096 layer (short graph replays, decode included, bf16 result): 113 us at 4096 tokens and 208 at 8192.
 //
 // The GEMM runs on pairs of CTAs (a cluster of two on the two SMs of a TPC) that share one instruction
 // stream of tcgen05.mma.cta_group::2: M = 256 tokens x N = 256 features x K = 16 per instruction.  CTA r of
@@ -23,10 +23,10 @@
 //   "full"  lives in rank 0 alone and counts the bytes of BOTH CTAs' tiles: rank 1's loads are cta_group::2 TMA
 //           copies that land in rank 1's shared memory and complete on rank 0's barrier;
 //   "empty" (and "done") are signalled by one tcgen05.commit that arrives on the barrier of either CTA.
-//   The issuing code sits behind elect.sync and on values that a shuffle has made uniform: behind a comparison of the lane's number a
-//   K step's four instructions and its commits took 450 cycles to issue, now 200, and the K loop runs at the tensor cores' rate
-//   (1060 cycles a step instead of about 1400); one multicast commit releases the stage in both CTAs.  With the epilogue below
-//   (16-byte stores) 4096 tokens took 88 us instead of 94 in short runs; in long ones the 1000 W limit lowers the clock and 1-2 % are left.
+//   The issuing code sits behind elect.sync and on values that a shuffle has made uniform, one multicast commit releases the stage in both
+//   CTAs, and the epilogue below stores 16 bytes a lane.  Together, decode included, short graph replays, before and now: bf16 result 64.2 -> 62.7 us at 2048
+//   tokens, 115.9 -> 113.3 at 4096, 213.6 -> 208.4 at 8192; float32 result 118.5 -> 119.2 at 4096.  In long runs the 1000 W limit lowers the clock and 1-2 %
+//   are left.  The counters at 2048 tokens are what they were: the tensor pipe is active in 79 % of the active cycles.
 // Every wait is bounded in time; on expiry the kernel sets the status word, skips its stores, frees its tensor
 // memory and returns.  Every TMA load lands in the CTA that issued it.
 // Measured and not kept: persistent clusters walking over tiles, (a) with 256-token tiles and the two accumulators

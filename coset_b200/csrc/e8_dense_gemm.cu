@@ -16,10 +16,10 @@
 // of its four instructions and one wait; stages of two steps below 160 tokens share the wait), 2 to 7 thousand cycles for the sums.  The kernel is
 // launched as a programmatic dependent, which hides about 2 us of that behind the kernel before it.
 // Two CTAs fit an SM (ten warps, at most 112 KB of stages) where there are more tiles than SMs.
-// Measured, 4096 x 4096 with a bias, torch's product and its bias cast against this kernel (graph replays, three weights in turn): 64 tokens 8.9 + 2.9
-// against 8.8 us, 256 tokens 11.1 + 2.9 against 12.6, 1024 tokens 25.2 + 2.9 against 25.5; a call of the layer with 256 tokens 20.7 -> 14.5 us, for
-// the host was what bounded it.  The products of a training step of a [3072, 768] layer with 4096 tokens: 22.7 + 16.3 + 15.1 us against 18.0 + 15.3 + 13.8 for
-// torch's, but 15 us of host time instead of 42, and the host bounds the step.
+// Measured on the device, 4096 x 4096 (graph replays, three weights in turn), this kernel / torch's product with its cast of the bias / without a bias: 64 tokens
+// 11.3 / 10.8 / 8.7 us, 256 tokens 14.5 / 13.1 / 10.9, 1024 tokens 26.9 / 26.6 / 25.1.  It costs the host one launch, and the host bounds such a call: the
+// layer's with 256 tokens 21.6 -> 14.6 us where weights alternate, 19.3 -> 11.7 on one weight, 14.8 -> 11.6 without a bias.  The products of a training
+// step of a [3072, 768] layer with 4096 tokens: 26.3 + 17.0 + 17.3 us against 18.4 + 16.0 + 14.7 for torch's, but the host bounds the step: 146 -> 118 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>

@@ -20,7 +20,7 @@
 // Guards: max|x| <= 1.96 and sum|x| <= 7.96 (which also makes the NEXT level the origin and keeps every
 // lane in range), max|d| < 1/2 - 2.96 * 2^-21 and min|d| > 2.96 * 2^-21 (rint equals the reference's
 // custom_round for x and x - 1/2), minimum of |d| unique by 2^-21 if coset 1 has a flip, |dist1 - dist0| > 2^-14.
-// Bound: instruction issue and the ALU pipe (80 and 70 % of the cycles in the encoder that has its rows in shared memory, e8_codec.cu).  What the
+// Bound: instruction issue (82 % of the cycles in the encoder that has its rows in shared memory, e8_codec.cu; ALU pipe 63 %).  What the
 // FMA pipe does on all eight coordinates is done in pairs (f32x2), floor comes from a round-down addition instead of a saturated product, the
 // uniqueness of the minimum is asked for only where it is used, the parities are sums of floats (2^25 float32 blocks 299 -> 294 us), and the signs at
 // the two flip coordinates are read by index where the caller has the row in memory (in the encoder 290 -> 283 us, bf16 293 -> 283).
