@@ -453,7 +453,7 @@ bool own_rows(const Tensor& t) {
            ((f32 && !tf32_allowed()) || (t.scalar_type() == at::kBFloat16 && t.size(1) % 8 == 0 && (uintptr_t)t.const_data_ptr() % 16 == 0));
 }
 // Whether they should multiply for a training step: where the host bounds it (110 us with them, 141 with torch's products) and the device, which they cost
-// more, does not.  Steps of a layer on this box, own / torch, us:
+// more, does not.  Eager steps of a layer, own / torch, us:
 //   bf16   the products take up to 40 % longer, most where rows are wide, and those of a wide input are read or written three times, of a wide
 //          output twice: T (n_out + 2 n_in) of 34 M values [8192 x 4096 x 64] 110 / 146, [8192 x 2048 x 1024] 126 / 141; 36 M [4096 x 8192 x 256]
 //          120 / 140; 42 M [8192 x 4096 x 512] 142 / 139; 50 M [16384 x 2048 x 512] 150 / 143; 68 M [4096 x 256 x 8192] 180 / 165; 101 M [8192 x 64 x 6144] 174 / 151.
